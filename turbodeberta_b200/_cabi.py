@@ -74,6 +74,14 @@ def _load() -> C.CDLL:
 
 lib = _load()
 
+# The operators' host path (argument checks, allocation, launch, status words) is native as well; it links against the
+# library above.
+try:
+    from . import _host as host
+except ImportError as e:
+    raise ImportError(f"the host extension is missing or stale ({e}): build it with `python -m turbodeberta_b200.build`. "
+                      "There is no fallback path.") from e
+
 
 def check(code: int) -> None:
     if code == 0:

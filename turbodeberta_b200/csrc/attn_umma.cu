@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(1024) build_tile_list_kernel(const int32_t* __
   __syncthreads();
   auto tiles_of = [&](int s) {
     const int a = cu[s], b = cu[s + 1];
-    if (a < 0 || b < a || (int64_t)b > total_tokens) { atomicExch(status + 1, 1); return 0; }
+    if (a < 0 || b < a || (int64_t)b > total_tokens) { *reinterpret_cast<volatile int32_t*>(status + 1) = 1; return 0; }
     return (b - a + BQ - 1) / BQ;
   };
   for (int s = threadIdx.x; s < n_seqs; s += blockDim.x) {
@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(1024) build_tile_list_kernel(const int32_t* __
     int run = 0;
     for (int bkt = LIST_BUCKETS - 1; bkt >= 0; --bkt) { const int c = hist[bkt]; hist[bkt] = run; run += c; }
     ws[0] = run < cap ? run : cap;
-    if (cu[n_seqs] != (int32_t)total_tokens) atomicExch(status + 1, 1);
+    if (cu[n_seqs] != (int32_t)total_tokens) *reinterpret_cast<volatile int32_t*>(status + 1) = 1;
   }
   __syncthreads();
   for (int s = threadIdx.x; s < n_seqs; s += blockDim.x) {
@@ -292,7 +292,7 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap tm_q, c
                                    : p.n_seqs * ((p.L + BQ - 1) / BQ);
   // An earlier CTA gave up: the scheduler lane (which reads the word while the CTA sets itself up) hands out no work.
   int32_t status_at_start = 0;
-  if (warp == NCW + 2 && lane == 0) status_at_start = *reinterpret_cast<volatile int32_t*>(p.status);
+  if (warp == NCW + 2 && lane == 0) status_at_start = *reinterpret_cast<volatile int32_t*>(p.gave_up);
 
   // ---- shared memory carve-up ----------------------------------------------------------------
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -442,13 +442,17 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap tm_q, c
     // The first item of a CTA is its own index (no round trip to the counter before the pipeline can start); the
     // counter hands out the items after those.
     // Padded form with lengths: the sequences are handed out in the order sorted above.
+    // Every CTA with an item of its own draws until the first draw past the end, so the counter is drawn from exactly
+    // as many times as there are items: a counter that wraps after that many draws is back at zero when the launch ends.
+    const unsigned int last_item = (unsigned int)(total_tiles * p.H - 1);
     int n = 0;
     bool first = true;
     while (true) {
       int w = 0;
       if (lane == 0)
         w = (*abort_flag || status_at_start != 0) ? 0x7fffffff
-                                                  : (first ? (int)blockIdx.x : (int)gridDim.x + atomicAdd(p.status + 2, 1));
+                                                  : (first ? (int)blockIdx.x
+                                                             : (int)gridDim.x + (int)atomicInc(reinterpret_cast<unsigned int*>(p.counter), last_item));
       first = false;
       w = __shfl_sync(0xffffffffu, w, 0);
       Work k;
@@ -979,6 +983,7 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap tm_q, c
 
   // ---- teardown ------------------------------------------------------------------------------
   if (*abort_flag) {                      // give copies that may still be in flight time to land
+    if (tid == 0 && p.gave_up != p.status) *reinterpret_cast<volatile int32_t*>(p.gave_up) = 1;
     const uint64_t t0 = globaltimer_ns();
     while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
   }
@@ -1028,6 +1033,17 @@ int table_map(CUtensorMap* m, const void* ptr, int rows, int H, int box_rows, co
   uint64_t strides[2] = {(uint64_t)HD * 2, (uint64_t)rows * HD * 2};
   uint32_t box[3] = {HD, (uint32_t)box_rows, 1};
   return encode_map(m, ptr, 3, dims, strides, box, what);
+}
+
+int device_sms(int* sms) {
+  constexpr int MAX_DEV = 64;
+  static int known[MAX_DEV] = {};                  // same value from every thread: a race writes it twice
+  int dev = 0, rc;
+  if ((rc = cuda_fail(cudaGetDevice(&dev), "cudaGetDevice"))) return rc;
+  if (dev < MAX_DEV && known[dev]) { *sms = known[dev]; return TDB_OK; }
+  if ((rc = cuda_fail(cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev), "cudaDeviceGetAttribute"))) return rc;
+  if (dev < MAX_DEV) known[dev] = *sms;
+  return TDB_OK;
 }
 
 // The kernel needs more dynamic shared memory than the default limit; the attribute is per device and per
@@ -1086,7 +1102,14 @@ size_t umma_workspace_bytes(int n_seqs, int64_t total_tokens) {
   return sizeof(TileListHeader) + (size_t)cap * sizeof(int2);
 }
 
-int launch_attn_umma(const AttnParams& p, cudaStream_t s) {
+int launch_attn_umma(const AttnParams& given, cudaStream_t s) {
+  AttnParams p = given;
+  if (!p.counter) { p.counter = p.status + 2; p.gave_up = p.status; }
+  // Saturated tiles exist only if a sequence exceeds the saturation distance by a tile; the variant that handles
+  // them specially is a little slower on ordinary tiles, so it is used from twice that length on (p.L is the
+  // padded length or the caller's max_seqlen).
+  const bool c2p = p.flags & TDB_FLAG_C2P, p2c = p.flags & TDB_FLAG_P2C;
+  const bool lng = (c2p || p2c) && p.L >= 2 * (p.exp_delta_max - TDB_EXPAND_MARGIN) + BK;
   if (p.H > 65535) { set_error("more than 65535 heads"); return TDB_ERR_SHAPE; }
   CUtensorMap maps[7];
   memset(maps, 0, sizeof(maps));
@@ -1098,18 +1121,17 @@ int launch_attn_umma(const AttnParams& p, cudaStream_t s) {
   if ((rc = token_map(&maps[2], p.v, tokens, p.H, B, p.v_sb, p.v_st, p.v_sh, "v"))) return rc;
   if (p.flags & TDB_FLAG_C2P) {
     if ((rc = table_map(&maps[3], p.kr_exp, p.exp_rows, p.H, BAND, "kr_exp"))) return rc;
-    if ((rc = table_map(&maps[5], p.kr_exp, p.exp_rows, p.H, SATN, "kr_exp (saturated tiles)"))) return rc;
+    if (lng && (rc = table_map(&maps[5], p.kr_exp, p.exp_rows, p.H, SATN, "kr_exp (saturated tiles)"))) return rc;
   } else { maps[3] = maps[0]; maps[5] = maps[0]; }
   if (p.flags & TDB_FLAG_P2C) {
     if ((rc = table_map(&maps[4], p.qr_exp, p.exp_rows, p.H, BAND, "qr_exp"))) return rc;
-    if ((rc = table_map(&maps[6], p.qr_exp, p.exp_rows, p.H, SATN, "qr_exp (saturated tiles)"))) return rc;
+    if (lng && (rc = table_map(&maps[6], p.qr_exp, p.exp_rows, p.H, SATN, "qr_exp (saturated tiles)"))) return rc;
   } else { maps[4] = maps[0]; maps[6] = maps[0]; }
 
   // Persistent CTAs: one per SM (201 KB of shared memory and all 512 tensor-memory columns each), never more
   // than there are work items (query tiles x heads).
-  int dev = 0, sms = 0;
-  if ((rc = cuda_fail(cudaGetDevice(&dev), "cudaGetDevice"))) return rc;
-  if ((rc = cuda_fail(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "cudaDeviceGetAttribute"))) return rc;
+  int sms = 0;
+  if ((rc = device_sms(&sms))) return rc;
   int64_t tiles;
   if (p.varlen) {
     tiles = (p.total_tokens + BQ - 1) / BQ + p.n_seqs + 1;           // upper bound; the device list has the real count
@@ -1123,13 +1145,9 @@ int launch_attn_umma(const AttnParams& p, cudaStream_t s) {
   }
   const int64_t items = tiles * p.H;
   dim3 grid((unsigned)(items < sms ? items : sms), 1, 1);
-  // status word 2 is the device-wide work counter of this launch; start it at zero even if the caller reuses the words
-  if ((rc = cuda_fail(cudaMemsetAsync(p.status + 2, 0, sizeof(int32_t), s), "cudaMemsetAsync(work counter)"))) return rc;
-  const bool c2p = p.flags & TDB_FLAG_C2P, p2c = p.flags & TDB_FLAG_P2C;
-  // Saturated tiles exist only if a sequence exceeds the saturation distance by a tile; the variant that handles
-  // them specially is a little slower on ordinary tiles, so it is used from twice that length on (p.L is the
-  // padded length or the caller's max_seqlen).
-  const bool lng = (c2p || p2c) && p.L >= 2 * (p.exp_delta_max - TDB_EXPAND_MARGIN) + BK;
+  // status word 2 as the work counter: start it at zero even if the caller reuses the words
+  if (p.counter == p.status + 2 &&
+      (rc = cuda_fail(cudaMemsetAsync(p.counter, 0, sizeof(int32_t), s), "cudaMemsetAsync(work counter)"))) return rc;
   if (c2p && p2c) return lng ? launch_variant<true, true, true>(p, grid, maps, s) : launch_variant<true, true, false>(p, grid, maps, s);
   if (c2p) return lng ? launch_variant<true, false, true>(p, grid, maps, s) : launch_variant<true, false, false>(p, grid, maps, s);
   if (p2c) return lng ? launch_variant<false, true, true>(p, grid, maps, s) : launch_variant<false, true, false>(p, grid, maps, s);

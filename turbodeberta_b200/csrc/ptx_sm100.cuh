@@ -69,7 +69,8 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     if (*abort_flag) return false;
     if (globaltimer_ns() - t0 > limit_ns) {
       *abort_flag = 1;
-      atomicCAS(status, 0, code);
+      // plain accesses: the word may live in host memory mapped into the device; of several reports at once one stays
+      if (*reinterpret_cast<volatile int*>(status) == 0) *reinterpret_cast<volatile int*>(status) = code;
       return false;
     }
   }

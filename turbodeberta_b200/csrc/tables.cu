@@ -157,4 +157,31 @@ int launch_relpos_expand(const void* table, const int16_t* idx, int idx_delta_ma
   return cuda_fail(cudaGetLastError(), "relpos_expand launch");
 }
 
+// Both tables of a layer in one launch, bf16 to bf16, head_dim 64: eight threads copy one 128-byte row, 16 bytes each.  Bound
+// by the launch itself at one layer's size (2 x 12 heads x 1544 rows = 4.7 MB written).  Either table may be null.
+__global__ void __launch_bounds__(256) relpos_expand_pair_kernel(const uint4* __restrict__ kr, const uint4* __restrict__ qr,
+                                                                 const int16_t* __restrict__ idx, int idx_delta_max, int H,
+                                                                 int two_span, int exp_delta_max, int exp_rows,
+                                                                 uint4* __restrict__ kr_out, uint4* __restrict__ qr_out) {
+  const uint4* table = blockIdx.y == 0 ? kr : qr;
+  uint4* out = blockIdx.y == 0 ? kr_out : qr_out;
+  if (!table) return;
+  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  const int64_t row = i >> 3;
+  if (row >= (int64_t)H * exp_rows) return;
+  const int h = (int)(row / exp_rows), x = (int)(row - (int64_t)h * exp_rows);
+  int delta = x - exp_delta_max;
+  delta = delta < -idx_delta_max ? -idx_delta_max : (delta > idx_delta_max ? idx_delta_max : delta);
+  out[i] = table[((int64_t)h * two_span + idx[delta + idx_delta_max]) * 8 + (i & 7)];
+}
+
+int launch_relpos_expand_pair(const void* kr, const void* qr, const int16_t* idx, int idx_delta_max, int H, int two_span,
+                              int exp_delta_max, int exp_rows, void* kr_out, void* qr_out, cudaStream_t s) {
+  const int64_t threads = (int64_t)H * exp_rows * 8;
+  dim3 grid((unsigned)((threads + 255) / 256), 2);
+  relpos_expand_pair_kernel<<<grid, 256, 0, s>>>((const uint4*)kr, (const uint4*)qr, idx, idx_delta_max, H, two_span,
+                                                 exp_delta_max, exp_rows, (uint4*)kr_out, (uint4*)qr_out);
+  return cuda_fail(cudaGetLastError(), "relpos_expand_pair launch");
+}
+
 }  // namespace tdb

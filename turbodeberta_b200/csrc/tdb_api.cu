@@ -89,6 +89,27 @@ static int check_umma(const AttnParams& p, int dtype) {
   return TDB_OK;
 }
 
+// The checks and the launch that every attention entry point shares (sizes are known to be non-empty here).
+static int run_attn(const AttnParams& p, int dtype, int kernel, cudaStream_t stream) {
+  int rc;
+  if (p.varlen) {
+    if (!p.cu_seqlens) { set_error("cu_seqlens is null"); return TDB_ERR_ARG; }
+    if (p.L <= 0 || p.L > p.total_tokens) { set_error("max_seqlen %d outside [1, total_tokens]", p.L); return TDB_ERR_ARG; }
+  }
+  if ((rc = check_common(p, dtype, kernel))) return rc;
+  if (!p.varlen && p.n_seqs > 1 && (p.q_sb <= 0 || p.k_sb <= 0 || p.v_sb <= 0 || p.o_sb <= 0)) {
+    set_error("batch stride must be positive when B > 1");
+    return TDB_ERR_ARG;
+  }
+  if (pick_kernel(dtype, kernel) == TDB_KERNEL_SIMT) return launch_attn_simt(p, dtype, stream);
+  if ((rc = check_umma(p, dtype))) return rc;
+  if (p.varlen && (!p.workspace || p.workspace_bytes < umma_workspace_bytes(p.n_seqs, p.total_tokens))) {
+    set_error("workspace of %zu bytes is smaller than the %zu required", p.workspace_bytes, umma_workspace_bytes(p.n_seqs, p.total_tokens));
+    return TDB_ERR_WORKSPACE;
+  }
+  return launch_attn_umma(p, stream);
+}
+
 }  // namespace tdb
 
 using namespace tdb;
@@ -180,13 +201,7 @@ TDB_API int tdb_attn_fwd_fixed(const void* q, const void* k, const void* v, void
   p.lse = lse; p.lse_sb = (int64_t)H * L; p.lse_sh = L; p.status = status;
   if (B < 0 || L < 0) { set_error("negative size"); return TDB_ERR_ARG; }
   if (B == 0 || L == 0) return TDB_OK;     // nothing to compute: pointers of empty tensors may be null
-  int rc = check_common(p, dtype, kernel);
-  if (rc) return rc;
-  if (B > 1 && (q_sb <= 0 || k_sb <= 0 || v_sb <= 0 || o_sb <= 0)) { set_error("batch stride must be positive when B > 1"); return TDB_ERR_ARG; }
-  int kn = pick_kernel(dtype, kernel);
-  if (kn == TDB_KERNEL_SIMT) return launch_attn_simt(p, dtype, (cudaStream_t)stream);
-  if ((rc = check_umma(p, dtype))) return rc;
-  return launch_attn_umma(p, (cudaStream_t)stream);
+  return run_attn(p, dtype, kernel, (cudaStream_t)stream);
 }
 
 TDB_API int tdb_attn_fwd_varlen(const void* q, const void* k, const void* v, void* o,
@@ -211,18 +226,7 @@ TDB_API int tdb_attn_fwd_varlen(const void* q, const void* k, const void* v, voi
     if (n_seqs < 0 || total_tokens < 0) { set_error("negative size"); return TDB_ERR_ARG; }
     return TDB_OK;
   }
-  if (!cu_seqlens) { set_error("cu_seqlens is null"); return TDB_ERR_ARG; }
-  if (max_seqlen <= 0 || max_seqlen > total_tokens) { set_error("max_seqlen %d outside [1, total_tokens]", max_seqlen); return TDB_ERR_ARG; }
-  int rc = check_common(p, dtype, kernel);
-  if (rc) return rc;
-  int kn = pick_kernel(dtype, kernel);
-  if (kn == TDB_KERNEL_SIMT) return launch_attn_simt(p, dtype, (cudaStream_t)stream);
-  if ((rc = check_umma(p, dtype))) return rc;
-  if (!workspace || workspace_bytes < umma_workspace_bytes(n_seqs, total_tokens)) {
-    set_error("workspace of %zu bytes is smaller than the %zu required", workspace_bytes, umma_workspace_bytes(n_seqs, total_tokens));
-    return TDB_ERR_WORKSPACE;
-  }
-  return launch_attn_umma(p, (cudaStream_t)stream);
+  return run_attn(p, dtype, kernel, (cudaStream_t)stream);
 }
 
 TDB_API int tdb_attn_fwd_fixed_scores(const void* q, const void* k, const void* v, void* o,
@@ -247,10 +251,7 @@ TDB_API int tdb_attn_fwd_fixed_scores(const void* q, const void* k, const void* 
   if (B < 0 || L < 0) { set_error("negative size"); return TDB_ERR_ARG; }
   if (B == 0 || L == 0) return TDB_OK;
   if (!c2p_scores && !p2c_scores) { set_error("no position scores given: use tdb_attn_fwd_fixed"); return TDB_ERR_ARG; }
-  int rc = check_common(p, dtype, TDB_KERNEL_SIMT);
-  if (rc) return rc;
-  if (B > 1 && (q_sb <= 0 || k_sb <= 0 || v_sb <= 0 || o_sb <= 0)) { set_error("batch stride must be positive when B > 1"); return TDB_ERR_ARG; }
-  return launch_attn_simt(p, dtype, (cudaStream_t)stream);
+  return run_attn(p, dtype, TDB_KERNEL_SIMT, (cudaStream_t)stream);
 }
 
 TDB_API int tdb_attn_fwd_varlen_scores(const void* q, const void* k, const void* v, void* o,
@@ -276,12 +277,8 @@ TDB_API int tdb_attn_fwd_varlen_scores(const void* q, const void* k, const void*
     if (n_seqs < 0 || total_tokens < 0) { set_error("negative size"); return TDB_ERR_ARG; }
     return TDB_OK;
   }
-  if (!cu_seqlens) { set_error("cu_seqlens is null"); return TDB_ERR_ARG; }
-  if (max_seqlen <= 0 || max_seqlen > total_tokens) { set_error("max_seqlen %d outside [1, total_tokens]", max_seqlen); return TDB_ERR_ARG; }
   if (!c2p_scores && !p2c_scores) { set_error("no position scores given: use tdb_attn_fwd_varlen"); return TDB_ERR_ARG; }
-  int rc = check_common(p, dtype, TDB_KERNEL_SIMT);
-  if (rc) return rc;
-  return launch_attn_simt(p, dtype, (cudaStream_t)stream);
+  return run_attn(p, dtype, TDB_KERNEL_SIMT, (cudaStream_t)stream);
 }
 
 // Same as tdb_attn_fwd_varlen, with the tile list kept in the library's fixed device array instead of a
@@ -308,6 +305,16 @@ TDB_API int tdb_attn_fwd_varlen_static(const void* q, const void* k, const void*
                              idx_delta_max, kr_exp, qr_exp, exp_delta_max, exp_rows, cu_seqlens, n_seqs, total_tokens,
                              max_seqlen, H, D, sm_scale, flags, dtype, kernel, scratch, (size_t)TDB_STATIC_SCRATCH_BYTES,
                              lse, status, stream);
+}
+
+int tdb_run_attn(const tdb::AttnParams* p, int dtype, int kernel, void* stream) {
+  return run_attn(*p, dtype, kernel, (cudaStream_t)stream);
+}
+
+int tdb_expand_pair(const void* kr, const void* qr, const int16_t* idx, int idx_delta_max, int H, int two_span,
+                    int exp_delta_max, int exp_rows, void* kr_out, void* qr_out, void* stream) {
+  return launch_relpos_expand_pair(kr, qr, idx, idx_delta_max, H, two_span, exp_delta_max, exp_rows, kr_out, qr_out,
+                                   (cudaStream_t)stream);
 }
 
 }  // extern "C"

@@ -35,7 +35,10 @@ struct AttnParams {
   float sm_scale;
   int flags;
   float* lse; int64_t lse_sb, lse_sh;                     // lse[b*lse_sb + h*lse_sh + t] or null
-  int32_t* status;
+  int32_t* status;                                        // device-visible words: 0 = gave-up code, 1 = malformed offsets
+  // Tensor-core kernel: the device-wide work counter (zero on entry, and zero again once the launch has finished) and the
+  // flag that makes CTAs starting after a wait gave up hand out no work.  Null: status words 2 (reset by the launch) and 0.
+  int32_t* counter; int32_t* gave_up;
   void* workspace; size_t workspace_bytes;
 };
 
@@ -54,6 +57,16 @@ int launch_bounded_wait_selftest(int32_t* status, int code, uint64_t limit_ns, c
 int launch_attn_simt(const AttnParams& p, int dtype, cudaStream_t s);
 int launch_attn_umma(const AttnParams& p, cudaStream_t s);
 size_t umma_workspace_bytes(int n_seqs, int64_t total_tokens);
+int launch_relpos_expand_pair(const void* kr, const void* qr, const int16_t* idx, int idx_delta_max, int H, int two_span,
+                              int exp_delta_max, int exp_rows, void* kr_out, void* qr_out, cudaStream_t s);
 int static_tile_scratch(void** ptr);   // device address of the library's fixed tile-list array on the current device
 
 }  // namespace tdb
+
+// What the host extension calls: the checks and the launch behind the tdb_attn_fwd_* entry points, on a filled AttnParams.
+extern "C" __attribute__((visibility("default"))) int tdb_run_attn(const tdb::AttnParams* p, int dtype, int kernel,
+                                                                   void* stream);
+extern "C" __attribute__((visibility("default"))) int tdb_expand_pair(const void* kr, const void* qr, const int16_t* idx,
+                                                                      int idx_delta_max, int H, int two_span,
+                                                                      int exp_delta_max, int exp_rows, void* kr_out,
+                                                                      void* qr_out, void* stream);

@@ -60,15 +60,25 @@ def _tables_from_args(q_pos, k_pos, q, position_buckets, max_relative_distance, 
             max_relative_distance = two_span // 2
         if two_span != 2 * max_relative_distance:
             raise ValueError(f"table has {two_span} rows but max_relative_distance={max_relative_distance}")
-    dev = q.device
-    sat = _relpos.saturation_distance(position_buckets, max_relative_distance)
-    idx = _relpos.bucket_index_table(position_buckets, max_relative_distance, sat + 1, dev)
-    exp_dm = sat + cabi.TDB_EXPAND_MARGIN
-    want_exp = q.dtype == torch.bfloat16
-    kr_exp = _relpos.expand(kr, idx, exp_dm) if (want_exp and kr is not None) else None
-    qr_exp = _relpos.expand(qr, idx, exp_dm) if (want_exp and qr is not None) else None
-    return _relpos.RelPosTables(position_buckets, max_relative_distance, two_span, idx, sat + 1, kr, qr, kr_exp,
-                                qr_exp, exp_dm, (2 * exp_dm + 1 + 7) // 8 * 8)
+    idx, idm, exp_dm, exp_rows = _geometry(position_buckets, max_relative_distance, q.device)
+    kr_exp, qr_exp = _relpos.expand_pair(kr, qr, idx, exp_dm) if q.dtype == torch.bfloat16 else (None, None)
+    return _relpos.RelPosTables(position_buckets, max_relative_distance, two_span, idx, idm, kr, qr, kr_exp, qr_exp,
+                                exp_dm, exp_rows)
+
+
+_GEOMETRY: dict = {}
+
+
+def _geometry(position_buckets, max_relative_distance, device):
+    """(index table, its delta_max, delta_max and rows of the expanded tables), kept per geometry and device."""
+    key = (position_buckets, max_relative_distance, device)
+    g = _GEOMETRY.get(key)
+    if g is None:
+        sat = _relpos.saturation_distance(position_buckets, max_relative_distance)
+        idx = _relpos.bucket_index_table(position_buckets, max_relative_distance, sat + 1, device)
+        exp_dm = sat + cabi.TDB_EXPAND_MARGIN
+        g = _GEOMETRY[key] = (idx, sat + 1, exp_dm, (2 * exp_dm + 1 + 7) // 8 * 8)
+    return g
 
 
 def _is_materialised(t, q, position_buckets=0, max_relative_distance=0) -> bool:
@@ -96,8 +106,7 @@ def _index_table_for_scores(two_span, position_buckets, max_relative_distance, d
             max_relative_distance = two_span // 2
         if two_span != 2 * max_relative_distance:
             raise ValueError(f"score tensors have {two_span} columns but max_relative_distance={max_relative_distance}")
-    sat = _relpos.saturation_distance(position_buckets, max_relative_distance)
-    return _relpos.bucket_index_table(position_buckets, max_relative_distance, sat + 1, dev), sat + 1
+    return _geometry(position_buckets, max_relative_distance, dev)[0]
 
 
 def refuse_gradients(*tensors) -> None:
@@ -114,45 +123,12 @@ def _scores_fixed(q, k, v, c2p_scores, p2c_scores, seqlens, sm_scale, position_b
     """Legacy form of the fixed-length op: gather from materialised ``(B, H, L, 2*span)`` score tensors."""
     dev = cabi.require_cuda(q, k, v, seqlens)
     refuse_gradients(q, k, v, c2p_scores, p2c_scores)
-    if q.dim() != 4 or k.shape != q.shape or v.shape != q.shape:
-        raise ValueError("q, k, v must share the shape (B, H, L, D)")
-    B, H, L, D = q.shape
-    code = cabi.dtype_code(q.dtype)
     some = c2p_scores if c2p_scores is not None else p2c_scores
-    two_span = some.shape[-1]
-    for t, name in ((c2p_scores, "q_pos"), (p2c_scores, "k_pos")):
-        if t is None:
-            continue
-        if tuple(t.shape) != (B, H, L, two_span) or t.dtype != q.dtype or t.stride(-1) != 1:
-            raise ValueError(f"{name} must be (B, H, L, 2*span) of q's dtype with a contiguous last dimension")
-    for t in (q, k, v):
-        if t.stride(-1) != 1:
-            raise ValueError("the head dimension must be contiguous")
-    idx, idm = _index_table_for_scores(two_span, position_buckets, max_relative_distance, dev)
-    o = torch.empty((B, L, H, D), dtype=q.dtype, device=dev).permute(0, 2, 1, 3)
-    lse = torch.empty((B, H, L), dtype=torch.float32, device=dev) if return_lse else None
-    status = torch.zeros(4, dtype=torch.int32, device=dev)
-    if B == 0 or L == 0:
-        return o, lse
-    if seqlens is not None:
-        seqlens = seqlens.to(device=dev, dtype=torch.int32).contiguous()
-    flags = ((cabi.TDB_FLAG_C2P if c2p_scores is not None else 0) | (cabi.TDB_FLAG_P2C if p2c_scores is not None else 0)
-             | (cabi.TDB_FLAG_P2C_MIRRORED if p2c_mirrored else 0))
-
-    def s(t):
-        return (t.stride(0), t.stride(2), t.stride(1)) if t is not None else (0, 0, 0)      # batch, token, head
-
-    with torch.cuda.device(dev):
-        rc = cabi.lib.tdb_attn_fwd_fixed_scores(
-            cabi.ptr(q), cabi.ptr(k), cabi.ptr(v), cabi.ptr(o), *s(q), *s(k), *s(v), *s(o),
-            cabi.ptr(c2p_scores), *s(c2p_scores), cabi.ptr(p2c_scores), *s(p2c_scores), two_span, cabi.ptr(idx), idm,
-            cabi.ptr(seqlens), B, L, H, D, float(sm_scale), flags, code, cabi.ptr(lse), cabi.ptr(status),
-            cabi.stream_ptr(dev))
-    cabi.check(rc)
-    if check_status:
-        _check_status(status)
-    else:
-        _PENDING_STATUS.append(status)
+    idx = _index_table_for_scores(some.shape[-1], position_buckets, max_relative_distance, dev)
+    o, lse, st = cabi.host.attn_fixed_scores(q, k, v, c2p_scores, p2c_scores, idx, p2c_mirrored, seqlens, sm_scale,
+                                             return_lse, check_status)
+    if st is not None:
+        finish_status(st, check_status)
     return o, lse
 
 
@@ -163,19 +139,22 @@ _PENDING_STATUS = _status.PENDING
 def check_pending_status() -> None:
     """Read (one synchronisation) the device status words of every call since the last check that was made
     with ``check_status=False`` and raise if any bounded device wait gave up or any ``cu_seqlens`` was malformed."""
-    pending = _PENDING_STATUS.drain()
-    if not pending:
-        return
+    pooled = cabi.host.drain_pending()
     by_dev = {}
-    for st in pending:
+    for st in _PENDING_STATUS.drain():
         by_dev.setdefault(st.device, []).append(st)
     for dev, sts in by_dev.items():
         _check_status(torch.stack(sts).amax(dim=0))
+    if pooled is not None:
+        _raise_for(pooled)
 
 
 def _check_status(status: torch.Tensor):
     """Read the device status words (synchronises); raise if a wait gave up or cu_seqlens was invalid."""
-    st = status.tolist()
+    _raise_for(status.tolist())
+
+
+def _raise_for(st):
     if st[0]:
         raise cabi.TdbError(cabi.ERR_TIMEOUT, f"a device-side wait gave up (barrier code {st[0]})")
     if st[1]:
@@ -183,57 +162,40 @@ def _check_status(status: torch.Tensor):
                          "differ from the query offsets, or max_seqlen is smaller than the longest sequence)")
 
 
+def finish_status(st, check: bool) -> None:
+    """What a native call left to the caller: an error code of the library, the words of a report, or (during a stream
+    capture, or with every pooled word in use) a tensor of words that nobody has read yet."""
+    if isinstance(st, torch.Tensor):
+        if check:
+            _check_status(st)
+        else:
+            _PENDING_STATUS.append(st)
+    elif isinstance(st, int):
+        cabi.check(st)
+    else:
+        _raise_for(st)
+
+
+def needs_graph(*tensors) -> bool:
+    """Whether autograd would record the call (its backward then raises)."""
+    return torch.is_grad_enabled() and any(t.requires_grad for t in tensors)
+
+
+def _call_fixed(q, k, v, tables, seqlens, sm_scale, kernel, return_lse, check):
+    o, lse, st = cabi.host.attn_fixed(q, k, v, None if tables is None else tables.native(), seqlens, sm_scale, kernel,
+                                      return_lse, check)
+    if st is not None:
+        finish_status(st, check)
+    return o, lse
+
+
 class _FixedFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, q, k, v, tables, seqlens, sm_scale, kernel, return_lse, check):
-        dev = cabi.require_cuda(q, k, v, seqlens)
-        if q.dim() != 4 or k.shape != q.shape or v.shape != q.shape:
-            raise ValueError("q, k, v must share the shape (B, H, L, D); cross-attention lengths are not supported")
-        B, H, L, D = q.shape
-        if not (q.dtype == k.dtype == v.dtype):
-            raise ValueError("q, k, v must share a dtype")
-        code = cabi.dtype_code(q.dtype)
-        for t in (q, k, v):
-            if t.stride(-1) != 1:
-                raise ValueError("the head dimension must be contiguous")
-        o = torch.empty((B, L, H, D), dtype=q.dtype, device=dev).permute(0, 2, 1, 3)     # (B,H,L,D) view of [B,L,H,D]
-        lse = torch.empty((B, H, L), dtype=torch.float32, device=dev) if return_lse else None
-        status = torch.zeros(4, dtype=torch.int32, device=dev)
-        if B == 0 or L == 0:                         # nothing to compute
-            return (o, lse, status)
-        if seqlens is not None:
-            seqlens = seqlens.to(device=dev, dtype=torch.int32).contiguous()
-            if seqlens.numel() != B:
-                raise ValueError("seqlens must have one entry per batch row")
-        flags = 0
-        kr = qr = idx = kr_exp = qr_exp = None
-        two_span = idm = edm = erows = 0
-        if tables is not None:
-            kr, qr, idx, kr_exp, qr_exp = tables.kr, tables.qr, tables.idx, tables.kr_exp, tables.qr_exp
-            two_span, idm, edm, erows = tables.two_span, tables.idx_delta_max, tables.exp_delta_max, tables.exp_rows
-            flags = (cabi.TDB_FLAG_C2P if kr is not None else 0) | (cabi.TDB_FLAG_P2C if qr is not None else 0)
-            for t in (kr, qr):
-                if t is not None and t.dtype != q.dtype:
-                    raise ValueError("relative tables must have the dtype of q")
-
-        def s(t):
-            return (t.stride(0), t.stride(2), t.stride(1))      # batch, token, head
-
-        with torch.cuda.device(dev):
-            rc = cabi.lib.tdb_attn_fwd_fixed(
-                cabi.ptr(q), cabi.ptr(k), cabi.ptr(v), cabi.ptr(o), *s(q), *s(k), *s(v), *s(o),
-                cabi.ptr(kr), cabi.ptr(qr), two_span, cabi.ptr(idx), idm, cabi.ptr(kr_exp), cabi.ptr(qr_exp), edm, erows,
-                cabi.ptr(seqlens), B, L, H, D, float(sm_scale), flags, code, kernel, cabi.ptr(lse), cabi.ptr(status),
-                cabi.stream_ptr(dev))
-        cabi.check(rc)
-        if check:
-            _check_status(status)
-        else:
-            _PENDING_STATUS.append(status)
-        ctx.mark_non_differentiable(status)
+    def forward(ctx, q, k, v, *args):
+        o, lse = _call_fixed(q, k, v, *args)
         if lse is not None:
             ctx.mark_non_differentiable(lse)
-        return (o, lse, status)
+        return o, lse
 
     @staticmethod
     def backward(ctx, *grads):
@@ -266,7 +228,8 @@ def flash_attention_with_disentangled(q, k, v, q_pos, k_pos, causal=False, sm_sc
     if p2c_mirrored:
         raise ValueError("p2c_mirrored applies to materialised score tensors only")
     tables = _tables_from_args(q_pos, k_pos, q, position_buckets, max_relative_distance, tables)
-    o, lse, status = _FixedFn.apply(q, k, v, tables, seqlens, sm_scale, kernel, return_lse, check_status)
+    call = _FixedFn.apply if needs_graph(q, k, v) else _call_fixed
+    o, lse = call(q, k, v, tables, seqlens, sm_scale, kernel, return_lse, check_status)
     if return_lse:
         return o, lse
     return o

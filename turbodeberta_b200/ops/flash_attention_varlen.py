@@ -20,75 +20,40 @@ import math
 import torch
 
 from .. import _cabi as cabi
-from .flash_attention import (_PENDING_STATUS, _check_status, _index_table_for_scores, _is_materialised,
-                              _tables_from_args, refuse_gradients)
+from .flash_attention import (_index_table_for_scores, _is_materialised, _tables_from_args, finish_status, needs_graph,
+                              refuse_gradients)
+
+
+def _call_varlen(q, k, v, tables, cu_seqlens, max_seqlen, sm_scale, kernel, return_lse, check, cu_seqlens_k=None):
+    o, lse, st = cabi.host.attn_packed(q, k, v, None if tables is None else tables.native(), cu_seqlens, max_seqlen,
+                                       sm_scale, kernel, return_lse, check)
+    if st is not None:
+        finish_status(st, check)
+    _check_key_offsets(cu_seqlens, cu_seqlens_k, check)
+    return o, lse
 
 
 class _VarlenFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, q, k, v, tables, cu_seqlens, max_seqlen, sm_scale, kernel, return_lse, check, cu_seqlens_k=None):
-        dev = cabi.require_cuda(q, k, v, cu_seqlens)
-        if q.dim() != 3 or k.shape != q.shape or v.shape != q.shape:
-            raise ValueError("q, k, v must share the shape (T, H, D)")
-        T, H, D = q.shape
-        if not (q.dtype == k.dtype == v.dtype):
-            raise ValueError("q, k, v must share a dtype")
-        code = cabi.dtype_code(q.dtype)
-        for t in (q, k, v):
-            if t.stride(-1) != 1:
-                raise ValueError("the head dimension must be contiguous")
-        if cu_seqlens.dtype != torch.int32 or cu_seqlens.dim() != 1 or cu_seqlens.numel() < 1:
-            raise ValueError("cu_seqlens must be a 1-D int32 tensor of n_seqs + 1 offsets")
-        cu_seqlens = cu_seqlens.contiguous()
-        n_seqs = cu_seqlens.numel() - 1
-        o = torch.empty((T, H, D), dtype=q.dtype, device=dev)
-        if T == 0 or n_seqs == 0:                    # nothing to compute
-            st = torch.zeros(4, dtype=torch.int32, device=dev)
-            return (o, torch.empty((H, T), dtype=torch.float32, device=dev) if return_lse else None, st)
-        lse = torch.empty((H, T), dtype=torch.float32, device=dev) if return_lse else None
-        status = torch.zeros(4, dtype=torch.int32, device=dev)
-        ws_bytes = int(cabi.lib.tdb_attn_workspace_bytes(n_seqs, T))
-        ws = torch.empty(max(ws_bytes, 16), dtype=torch.uint8, device=dev)
-        flags = 0
-        kr = qr = idx = kr_exp = qr_exp = None
-        two_span = idm = edm = erows = 0
-        if tables is not None:
-            kr, qr, idx, kr_exp, qr_exp = tables.kr, tables.qr, tables.idx, tables.kr_exp, tables.qr_exp
-            two_span, idm, edm, erows = tables.two_span, tables.idx_delta_max, tables.exp_delta_max, tables.exp_rows
-            flags = (cabi.TDB_FLAG_C2P if kr is not None else 0) | (cabi.TDB_FLAG_P2C if qr is not None else 0)
-            for t in (kr, qr):
-                if t is not None and t.dtype != q.dtype:
-                    raise ValueError("relative tables must have the dtype of q")
-        with torch.cuda.device(dev):
-            rc = cabi.lib.tdb_attn_fwd_varlen(
-                cabi.ptr(q), cabi.ptr(k), cabi.ptr(v), cabi.ptr(o),
-                q.stride(0), q.stride(1), k.stride(0), k.stride(1), v.stride(0), v.stride(1), o.stride(0), o.stride(1),
-                cabi.ptr(kr), cabi.ptr(qr), two_span, cabi.ptr(idx), idm, cabi.ptr(kr_exp), cabi.ptr(qr_exp), edm, erows,
-                cabi.ptr(cu_seqlens), n_seqs, T, int(max_seqlen), H, D, float(sm_scale), flags, code, kernel,
-                cabi.ptr(ws), ws_bytes, cabi.ptr(lse), cabi.ptr(status), cabi.stream_ptr(dev))
-        cabi.check(rc)
-        _flag_offset_mismatch(status, cu_seqlens, cu_seqlens_k)
-        if check:
-            _check_status(status)
-        else:
-            _PENDING_STATUS.append(status)
-        ctx.mark_non_differentiable(status)
+    def forward(ctx, q, k, v, *args):
+        o, lse = _call_varlen(q, k, v, *args)
         if lse is not None:
             ctx.mark_non_differentiable(lse)
-        return (o, lse, status)
+        return o, lse
 
     @staticmethod
     def backward(ctx, *grads):
         raise RuntimeError("turbodeberta_b200 attention is forward-only (as in the reference: no backward kernel)")
 
 
-def _flag_offset_mismatch(status, cu_q, cu_k) -> None:
+def _check_key_offsets(cu_q, cu_k, check) -> None:
     """Self-attention only: key offsets must equal the query offsets.  When the caller passes two different tensors
-    the comparison runs on the device and lands in status word 1 (the malformed-offsets word), so the call itself
-    never waits for the GPU."""
+    the comparison runs on the device and counts as a malformed-offsets report of this call."""
     if cu_k is None or cu_k is cu_q or (cu_k.data_ptr() == cu_q.data_ptr() and cu_k.shape == cu_q.shape):
         return
-    status[1:2].add_((cu_k.to(cu_q.device) != cu_q).any().to(torch.int32))
+    words = torch.zeros(4, dtype=torch.int32, device=cu_q.device)
+    words[1:2].add_((cu_k.to(cu_q.device) != cu_q).any().to(torch.int32))
+    finish_status(words, check)
 
 
 def _scores_varlen(q, k, v, c2p_scores, p2c_scores, cu_seqlens, max_seqlen, sm_scale, position_buckets,
@@ -96,46 +61,13 @@ def _scores_varlen(q, k, v, c2p_scores, p2c_scores, cu_seqlens, max_seqlen, sm_s
     """Legacy form of the packed op: gather from materialised ``(T, H, 2*span)`` score tensors."""
     dev = cabi.require_cuda(q, k, v, cu_seqlens)
     refuse_gradients(q, k, v, c2p_scores, p2c_scores)
-    if q.dim() != 3 or k.shape != q.shape or v.shape != q.shape:
-        raise ValueError("q, k, v must share the shape (T, H, D)")
-    T, H, D = q.shape
-    code = cabi.dtype_code(q.dtype)
     some = c2p_scores if c2p_scores is not None else p2c_scores
-    two_span = some.shape[-1]
-    for t, name in ((c2p_scores, "q_pos"), (p2c_scores, "k_pos")):
-        if t is not None and (tuple(t.shape) != (T, H, two_span) or t.dtype != q.dtype or t.stride(-1) != 1):
-            raise ValueError(f"{name} must be (T, H, 2*span) of q's dtype with a contiguous last dimension")
-    for t in (q, k, v):
-        if t.stride(-1) != 1:
-            raise ValueError("the head dimension must be contiguous")
-    if cu_seqlens.dtype != torch.int32 or cu_seqlens.dim() != 1 or cu_seqlens.numel() < 1:
-        raise ValueError("cu_seqlens must be a 1-D int32 tensor of n_seqs + 1 offsets")
-    cu_seqlens = cu_seqlens.contiguous()
-    n_seqs = cu_seqlens.numel() - 1
-    idx, idm = _index_table_for_scores(two_span, position_buckets, max_relative_distance, dev)
-    o = torch.empty((T, H, D), dtype=q.dtype, device=dev)
-    lse = torch.empty((H, T), dtype=torch.float32, device=dev) if return_lse else None
-    if T == 0 or n_seqs == 0:
-        return o, lse
-    status = torch.zeros(4, dtype=torch.int32, device=dev)
-    flags = ((cabi.TDB_FLAG_C2P if c2p_scores is not None else 0) | (cabi.TDB_FLAG_P2C if p2c_scores is not None else 0)
-             | (cabi.TDB_FLAG_P2C_MIRRORED if p2c_mirrored else 0))
-
-    def s(t):
-        return (t.stride(0), t.stride(1)) if t is not None else (0, 0)
-
-    with torch.cuda.device(dev):
-        rc = cabi.lib.tdb_attn_fwd_varlen_scores(
-            cabi.ptr(q), cabi.ptr(k), cabi.ptr(v), cabi.ptr(o), *s(q), *s(k), *s(v), *s(o),
-            cabi.ptr(c2p_scores), *s(c2p_scores), cabi.ptr(p2c_scores), *s(p2c_scores), two_span, cabi.ptr(idx), idm,
-            cabi.ptr(cu_seqlens), n_seqs, T, max_seqlen, H, D, float(sm_scale), flags, code, cabi.ptr(lse),
-            cabi.ptr(status), cabi.stream_ptr(dev))
-    cabi.check(rc)
-    _flag_offset_mismatch(status, cu_seqlens, cu_seqlens_k)
-    if check_status:
-        _check_status(status)
-    else:
-        _PENDING_STATUS.append(status)
+    idx = _index_table_for_scores(some.shape[-1], position_buckets, max_relative_distance, dev)
+    o, lse, st = cabi.host.attn_packed_scores(q, k, v, c2p_scores, p2c_scores, idx, p2c_mirrored, cu_seqlens, max_seqlen,
+                                              sm_scale, return_lse, check_status)
+    if st is not None:
+        finish_status(st, check_status)
+    _check_key_offsets(cu_seqlens, cu_seqlens_k, check_status)
     return o, lse
 
 
@@ -164,8 +96,8 @@ def flash_attention_with_disentangled_varlen(q, k, v, q_pos, k_pos, cu_seqlens_q
     if p2c_mirrored:
         raise ValueError("p2c_mirrored applies to materialised score tensors only")
     tables = _tables_from_args(q_pos, k_pos, q, position_buckets, max_relative_distance, tables)
-    o, lse, status = _VarlenFn.apply(q, k, v, tables, cu_seqlens_q, max_seqlen, sm_scale, kernel, return_lse,
-                                     check_status, cu_seqlens_k)
+    call = _VarlenFn.apply if needs_graph(q, k, v) else _call_varlen
+    o, lse = call(q, k, v, tables, cu_seqlens_q, max_seqlen, sm_scale, kernel, return_lse, check_status, cu_seqlens_k)
     if return_lse:
         return o, lse
     return o

@@ -18,6 +18,7 @@ from dataclasses import dataclass
 import torch
 
 from . import _cabi as cabi
+from ._cabi import host
 from .status import PENDING as PENDING_STATUS
 
 _IDX_CACHE: dict = {}
@@ -92,6 +93,16 @@ def expand(table: torch.Tensor, idx: torch.Tensor, exp_delta_max: int) -> torch.
     return out
 
 
+def expand_pair(kr: torch.Tensor | None, qr: torch.Tensor | None, idx: torch.Tensor, exp_delta_max: int):
+    """``expand`` of both tables of a layer (either may be None); bf16 tables of head_dim 64 take one launch."""
+    some = kr if kr is not None else qr
+    if some is None:
+        return None, None
+    if some.dtype == torch.bfloat16 and some.shape[-1] == 64:
+        return host.expand_pair(kr, qr, idx, exp_delta_max)
+    return tuple(None if t is None else expand(t, idx, exp_delta_max) for t in (kr, qr))
+
+
 @dataclass
 class RelPosTables:
     position_buckets: int
@@ -105,6 +116,19 @@ class RelPosTables:
     qr_exp: torch.Tensor | None
     exp_delta_max: int
     exp_rows: int
+
+    def native(self):
+        """The same fields as one object of the host extension (built on first use, again after a field is set)."""
+        n = self.__dict__.get("_native")
+        if n is None:
+            n = host.Tables(self.kr, self.qr, self.idx, self.kr_exp, self.qr_exp, self.two_span, self.idx_delta_max,
+                            self.exp_delta_max, self.exp_rows)
+            self.__dict__["_native"] = n
+        return n
+
+    def __setattr__(self, name, value):
+        self.__dict__.pop("_native", None)
+        self.__dict__[name] = value
 
 
 def build_tables(rel_embeddings: torch.Tensor, *, num_heads: int, position_buckets: int,
@@ -126,7 +150,6 @@ def build_tables(rel_embeddings: torch.Tensor, *, num_heads: int, position_bucke
         expanded = rel.dtype == torch.bfloat16
     exp_delta_max = sat + cabi.TDB_EXPAND_MARGIN
     exp_rows = (2 * exp_delta_max + 1 + 7) // 8 * 8
-    kr_exp = expand(kr, idx, exp_delta_max) if (expanded and kr is not None) else None
-    qr_exp = expand(qr, idx, exp_delta_max) if (expanded and qr is not None) else None
+    kr_exp, qr_exp = expand_pair(kr, qr, idx, exp_delta_max) if expanded else (None, None)
     return RelPosTables(position_buckets, max_relative_positions, 2 * span, idx, idx_delta_max, kr, qr,
                         kr_exp, qr_exp, exp_delta_max, exp_rows)
