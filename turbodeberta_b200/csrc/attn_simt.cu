@@ -1,56 +1,99 @@
-// CUDA-core disentangled attention: exact fp32 arithmetic, any I/O dtype.
+// CUDA-core disentangled attention: exact fp32 arithmetic on f32 or bf16 inputs.
 //
-// This is the full-precision path (fp32 inputs must land within 1e-4 of the eager module, which the
-// bf16 tensor-core pipeline cannot do) and the cross-check for the tensor-core kernel.  One warp owns
-// one query row; lane l scores keys l, l+32, ... with its own online softmax state (max, sum, 64
-// output partials) and the 32 states are merged once at the end.  All operands are read through the
-// read-only cache; nothing is staged, so it is latency/L1-bound and is not the throughput path.
+// This is the full-precision path (fp32 inputs must land within 1e-4 of the eager module, which the bf16 tensor-core
+// pipeline cannot do), the path of materialised position scores, and the cross-check for the tensor-core kernel.
 //
 //   score[q,k] = (Q[q].K[k] + Q[q].Kr[r] + K[k].Qr[r]) * sm_scale,  r = idx[clamp(q-k)]
 //
 // Legacy form: the two position products arrive materialised (c2p_scores[q, r], p2c_scores[k, r]) and are only
 // gathered; with TDB_FLAG_P2C_MIRRORED the p2c term is read at idx[clamp(k-q)], the reference kernel's convention.
+//
+// Bound by the FMA pipes and, close behind, by shared-memory reads (256 fp32 multiply-adds per score with both terms).
+// A block of two warps owns 8R query rows and walks the keys in tiles of 64.  A thread owns R x 8 scores at rows ti + 8r and
+// keys tj + 8s, so that the distance of each of them is (ti - tj) + 8 (r - s): R + 7 table rows per term serve all 8R
+// scores, every product that is formed is a score's own (a band of q.Kr products over all distances of a tile would be
+// twice as many), and nothing has to be skewed or gathered afterwards.  Operand rows are staged fp32, 36-word pitch, half a
+// head (32 columns) at a time: eight consecutive rows fall on different banks, and four blocks fit on an SM, which cover
+// each other's loads.  The rows of one query tile stay inside one warp, so the softmax needs shuffles only.
+// One call of 8 x (48..387) fp32 tokens with 12 heads and both terms: 245 us, 23 TFLOP/s (one warp per query row, keys spread
+// over its lanes, every operand read row by row through L1: 1852 us).
 #include "tdb_internal.h"
 #include <math_constants.h>
 
 namespace tdb {
 
-template <typename T> __device__ __forceinline__ void load64(const T* p, float* dst);
-template <> __device__ __forceinline__ void load64<float>(const float* p, float* dst) {
-  const float4* p4 = reinterpret_cast<const float4*>(p);
-#pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    float4 t = __ldg(p4 + i);
-    dst[4 * i] = t.x; dst[4 * i + 1] = t.y; dst[4 * i + 2] = t.z; dst[4 * i + 3] = t.w;
-  }
-}
-template <> __device__ __forceinline__ void load64<__nv_bfloat16>(const __nv_bfloat16* p, float* dst) {
-  const uint4* p4 = reinterpret_cast<const uint4*>(p);
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    uint4 t = __ldg(p4 + i);
-    uint32_t w[4] = {t.x, t.y, t.z, t.w};
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      dst[8 * i + 2 * j] = __uint_as_float(w[j] << 16);
-      dst[8 * i + 2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u);
-    }
-  }
-}
-template <typename T> __device__ __forceinline__ T cast_out(float x);
-template <> __device__ __forceinline__ float cast_out<float>(float x) { return x; }
-template <> __device__ __forceinline__ __nv_bfloat16 cast_out<__nv_bfloat16>(float x) { return __float2bfloat16_rn(x); }
+namespace {
+
+constexpr int KT = 64, HALF = 32, HP = HALF + 4, DP = 64 + 4, THREADS = 64;
 
 __device__ __forceinline__ float to_float(float x) { return x; }
 __device__ __forceinline__ float to_float(__nv_bfloat16 x) { return __bfloat162float(x); }
 
-constexpr int SIMT_WARPS = 4;
+__device__ __forceinline__ void cp_async16(float* dst, const void* src, bool real) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(real ? 16 : 0) : "memory");
+}
 
-template <typename T>
-__global__ void __launch_bounds__(SIMT_WARPS * 32) attn_simt_kernel(const AttnParams p) {
+// COLS columns of ROWS rows to shared memory as fp32; src(row) is the row's first element, or null for a row of zeros.
+template <typename T, int COLS, int PITCH, typename F>
+__device__ __forceinline__ void stage_rows(float* dst, int rows, const T* any, F src) {
+  constexpr int PER = 16 / sizeof(T), CH = COLS / PER;
+  for (int e = threadIdx.x; e < rows * CH; e += THREADS) {
+    const int row = e / CH, c = e % CH;
+    const T* s = src(row);
+    float* d = dst + row * PITCH + c * PER;
+    if constexpr (sizeof(T) == 4) {
+      cp_async16(d, s ? s + c * PER : any, s != nullptr);
+    } else {
+      uint4 t = make_uint4(0, 0, 0, 0);
+      if (s) t = __ldg(reinterpret_cast<const uint4*>(s) + c);
+      const uint32_t w[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+        *reinterpret_cast<float4*>(d + 4 * i) =
+            make_float4(__uint_as_float(w[2 * i] << 16), __uint_as_float(w[2 * i] & 0xffff0000u),
+                        __uint_as_float(w[2 * i + 1] << 16), __uint_as_float(w[2 * i + 1] & 0xffff0000u));
+    }
+  }
+}
+__device__ __forceinline__ void staged() {
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+}
+
+__device__ __forceinline__ void fma4(float& acc, const float4& a, const float4& b) {
+  acc = fmaf(a.x, b.x, acc); acc = fmaf(a.y, b.y, acc); acc = fmaf(a.z, b.z, acc); acc = fmaf(a.w, b.w, acc);
+}
+
+__device__ __forceinline__ void store4(float* d, float a, float b, float c, float e) { *reinterpret_cast<float4*>(d) = make_float4(a, b, c, e); }
+__device__ __forceinline__ void store4(__nv_bfloat16* d, float a, float b, float c, float e) {
+  __nv_bfloat162 lo = __floats2bfloat162_rn(a, b), hi = __floats2bfloat162_rn(c, e);
+  uint2 v;
+  v.x = *reinterpret_cast<uint32_t*>(&lo); v.y = *reinterpret_cast<uint32_t*>(&hi);
+  *reinterpret_cast<uint2*>(d) = v;
+}
+
+template <int R> constexpr int smem_floats(bool tables) {
+  const int half = (KT + (tables ? 2 * (8 * R + KT) : 0)) * HP;
+  const int values = KT * DP;
+  return 2 * 8 * R * DP + (half > values ? half : values);
+}
+
+// TABLES: position terms from the projected tables (either may be absent); otherwise none, or gathered scores.
+template <typename T, int R, bool TABLES>
+__global__ void __launch_bounds__(THREADS, 4) attn_simt_kernel(const AttnParams p) {
+  constexpr int QT = 8 * R, XR = QT + KT;           // XR: table rows a tile can touch (QT + KT - 1, padded)
+  extern __shared__ __align__(16) float smem[];
+  float* const sQ = smem;                            // [QT][DP]
+  float* const sP = sQ + QT * DP;                    // [QT][DP]
+  float* const sK = sP + QT * DP;                    // [KT][HP], half a head
+  float* const sKr = sK + KT * HP;                   // [XR][HP]
+  float* const sQr = sKr + XR * HP;                  // [XR][HP]
+  float* const sV = sK;                              // [KT][DP], over the three above
+
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-  const int s = blockIdx.z, h = blockIdx.y;
-  const int qi = blockIdx.x * SIMT_WARPS + warp;
+  const int ti = warp * 4 + lane / 8, tj = lane % 8;
+  const int s = blockIdx.z, h = blockIdx.y, q0 = blockIdx.x * QT;
   int len, rows;                 // valid length; rows that exist in the output
   int64_t tok0; int b;
   if (p.varlen) {
@@ -69,109 +112,196 @@ __global__ void __launch_bounds__(SIMT_WARPS * 32) attn_simt_kernel(const AttnPa
     len = p.seqlens ? p.seqlens[s] : p.L; rows = p.L; tok0 = 0; b = s;
     len = len < 0 ? 0 : (len > p.L ? p.L : len);
   }
-  if (qi >= rows) return;
-  T* orow = reinterpret_cast<T*>(p.o) + b * p.o_sb + (tok0 + qi) * p.o_st + h * p.o_sh;
-  if (qi >= len) {               // padded query row of the padded form: zeros
-    orow[lane] = cast_out<T>(0.f); orow[lane + 32] = cast_out<T>(0.f);
-    if (p.lse) p.lse[b * p.lse_sb + h * p.lse_sh + tok0 + qi] = 0.f;
-    return;
-  }
-  const T* qb = reinterpret_cast<const T*>(p.q) + b * p.q_sb + (tok0 + qi) * p.q_st + h * p.q_sh;
-  const T* kb = reinterpret_cast<const T*>(p.k) + b * p.k_sb + tok0 * p.k_st + h * p.k_sh;
-  const T* vb = reinterpret_cast<const T*>(p.v) + b * p.v_sb + tok0 * p.v_st + h * p.v_sh;
-  const bool gathered = p.c2p_scores || p.p2c_scores;
-  const T* krh = (!gathered && (p.flags & TDB_FLAG_C2P)) ? reinterpret_cast<const T*>(p.kr) + (int64_t)h * p.two_span * 64 : nullptr;
-  const T* qrh = (!gathered && (p.flags & TDB_FLAG_P2C)) ? reinterpret_cast<const T*>(p.qr) + (int64_t)h * p.two_span * 64 : nullptr;
-  // materialised scores: this query's row of c2p, and the base of this head's p2c rows (one per key)
-  const T* c2p_row = ((p.flags & TDB_FLAG_C2P) && p.c2p_scores)
-      ? reinterpret_cast<const T*>(p.c2p_scores) + b * p.c2p_sb + (tok0 + qi) * p.c2p_st + h * p.c2p_sh : nullptr;
-  const T* p2c_base = ((p.flags & TDB_FLAG_P2C) && p.p2c_scores)
+  if (q0 >= rows) return;
+  T* const ob = reinterpret_cast<T*>(p.o) + b * p.o_sb + tok0 * p.o_st + h * p.o_sh;
+  float* const lse = p.lse ? p.lse + b * p.lse_sb + h * p.lse_sh + tok0 : nullptr;
+
+  const T* const qb = reinterpret_cast<const T*>(p.q) + b * p.q_sb + tok0 * p.q_st + h * p.q_sh;
+  const T* const kb = reinterpret_cast<const T*>(p.k) + b * p.k_sb + tok0 * p.k_st + h * p.k_sh;
+  const T* const vb = reinterpret_cast<const T*>(p.v) + b * p.v_sb + tok0 * p.v_st + h * p.v_sh;
+  const T* const krh = (TABLES && (p.flags & TDB_FLAG_C2P)) ? reinterpret_cast<const T*>(p.kr) + (int64_t)h * p.two_span * 64 : nullptr;
+  const T* const qrh = (TABLES && (p.flags & TDB_FLAG_P2C)) ? reinterpret_cast<const T*>(p.qr) + (int64_t)h * p.two_span * 64 : nullptr;
+  // materialised scores: the base of this head's c2p rows (one per query) and p2c rows (one per key)
+  const T* const c2p_base = (!TABLES && (p.flags & TDB_FLAG_C2P))
+      ? reinterpret_cast<const T*>(p.c2p_scores) + b * p.c2p_sb + tok0 * p.c2p_st + h * p.c2p_sh : nullptr;
+  const T* const p2c_base = (!TABLES && (p.flags & TDB_FLAG_P2C))
       ? reinterpret_cast<const T*>(p.p2c_scores) + b * p.p2c_sb + tok0 * p.p2c_st + h * p.p2c_sh : nullptr;
+  const int dm = p.idx_delta_max;
+  auto clamped = [&](int delta) { return delta < -dm ? 0 : (delta > dm ? 2 * dm : delta + dm); };
 
-  float qv[64], acc[64], kv[64], tv[64];
-  load64<T>(qb, qv);
+  float o[R][8], m[R], l[R];
 #pragma unroll
-  for (int d = 0; d < 64; ++d) acc[d] = 0.f;
-  float m = -CUDART_INF_F, l = 0.f;
+  for (int r = 0; r < R; ++r) {
+    m[r] = -CUDART_INF_F; l[r] = 0.f;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) o[r][c] = 0.f;
+  }
 
-  for (int kj = lane; kj < len; kj += 32) {
-    load64<T>(kb + (int64_t)kj * p.k_st, kv);
-    float sc = 0.f;
+  if (q0 < len) {
+    stage_rows<T, 64, DP>(sQ, QT, qb, [&](int row) { return q0 + row < len ? qb + (int64_t)(q0 + row) * p.q_st : nullptr; });
+    for (int k0 = 0; k0 < len; k0 += KT) {
+      float acc[R][8];
 #pragma unroll
-    for (int d = 0; d < 64; ++d) sc = fmaf(qv[d], kv[d], sc);
-    if (c2p_row || p2c_base) {
-      int delta = qi - kj;
-      delta = delta < -p.idx_delta_max ? -p.idx_delta_max : (delta > p.idx_delta_max ? p.idx_delta_max : delta);
-      if (c2p_row) sc += to_float(c2p_row[p.idx[delta + p.idx_delta_max]]);
-      if (p2c_base) {
-        const int r = (p.flags & TDB_FLAG_P2C_MIRRORED) ? p.idx[p.idx_delta_max - delta] : p.idx[delta + p.idx_delta_max];
-        sc += to_float(p2c_base[(int64_t)kj * p.p2c_st + r]);
+      for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int c = 0; c < 8; ++c) acc[r][c] = 0.f;
+#pragma unroll 1
+      for (int half = 0; half < 2; ++half) {
+        const int d0 = half * HALF;
+        stage_rows<T, HALF, HP>(sK, KT, kb, [&](int row) { return k0 + row < len ? kb + (int64_t)(k0 + row) * p.k_st + d0 : nullptr; });
+        if (TABLES) {
+          auto table_row = [&](const T* t, int x) { return t + (int64_t)p.idx[clamped(q0 - k0 - (KT - 1) + x)] * 64 + d0; };
+          if (krh) stage_rows<T, HALF, HP>(sKr, XR, krh, [&](int x) { return table_row(krh, x); });
+          if (qrh) stage_rows<T, HALF, HP>(sQr, XR, qrh, [&](int x) { return table_row(qrh, x); });
+        }
+        staged();
+        const float* const kp = sK + tj * HP;
+        const float* const qp = sQ + ti * DP + d0;
+        const int x0 = ti - tj + (KT - 1) - 56;      // table row of (r, s) is x0 + 8 (r - s + 7)
+#pragma unroll 1
+        for (int d = 0; d < HALF; d += 4) {
+          float4 kf[8];
+#pragma unroll
+          for (int c = 0; c < 8; ++c) kf[c] = *reinterpret_cast<const float4*>(kp + 8 * c * HP + d);
+          if (TABLES && krh) {
+            float4 t[R + 7];
+#pragma unroll
+            for (int x = 0; x < R + 7; ++x) t[x] = *reinterpret_cast<const float4*>(sKr + (x0 + 8 * x) * HP + d);
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+              const float4 qf = *reinterpret_cast<const float4*>(qp + 8 * r * DP + d);
+#pragma unroll
+              for (int c = 0; c < 8; ++c) { fma4(acc[r][c], qf, kf[c]); fma4(acc[r][c], qf, t[r - c + 7]); }
+            }
+          } else {
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+              const float4 qf = *reinterpret_cast<const float4*>(qp + 8 * r * DP + d);
+#pragma unroll
+              for (int c = 0; c < 8; ++c) fma4(acc[r][c], qf, kf[c]);
+            }
+          }
+          if (TABLES && qrh) {
+            float4 t[R + 7];
+#pragma unroll
+            for (int x = 0; x < R + 7; ++x) t[x] = *reinterpret_cast<const float4*>(sQr + (x0 + 8 * x) * HP + d);
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+#pragma unroll
+              for (int c = 0; c < 8; ++c) fma4(acc[r][c], kf[c], t[r - c + 7]);
+          }
+        }
+        __syncthreads();
       }
-    }
-    if (krh || qrh) {
-      int delta = qi - kj;
-      delta = delta < -p.idx_delta_max ? -p.idx_delta_max : (delta > p.idx_delta_max ? p.idx_delta_max : delta);
-      int r = p.idx[delta + p.idx_delta_max];
-      if (krh) {
-        load64<T>(krh + (int64_t)r * 64, tv);
-        float c = 0.f;
+      // V replaces the operand rows while the softmax runs
+      stage_rows<T, 64, DP>(sV, KT, vb, [&](int row) { return k0 + row < len ? vb + (int64_t)(k0 + row) * p.v_st : nullptr; });
 #pragma unroll
-        for (int d = 0; d < 64; ++d) c = fmaf(qv[d], tv[d], c);
-        sc += c;
+      for (int r = 0; r < R; ++r) {
+        const int qi = q0 + ti + 8 * r;
+        float mx = -CUDART_INF_F;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          const int kj = k0 + tj + 8 * c;
+          float sc = acc[r][c];
+          if (!TABLES && kj < len && qi < len) {
+            const int x = clamped(qi - kj);
+            if (c2p_base) sc += to_float(c2p_base[(int64_t)qi * p.c2p_st + p.idx[x]]);
+            if (p2c_base) sc += to_float(p2c_base[(int64_t)kj * p.p2c_st + p.idx[(p.flags & TDB_FLAG_P2C_MIRRORED) ? 2 * dm - x : x]]);
+          }
+          sc = kj < len ? sc * p.sm_scale : -CUDART_INF_F;
+          acc[r][c] = sc;
+          mx = fmaxf(mx, sc);
+        }
+#pragma unroll
+        for (int off = 1; off < 8; off *= 2) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+        const float mn = fmaxf(m[r], mx);            // finite: every key tile has a valid key
+        const float corr = expf(m[r] - mn);          // first tile: m = -inf -> 0
+        m[r] = mn;
+        float sum = 0.f;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          const float e = expf(acc[r][c] - mn);
+          sum += e;
+          sP[(ti + 8 * r) * DP + tj + 8 * c] = e;
+        }
+        l[r] = l[r] * corr + sum;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) o[r][c] *= corr;
       }
-      if (qrh) {
-        load64<T>(qrh + (int64_t)r * 64, tv);
-        float c = 0.f;
+      staged();                                      // also makes the warp's own rows of P visible to its lanes
+#pragma unroll 1
+      for (int j = 0; j < KT; j += 4) {
+        float4 pf[R];
 #pragma unroll
-        for (int d = 0; d < 64; ++d) c = fmaf(kv[d], tv[d], c);
-        sc += c;
+        for (int r = 0; r < R; ++r) pf[r] = *reinterpret_cast<const float4*>(sP + (ti + 8 * r) * DP + j);
+#pragma unroll
+        for (int jj = 0; jj < 4; ++jj) {
+          const float4 a = *reinterpret_cast<const float4*>(sV + (j + jj) * DP + 4 * tj);
+          const float4 c = *reinterpret_cast<const float4*>(sV + (j + jj) * DP + 32 + 4 * tj);
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            const float w = jj == 0 ? pf[r].x : jj == 1 ? pf[r].y : jj == 2 ? pf[r].z : pf[r].w;
+            o[r][0] = fmaf(w, a.x, o[r][0]); o[r][1] = fmaf(w, a.y, o[r][1]);
+            o[r][2] = fmaf(w, a.z, o[r][2]); o[r][3] = fmaf(w, a.w, o[r][3]);
+            o[r][4] = fmaf(w, c.x, o[r][4]); o[r][5] = fmaf(w, c.y, o[r][5]);
+            o[r][6] = fmaf(w, c.z, o[r][6]); o[r][7] = fmaf(w, c.w, o[r][7]);
+          }
+        }
       }
+      __syncthreads();                               // the next tile's operand rows go where V is
     }
-    sc *= p.sm_scale;
-    float mn = fmaxf(m, sc);
-    float corr = expf(m - mn);                            // first key: m = -inf -> 0
-    float pe = expf(sc - mn);
-    l = l * corr + pe;
-    load64<T>(vb + (int64_t)kj * p.v_st, tv);
-#pragma unroll
-    for (int d = 0; d < 64; ++d) acc[d] = fmaf(pe, tv[d], acc[d] * corr);
-    m = mn;
   }
-  // merge the 32 lane-local softmax states
 #pragma unroll
-  for (int off = 16; off >= 1; off >>= 1) {
-    float mo = __shfl_xor_sync(0xffffffffu, m, off);
-    float lo = __shfl_xor_sync(0xffffffffu, l, off);
-    float mn = fmaxf(m, mo);
-    float a = (m == -CUDART_INF_F) ? 0.f : expf(m - mn);
-    float bb = (mo == -CUDART_INF_F) ? 0.f : expf(mo - mn);
-    l = l * a + lo * bb;
+  for (int r = 0; r < R; ++r) {
+    const int qi = q0 + ti + 8 * r;
+    float sum = l[r];
 #pragma unroll
-    for (int d = 0; d < 64; ++d) {
-      float oo = __shfl_xor_sync(0xffffffffu, acc[d], off);
-      acc[d] = acc[d] * a + oo * bb;
+    for (int off = 1; off < 8; off *= 2) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+    if (qi >= rows) continue;
+    const bool valid = qi < len;                     // padded query rows of the padded form: zeros
+    const float inv = valid ? 1.f / sum : 0.f;
+    T* const orow = ob + (int64_t)qi * p.o_st;
+    if (valid) {
+      store4(orow + 4 * tj, o[r][0] * inv, o[r][1] * inv, o[r][2] * inv, o[r][3] * inv);
+      store4(orow + 32 + 4 * tj, o[r][4] * inv, o[r][5] * inv, o[r][6] * inv, o[r][7] * inv);
+    } else {
+      store4(orow + 4 * tj, 0.f, 0.f, 0.f, 0.f);
+      store4(orow + 32 + 4 * tj, 0.f, 0.f, 0.f, 0.f);
     }
-    m = mn;
+    if (lse && tj == 0) lse[qi] = valid ? m[r] + logf(sum) : 0.f;
   }
-  float inv = 1.f / l;
-  // every lane now holds the whole row; lane l writes elements l and l+32
-  float o0 = 0.f, o1 = 0.f;
-#pragma unroll
-  for (int d = 0; d < 32; ++d) {
-    if (d == lane) { o0 = acc[d]; o1 = acc[d + 32]; }
-  }
-  orow[lane] = cast_out<T>(o0 * inv);
-  orow[lane + 32] = cast_out<T>(o1 * inv);
-  if (p.lse && lane == 0) p.lse[b * p.lse_sb + h * p.lse_sh + tok0 + qi] = m + logf(l);
 }
+
+template <typename T, int R, bool TABLES>
+int launch_variant(const AttnParams& p, cudaStream_t s) {
+  constexpr int SMEM = smem_floats<R>(TABLES) * 4;
+  auto kern = attn_simt_kernel<T, R, TABLES>;
+  if (SMEM > 48 * 1024) {
+    int rc = opt_in_smem(reinterpret_cast<const void*>(kern), SMEM);
+    if (rc) return rc;
+  }
+  dim3 grid((p.L + 8 * R - 1) / (8 * R), p.H, p.n_seqs);
+  kern<<<grid, THREADS, SMEM, s>>>(p);
+  return cuda_fail(cudaGetLastError(), "attn_simt launch");
+}
+
+template <typename T>
+int launch_dtype(const AttnParams& p, cudaStream_t s) {
+  const bool tables = p.flags && !p.c2p_scores && !p.p2c_scores;
+  // 32 query rows per block re-use each staged row twice as often as 16; 16 rows where 32 would leave SMs without a block.
+  int sms = 0, rc;
+  if ((rc = device_sms(&sms))) return rc;
+  const bool small = (int64_t)((p.L + 31) / 32) * p.H * p.n_seqs < 2 * (int64_t)sms;
+  if (tables) return small ? launch_variant<T, 2, true>(p, s) : launch_variant<T, 4, true>(p, s);
+  return small ? launch_variant<T, 2, false>(p, s) : launch_variant<T, 4, false>(p, s);
+}
+
+}  // namespace
 
 int launch_attn_simt(const AttnParams& p, int dtype, cudaStream_t s) {
   if (p.n_seqs == 0 || p.L == 0) return TDB_OK;
-  dim3 grid((p.L + SIMT_WARPS - 1) / SIMT_WARPS, p.H, p.n_seqs);
-  if (grid.z > 65535 || grid.y > 65535) { set_error("attn_simt: more than 65535 sequences or heads"); return TDB_ERR_SHAPE; }
-  if (dtype == TDB_DTYPE_F32) attn_simt_kernel<float><<<grid, SIMT_WARPS * 32, 0, s>>>(p);
-  else attn_simt_kernel<__nv_bfloat16><<<grid, SIMT_WARPS * 32, 0, s>>>(p);
-  return cuda_fail(cudaGetLastError(), "attn_simt launch");
+  if (p.n_seqs > 65535 || p.H > 65535) { set_error("attn_simt: more than 65535 sequences or heads"); return TDB_ERR_SHAPE; }
+  return dtype == TDB_DTYPE_F32 ? launch_dtype<float>(p, s) : launch_dtype<__nv_bfloat16>(p, s);
 }
 
 }  // namespace tdb

@@ -1035,36 +1035,11 @@ int table_map(CUtensorMap* m, const void* ptr, int rows, int H, int box_rows, co
   return encode_map(m, ptr, 3, dims, strides, box, what);
 }
 
-int device_sms(int* sms) {
-  constexpr int MAX_DEV = 64;
-  static int known[MAX_DEV] = {};                  // same value from every thread: a race writes it twice
-  int dev = 0, rc;
-  if ((rc = cuda_fail(cudaGetDevice(&dev), "cudaGetDevice"))) return rc;
-  if (dev < MAX_DEV && known[dev]) { *sms = known[dev]; return TDB_OK; }
-  if ((rc = cuda_fail(cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev), "cudaDeviceGetAttribute"))) return rc;
-  if (dev < MAX_DEV) known[dev] = *sms;
-  return TDB_OK;
-}
-
-// The kernel needs more dynamic shared memory than the default limit; the attribute is per device and per
-// instantiation, so it is set once for each pair, under a lock (entry points may be called from several host threads).
 template <bool C2P, bool P2C, bool LONG>
 int launch_variant(const AttnParams& p, dim3 grid, const CUtensorMap* maps, cudaStream_t s) {
   auto kern = attn_umma_kernel<C2P, P2C, LONG>;
-  constexpr int MAX_DEV = 64;
-  static std::mutex mu;
-  static bool configured[MAX_DEV] = {};
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return cuda_fail(e, "cudaGetDevice");
-  {
-    std::lock_guard<std::mutex> lock(mu);
-    if (dev < 0 || dev >= MAX_DEV || !configured[dev]) {
-      e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
-      if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(max dynamic shared memory)");
-      if (dev >= 0 && dev < MAX_DEV) configured[dev] = true;
-    }
-  }
+  const int rc = opt_in_smem(reinterpret_cast<const void*>(kern), (int)SMEM_BYTES);
+  if (rc) return rc;
   kern<<<grid, NTHREADS, SMEM_BYTES, s>>>(p, maps[0], maps[1], maps[2], maps[3], maps[4], maps[5], maps[6]);
   return cuda_fail(cudaGetLastError(), "attn_umma launch");
 }

@@ -182,18 +182,7 @@ int launch_relpos_project_umma(const void* rel, const void* W, const void* bias,
   int rc;
   if ((rc = map_2d(&tm_rel, rel, (uint64_t)hidden, (uint64_t)two_span, PM, "rel"))) return rc;
   if ((rc = map_2d(&tm_w, W, (uint64_t)hidden, (uint64_t)H * PN, PN, "W"))) return rc;
-  {                                   // the shared-memory opt-in is a per-device attribute: set once per device
-    static std::mutex mu;
-    static bool configured[64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    std::lock_guard<std::mutex> lock(mu);
-    if (dev < 0 || dev >= 64 || !configured[dev]) {
-      cudaError_t e = cudaFuncSetAttribute(relpos_project_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P_SMEM);
-      if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(relpos projection)");
-      if (dev >= 0 && dev < 64) configured[dev] = true;
-    }
-  }
+  if ((rc = opt_in_smem(reinterpret_cast<const void*>(relpos_project_umma_kernel), (int)P_SMEM))) return rc;
   dim3 grid((two_span + PM - 1) / PM, H);
   relpos_project_umma_kernel<<<grid, P_THREADS, P_SMEM, s>>>(tm_rel, tm_w, (const __nv_bfloat16*)bias, two_span, hidden, H,
                                                              (__nv_bfloat16*)out, status);

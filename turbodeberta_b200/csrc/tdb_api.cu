@@ -3,6 +3,8 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
+#include <vector>
 
 namespace tdb {
 
@@ -18,6 +20,34 @@ int cuda_fail(cudaError_t e, const char* what) {
   if (e == cudaSuccess) return TDB_OK;
   set_error("%s: %s", what, cudaGetErrorString(e));
   return TDB_ERR_CUDA;
+}
+
+int device_sms(int* sms) {
+  constexpr int MAX_DEV = 64;
+  static int known[MAX_DEV] = {};                  // same value from every thread: a race writes it twice
+  int dev = 0, rc;
+  if ((rc = cuda_fail(cudaGetDevice(&dev), "cudaGetDevice"))) return rc;
+  if (dev < MAX_DEV && known[dev]) { *sms = known[dev]; return TDB_OK; }
+  if ((rc = cuda_fail(cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev), "cudaDeviceGetAttribute"))) return rc;
+  if (dev < MAX_DEV) known[dev] = *sms;
+  return TDB_OK;
+}
+
+int opt_in_smem(const void* kernel, int bytes) {
+  constexpr int MAX_DEV = 64;
+  static std::mutex mu;
+  static std::vector<const void*> done[MAX_DEV];   // a handful of kernels per device
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return cuda_fail(e, "cudaGetDevice");
+  std::lock_guard<std::mutex> lock(mu);
+  if (dev < MAX_DEV)
+    for (const void* k : done[dev])
+      if (k == kernel) return TDB_OK;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(max dynamic shared memory)");
+  if (dev < MAX_DEV) done[dev].push_back(kernel);
+  return TDB_OK;
 }
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }

@@ -45,6 +45,9 @@ struct AttnParams {
 void set_error(const char* fmt, ...);
 int cuda_fail(cudaError_t e, const char* what);
 
+int device_sms(int* sms);                                            // of the current device; asked once per device
+int opt_in_smem(const void* kernel, int bytes);                      // dynamic shared memory beyond 48 KB, set once per device
+
 int launch_bucket_table(int buckets, int max_pos, int delta_max, int16_t* out, cudaStream_t s);
 int launch_relpos_project(const void* rel, const void* W, const void* bias, int two_span, int hidden,
                           int H, int D, int dtype, void* out, cudaStream_t s);
