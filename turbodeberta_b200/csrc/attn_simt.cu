@@ -73,6 +73,23 @@ __device__ __forceinline__ void store4(__nv_bfloat16* d, float a, float b, float
   *reinterpret_cast<uint2*>(d) = v;
 }
 
+// The sequence that block row z works on.  Blocks start in grid order, and those of a long sequence last longest: with the
+// sequences taken by decreasing length (up to 64 of them, one per thread) the last blocks to start are the cheapest.
+__device__ __forceinline__ int longest_first(const AttnParams& p, int z) {
+  __shared__ int lens[THREADS], mine;
+  if (p.n_seqs == 1 || p.n_seqs > THREADS || !(p.varlen || p.seqlens)) return z;
+  const int t = threadIdx.x;
+  int len = -1;
+  if (t < p.n_seqs) len = p.varlen ? p.cu_seqlens[t + 1] - p.cu_seqlens[t] : p.seqlens[t];
+  lens[t] = len;
+  __syncthreads();
+  int rank = 0;
+  for (int j = 0; j < p.n_seqs; ++j) rank += lens[j] > len || (lens[j] == len && j < t);
+  if (t < p.n_seqs && rank == z) mine = t;
+  __syncthreads();
+  return mine;
+}
+
 template <int R> constexpr int smem_floats(bool tables) {
   const int half = (KT + (tables ? 2 * (8 * R + KT) : 0)) * HP;
   const int values = KT * DP;
@@ -93,7 +110,7 @@ __global__ void __launch_bounds__(THREADS, 4) attn_simt_kernel(const AttnParams 
 
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int ti = warp * 4 + lane / 8, tj = lane % 8;
-  const int s = blockIdx.z, h = blockIdx.y, q0 = blockIdx.x * QT;
+  const int s = longest_first(p, blockIdx.z), h = blockIdx.y, q0 = blockIdx.x * QT;
   int len, rows;                 // valid length; rows that exist in the output
   int64_t tok0; int b;
   if (p.varlen) {
