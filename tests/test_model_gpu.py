@@ -253,3 +253,66 @@ def test_task_head_classes_run_on_the_gpu():
                     a, b = a[v], b[v]
                 assert (a - b).abs().max().item() / max(b.abs().max().item(), 1e-6) < 5e-4, (name, f)
         del hf, fl
+
+
+def _generic_route(model, **kw):
+    """The layer-by-layer route: a hook anywhere in the stack takes the native layer loop out of the way."""
+    handle = model.encoder.layer[0].register_forward_hook(lambda *a: None)
+    try:
+        return model(**kw)
+    finally:
+        handle.remove()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("lengths,L", [([1], 1), ([128, 128], 128), ([129, 1, 64], 129), ([33, 0, 7, 200], 200)])
+def test_native_layer_loop_matches_the_module_route(dtype, lengths, L):
+    """The encoder's native loop against the modules it stands in for: one token, full rows, ragged rows, an empty row,
+    holes in the mask; hooks and replaced parameters must be seen."""
+    import copy
+    from turbodeberta_b200.model import FlashDebertaV2Model
+    torch.manual_seed(12)
+    model = FlashDebertaV2Model(_cfg(num_hidden_layers=3)).eval().to("cuda", dtype)
+    ids = torch.randint(0, 500, (len(lengths), L), device="cuda")
+    mask = (torch.arange(L, device="cuda")[None] < torch.tensor(lengths, device="cuda")[:, None]).long()
+    if L == 129:
+        mask[0, 5:40] = 0                                            # not right padded
+    v = mask.bool()
+    tol = 1e-4 if dtype == torch.float32 else 4e-2
+    with torch.no_grad():
+        for _ in range(2):
+            got = model(input_ids=ids, attention_mask=mask, output_hidden_states=True)
+            want = _generic_route(model, input_ids=ids, attention_mask=mask, output_hidden_states=True)
+            assert len(got.hidden_states) == len(want.hidden_states) == 4
+            for a, b in zip(got.hidden_states, want.hidden_states):
+                assert a.shape == b.shape
+                assert (a.float() - b.float())[v].abs().max().item() <= tol * b.float()[v].abs().max().item()
+            assert torch.equal(got.last_hidden_state, got.hidden_states[-1])
+            assert torch.count_nonzero(got.last_hidden_state[~v]).item() == 0
+            # a replaced parameter and an in-place update, both behind a plan that was made before
+            model.encoder.layer[1].output.dense.weight = torch.nn.Parameter(model.encoder.layer[1].output.dense.weight * 1.25)
+            model.encoder.layer[0].attention.self.key_proj.weight.mul_(1.1)
+        plain = model(input_ids=ids, attention_mask=mask)
+        assert plain.hidden_states is None
+        twin = copy.deepcopy(model)
+        assert torch.equal(twin(input_ids=ids, attention_mask=mask).last_hidden_state, plain.last_hidden_state)
+        called = []
+        model.encoder.layer[2].output.dense.register_forward_hook(lambda *a: called.append(1))
+        model(input_ids=ids, attention_mask=mask)
+        assert called
+
+
+@pytest.mark.parametrize("rows,hidden", [(1, 8), (3, 768), (2400, 1024), (2401, 264), (5, 2048)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_residual_layernorm_kernel(rows, hidden, dtype):
+    from turbodeberta_b200 import _cabi as cabi
+    if dtype == torch.float32 and hidden > 1024:
+        pytest.skip("fp32 rows go up to 1024 columns")
+    torch.manual_seed(13)
+    x, r = (torch.randn(rows, hidden, device="cuda").to(dtype) * 3 for _ in range(2))
+    w, b = (torch.randn(hidden, device="cuda").to(dtype) for _ in range(2))
+    out = torch.empty_like(x)
+    cabi.check(cabi.host.add_layernorm(x, r, w, b, 1e-7, out))
+    want = torch.nn.functional.layer_norm(x.double() + r.double(), (hidden,), w.double(), b.double(), 1e-7)
+    tol = 1e-5 if dtype == torch.float32 else 1e-2
+    assert (out.double() - want).abs().max().item() <= tol * want.abs().max().item()

@@ -116,6 +116,8 @@ constexpr int LIST_BUCKETS = 1024;
 __global__ void __launch_bounds__(1024) build_tile_list_kernel(const int32_t* __restrict__ cu, int n_seqs,
                                                                 int64_t total_tokens, int32_t* ws, int cap,
                                                                 int32_t* status) {
+  static_assert(LIST_BUCKETS == 1024, "one bucket per thread");
+  __shared__ int warp_total[32];
   __shared__ int hist[LIST_BUCKETS];       // tiles per bucket, then the write cursor of the bucket
   int2* entries = reinterpret_cast<int2*>(ws + 4);
   for (int i = threadIdx.x; i < LIST_BUCKETS; i += blockDim.x) hist[i] = 0;
@@ -130,11 +132,25 @@ __global__ void __launch_bounds__(1024) build_tile_list_kernel(const int32_t* __
     if (nt > 0) atomicAdd(&hist[nt < LIST_BUCKETS ? nt : LIST_BUCKETS - 1], nt);
   }
   __syncthreads();
-  if (threadIdx.x == 0) {                  // exclusive scan from the largest bucket down
-    int run = 0;
-    for (int bkt = LIST_BUCKETS - 1; bkt >= 0; --bkt) { const int c = hist[bkt]; hist[bkt] = run; run += c; }
-    ws[0] = run < cap ? run : cap;
-    if (cu[n_seqs] != (int32_t)total_tokens) *reinterpret_cast<volatile int32_t*>(status + 1) = 1;
+  {                                        // exclusive scan from the largest bucket down, one bucket per thread
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int own = hist[LIST_BUCKETS - 1 - threadIdx.x];
+    int inc = own;
+#pragma unroll
+    for (int off = 1; off < 32; off *= 2) {
+      const int o = __shfl_up_sync(0xffffffffu, inc, off);
+      if (lane >= off) inc += o;
+    }
+    if (lane == 31) warp_total[wid] = inc;
+    __syncthreads();
+    int before = lane < wid ? warp_total[lane] : 0;
+#pragma unroll
+    for (int off = 16; off >= 1; off >>= 1) before += __shfl_xor_sync(0xffffffffu, before, off);
+    hist[LIST_BUCKETS - 1 - threadIdx.x] = before + inc - own;
+    if (threadIdx.x == LIST_BUCKETS - 1) {
+      ws[0] = before + inc < cap ? before + inc : cap;
+      if (cu[n_seqs] != (int32_t)total_tokens) *reinterpret_cast<volatile int32_t*>(status + 1) = 1;
+    }
   }
   __syncthreads();
   for (int s = threadIdx.x; s < n_seqs; s += blockDim.x) {
@@ -1111,9 +1127,11 @@ int launch_attn_umma(const AttnParams& given, cudaStream_t s) {
   if (p.varlen) {
     tiles = (p.total_tokens + BQ - 1) / BQ + p.n_seqs + 1;           // upper bound; the device list has the real count
     if (tiles * p.H > 0x7fffffff) { set_error("too many tiles"); return TDB_ERR_SHAPE; }
-    build_tile_list_kernel<<<1, 1024, 0, s>>>(p.cu_seqlens, p.n_seqs, p.total_tokens,
-                                              reinterpret_cast<int32_t*>(p.workspace), (int)tiles, p.status);
-    if ((rc = cuda_fail(cudaGetLastError(), "build_tile_list launch"))) return rc;
+    if (!p.tiles_listed) {
+      build_tile_list_kernel<<<1, 1024, 0, s>>>(p.cu_seqlens, p.n_seqs, p.total_tokens,
+                                                reinterpret_cast<int32_t*>(p.workspace), (int)tiles, p.status);
+      if ((rc = cuda_fail(cudaGetLastError(), "build_tile_list launch"))) return rc;
+    }
   } else {
     tiles = (int64_t)p.n_seqs * ((p.L + BQ - 1) / BQ);
     if (tiles * p.H > 0x7fffffff) { set_error("too many tiles"); return TDB_ERR_SHAPE; }

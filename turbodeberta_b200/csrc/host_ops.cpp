@@ -106,6 +106,12 @@ struct Status {
       p.status = own.data_ptr<int32_t>();
     }
   }
+  // Leave the check to drain_pending(); words of the call's own go to `words`.  Needs no interpreter lock.
+  void defer(cudaStream_t stream, std::vector<Tensor>& words) {
+    if (slot < 0) { words.push_back(own); return; }
+    std::lock_guard<std::mutex> lock(g_pools[dev].mu);
+    g_pools[dev].pending.push_back({slot, stream});
+  }
   // What the caller in Python gets to see: None (fine, or deferred into the pool), (word 0, word 1), or the tensor of words.
   py::object finish(bool check, cudaStream_t stream) {
     if (slot < 0) return py::cast(own);
@@ -392,6 +398,227 @@ std::pair<OptTensor, OptTensor> expand_pair(const OptTensor& kr, const OptTensor
   return {ko, qo};
 }
 
+// ------------------------------------------------------------------------------------------------------- the encoder
+Tensor mask_bytes(const Tensor& mask) {
+  if (mask.scalar_type() == at::kLong || mask.scalar_type() == at::kBool || mask.scalar_type() == at::kByte) return mask.contiguous();
+  return mask.ne(0).contiguous();
+}
+
+// A set of modules whose forward the native encoder stands in for, as it was when the plan was made.  The plan holds as long
+// as nobody has put a hook, a new child or parameter, or another forward on any of them, and all are in eval mode.
+class Watch {
+ public:
+  explicit Watch(const py::list& modules) {
+    for (py::handle m : modules) {
+      Entry e;
+      e.module = py::reinterpret_borrow<py::object>(m);
+      e.type = Py_TYPE(m.ptr());
+      e.dict = m.attr("__dict__");
+      for (const char* part : {"_modules", "_parameters"}) {
+        py::dict d = e.dict[part];
+        std::vector<std::pair<py::object, py::object>> items;
+        for (auto kv : d) items.emplace_back(py::reinterpret_borrow<py::object>(kv.first), py::reinterpret_borrow<py::object>(kv.second));
+        e.parts.emplace_back(d, std::move(items));
+      }
+      entries_.push_back(std::move(e));
+    }
+    for (const char* n : {"_forward_hooks", "_forward_pre_hooks", "_backward_hooks", "_backward_pre_hooks"}) hooks_.push_back(py::str(n));
+    training_ = py::str("training");
+    forward_ = py::str("forward");
+  }
+  bool holds() const {
+    for (const Entry& e : entries_) {
+      if (Py_TYPE(e.module.ptr()) != e.type) return false;
+      PyObject* d = e.dict.ptr();
+      if (PyDict_GetItem(d, training_.ptr()) != Py_False || PyDict_Contains(d, forward_.ptr())) return false;
+      for (const py::object& h : hooks_) {
+        PyObject* v = PyDict_GetItem(d, h.ptr());
+        if (v && PyDict_Size(v) != 0) return false;
+      }
+      for (const auto& [dict, items] : e.parts) {
+        if ((size_t)PyDict_Size(dict.ptr()) != items.size()) return false;
+        for (const auto& [k, v] : items)
+          if (PyDict_GetItem(dict.ptr(), k.ptr()) != v.ptr()) return false;
+      }
+    }
+    return true;
+  }
+
+ private:
+  struct Entry {
+    py::object module;
+    PyTypeObject* type;
+    py::dict dict;
+    std::vector<std::pair<py::dict, std::vector<std::pair<py::object, py::object>>>> parts;
+  };
+  std::vector<Entry> entries_;
+  std::vector<py::object> hooks_;
+  py::object training_, forward_;
+};
+
+int64_t version_of(const Tensor& t) { return t.is_inference() ? 0 : (int64_t)t._version(); }
+
+struct Layer {
+  Tensor out_w, out_b, ln1_w, ln1_b, up_w, up_b, down_w, down_b, ln2_w, ln2_b;
+  double eps1, eps2, sm_scale;
+  std::vector<Tensor> sources;                       // what the derived tensors below were made from
+  std::vector<std::pair<void*, int64_t>> seen;
+  Tensor qkv_w, qkv_b;
+  py::object tables_ref;                             // keeps `tables` alive
+  const Tables* tables = nullptr;
+};
+
+// The encoder's layer loop on a token-major [T, hidden] stream: four library matrix products per layer, the fused attention,
+// and two residual + LayerNorm kernels and a GELU in between.
+class Encoder {
+ public:
+  Encoder(int heads) : heads_(heads) {}
+  void add_layer(std::vector<Tensor> w, double eps1, double eps2, double sm_scale, std::vector<Tensor> sources) {
+    TORCH_CHECK(w.size() == 10);
+    layers_.push_back(Layer{w[0], w[1], w[2], w[3], w[4], w[5], w[6], w[7], w[8], w[9], eps1, eps2, sm_scale, std::move(sources), {}, {}, {}, py::none(), nullptr});
+  }
+  // Layers whose derived tensors are missing, or older than what they were made from.
+  std::vector<int> stale() const {
+    std::vector<int> r;
+    for (size_t i = 0; i < layers_.size(); ++i)
+      if (layers_[i].seen != stamp(layers_[i])) r.push_back((int)i);
+    return r;
+  }
+  void set_derived(int i, Tensor qkv_w, Tensor qkv_b, py::object tables) {
+    Layer& l = layers_.at(i);
+    l.qkv_w = std::move(qkv_w); l.qkv_b = std::move(qkv_b);
+    l.tables_ref = tables;
+    l.tables = tables.is_none() ? nullptr : tables.cast<const Tables*>();
+    l.seen = stamp(l);
+  }
+  bool fits(const Tensor& x) const {
+    for (const Layer& l : layers_)
+      for (const Tensor* t : {&l.out_w, &l.out_b, &l.ln1_w, &l.ln1_b, &l.up_w, &l.up_b, &l.down_w, &l.down_b, &l.ln2_w, &l.ln2_b})
+        if (t->scalar_type() != x.scalar_type() || t->device() != x.device() || !t->is_contiguous()) return false;
+    return true;
+  }
+  // x: [T, hidden].  Packed form: cu_seqlens; padded form: batch rows of `length` tokens, all valid.  Returns the outputs of
+  // all layers (or of the last one), and the status words that the caller has to look at (see Status).
+  std::pair<std::vector<Tensor>, std::vector<Tensor>> run(Tensor x, const OptTensor& cu_seqlens, int64_t length, bool every) {
+    std::vector<Tensor> outs, words;
+    const int dev = x.get_device();
+    const int64_t T = x.size(0), hidden = x.size(1);
+    const int code = dtype_code(x);
+    py::gil_scoped_release nogil;
+    c10::cuda::CUDAGuard guard((c10::DeviceIndex)dev);
+    at::AutoDispatchBelowAutograd below;
+    cudaStream_t stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream();
+    Tensor ws;
+    int64_t n_seqs = 0;
+    if (cu_seqlens) {
+      n_seqs = cu_seqlens->numel() - 1;
+      ws = at::empty({(int64_t)tdb_attn_workspace_bytes((int)n_seqs, T)}, x.options().dtype(at::kByte));
+    }
+    bool listed = false;
+    for (const Layer& l : layers_) {
+      const Tensor qkv = at::linear(x, l.qkv_w, l.qkv_b);
+      Tensor ctx = at::empty({T, hidden}, x.options());
+      {
+        tdb::AttnParams p{};
+        const int64_t e = x.element_size();
+        char* base = static_cast<char*>(qkv.data_ptr());
+        p.q = base; p.k = base + e * hidden; p.v = base + 2 * e * hidden; p.o = ctx.data_ptr();
+        p.q_st = p.k_st = p.v_st = 3 * hidden; p.q_sh = p.k_sh = p.v_sh = p.o_sh = hidden / heads_; p.o_st = hidden;
+        if (l.tables) l.tables->fill(p, x);
+        p.H = heads_; p.D = (int)(hidden / heads_); p.sm_scale = (float)l.sm_scale; p.total_tokens = T;
+        if (cu_seqlens) {
+          p.varlen = 1; p.cu_seqlens = cu_seqlens->data_ptr<int32_t>(); p.n_seqs = (int)n_seqs; p.L = (int)length;
+          p.workspace = ws.data_ptr(); p.workspace_bytes = ws.numel(); p.tiles_listed = listed;
+        } else {
+          p.n_seqs = (int)(T / length); p.L = (int)length;
+          p.q_sb = p.k_sb = p.v_sb = 3 * hidden * length; p.o_sb = hidden * length;
+        }
+        Status st(dev, p);
+        const int rc = tdb_run_attn(&p, code, TDB_KERNEL_AUTO, stream);
+        if (rc) release_unused(dev, st.slot);
+        ok(rc);
+        st.defer(stream, words);
+        listed = true;
+      }
+      Tensor y = at::linear(ctx, l.out_w, l.out_b);
+      add_norm(y, x, l.ln1_w, l.ln1_b, l.eps1, code, stream);
+      Tensor u = at::linear(y, l.up_w, l.up_b);
+      ok(tdb_gelu(u.data_ptr(), u.numel(), code, stream));
+      Tensor z = at::linear(u, l.down_w, l.down_b);
+      add_norm(z, y, l.ln2_w, l.ln2_b, l.eps2, code, stream);
+      x = z;
+      if (every) outs.push_back(x);
+    }
+    if (!every) outs.push_back(x);
+    return {std::move(outs), std::move(words)};
+  }
+
+ private:
+  static std::vector<std::pair<void*, int64_t>> stamp(const Layer& l) {
+    std::vector<std::pair<void*, int64_t>> s;
+    s.reserve(l.sources.size());
+    for (const Tensor& t : l.sources) s.emplace_back(t.data_ptr(), version_of(t));
+    return s;
+  }
+  static void ok(int rc) { TORCH_CHECK(rc == 0, "libtdb_b200: ", tdb_last_error(), " (code ", rc, ")"); }
+  static void add_norm(Tensor& x, const Tensor& res, const Tensor& w, const Tensor& b, double eps, int code, cudaStream_t stream) {
+    ok(tdb_add_layernorm(x.data_ptr(), res.data_ptr(), w.data_ptr(), b.data_ptr(), (float)eps, x.size(0), (int)x.size(1), code, x.data_ptr(), stream));
+  }
+  int heads_;
+  std::vector<Layer> layers_;
+};
+
+// (all ones, right padded, tokens, longest, seqlens, cu_seqlens) of a [B, L] padding mask; one synchronisation.
+py::object mask_rows(const Tensor& mask) {
+  const Tensor m = mask_bytes(mask);
+  const int dev = m.get_device();
+  c10::cuda::CUDAGuard guard((c10::DeviceIndex)dev);
+  cudaStream_t stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream();
+  const int64_t B = m.size(0), L = m.size(1);
+  const int slot = acquire(dev);
+  if (slot < 0) return py::none();
+  int32_t* out = g_pools[dev].host + slot * SLOT_WORDS;
+  Tensor both;
+  int rc;
+  cudaError_t e = cudaSuccess;
+  int32_t w[4];
+  {
+    py::gil_scoped_release nogil;
+    both = at::empty({2 * B + 1}, m.options().dtype(at::kInt));
+    int32_t* lens = both.data_ptr<int32_t>();
+    rc = tdb_mask_rows(m.data_ptr(), (int)m.element_size(), (int)B, (int)L, lens, lens + B, g_pools[dev].ctl + slot * SLOT_WORDS, out, stream);
+    if (!rc) e = cudaStreamSynchronize(stream);
+    for (int i = 0; i < 4; ++i) { w[i] = reinterpret_cast<volatile int32_t*>(out)[i]; out[i] = 0; }
+  }
+  release_unused(dev, slot);
+  TORCH_CHECK(rc == 0, "libtdb_b200: ", tdb_last_error());
+  cuda_ok(e, "cudaStreamSynchronize");
+  return py::make_tuple((bool)w[0], (bool)w[1], w[2], w[3], both.narrow(0, 0, B), both.narrow(0, B, B + 1));
+}
+
+// The valid rows of x [B, L, hidden] back to back, and each token's place in that stream (-1: padding).
+std::pair<Tensor, Tensor> pack_rows(const Tensor& x, const Tensor& mask, const Tensor& cu, int64_t tokens) {
+  c10::cuda::CUDAGuard guard(x.device());
+  cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
+  const Tensor m = mask_bytes(mask), xc = x.contiguous();
+  const int64_t B = x.size(0), L = x.size(1), hidden = x.size(2);
+  Tensor pos = at::empty({B * L}, cu.options()), out = at::empty({tokens, hidden}, x.options());
+  int rc = tdb_mask_positions(m.data_ptr(), (int)m.element_size(), cu.data_ptr<int32_t>(), (int)B, (int)L, pos.data_ptr<int32_t>(), stream);
+  if (!rc) rc = tdb_repack(1, xc.data_ptr(), pos.data_ptr<int32_t>(), B * L, (int)(hidden * x.element_size()), out.data_ptr(), stream);
+  TORCH_CHECK(rc == 0, "libtdb_b200: ", tdb_last_error());
+  return {out, pos};
+}
+
+// The inverse: [B, L, hidden] with zeros at the padding.
+Tensor unpack_rows(const Tensor& x, const Tensor& pos, int64_t B, int64_t L) {
+  c10::cuda::CUDAGuard guard(x.device());
+  Tensor out = at::empty({B, L, x.size(1)}, x.options());
+  const int rc = tdb_repack(0, x.data_ptr(), pos.data_ptr<int32_t>(), B * L, (int)(x.size(1) * x.element_size()), out.data_ptr(),
+                            c10::cuda::getCurrentCUDAStream().stream());
+  TORCH_CHECK(rc == 0, "libtdb_b200: ", tdb_last_error());
+  return out;
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
@@ -406,4 +633,20 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("attn_packed_scores", &attn_packed_scores);
   m.def("expand_pair", &expand_pair);
   m.def("drain_pending", &drain_pending);
+  py::class_<Watch>(m, "Watch").def(py::init<const py::list&>()).def("holds", &Watch::holds);
+  py::class_<Encoder>(m, "Encoder")
+      .def(py::init<int>())
+      .def("add_layer", &Encoder::add_layer)
+      .def("stale", &Encoder::stale)
+      .def("set_derived", &Encoder::set_derived)
+      .def("fits", &Encoder::fits)
+      .def("run", &Encoder::run);
+  m.def("add_layernorm", [](const Tensor& x, const Tensor& res, const Tensor& w, const Tensor& b, double eps, const Tensor& out) {
+    c10::cuda::CUDAGuard guard(x.device());
+    return tdb_add_layernorm(x.data_ptr(), res.data_ptr(), w.data_ptr(), b.data_ptr(), (float)eps, x.size(0), (int)x.size(1), dtype_code(x),
+                             out.data_ptr(), c10::cuda::getCurrentCUDAStream().stream());
+  });
+  m.def("mask_rows", &mask_rows);
+  m.def("pack_rows", &pack_rows);
+  m.def("unpack_rows", &unpack_rows);
 }

@@ -40,6 +40,7 @@ struct AttnParams {
   // flag that makes CTAs starting after a wait gave up hand out no work.  Null: status words 2 (reset by the launch) and 0.
   int32_t* counter; int32_t* gave_up;
   void* workspace; size_t workspace_bytes;
+  int tiles_listed;                                       // packed form: the workspace already holds this batch's tile list
 };
 
 void set_error(const char* fmt, ...);
@@ -66,10 +67,18 @@ int static_tile_scratch(void** ptr);   // device address of the library's fixed 
 
 }  // namespace tdb
 
-// What the host extension calls: the checks and the launch behind the tdb_attn_fwd_* entry points, on a filled AttnParams.
-extern "C" __attribute__((visibility("default"))) int tdb_run_attn(const tdb::AttnParams* p, int dtype, int kernel,
-                                                                   void* stream);
-extern "C" __attribute__((visibility("default"))) int tdb_expand_pair(const void* kr, const void* qr, const int16_t* idx,
-                                                                      int idx_delta_max, int H, int two_span,
-                                                                      int exp_delta_max, int exp_rows, void* kr_out,
-                                                                      void* qr_out, void* stream);
+// What the host extension calls (the checks and the launch behind the tdb_attn_fwd_* entry points on a filled AttnParams,
+// and kernels that have no C entry point of their own).
+#define TDB_HOST_API __attribute__((visibility("default")))
+extern "C" {
+TDB_HOST_API int tdb_run_attn(const tdb::AttnParams* p, int dtype, int kernel, void* stream);
+TDB_HOST_API int tdb_expand_pair(const void* kr, const void* qr, const int16_t* idx, int idx_delta_max, int H, int two_span,
+                                 int exp_delta_max, int exp_rows, void* kr_out, void* qr_out, void* stream);
+TDB_HOST_API int tdb_add_layernorm(const void* x, const void* res, const void* w, const void* b, float eps, int64_t rows, int hidden,
+                                   int dtype, void* out, void* stream);
+TDB_HOST_API int tdb_gelu(void* x, int64_t elements, int dtype, void* stream);
+TDB_HOST_API int tdb_mask_rows(const void* mask, int elem_bytes, int B, int L, int32_t* seqlens, int32_t* cu, int32_t* ticket,
+                               int32_t* out, void* stream);
+TDB_HOST_API int tdb_mask_positions(const void* mask, int elem_bytes, const int32_t* cu, int B, int L, int32_t* pos, void* stream);
+TDB_HOST_API int tdb_repack(int pack, const void* src, const int32_t* pos, int64_t rows, int row_bytes, void* dst, void* stream);
+}

@@ -17,6 +17,7 @@ one fused kernel call.  Differences from the reference module, all on the host s
 from __future__ import annotations
 
 import math
+import threading
 import warnings
 import weakref
 
@@ -25,10 +26,12 @@ from torch import nn
 from transformers.models.deberta_v2.modeling_deberta_v2 import (
     DebertaV2Attention, DebertaV2Encoder, DebertaV2ForMaskedLM, DebertaV2ForMultipleChoice,
     DebertaV2ForQuestionAnswering, DebertaV2ForSequenceClassification, DebertaV2ForTokenClassification,
-    DebertaV2Layer, DebertaV2Model, DisentangledSelfAttention)
+    DebertaV2Intermediate, DebertaV2Layer, DebertaV2Model, DebertaV2Output, DebertaV2SelfOutput,
+    DisentangledSelfAttention)
 
 from . import relpos as _relpos
-from .ops.flash_attention import check_pending_status, flash_attention_with_disentangled
+from ._cabi import host
+from .ops.flash_attention import _PENDING_STATUS, check_pending_status, flash_attention_with_disentangled
 from .ops.flash_attention_varlen import flash_attention_with_disentangled_varlen
 from .padding import _get_unpad_data, _upad_input, index_first_axis, pad_input
 
@@ -43,11 +46,13 @@ class PackedSequences:
 
 
 class MaskInfo:
-    """Key validity derived from an attention mask: lengths, and the packing indices when needed."""
-    __slots__ = ("all_ones", "right_padded", "seqlens", "key_mask")
+    """Key validity derived from an attention mask: lengths, and the packing indices when needed.  ``packed`` (only from
+    the native analysis of a 2-D mask): token count, longest sequence and the sequences' offsets."""
+    __slots__ = ("all_ones", "right_padded", "seqlens", "key_mask", "packed")
 
-    def __init__(self, all_ones, right_padded, seqlens, key_mask):
+    def __init__(self, all_ones, right_padded, seqlens, key_mask, packed=None):
         self.all_ones, self.right_padded, self.seqlens, self.key_mask = all_ones, right_padded, seqlens, key_mask
+        self.packed = packed
 
 
 _MASK_CACHE: dict = {}
@@ -118,6 +123,24 @@ def analyse_mask(attention_mask: torch.Tensor | None, batch: int, length: int, r
     return info
 
 
+def _analyse_2d(attention_mask: torch.Tensor, batch: int, length: int) -> MaskInfo | None:
+    """``analyse_mask`` of a CUDA ``[B, L]`` mask in one kernel and one synchronisation, offsets of the packed stream
+    included.  A mask that is already known to be all ones costs neither."""
+    if attention_mask.shape != (batch, length) or batch == 0 or length == 0:
+        return None
+    hit = _MASK_CACHE.get(id(attention_mask))
+    if hit is not None and hit[0]() is attention_mask and hit[1] == attention_mask._version and hit[2].all_ones:
+        return hit[2]
+    rows = host.mask_rows(attention_mask)
+    if rows is None:
+        return None
+    all_ones, right, tokens, longest, seqlens, cu = rows
+    info = MaskInfo(all_ones, right, seqlens, attention_mask != 0 if all_ones else None, (tokens, longest, cu))
+    if all_ones and not attention_mask.is_inference():
+        _mask_cache_put(attention_mask, info)
+    return info
+
+
 _WARNED: set = set()
 
 
@@ -145,19 +168,23 @@ class FlashDisentangledSelfAttention(DisentangledSelfAttention):
         H, D = self.num_attention_heads, self.attention_head_size
         lead = hidden_states.shape[:-1]
         if query_states is hidden_states and not torch.is_grad_enabled():
-            params = (self.query_proj.weight, self.query_proj.bias, self.key_proj.weight, self.key_proj.bias,
-                      self.value_proj.weight, self.value_proj.bias)
-            key = tuple((t.data_ptr(), t._version, t.dtype, t.device) for t in params)
-            if self._qkv is None or self._qkv_key != key:
-                w = torch.cat([params[0], params[2], params[4]], 0).detach()
-                b = torch.cat([params[1], params[3], params[5]], 0).detach()
-                self._qkv, self._qkv_key = (w, b), key
-            qkv = torch.nn.functional.linear(hidden_states, *self._qkv).view(*lead, 3, H, D)
+            qkv = torch.nn.functional.linear(hidden_states, *self._qkv_weights()).view(*lead, 3, H, D)
             return qkv.select(-3, 0), qkv.select(-3, 1), qkv.select(-3, 2)
         q = self.query_proj(query_states).view(*query_states.shape[:-1], H, D)
         k = self.key_proj(hidden_states).view(*lead, H, D)
         v = self.value_proj(hidden_states).view(*lead, H, D)
         return q, k, v
+
+    def _qkv_weights(self):
+        """Weight and bias of the three projections as one GEMM's (cached until one of them changes)."""
+        params = (self.query_proj.weight, self.query_proj.bias, self.key_proj.weight, self.key_proj.bias,
+                  self.value_proj.weight, self.value_proj.bias)
+        key = tuple((t.data_ptr(), t._version, t.dtype, t.device) for t in params)
+        if self._qkv is None or self._qkv_key != key:
+            w = torch.cat([params[0], params[2], params[4]], 0).detach()
+            b = torch.cat([params[1], params[3], params[5]], 0).detach()
+            self._qkv, self._qkv_key = (w, b), key
+        return self._qkv
 
     # -- relative tables ---------------------------------------------------------------------------
     def _relative_tables(self, rel_embeddings: torch.Tensor, dtype: torch.dtype):
@@ -248,6 +275,10 @@ class FlashDebertaV2Layer(DebertaV2Layer):
         self.attention = FlashDebertaV2Attention(config)
 
 
+# Native plans of live encoders; kept outside the modules, which stay plain data to copy and pickle.
+_PLANS: "weakref.WeakKeyDictionary" = weakref.WeakKeyDictionary()
+
+
 class FlashDebertaV2Encoder(DebertaV2Encoder):
     """HF encoder whose layers use the fused attention.  Two host-side savings: the ``[L, L]`` relative
     position matrix is not built (the kernels do not read it), and in eval mode the LayerNorm'd relative
@@ -273,6 +304,11 @@ class FlashDebertaV2Encoder(DebertaV2Encoder):
         self._mask_info = None
         if (query_states is None and self.conv is None and not output_attentions
                 and hidden_states.is_cuda and hidden_states.dim() == 3):
+            if not torch.is_grad_enabled():
+                out = self._forward_native(hidden_states, attention_mask, output_hidden_states, return_dict)
+                if out is not None:
+                    self._check_status_unless_capturing()
+                    return out
             # One analysis of the user's mask per forward (cached per mask tensor, so a repeated call with the same
             # tensor - e.g. while the forward is being captured into a CUDA graph - costs no synchronisation); the
             # expanded mask that the HF encoder builds from it inherits the result in get_attention_mask().
@@ -302,6 +338,111 @@ class FlashDebertaV2Encoder(DebertaV2Encoder):
         ``check_pending_status()`` outside a capture reads them."""
         if not torch.cuda.is_current_stream_capturing():
             check_pending_status()
+
+    # -- the whole layer loop in one native call -------------------------------------------------------
+    def _native_layers(self):
+        """(watched modules, native encoder, attention modules) for a stack made of the stock modules only, else None."""
+        layers = list(self.layer)
+        native, attns = None, []
+        for layer in layers:
+            att, up, down = layer.attention, layer.intermediate, layer.output
+            sa, so, act = att.self, att.output, layer.intermediate.intermediate_act_fn
+            stock = (type(layer) in (DebertaV2Layer, FlashDebertaV2Layer)
+                     and type(att) in (DebertaV2Attention, FlashDebertaV2Attention)
+                     and type(sa) is FlashDisentangledSelfAttention and type(so) is DebertaV2SelfOutput
+                     and type(up) is DebertaV2Intermediate and type(down) is DebertaV2Output
+                     and (getattr(act, "act", None) is nn.functional.gelu
+                          or (type(act) is nn.GELU and act.approximate == "none")))
+            if not stock or sa.attention_head_size != 64:
+                return None
+            lins = [sa.query_proj, sa.key_proj, sa.value_proj, so.dense, up.dense, down.dense]
+            if not sa.share_att_key and sa.relative_attention:
+                lins += [lin for lin in (getattr(sa, "pos_key_proj", None), getattr(sa, "pos_query_proj", None)) if lin is not None]
+            norms = [so.LayerNorm, down.LayerNorm]
+            if any(type(m) is not nn.Linear or m.bias is None for m in lins):
+                return None
+            if any(type(m) is not nn.LayerNorm or m.weight is None or m.bias is None for m in norms):
+                return None
+            hidden = so.dense.out_features
+            widest = 1024 if so.dense.weight.dtype == torch.float32 else 2048
+            if hidden % 8 or hidden > widest or up.dense.out_features % 8 or hidden != 64 * sa.num_attention_heads:
+                return None
+            if native is None:
+                native = host.Encoder(sa.num_attention_heads)
+            terms = 1 + int("c2p" in sa.pos_att_type) + int("p2c" in sa.pos_att_type)
+            native.add_layer([so.dense.weight, so.dense.bias, norms[0].weight, norms[0].bias, up.dense.weight, up.dense.bias,
+                              down.dense.weight, down.dense.bias, norms[1].weight, norms[1].bias], norms[0].eps,
+                             norms[1].eps, 1.0 / math.sqrt(64 * terms), [t for m in lins[:3] + lins[6:] for t in (m.weight, m.bias)])
+            attns.append(sa)
+        if native is None:
+            return None
+        return host.Watch([m for m in self.layer.modules()]), native, attns
+
+    def _native_plan(self, hidden_states, rel_embeddings):
+        """The native encoder with every layer's derived tensors up to date, or None where it does not apply."""
+        plan = _PLANS.get(self)
+        if plan is None or not plan[0].holds():
+            made = self._native_layers()
+            if made is None or not made[0].holds():
+                return None
+            plan = _PLANS[self] = [*made, None]      # the last entry: stamp of the relative embeddings behind its tables
+        _, native, attns, stamp = plan
+        if not native.fits(hidden_states):
+            return None
+        dtype = hidden_states.dtype
+        stamp_now = (getattr(rel_embeddings, "_tdb_stamp", None), dtype)
+        if stamp != stamp_now:
+            todo = range(len(attns))
+            if rel_embeddings is not None and stamp_now[0] is None:
+                return None
+        else:
+            todo = native.stale()
+        for i in todo:
+            w, b = attns[i]._qkv_weights()
+            tables = attns[i]._relative_tables(rel_embeddings, dtype) if attns[i].relative_attention else None
+            if w.dtype != dtype or w.device != hidden_states.device:
+                return None
+            native.set_derived(i, w, b, None if tables is None else tables.native())
+        plan[3] = stamp_now
+        return native
+
+    def _forward_native(self, hidden_states, attention_mask, output_hidden_states, return_dict):
+        """The encoder as one native call on the token-major stream: packed (valid tokens only) for padded batches,
+        ``[B * L, hidden]`` otherwise.  None where the generic route has to take over."""
+        if (self.training or hidden_states.dtype not in (torch.float32, torch.bfloat16) or torch.is_autocast_enabled()
+                or torch.nn.modules.module._has_any_global_hook() or hidden_states.numel() == 0):
+            return None
+        B, L, hid = hidden_states.shape
+        if torch.cuda.is_current_stream_capturing() or attention_mask is None or attention_mask.dim() != 2:
+            info = analyse_mask(attention_mask, B, L, refresh=True)
+            if not info.all_ones:
+                return None
+        else:
+            info = _analyse_2d(attention_mask, B, L)
+            if info is None or (not info.all_ones and (not self.pack_padded_batches or info.packed[0] == 0)):
+                return None
+        native = self._native_plan(hidden_states, self.get_rel_embedding())
+        if native is None:
+            return None
+        every = output_hidden_states and _WANTED.hidden_states
+        if info.all_ones:
+            outs, words = native.run(hidden_states.reshape(B * L, hid), None, L, every)
+            padded = [o.view(B, L, hid) for o in outs]
+        else:
+            tokens, longest, cu = info.packed
+            x, pos = host.pack_rows(hidden_states, attention_mask, cu, tokens)
+            outs, words = native.run(x, cu, longest, every)
+            keep = [o[None] for o in outs[:-1]] if self.skip_intermediate_padding else [host.unpack_rows(o, pos, B, L) for o in outs[:-1]]
+            padded = keep + [host.unpack_rows(outs[-1], pos, B, L)]
+        for w in words:
+            _PENDING_STATUS.append(w)
+        all_hidden = None
+        if output_hidden_states:
+            all_hidden = (hidden_states, *padded) if every else (padded[-1],)
+        from transformers.modeling_outputs import BaseModelOutput
+        if not return_dict:
+            return tuple(v for v in [padded[-1], all_hidden, None] if v is not None)
+        return BaseModelOutput(last_hidden_state=padded[-1], hidden_states=all_hidden, attentions=None)
 
     def _forward_packed(self, hidden_states, info: MaskInfo, output_hidden_states: bool, return_dict: bool):
         """The layer loop of the HF encoder (``modeling_deberta_v2.py:630-682``) on valid tokens only.  The reference
@@ -345,11 +486,31 @@ class FlashDebertaV2Encoder(DebertaV2Encoder):
         return self._rel_cache
 
 
+class _Wanted(threading.local):
+    """What the model around the encoder will use of the layers' outputs (the HF model asks its encoder for all of them and
+    then drops them unless its caller asked, which for a padded batch costs one re-padding per layer)."""
+    hidden_states = True
+
+
+_WANTED = _Wanted()
+
+
 class FlashDebertaV2Model(DebertaV2Model):
     def __init__(self, config):
         super().__init__(config)
         self.encoder = FlashDebertaV2Encoder(config)
         self.post_init()
+
+    def forward(self, *args, **kwargs):
+        wanted = kwargs.get("output_hidden_states")
+        if wanted is None:
+            wanted = len(args) > 1 or bool(getattr(self.config, "output_hidden_states", False))
+        before = _WANTED.hidden_states
+        _WANTED.hidden_states = bool(wanted) or getattr(self, "z_steps", 0) != 0
+        try:
+            return super().forward(*args, **kwargs)
+        finally:
+            _WANTED.hidden_states = before
 
 
 def patch_model(model: nn.Module) -> nn.Module:
@@ -365,6 +526,8 @@ def patch_model(model: nn.Module) -> nn.Module:
         if type(mod) is DebertaV2Encoder:
             mod.__class__ = FlashDebertaV2Encoder
             mod._rel_cache, mod._rel_cache_key, mod._rel_stamp = None, None, 0
+        if type(mod) is DebertaV2Model:
+            mod.__class__ = FlashDebertaV2Model
     return model
 
 

@@ -126,6 +126,9 @@ class RelPosTables:
             self.__dict__["_native"] = n
         return n
 
+    def __getstate__(self):
+        return {k: v for k, v in self.__dict__.items() if k != "_native"}
+
     def __setattr__(self, name, value):
         self.__dict__.pop("_native", None)
         self.__dict__[name] = value
