@@ -316,3 +316,51 @@ def test_residual_layernorm_kernel(rows, hidden, dtype):
     want = torch.nn.functional.layer_norm(x.double() + r.double(), (hidden,), w.double(), b.double(), 1e-7)
     tol = 1e-5 if dtype == torch.float32 else 1e-2
     assert (out.double() - want).abs().max().item() <= tol * want.abs().max().item()
+
+
+@pytest.mark.parametrize("n", [8, 4096, 8 * 257])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_gelu_kernel(n, dtype):
+    from turbodeberta_b200 import _cabi as cabi
+    x = torch.linspace(-9, 9, n, device="cuda").to(dtype)
+    want = torch.nn.functional.gelu(x.double())
+    cabi.check(cabi.host.gelu_(x))
+    bound = (1e-6 if dtype == torch.float32 else 5e-3) * want.abs() + (2e-7 if dtype == torch.float32 else 1e-6)
+    assert ((x.double() - want).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("lengths,L", [([40], 40), ([1, 90, 33], 90), ([128, 128], 128)])
+def test_repeated_shapes_replay_a_recorded_graph(lengths, L):
+    """From its second pass on a small shape runs as a recorded graph: new inputs, more shapes than are kept, other
+    streams and replaced weights must all give what the first (unrecorded) pass gives."""
+    from turbodeberta_b200.model import FlashDebertaV2Model
+    from turbodeberta_b200.ops.flash_attention import check_pending_status
+    torch.manual_seed(14)
+    model = FlashDebertaV2Model(_cfg(num_hidden_layers=2)).eval().to("cuda", torch.bfloat16)
+
+    def inputs(extra=0):
+        ids = torch.randint(1, 500, (len(lengths), L + extra), device="cuda")
+        mask = (torch.arange(L + extra, device="cuda")[None] < torch.tensor(lengths, device="cuda")[:, None] + extra).long()
+        return dict(input_ids=ids, attention_mask=mask)
+
+    @torch.no_grad()
+    def fresh(kw):
+        with torch.cuda.stream(torch.cuda.Stream()):                 # a stream's first pass is not recorded
+            out = model(**kw).last_hidden_state
+        torch.cuda.synchronize()
+        return out
+
+    with torch.no_grad():
+        for step in range(4):
+            kw = inputs()
+            assert torch.equal(model(**kw).last_hidden_state, fresh(kw)), step
+        for extra in list(range(1, 12)) * 2:
+            kw = inputs(extra)
+            a = model(**kw).last_hidden_state
+            assert torch.equal(a, model(**kw).last_hidden_state)
+        model.encoder.layer[1].intermediate.dense.weight = torch.nn.Parameter(model.encoder.layer[1].intermediate.dense.weight * 1.5)
+        model.encoder.layer[0].attention.self.value_proj.weight.mul_(0.5)
+        kw = inputs()
+        a = model(**kw).last_hidden_state
+        assert torch.equal(a, fresh(kw))
+    check_pending_status()

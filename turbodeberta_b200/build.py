@@ -49,7 +49,8 @@ def build_host(verbose: bool = False) -> str:
            "-DTORCH_API_INCLUDE_EXTENSION_H", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
            *[f"-I{i}" for i in inc], *[os.path.join(CSRC, s) for s in HOST_SOURCES], "-o", HOST,
            f"-L{HERE}", "-l:libtdb_b200.so", "-Wl,-rpath,$ORIGIN", f"-L{torch_lib}", "-ltorch_python", "-ltorch",
-           "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", f"-L{os.path.join(cuda_home, 'lib64')}", "-lcudart"]
+           "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", f"-L{os.path.join(cuda_home, 'lib64')}", "-lcudart",
+           "-lcublasLt"]
     r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     if verbose or r.returncode:
         sys.stderr.write(r.stdout)

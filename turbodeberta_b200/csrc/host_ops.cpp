@@ -14,8 +14,11 @@
 #include <c10/cuda/CUDAStream.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/CUDAGraphsUtils.cuh>
+#include <cublasLt.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <map>
 #include <mutex>
 #include <vector>
 
@@ -34,7 +37,7 @@ struct StatusPool {
   int32_t* host = nullptr;        // SLOTS x 4 words, pinned and mapped
   int32_t* ctl = nullptr;         // SLOTS x 4 words on the device: work counter, gave-up flag
   std::vector<int> free;
-  struct Pending { int slot; cudaStream_t stream; };
+  struct Pending { int slot; cudaStream_t stream; bool keep; };   // keep: the slot stays its owner's
   std::vector<Pending> pending;   // launches whose check was deferred
 };
 StatusPool g_pools[MAX_DEV];
@@ -70,7 +73,7 @@ int acquire(int dev) {
 }
 
 // Read the words of a slot whose launch has finished, and hand the slot back clean.
-std::pair<int, int> collect(int dev, int slot) {
+std::pair<int, int> collect(int dev, int slot, bool keep = false) {
   StatusPool& p = g_pools[dev];
   volatile int32_t* w = p.host + slot * SLOT_WORDS;
   const std::pair<int, int> r(w[0], w[1]);
@@ -80,6 +83,7 @@ std::pair<int, int> collect(int dev, int slot) {
     cudaMemset(p.ctl + slot * SLOT_WORDS, 0, SLOT_WORDS * 4);
     cudaDeviceSynchronize();
   }
+  if (keep) return r;
   std::lock_guard<std::mutex> lock(p.mu);
   p.free.push_back(slot);
   return r;
@@ -110,14 +114,14 @@ struct Status {
   void defer(cudaStream_t stream, std::vector<Tensor>& words) {
     if (slot < 0) { words.push_back(own); return; }
     std::lock_guard<std::mutex> lock(g_pools[dev].mu);
-    g_pools[dev].pending.push_back({slot, stream});
+    g_pools[dev].pending.push_back({slot, stream, false});
   }
   // What the caller in Python gets to see: None (fine, or deferred into the pool), (word 0, word 1), or the tensor of words.
   py::object finish(bool check, cudaStream_t stream) {
     if (slot < 0) return py::cast(own);
     if (!check) {
       std::lock_guard<std::mutex> lock(g_pools[dev].mu);
-      g_pools[dev].pending.push_back({slot, stream});
+      g_pools[dev].pending.push_back({slot, stream, false});
       return py::none();
     }
     cudaError_t e;
@@ -158,7 +162,7 @@ py::object drain_pending() {
       }
     }
     for (const auto& t : take) {
-      const auto r = collect(dev, t.slot);
+      const auto r = collect(dev, t.slot, t.keep);
       w0 = std::max(w0, r.first); w1 = std::max(w1, r.second);
     }
     cuda_ok(e, "synchronisation");
@@ -405,58 +409,162 @@ Tensor mask_bytes(const Tensor& mask) {
 }
 
 // A set of modules whose forward the native encoder stands in for, as it was when the plan was made.  The plan holds as long
-// as nobody has put a hook, a new child or parameter, or another forward on any of them, and all are in eval mode.
+// as nobody has put a hook, a new child or parameter, or another forward on any of them, and all are in eval mode.  Checked
+// on every forward, so it follows pointers instead of looking names up: a module keeps its hook, child and parameter dicts.
 class Watch {
  public:
   explicit Watch(const py::list& modules) {
+    training_ = py::str("training");
+    forward_ = py::str("forward");
     for (py::handle m : modules) {
       Entry e;
       e.module = py::reinterpret_borrow<py::object>(m);
       e.type = Py_TYPE(m.ptr());
       e.dict = m.attr("__dict__");
+      for (const char* n : {"_forward_hooks", "_forward_pre_hooks"})       // no gradients here, so no backward hooks
+        if (e.dict.contains(n)) e.hooks.push_back(e.dict[n]);
       for (const char* part : {"_modules", "_parameters"}) {
         py::dict d = e.dict[part];
-        std::vector<std::pair<py::object, py::object>> items;
-        for (auto kv : d) items.emplace_back(py::reinterpret_borrow<py::object>(kv.first), py::reinterpret_borrow<py::object>(kv.second));
-        e.parts.emplace_back(d, std::move(items));
+        std::vector<py::object> values;
+        for (auto kv : d) values.push_back(py::reinterpret_borrow<py::object>(kv.second));
+        e.parts.emplace_back(d, std::move(values));
       }
       entries_.push_back(std::move(e));
     }
-    for (const char* n : {"_forward_hooks", "_forward_pre_hooks", "_backward_hooks", "_backward_pre_hooks"}) hooks_.push_back(py::str(n));
-    training_ = py::str("training");
-    forward_ = py::str("forward");
   }
   bool holds() const {
+    // Some two hundred modules whose objects the last forward has long pushed out of the core's caches: fetched side by side
+    // first, since one after the other they cost 95 us.
+    for (const Entry& e : entries_) {
+      __builtin_prefetch(e.module.ptr());
+      prefetch_dict(e.dict.ptr());
+      for (const py::dict& h : e.hooks) prefetch_dict(h.ptr());
+      for (const auto& part : e.parts) prefetch_dict(part.first.ptr());
+    }
+    for (const Entry& e : entries_) {
+      prefetch_keys(e.dict.ptr());
+      for (const auto& part : e.parts)
+        if (!part.second.empty()) prefetch_keys(part.first.ptr());
+    }
     for (const Entry& e : entries_) {
       if (Py_TYPE(e.module.ptr()) != e.type) return false;
       PyObject* d = e.dict.ptr();
       if (PyDict_GetItem(d, training_.ptr()) != Py_False || PyDict_Contains(d, forward_.ptr())) return false;
-      for (const py::object& h : hooks_) {
-        PyObject* v = PyDict_GetItem(d, h.ptr());
-        if (v && PyDict_Size(v) != 0) return false;
-      }
-      for (const auto& [dict, items] : e.parts) {
-        if ((size_t)PyDict_Size(dict.ptr()) != items.size()) return false;
-        for (const auto& [k, v] : items)
-          if (PyDict_GetItem(dict.ptr(), k.ptr()) != v.ptr()) return false;
+      for (const py::dict& h : e.hooks)
+        if (PyDict_Size(h.ptr()) != 0) return false;
+      for (const auto& [dict, values] : e.parts) {
+        if ((size_t)PyDict_Size(dict.ptr()) != values.size()) return false;
+        Py_ssize_t pos = 0;
+        PyObject *k, *v;
+        for (size_t i = 0; PyDict_Next(dict.ptr(), &pos, &k, &v); ++i)
+          if (v != values[i].ptr()) return false;
       }
     }
     return true;
   }
 
  private:
+  static void prefetch_dict(PyObject* d) { __builtin_prefetch(&reinterpret_cast<PyDictObject*>(d)->ma_used); }
+  static void prefetch_keys(PyObject* d) {
+    const char* k = reinterpret_cast<const char*>(reinterpret_cast<PyDictObject*>(d)->ma_keys);
+    for (int i = 0; i < 8; ++i) __builtin_prefetch(k + 64 * i);
+    if (reinterpret_cast<PyDictObject*>(d)->ma_values) __builtin_prefetch(reinterpret_cast<PyDictObject*>(d)->ma_values);
+  }
   struct Entry {
     py::object module;
     PyTypeObject* type;
     py::dict dict;
-    std::vector<std::pair<py::dict, std::vector<std::pair<py::object, py::object>>>> parts;
+    std::vector<py::dict> hooks;
+    std::vector<std::pair<py::dict, std::vector<py::object>>> parts;
   };
   std::vector<Entry> entries_;
-  std::vector<py::object> hooks_;
   py::object training_, forward_;
 };
 
 int64_t version_of(const Tensor& t) { return t.is_inference() ? 0 : (int64_t)t._version(); }
+
+// y = x W^T + b for bf16, straight through cuBLASLt: the library picks the kernel as it does behind torch's linear, but the
+// choice is kept per shape and nothing else is looked up per call (about 3 us of host time instead of 9).
+class Linear {
+ public:
+  // One per run, with a workspace that nobody else uses on another stream meanwhile.  recording: `stream` is not torch's
+  // current one, so what torch would have to do cannot be done.
+  Linear(const Tensor& x, cudaStream_t stream, Tensor ws = {}, bool recording = false) : stream_(stream), recording_(recording) {
+    own_ = applies(x);
+    if (!own_) return;
+    handle_ = at::cuda::getCurrentCUDABlasLtHandle();
+    ws_ = ws.defined() ? ws : at::empty({(int64_t)WORKSPACE}, x.options().dtype(at::kByte));
+  }
+  static bool applies(const Tensor& x) {
+    return x.scalar_type() == at::kBFloat16 && at::globalContext().allowBF16ReductionCuBLAS() == at::CuBLASReductionOption::AllowReducedPrecisionWithSplitK;
+  }
+  // False: the caller's torch has to do it.
+  bool try_run(Tensor& y, const Tensor& x, const Tensor& w, const Tensor& b) {
+    if (!own_ || (reinterpret_cast<uintptr_t>(x.data_ptr()) | reinterpret_cast<uintptr_t>(w.data_ptr()) | reinterpret_cast<uintptr_t>(b.data_ptr())) & 15)
+      return false;
+    const int64_t T = x.size(0), k = x.size(1), n = w.size(0);
+    Plan& p = plan(T, k, n);
+    if (!p.usable) return false;
+    const void* bias = b.data_ptr();
+    const float one = 1.f, zero = 0.f;
+    bool good = cublasLtMatmulDescSetAttribute(p.op, CUBLASLT_MATMUL_DESC_BIAS_POINTER, &bias, sizeof(bias)) == CUBLAS_STATUS_SUCCESS;
+    good = good && cublasLtMatmul(handle_, p.op, &one, w.data_ptr(), p.w, x.data_ptr(), p.x, &zero, y.data_ptr(), p.y, y.data_ptr(), p.y, &p.algo,
+                                  ws_.data_ptr(), WORKSPACE, stream_) == CUBLAS_STATUS_SUCCESS;
+    return good;
+  }
+  void operator()(Tensor& y, const Tensor& x, const Tensor& w, const Tensor& b) {
+    if (try_run(y, x, w, b)) return;
+    TORCH_CHECK(!recording_, "not recordable");
+    at::addmm_out(y, b, x, w.t());
+  }
+  static constexpr size_t WORKSPACE = 32u << 20;
+
+ private:
+  struct Plan {
+    bool usable = false;
+    cublasLtMatmulDesc_t op = nullptr;
+    cublasLtMatrixLayout_t w = nullptr, x = nullptr, y = nullptr;
+    cublasLtMatmulAlgo_t algo;
+    ~Plan() {
+      if (op) cublasLtMatmulDescDestroy(op);
+      for (auto l : {w, x, y})
+        if (l) cublasLtMatrixLayoutDestroy(l);
+    }
+  };
+  Plan& plan(int64_t T, int64_t k, int64_t n) {
+    // per thread (a descriptor is written to before each launch), and bounded: a packed batch brings a new T each time
+    thread_local std::map<std::tuple<int, int64_t, int64_t, int64_t>, std::unique_ptr<Plan>> plans;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const auto key = std::make_tuple(dev, T, k, n);
+    auto it = plans.find(key);
+    if (it != plans.end()) return *it->second;
+    if (plans.size() >= 256) plans.clear();
+    auto p = std::make_unique<Plan>();
+    const cublasOperation_t trans = CUBLAS_OP_T;
+    const cublasLtEpilogue_t epilogue = CUBLASLT_EPILOGUE_BIAS;
+    cublasLtMatmulPreference_t pref = nullptr;
+    cublasLtMatmulHeuristicResult_t found{};
+    int count = 0;
+    bool good = cublasLtMatmulDescCreate(&p->op, CUBLAS_COMPUTE_32F, CUDA_R_32F) == CUBLAS_STATUS_SUCCESS &&
+                cublasLtMatmulDescSetAttribute(p->op, CUBLASLT_MATMUL_DESC_TRANSA, &trans, sizeof(trans)) == CUBLAS_STATUS_SUCCESS &&
+                cublasLtMatmulDescSetAttribute(p->op, CUBLASLT_MATMUL_DESC_EPILOGUE, &epilogue, sizeof(epilogue)) == CUBLAS_STATUS_SUCCESS &&
+                cublasLtMatrixLayoutCreate(&p->w, CUDA_R_16BF, k, n, k) == CUBLAS_STATUS_SUCCESS &&
+                cublasLtMatrixLayoutCreate(&p->x, CUDA_R_16BF, k, T, k) == CUBLAS_STATUS_SUCCESS &&
+                cublasLtMatrixLayoutCreate(&p->y, CUDA_R_16BF, n, T, n) == CUBLAS_STATUS_SUCCESS &&
+                cublasLtMatmulPreferenceCreate(&pref) == CUBLAS_STATUS_SUCCESS &&
+                cublasLtMatmulPreferenceSetAttribute(pref, CUBLASLT_MATMUL_PREF_MAX_WORKSPACE_BYTES, &WORKSPACE_BYTES, sizeof(WORKSPACE_BYTES)) == CUBLAS_STATUS_SUCCESS &&
+                cublasLtMatmulAlgoGetHeuristic(handle_, p->op, p->w, p->x, p->y, p->y, pref, 1, &found, &count) == CUBLAS_STATUS_SUCCESS && count == 1;
+    if (pref) cublasLtMatmulPreferenceDestroy(pref);
+    if (good) { p->algo = found.algo; p->usable = true; }
+    return *(plans[key] = std::move(p));
+  }
+  static constexpr uint64_t WORKSPACE_BYTES = WORKSPACE;
+  bool own_, recording_;
+  cublasLtHandle_t handle_ = nullptr;
+  cudaStream_t stream_;
+  Tensor ws_;
+};
 
 struct Layer {
   Tensor out_w, out_b, ln1_w, ln1_b, up_w, up_b, down_w, down_b, ln2_w, ln2_b;
@@ -481,7 +589,7 @@ class Encoder {
   std::vector<int> stale() const {
     std::vector<int> r;
     for (size_t i = 0; i < layers_.size(); ++i)
-      if (layers_[i].seen != stamp(layers_[i])) r.push_back((int)i);
+      if (!current(layers_[i])) r.push_back((int)i);
     return r;
   }
   void set_derived(int i, Tensor qkv_w, Tensor qkv_b, py::object tables) {
@@ -499,58 +607,38 @@ class Encoder {
   }
   // x: [T, hidden].  Packed form: cu_seqlens; padded form: batch rows of `length` tokens, all valid.  Returns the outputs of
   // all layers (or of the last one), and the status words that the caller has to look at (see Status).
-  std::pair<std::vector<Tensor>, std::vector<Tensor>> run(Tensor x, const OptTensor& cu_seqlens, int64_t length, bool every) {
-    std::vector<Tensor> outs, words;
-    const int dev = x.get_device();
-    const int64_t T = x.size(0), hidden = x.size(1);
-    const int code = dtype_code(x);
+  std::pair<std::vector<Tensor>, std::vector<Tensor>> run(const Tensor& x, const OptTensor& cu_seqlens, int64_t length, bool every) {
+    std::pair<std::vector<Tensor>, std::vector<Tensor>> r;
+    auto& [outs, words] = r;
     py::gil_scoped_release nogil;
-    c10::cuda::CUDAGuard guard((c10::DeviceIndex)dev);
+    c10::cuda::CUDAGuard guard(x.device());
     at::AutoDispatchBelowAutograd below;
-    cudaStream_t stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream();
-    Tensor ws;
-    int64_t n_seqs = 0;
-    if (cu_seqlens) {
-      n_seqs = cu_seqlens->numel() - 1;
-      ws = at::empty({(int64_t)tdb_attn_workspace_bytes((int)n_seqs, T)}, x.options().dtype(at::kByte));
+    cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
+    if (!every) {
+      Tensor y = replay(x, cu_seqlens, length, stream);
+      if (y.defined()) {
+        outs.push_back(y);
+        return r;
+      }
     }
-    bool listed = false;
-    for (const Layer& l : layers_) {
-      const Tensor qkv = at::linear(x, l.qkv_w, l.qkv_b);
-      Tensor ctx = at::empty({T, hidden}, x.options());
-      {
-        tdb::AttnParams p{};
-        const int64_t e = x.element_size();
-        char* base = static_cast<char*>(qkv.data_ptr());
-        p.q = base; p.k = base + e * hidden; p.v = base + 2 * e * hidden; p.o = ctx.data_ptr();
-        p.q_st = p.k_st = p.v_st = 3 * hidden; p.q_sh = p.k_sh = p.v_sh = p.o_sh = hidden / heads_; p.o_st = hidden;
-        if (l.tables) l.tables->fill(p, x);
-        p.H = heads_; p.D = (int)(hidden / heads_); p.sm_scale = (float)l.sm_scale; p.total_tokens = T;
-        if (cu_seqlens) {
-          p.varlen = 1; p.cu_seqlens = cu_seqlens->data_ptr<int32_t>(); p.n_seqs = (int)n_seqs; p.L = (int)length;
-          p.workspace = ws.data_ptr(); p.workspace_bytes = ws.numel(); p.tiles_listed = listed;
-        } else {
-          p.n_seqs = (int)(T / length); p.L = (int)length;
-          p.q_sb = p.k_sb = p.v_sb = 3 * hidden * length; p.o_sb = hidden * length;
-        }
+    Scratch s(*this, x, cu_seqlens);
+    Linear linear(x, stream);
+    const int dev = x.get_device();
+    Tensor in = x;
+    for (size_t i = 0; i < layers_.size(); ++i) {
+      Tensor out = every || i + 1 == layers_.size() ? at::empty_like(x) : s.z[i & 1];
+      layer(layers_[i], in, out, s, cu_seqlens, length, linear, stream, i > 0, [&](tdb::AttnParams& p) {
         Status st(dev, p);
-        const int rc = tdb_run_attn(&p, code, TDB_KERNEL_AUTO, stream);
+        const int rc = tdb_run_attn(&p, dtype_code(x), TDB_KERNEL_AUTO, stream);
         if (rc) release_unused(dev, st.slot);
         ok(rc);
         st.defer(stream, words);
-        listed = true;
-      }
-      Tensor y = at::linear(ctx, l.out_w, l.out_b);
-      add_norm(y, x, l.ln1_w, l.ln1_b, l.eps1, code, stream);
-      Tensor u = at::linear(y, l.up_w, l.up_b);
-      ok(tdb_gelu(u.data_ptr(), u.numel(), code, stream));
-      Tensor z = at::linear(u, l.down_w, l.down_b);
-      add_norm(z, y, l.ln2_w, l.ln2_b, l.eps2, code, stream);
-      x = z;
-      if (every) outs.push_back(x);
+      });
+      in = out;
+      if (every) outs.push_back(out);
     }
-    if (!every) outs.push_back(x);
-    return {std::move(outs), std::move(words)};
+    if (!every) outs.push_back(in);
+    return r;
   }
 
  private:
@@ -560,13 +648,206 @@ class Encoder {
     for (const Tensor& t : l.sources) s.emplace_back(t.data_ptr(), version_of(t));
     return s;
   }
+  static bool current(const Layer& l) {
+    if (l.seen.size() != l.sources.size()) return false;
+    for (size_t i = 0; i < l.seen.size(); ++i)
+      if (l.seen[i].first != l.sources[i].data_ptr() || l.seen[i].second != version_of(l.sources[i])) return false;
+    return true;
+  }
   static void ok(int rc) { TORCH_CHECK(rc == 0, "libtdb_b200: ", tdb_last_error(), " (code ", rc, ")"); }
   static void add_norm(Tensor& x, const Tensor& res, const Tensor& w, const Tensor& b, double eps, int code, cudaStream_t stream) {
     ok(tdb_add_layernorm(x.data_ptr(), res.data_ptr(), w.data_ptr(), b.data_ptr(), (float)eps, x.size(0), (int)x.size(1), code, x.data_ptr(), stream));
   }
+  // The buffers of one pass: every layer writes over those of the layer before it.
+  struct Scratch {
+    Tensor qkv, ctx, y, u, z[2], tiles;
+    Scratch(const Encoder& e, const Tensor& x, const OptTensor& cu) {
+      const int64_t T = x.size(0), hidden = x.size(1);
+      qkv = at::empty({T, 3 * hidden}, x.options());
+      ctx = at::empty({T, hidden}, x.options());
+      y = at::empty({T, hidden}, x.options());
+      u = at::empty({T, e.layers_[0].up_w.size(0)}, x.options());
+      z[0] = at::empty({T, hidden}, x.options());
+      z[1] = at::empty({T, hidden}, x.options());
+      if (cu) tiles = at::empty({(int64_t)tdb_attn_workspace_bytes((int)(cu->numel() - 1), T)}, x.options().dtype(at::kByte));
+    }
+  };
+
+  template <typename Attention>
+  void layer(const Layer& l, const Tensor& x, Tensor& out, Scratch& s, const OptTensor& cu_seqlens, int64_t length, Linear& linear,
+             cudaStream_t stream, bool tiles_listed, Attention attention) {
+    const int code = dtype_code(x);
+    const int64_t T = x.size(0), hidden = x.size(1), e = x.element_size();
+    linear(s.qkv, x, l.qkv_w, l.qkv_b);
+    tdb::AttnParams p{};
+    char* base = static_cast<char*>(s.qkv.data_ptr());
+    p.q = base; p.k = base + e * hidden; p.v = base + 2 * e * hidden; p.o = s.ctx.data_ptr();
+    p.q_st = p.k_st = p.v_st = 3 * hidden; p.q_sh = p.k_sh = p.v_sh = p.o_sh = hidden / heads_; p.o_st = hidden;
+    if (l.tables) l.tables->fill(p, x);
+    p.H = heads_; p.D = (int)(hidden / heads_); p.sm_scale = (float)l.sm_scale; p.total_tokens = T;
+    if (cu_seqlens) {
+      p.varlen = 1; p.cu_seqlens = cu_seqlens->data_ptr<int32_t>(); p.n_seqs = (int)(cu_seqlens->numel() - 1); p.L = (int)length;
+      p.workspace = s.tiles.data_ptr(); p.workspace_bytes = s.tiles.numel(); p.tiles_listed = tiles_listed;
+    } else {
+      p.n_seqs = (int)(T / length); p.L = (int)length;
+      p.q_sb = p.k_sb = p.v_sb = 3 * hidden * length; p.o_sb = hidden * length;
+    }
+    attention(p);
+    linear(s.y, s.ctx, l.out_w, l.out_b);
+    add_norm(s.y, x, l.ln1_w, l.ln1_b, l.eps1, code, stream);
+    linear(s.u, s.y, l.up_w, l.up_b);
+    ok(tdb_gelu(s.u.data_ptr(), s.u.numel(), code, stream));
+    linear(out, s.u, l.down_w, l.down_b);
+    add_norm(out, s.y, l.ln2_w, l.ln2_b, l.eps2, code, stream);
+  }
+
+  // Small passes are bound by the host: eight launches per layer of some 4 us each, for kernels of 2 to 8 us.  A shape that
+  // comes a second time on a stream is recorded into a CUDA graph, which belongs to that stream (its buffers are in use until
+  // the replay is over), as long as the weights stay where they are.  At most GRAPHS of them, the longest unused one goes first.
+  static constexpr int GRAPHS = 8;
+  static constexpr int64_t GRAPH_MAX_ELEMENTS = 2048 * 1024;      // T * hidden: beyond it the GPU needs longer than the host
+  struct Graph {
+    int dev = 0, slot = -1;
+    Tensor x, out, cu, lt_ws;
+    std::unique_ptr<Scratch> scratch;
+    std::vector<const void*> weights;
+    cudaGraphExec_t exec = nullptr;
+    uint64_t used = 0;
+    ~Graph() {
+      if (!exec && slot < 0) return;
+      int before = 0;
+      cudaGetDevice(&before);
+      cudaSetDevice(dev);
+      cudaDeviceSynchronize();                                    // it may still be running
+      if (exec) cudaGraphExecDestroy(exec);
+      cudaSetDevice(before);
+      (void)cudaGetLastError();
+      if (slot < 0) return;
+      StatusPool& p = g_pools[dev];
+      std::lock_guard<std::mutex> lock(p.mu);
+      bool listed = false;
+      for (auto& t : p.pending)
+        if (t.slot == slot) {                                     // an unread report: reading it frees the slot
+          t.keep = listed;                                        // (once, should two streams have listed it)
+          listed = true;
+        }
+      if (!listed) p.free.push_back(slot);
+    }
+  };
+  using Key = std::tuple<int, cudaStream_t, int64_t, int64_t, int64_t>;   // device, stream, tokens, sequences (0: padded form), length
+
+  std::vector<const void*> weight_pointers() const {
+    std::vector<const void*> w;
+    w.reserve(layers_.size() * 14);
+    for (const Layer& l : layers_) {
+      for (const Tensor* t : {&l.qkv_w, &l.qkv_b, &l.out_w, &l.out_b, &l.ln1_w, &l.ln1_b, &l.up_w, &l.up_b, &l.down_w, &l.down_b, &l.ln2_w, &l.ln2_b})
+        w.push_back(t->data_ptr());
+      w.push_back(l.tables ? ptr(l.tables->kr_exp) : nullptr);
+      w.push_back(l.tables ? ptr(l.tables->qr_exp) : nullptr);
+    }
+    return w;
+  }
+
+  Tensor replay(const Tensor& x, const OptTensor& cu_seqlens, int64_t length, cudaStream_t stream) {
+    if (x.numel() > GRAPH_MAX_ELEMENTS || !Linear::applies(x) || !x.is_contiguous() ||
+        at::cuda::currentStreamCaptureStatusMayInitCtx() != at::cuda::CaptureStatus::None)
+      return {};
+    const int dev = x.get_device();
+    const Key key(dev, stream, x.size(0), cu_seqlens ? cu_seqlens->numel() - 1 : 0, length);
+    std::lock_guard<std::mutex> lock(graph_mu_);
+    auto it = graphs_.find(key);
+    if (it == graphs_.end()) {
+      if (std::find(seen_.begin(), seen_.end(), key) == seen_.end()) {      // first time: not worth recording yet
+        seen_.push_back(key);
+        if (seen_.size() > 64) seen_.erase(seen_.begin());
+        return {};
+      }
+      if (graphs_.size() >= GRAPHS) {
+        auto oldest = graphs_.begin();
+        for (auto g = graphs_.begin(); g != graphs_.end(); ++g)
+          if (g->second->used < oldest->second->used) oldest = g;
+        graphs_.erase(oldest);
+      }
+      it = graphs_.emplace(key, std::make_unique<Graph>()).first;
+    }
+    Graph& g = *it->second;
+    if (!g.exec || g.weights != weight_pointers()) {
+      it->second = std::make_unique<Graph>();
+      if (!record(*it->second, x, cu_seqlens, length, stream)) {
+        graphs_.erase(key);
+        return {};
+      }
+    }
+    return launch_graph(*it->second, x, cu_seqlens, stream);
+  }
+
+  bool record(Graph& g, const Tensor& x, const OptTensor& cu_seqlens, int64_t length, cudaStream_t stream) {
+    g.dev = x.get_device();
+    g.slot = acquire(g.dev);
+    if (g.slot < 0) return false;
+    g.x = at::empty_like(x);
+    g.out = at::empty_like(x);
+    OptTensor cu;
+    if (cu_seqlens) cu = g.cu = at::empty_like(*cu_seqlens);
+    g.scratch = std::make_unique<Scratch>(*this, x, cu_seqlens);
+    Tensor& ws = lt_workspaces_[{g.dev, stream}];
+    if (!ws.defined()) ws = at::empty({(int64_t)Linear::WORKSPACE}, x.options().dtype(at::kByte));
+    g.lt_ws = ws;
+    g.weights = weight_pointers();
+    cudaStream_t side = nullptr;
+    cudaGraph_t graph = nullptr;
+    if (cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking) != cudaSuccess) return false;
+    bool good = cudaStreamBeginCapture(side, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
+    if (good) {
+      Linear linear(x, side, g.lt_ws, true);
+      try {
+        Tensor in = g.x;
+        for (size_t i = 0; good && i < layers_.size(); ++i) {
+          Tensor out = i + 1 == layers_.size() ? g.out : g.scratch->z[i & 1];
+          layer(layers_[i], in, out, *g.scratch, cu, length, linear, side, i > 0, [&](tdb::AttnParams& p) {
+            p.status = g_pools[g.dev].host + g.slot * SLOT_WORDS;
+            p.counter = g_pools[g.dev].ctl + g.slot * SLOT_WORDS;
+            p.gave_up = p.counter + 1;
+            ok(tdb_run_attn(&p, dtype_code(x), TDB_KERNEL_AUTO, side));
+          });
+          in = out;
+        }
+      } catch (const std::exception&) {
+        good = false;                                             // e.g. a shape that cuBLASLt leaves to torch: stays eager
+      }
+      good = (cudaStreamEndCapture(side, &graph) == cudaSuccess) && good && graph;
+    }
+    good = good && cudaGraphInstantiate(&g.exec, graph, 0) == cudaSuccess;
+    if (graph) cudaGraphDestroy(graph);
+    cudaStreamDestroy(side);
+    if (!good) (void)cudaGetLastError();
+    return good;
+  }
+
+  Tensor launch_graph(Graph& g, const Tensor& x, const OptTensor& cu_seqlens, cudaStream_t stream) {
+    g.used = ++uses_;
+    Tensor y = at::empty_like(x);
+    cuda_ok(cudaMemcpyAsync(g.x.data_ptr(), x.data_ptr(), x.nbytes(), cudaMemcpyDeviceToDevice, stream), "copy of the encoder's input");
+    if (cu_seqlens) cuda_ok(cudaMemcpyAsync(g.cu.data_ptr(), cu_seqlens->data_ptr(), cu_seqlens->nbytes(), cudaMemcpyDeviceToDevice, stream), "copy of the offsets");
+    cuda_ok(cudaGraphLaunch(g.exec, stream), "cudaGraphLaunch");
+    cuda_ok(cudaMemcpyAsync(y.data_ptr(), g.out.data_ptr(), y.nbytes(), cudaMemcpyDeviceToDevice, stream), "copy of the encoder's output");
+    StatusPool& p = g_pools[g.dev];
+    std::lock_guard<std::mutex> lock(p.mu);
+    bool listed = false;
+    for (const auto& t : p.pending) listed = listed || (t.slot == g.slot && t.keep && t.stream == stream);
+    if (!listed) p.pending.push_back({g.slot, stream, true});
+    return y;
+  }
+
   int heads_;
   std::vector<Layer> layers_;
+  std::mutex graph_mu_;
+  std::map<Key, std::unique_ptr<Graph>> graphs_;
+  std::vector<Key> seen_;
+  std::map<std::pair<int, cudaStream_t>, Tensor> lt_workspaces_;
+  uint64_t uses_ = 0;
 };
+
 
 // (all ones, right padded, tokens, longest, seqlens, cu_seqlens) of a [B, L] padding mask; one synchronisation.
 py::object mask_rows(const Tensor& mask) {
@@ -645,6 +926,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     c10::cuda::CUDAGuard guard(x.device());
     return tdb_add_layernorm(x.data_ptr(), res.data_ptr(), w.data_ptr(), b.data_ptr(), (float)eps, x.size(0), (int)x.size(1), dtype_code(x),
                              out.data_ptr(), c10::cuda::getCurrentCUDAStream().stream());
+  });
+  m.def("gelu_", [](const Tensor& x) {
+    c10::cuda::CUDAGuard guard(x.device());
+    return tdb_gelu(x.data_ptr(), x.numel(), dtype_code(x), c10::cuda::getCurrentCUDAStream().stream());
   });
   m.def("mask_rows", &mask_rows);
   m.def("pack_rows", &pack_rows);
