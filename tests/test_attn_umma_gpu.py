@@ -299,3 +299,48 @@ def test_long_sequences_with_one_position_term(c2p, p2c):
     score product, band tiles drain only that band."""
     o, ref = _fixed(_wl([1408, 700], 1408, hidden=64, heads=1), c2p=c2p, p2c=p2c)
     util.assert_close(o, ref, DT, f"long sequences, c2p={c2p}, p2c={p2c}")
+
+
+@pytest.mark.parametrize("lengths,geometry,heads", [([384, 383, 1, 0], (64, 128), 2), ([641, 896], (64, 128), 1),
+                                                    ([1152, 1025, 1279], (256, 512), 1), ([2047, 1300], (0, 512), 1)])
+def test_far_tiles_take_over_from_near_tiles(lengths, geometry, heads):
+    """Key tiles beyond the saturation distance have a kernel of their own that carries on from the near tiles' state:
+    sizes around its pairs of query tiles (an odd last tile, one row in the last tile, far tiles on one side only, no far
+    tiles), padded and packed, against the exact kernel."""
+    from turbodeberta_b200.ops.flash_attention import flash_attention_with_disentangled
+    from turbodeberta_b200.ops.flash_attention_varlen import flash_attention_with_disentangled_varlen
+    L = max(lengths)
+    w = _wl(lengths, L, hidden=64 * heads, heads=heads, buckets=geometry[0], maxpos=geometry[1])
+    q, k, v, rel, P = util.device_inputs(w, DT)
+    tables = util.make_tables(w, rel, P)
+    lens = torch.tensor(lengths, dtype=torch.int32, device="cuda")
+    args = [t.permute(0, 2, 1, 3) for t in (q, k, v)] + [None, None, False, 0.0722, *geometry]
+    o, lse = flash_attention_with_disentangled(*args, seqlens=lens, tables=tables, kernel=UMMA, return_lse=True)
+    o2, lse2 = flash_attention_with_disentangled(*args, seqlens=lens, tables=tables, kernel=SIMT, return_lse=True)
+    assert (o.float() - o2.float()).abs().max().item() < 8e-3
+    for b, n in enumerate(lengths):
+        assert torch.count_nonzero(o[b, :, n:]).item() == 0
+        assert n == 0 or (lse[b, :, :n] - lse2[b, :, :n]).abs().max().item() < 1e-3
+    keep = torch.arange(L, device="cuda")[None] < lens[:, None]
+    cu = torch.tensor(np.concatenate([[0], np.cumsum(lengths)]), dtype=torch.int32, device="cuda")
+    packed = flash_attention_with_disentangled_varlen(q[keep], k[keep], v[keep], None, None, cu, cu, L, L, False, 0.0722,
+                                                      *geometry, tables=tables, kernel=UMMA)
+    assert torch.equal(packed, o.permute(0, 2, 1, 3)[keep])
+
+
+@pytest.mark.parametrize("level", [4.0, 16.0, 60.0])
+def test_far_scores_far_above_the_near_ones(level):
+    """Far keys whose scores lie up to hundreds of powers of two above the near tiles': within what the near tiles'
+    exponent can carry, and beyond it (rows move their exponent in the far kernel)."""
+    from turbodeberta_b200.ops.flash_attention import flash_attention_with_disentangled
+    w = _wl([1500], 1500, hidden=64, heads=1, seed=78)
+    q, k, v, rel, P = util.device_inputs(w, DT)
+    tables = util.make_tables(w, rel, P)
+    q = (torch.ones_like(q).float() + 0.05 * q.float()).to(DT)
+    k = (0.1 * k.float()).to(DT)
+    k[:, 1400:] = level
+    args = [t.permute(0, 2, 1, 3) for t in (q, k, v)] + [None, None, False, 0.0722, 256, 512]
+    o = flash_attention_with_disentangled(*args, tables=tables, kernel=UMMA)
+    o2 = flash_attention_with_disentangled(*args, tables=tables, kernel=SIMT)
+    assert torch.isfinite(o.float()).all()
+    assert (o.float() - o2.float()).abs().max().item() < 2e-2

@@ -1,0 +1,557 @@
+// Far key tiles of long sequences on the sm_100a tensor cores (tcgen05 UMMA, accumulators in tensor memory).
+//
+// Where every distance of a 128x128 score tile lies at or beyond the saturation distance, on one side, all its scores use
+// the same table row r of that side, and nothing has to be gathered:
+//
+//   s[i][j] = (Q[i].K[j] + Qr[r].K[j] + Q[i].Kr[r]) * scale
+//
+// The first two terms are two accumulating products (Qr[r] as an operand of 128 identical rows, which the expanded tables
+// hold), the third is a constant of the query row that is added to its exponent.  What is left is plain attention, so this
+// kernel is built like one: a persistent CTA takes pairs of query tiles (256 rows) of one head; two groups of eight warps own a
+// tile each, two threads per row; while one group takes exponentials the tensor cores form the other's scores.
+//
+// The kernel for near key tiles (attn_umma.cu) has left each row's unnormalised output, reference exponent and sum in fp32;
+// a group starts from that exponent, adds the near output at the end and writes the finished rows.
+//
+// Bound: the special-function unit, 16384 exponentials per tile = 1024 clocks, beside 768 clocks of tensor work.  What matters
+// is that neither waits for the other: three score buffers go round the two groups, so a group's next scores are complete
+// before it has finished with the last ones, and only P.V follows its hand-off.  (With one buffer per group a pair of tiles
+// took 4300 clocks, of which 1400 were spent waiting for scores; in the one kernel for all tiles, with one accumulator and all
+// sixteen warps in step, a saturated tile took 3700.)
+//
+// Half-step t is group t & 1 at its tile t / 2.  Tensor-memory columns: three buffers of 128, S(t) in buffer t % 3 and P(t) (bf16)
+// over the columns of S(t) that its own thread has read; O of the two groups at [384,448) [448,512).  The MMA lane runs
+// S(0) S(1) S(2) | PV(0) S(3) | PV(1) S(4) | ...: S(t + 3) goes into the buffer that PV(t) reads, right behind it in the pipe.
+// All hand-offs are mbarriers with bounded waits; a wait that gives up sets the CTA's abort flag, after which every role runs
+// out its loops (the groups take their trip counts from one copy of the work item, so their named barriers still match), tensor
+// memory is freed and the host reports it.
+#include "attn_common.cuh"
+#include <math_constants.h>
+
+namespace tdb {
+using namespace ptx;
+
+namespace {
+
+constexpr int GW = 8, GT = GW * 32;                  // warps, threads of a group
+constexpr int F_THREADS = 2 * GT + 4 * 32;           // + Q and K warp, MMA warp, scheduler warp, V warp
+constexpr int F_RING = 3, STAGES = 2, BUFS = 3;
+constexpr uint32_t TILE = BQ * HD * 2;               // bytes of a 128 x 64 bf16 tile
+// Q buffer b: query tile A, query tile B, left row of Qr, right row of Qr
+constexpr uint32_t F_OFF_Q = 0, F_OFF_K = 2 * 4 * TILE, F_OFF_V = F_OFF_K + STAGES * TILE, F_OFF_BAR = F_OFF_V + STAGES * TILE;
+constexpr uint32_t F_OFF_WORK = F_OFF_BAR + 256, F_OFF_ITEM = F_OFF_WORK + F_RING * 64, F_OFF_X = F_OFF_ITEM + 4 * 64;
+constexpr uint32_t F_OFF_FLAG = F_OFF_X + 2 * 2 * BQ * 4;    // exchange: [group][half][row]
+constexpr uint32_t F_SMEM = F_OFF_FLAG + 64 + 1024;
+static_assert(F_SMEM <= 227 * 1024, "shared memory budget");
+constexpr uint32_t F_TM_S = 0, F_TM_O = 384, F_TM_COLS = 512;
+constexpr uint64_t F_WAIT_NS = 1000ull * 1000ull * 1000ull;
+
+enum FBar { FQ_FULL = 0, FQ_EMPTY = 2, FK_FULL = 4, FK_EMPTY = 6, FV_FULL = 8, FV_EMPTY = 10, FS_FULL = 12 /* per buffer */,
+            FP_READY = 15 /* per group */, FPV_DONE = 17, FWORK_FULL = 19, FWORK_EMPTY = 22, FDONE = 25, F_NBARS };
+constexpr int F_READERS = 3 + 1;                     // K lane, V lane, MMA lane, the groups' leader
+
+// A pair of query tiles of one head and its far key tiles: [0, n_left) and [right, right + n_far - n_left).
+struct FarWork {
+  int q0, len, rows, bcoord, h, n_left, right, n_far;          // n_far < 0: end of the stream
+  int64_t tok0;
+  int32_t seq, pad[5];
+};
+static_assert(sizeof(FarWork) == 64, "a ring slot");
+
+// False: past the last index.  n_far == 0: nothing to do at this index.
+__device__ __forceinline__ bool far_work(const AttnParams& p, int total_tiles, int w, FarWork& k) {
+  const int tile = w / p.H;
+  if (tile >= total_tiles) return false;
+  k.h = w - tile * p.H;
+  if (p.varlen) {
+    const int2 e = reinterpret_cast<const int2*>(reinterpret_cast<const int32_t*>(p.workspace) + 4)[tile];
+    const int c0 = p.cu_seqlens[e.x];
+    k.len = p.cu_seqlens[e.x + 1] - c0; k.rows = k.len; k.tok0 = c0; k.bcoord = 0; k.q0 = e.y; k.seq = e.x;
+  } else {
+    const int qtiles = (p.L + BQ - 1) / BQ;
+    const int seq = tile / qtiles;
+    k.q0 = (tile - seq * qtiles) * BQ;
+    const int len = p.seqlens ? p.seqlens[seq] : p.L;
+    k.len = len < 0 ? 0 : (len > p.L ? p.L : len);
+    k.rows = p.L; k.tok0 = 0; k.bcoord = seq; k.seq = seq;
+  }
+  k.n_left = 0; k.right = 0; k.n_far = 0;
+  if ((k.q0 & BQ) || k.q0 >= k.len) return true;     // the second tile of a pair, or padding
+  const int all = (k.len + BK - 1) / BK;
+  k.n_left = near_first(k.q0, p.split_sat);
+  k.right = near_end(k.q0, p.split_sat);
+  k.n_far = k.n_left + (all > k.right ? all - k.right : 0);
+  return true;
+}
+
+__device__ __forceinline__ int far_tile(const FarWork& k, int it) { return it < k.n_left ? it : k.right + (it - k.n_left); }
+
+__device__ __forceinline__ bool group_vote(int grp, bool flag) {
+  uint32_t r;
+  asm volatile(
+      "{\n"
+      ".reg .pred p, q;\n"
+      "setp.ne.u32 q, %1, 0;\n"
+      "bar.red.or.pred p, %2, %3, q;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}"
+      : "=r"(r) : "r"((uint32_t)flag), "r"(1 + grp), "n"(GT) : "memory");
+  return r != 0;
+}
+// The right to take exponentials, one token per scheduler (both groups have two warps on each): side by side the groups would
+// each get half of the special-function unit and then leave it idle together.
+__device__ __forceinline__ void token_wait(int grp, int qd) { asm volatile("bar.sync %0, 128;" ::"r"(3 + 4 * grp + qd) : "memory"); }
+__device__ __forceinline__ void token_pass(int grp, int qd) { asm volatile("bar.arrive %0, 128;" ::"r"(3 + 4 * (grp ^ 1) + qd) : "memory"); }
+__device__ __forceinline__ void groups_sync() { asm volatile("bar.sync 11, %0;" ::"n"(2 * GT) : "memory"); }
+__device__ __forceinline__ void group_sync(int grp) { asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "n"(GT) : "memory"); }
+
+// A far score without the row's constant, from global memory (rare path only): key . (query row + saturated row of Qr).
+template <bool P2C>
+__device__ __noinline__ float far_score(const __nv_bfloat16* q, const __nv_bfloat16* k, const __nv_bfloat16* r) {
+  float acc = 0.f;
+#pragma unroll 1
+  for (int d = 0; d < HD; ++d) {
+    const float kv = __bfloat162float(k[d]);
+    acc = fmaf(__bfloat162float(q[d]), kv, acc);
+    if (P2C) acc = fmaf(__bfloat162float(r[d]), kv, acc);
+  }
+  return acc;
+}
+
+template <bool C2P, bool P2C>
+__global__ void __launch_bounds__(F_THREADS, 1)
+attn_far_kernel(const AttnParams p, int32_t* counter, const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
+                const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_qr) {
+  extern __shared__ uint8_t smem_raw[];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int total_tiles = p.varlen ? reinterpret_cast<const int32_t*>(p.workspace)[0] : p.n_seqs * ((p.L + BQ - 1) / BQ);
+  const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  uint8_t* gbase = smem_raw + (sbase - smem_u32(smem_raw));
+  const uint32_t bars = sbase + F_OFF_BAR;
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(gbase + F_OFF_FLAG);
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gbase + F_OFF_FLAG + 8);
+  FarWork* ring = reinterpret_cast<FarWork*>(gbase + F_OFF_WORK);
+  auto bar = [&](int i) { return bars + 8u * (uint32_t)i; };
+  auto wait = [&](int i, uint32_t parity) { return mbar_wait(bar(i), parity, abort_flag, p.status, 201 + i, F_WAIT_NS); };
+  int32_t gave_up_before = 0;
+  if (warp == 2 * GW + 2 && lane == 0) gave_up_before = *reinterpret_cast<volatile int32_t*>(p.gave_up);
+
+  if (tid == 0) {
+    *abort_flag = 0;
+    for (int i = 0; i < F_NBARS; ++i) {
+      const bool by_warps = i >= FP_READY && i < FP_READY + 2, by_readers = i >= FWORK_EMPTY && i < FWORK_EMPTY + F_RING;
+      // a Q buffer is free when its products are done and both groups have taken their rows' constants from it
+      const bool q_empty = i >= FQ_EMPTY && i < FQ_EMPTY + 2;
+      mbar_init(bar(i), by_readers ? (uint32_t)F_READERS : by_warps ? (uint32_t)GW : q_empty ? 3u : 1u);
+    }
+    fence_mbar_init();
+  }
+  if (warp == 2 * GW && lane == 0) {
+    prefetch_tmap(&tm_q); prefetch_tmap(&tm_k); prefetch_tmap(&tm_v);
+    if (P2C) prefetch_tmap(&tm_qr);
+  }
+  if (warp == 2 * GW + 1) {
+    tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), F_TM_COLS);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+
+  auto fetch = [&](int n, FarWork& k) {
+    wait(FWORK_FULL + (n % F_RING), (uint32_t)((n / F_RING) & 1));
+    k = ring[n % F_RING];
+    if (*abort_flag) k.n_far = -1;
+    return k.n_far > 0;
+  };
+  auto release = [&](int n) { mbar_arrive(bar(FWORK_EMPTY + (n % F_RING))); };
+
+  if (warp == 2 * GW) {
+    // ================================ TMA producers ==========================================
+    if (lane == 0) {                                 // per item both query tiles and both saturated rows, then K
+      FarWork k;
+      int g = 0, n = 0;
+      for (; fetch(n, k); release(n), ++n) {
+        const int b = n & 1;
+        const uint32_t q = sbase + F_OFF_Q + (uint32_t)b * 4 * TILE;
+        if (n >= 2) wait(FQ_EMPTY + b, (uint32_t)(((n >> 1) - 1) & 1));
+        if (!*abort_flag) {
+          mbar_expect_tx(bar(FQ_FULL + b), (P2C ? 4 : 2) * TILE);
+          tma_load_4d(q, &tm_q, bar(FQ_FULL + b), 0, (int)k.tok0 + k.q0, k.h, k.bcoord);
+          tma_load_4d(q + TILE, &tm_q, bar(FQ_FULL + b), 0, (int)k.tok0 + k.q0 + BQ, k.h, k.bcoord);
+          if (P2C) {
+            tma_load_3d(q + 2 * TILE, &tm_qr, bar(FQ_FULL + b), 0, p.exp_rows - BQ, k.h);     // distances far above zero
+            tma_load_3d(q + 3 * TILE, &tm_qr, bar(FQ_FULL + b), 0, 0, k.h);                    // far below
+          }
+        }
+        for (int it = 0; it < k.n_far; ++it, ++g) {
+          const int st = g % STAGES;
+          if (g >= STAGES) wait(FK_EMPTY + st, (uint32_t)((g / STAGES - 1) & 1));
+          if (!*abort_flag) {
+            mbar_expect_tx(bar(FK_FULL + st), TILE);
+            tma_load_4d(sbase + F_OFF_K + st * TILE, &tm_k, bar(FK_FULL + st), 0, (int)k.tok0 + far_tile(k, it) * BK, k.h, k.bcoord);
+          }
+        }
+      }
+      release(n);
+    }
+  } else if (warp == 2 * GW + 3) {
+    if (lane == 0) {                                 // V
+      FarWork k;
+      int g = 0, n = 0;
+      for (; fetch(n, k); release(n), ++n)
+        for (int it = 0; it < k.n_far; ++it, ++g) {
+          const int st = g % STAGES;
+          if (g >= STAGES) wait(FV_EMPTY + st, (uint32_t)((g / STAGES - 1) & 1));
+          if (!*abort_flag) {
+            mbar_expect_tx(bar(FV_FULL + st), TILE);
+            tma_load_4d(sbase + F_OFF_V + st * TILE, &tm_v, bar(FV_FULL + st), 0, (int)k.tok0 + far_tile(k, it) * BK, k.h, k.bcoord);
+          }
+        }
+      release(n);
+    }
+  } else if (warp == 2 * GW + 2) {
+    // ================================ scheduler ==============================================
+    // Every CTA with an index of its own draws until its first draw past the end: as many draws as indices, and the counter
+    // wraps back to zero (see attn_umma.cu).
+    if (lane == 0) {
+      const unsigned int last_item = (unsigned int)(total_tiles * p.H - 1);
+      int n = 0;
+      bool first = true;
+      while (true) {
+        const int w = (*abort_flag || gave_up_before != 0) ? 0x7fffffff
+                      : first ? (int)blockIdx.x
+                              : (int)gridDim.x + (int)atomicInc(reinterpret_cast<unsigned int*>(counter), last_item);
+        first = false;
+        FarWork k;
+        if (!far_work(p, total_tiles, w, k)) k.n_far = -1;
+        if (k.n_far == 0) continue;
+        if (n >= F_RING) wait(FWORK_EMPTY + (n % F_RING), (uint32_t)(((n / F_RING) - 1) & 1));
+        ring[n % F_RING] = k;
+        mbar_arrive(bar(FWORK_FULL + (n % F_RING)));
+        ++n;
+        if (k.n_far < 0) break;
+      }
+    }
+  } else if (warp == 2 * GW + 1) {
+    // ================================ MMA issuer ============================================
+    // The whole warp walks the loop and one elected lane issues: 6 % of the kernel's time against a single-lane branch.
+    constexpr uint32_t ID_S = make_idesc_bf16(128, BK, 0), ID_PV = make_idesc_bf16(128, HD, 1);
+    const uint64_t dQ = smem_desc_sw128(sbase + F_OFF_Q), dK = smem_desc_sw128(sbase + F_OFF_K), dV = smem_desc_sw128(sbase + F_OFF_V);
+    constexpr uint64_t STEP = TILE >> 4;
+    const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+    struct Cur { int n, it, n_far, n_left; };          // item, its tile; n_far <= 0: end of the stream
+    auto load_item = [&](Cur& c) {
+      FarWork k;
+      fetch(c.n, k);
+      __syncwarp();
+      c.n_far = __shfl_sync(0xffffffffu, k.n_far, 0);
+      c.n_left = __shfl_sync(0xffffffffu, k.n_left, 0);
+    };
+    Cur cs{0, 0, 0, 0}, cv;                            // scores, three half-steps ahead of P.V
+    load_item(cs);
+    cv = cs;
+    int ts = 0;
+    auto issue_s = [&]() {
+      if (cs.n_far <= 0) return;
+      const int grp = ts & 1, g = ts >> 1, buf = ts % BUFS;
+      if (grp == 0) {
+        if (cs.it == 0) wait(FQ_FULL + (cs.n & 1), (uint32_t)((cs.n >> 1) & 1));
+        wait(FK_FULL + (g % STAGES), (uint32_t)((g / STAGES) & 1));
+        tc_fence_after();
+      }
+      const uint32_t tS = tm + F_TM_S + 128u * (uint32_t)buf;
+      const uint64_t q = dQ + (uint64_t)((cs.n & 1) * 4) * STEP, kd = dK + (uint64_t)(g % STAGES) * STEP;
+#pragma unroll
+      for (int i = 0; i < HD / 16; ++i) mma_ss_warp(tS, q + (uint64_t)grp * STEP + 2 * i, kd + 2 * i, ID_S, i > 0);
+      if (P2C) {
+        const uint64_t r = q + (cs.it < cs.n_left ? 2 : 3) * STEP;
+#pragma unroll
+        for (int i = 0; i < HD / 16; ++i) mma_ss_warp(tS, r + 2 * i, kd + 2 * i, ID_S, 1u);
+      }
+      tc_commit_warp(bar(FS_FULL + buf));
+      ++ts;
+      if (grp == 1) {
+        tc_commit_warp(bar(FK_EMPTY + (g % STAGES)));
+        if (++cs.it == cs.n_far) {
+          tc_commit_warp(bar(FQ_EMPTY + (cs.n & 1)));
+          ++cs.n; cs.it = 0;
+          load_item(cs);
+        }
+      }
+    };
+#pragma unroll 1
+    for (int i = 0; i < BUFS; ++i) issue_s();
+#pragma unroll 1
+    for (int t = 0; cv.n_far > 0; ++t) {
+      const int grp = t & 1, g = t >> 1;
+      if (grp == 0) wait(FV_FULL + (g % STAGES), (uint32_t)((g / STAGES) & 1));
+      wait(FP_READY + grp, (uint32_t)(g & 1));
+      tc_fence_after();
+      const uint64_t vd = dV + (uint64_t)(g % STAGES) * STEP;
+      const uint32_t tP = tm + F_TM_S + 128u * (uint32_t)(t % BUFS), tO = tm + F_TM_O + 64u * (uint32_t)grp;
+#pragma unroll
+      for (int i = 0; i < BK / 16; ++i)                // keys 64.. of P lie over columns 64.. of the scores
+        mma_ts_warp(tO, tP + 8u * (uint32_t)(i & 3) + 64u * (uint32_t)(i >> 2), vd + (uint64_t)(128 * i), ID_PV, (cv.it > 0 || i > 0) ? 1u : 0u);
+      tc_commit_warp(bar(FPV_DONE + grp));
+      if (grp == 1) {
+        tc_commit_warp(bar(FV_EMPTY + (g % STAGES)));
+        if (++cv.it == cv.n_far) {
+          if (lane == 0) release(cv.n);
+          ++cv.n; cv.it = 0;
+          load_item(cv);
+        }
+      }
+      issue_s();
+    }
+    if (lane == 0) release(cv.n);                      // the end-of-stream marker
+    tc_commit_warp(bar(FDONE));
+    int never = 0;                                     // this wait runs even after an abort, with its own limit
+    mbar_wait(bar(FDONE), 0, &never, p.status, 201 + FDONE, F_WAIT_NS);
+  } else {
+    // ================================ softmax groups ========================================
+    const int grp = warp / GW, gw = warp % GW, gt = tid - grp * GT;
+    const int qd = gw & 3, half = gw >> 2;
+    const int row_t = qd * 32 + lane;
+    const uint32_t lane_base = ((uint32_t)(qd * 32)) << 16;
+    const uint32_t tO = tmem + lane_base + F_TM_O + 64u * (uint32_t)grp + 32u * (uint32_t)half;
+    const uint32_t x_row = sbase + F_OFF_X + 4u * (uint32_t)(grp * 2 * BQ + row_t);             // + half * BQ * 4
+    const float sl2 = p.sm_scale * 1.4426950408889634f;
+    // All threads take their trip counts from one copy of the items, which thread 0 keeps one item ahead of the stream: it is
+    // written before thread 0 passes its token in an item's first tile, and read after that tile's vote at the earliest.
+    FarWork* const items = reinterpret_cast<FarWork*>(gbase + F_OFF_ITEM);
+    auto publish = [&](int n) {
+      FarWork k;
+      k.n_far = -1;
+      if (n == 0 || items[(n - 1) & 3].n_far > 0) {    // nothing follows the end of the stream
+        fetch(n, k);
+        release(n);
+      }
+      items[n & 3] = k;
+    };
+    if (tid == 0) publish(0);
+    groups_sync();
+    if (grp == 1) token_pass(1, qd);                 // group A goes first
+    int g = 0;
+    for (int n = 0;; ++n) {
+      const FarWork* const item = items + (n & 3);
+      const int n_far = item->n_far, n_left = item->n_left, right = item->right, len = item->len, h = item->h;
+      const int row = item->q0 + BQ * grp + row_t;
+      if (n_far <= 0) break;
+      const int64_t tok = item->tok0 + row;                          // of the packed stream, or of its batch row
+      const int64_t part = partial_tile(p, item->tok0, item->seq, item->bcoord, item->q0 + BQ * grp) * p.H + h;
+      const bool valid = row < len;
+      float2 near = make_float2(0.f, 0.f);                           // the near tiles' exponent and sum
+      if (valid) near = __ldg(reinterpret_cast<const float2*>(p.part_ml) + part * BQ + row_t);
+      float c_left = 0.f, c_right = 0.f;
+      wait(FQ_FULL + (n & 1), (uint32_t)((n >> 1) & 1));
+      if (C2P) {                                                     // Q[i].Kr[r] of both sides
+        const uint4* kl = reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(p.kr_exp) +
+                                                         ((int64_t)h * p.exp_rows + p.exp_rows - 1) * HD);
+        const uint4* kr = reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(p.kr_exp) + (int64_t)h * p.exp_rows * HD);
+        const uint32_t qrow = sbase + F_OFF_Q + (uint32_t)((n & 1) * 4 + grp) * TILE + 128u * (uint32_t)row_t;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const uint4 a = lds_128(qrow + 16u * (uint32_t)(i ^ (row_t & 7))), b = __ldg(kl + i), c = __ldg(kr + i);
+          const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w}, cw[4] = {c.x, c.y, c.z, c.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float a0 = __uint_as_float(aw[e] << 16), a1 = __uint_as_float(aw[e] & 0xffff0000u);
+            c_left = fmaf(a0, __uint_as_float(bw[e] << 16), c_left);
+            c_left = fmaf(a1, __uint_as_float(bw[e] & 0xffff0000u), c_left);
+            c_right = fmaf(a0, __uint_as_float(cw[e] << 16), c_right);
+            c_right = fmaf(a1, __uint_as_float(cw[e] & 0xffff0000u), c_right);
+          }
+        }
+        c_left *= sl2; c_right *= sl2;
+      }
+      float m = near.x, l = 0.f;
+      for (int it = 0; it < n_far; ++it, ++g) {
+        const int kt = it < n_left ? it : right + (it - n_left);
+        const int nv_tile = len - kt * BK, nvalid = nv_tile - 64 * half;   // keys e >= nvalid of this thread are masked
+        const float c = it < n_left ? c_left : c_right;
+        const int t = 2 * g + grp, buf = t % BUFS;
+        const uint32_t tS = tmem + lane_base + F_TM_S + 128u * (uint32_t)buf + 64u * (uint32_t)half;
+        wait(FS_FULL + buf, (uint32_t)((t / BUFS) & 1));
+        tc_fence_after();
+        if (it == 0 && tid == 0) publish(n + 1);
+        token_wait(grp, qd);
+        // P of the thread's 64 keys, sixteen at a time: the next sixteen scores are on their way from tensor memory while the
+        // exponentials (against the row's reference exponent) of these are taken.  P goes over scores that have been read.
+        float sum;
+        {
+          float s[2][16];
+          const float bias = c - m;
+          float s0 = 0.f, s1 = 0.f;
+          tmem_ld16(tS, reinterpret_cast<uint32_t*>(s[0]));
+#pragma unroll
+          for (int part = 0; part < 4; ++part) {
+            float* x = s[part & 1];
+            tmem_ld_wait16(reinterpret_cast<uint32_t*>(x));
+            if (part < 3) tmem_ld16(tS + 16u * (uint32_t)(part + 1), reinterpret_cast<uint32_t*>(s[(part + 1) & 1]));
+            if (nvalid < 64) {
+#pragma unroll
+              for (int e = 0; e < 16; ++e) x[e] = 16 * part + e < nvalid ? x[e] : -CUDART_INF_F;
+            }
+            uint32_t pk[8];
+#pragma unroll
+            for (int e = 0; e < 16; e += 2) {
+              const float a = ex2(fmaf(x[e], sl2, bias)), b = ex2(fmaf(x[e + 1], sl2, bias));
+              s0 += a; s1 += b;
+              pk[e / 2] = pack_bf16x2(a, b);
+            }
+            tmem_st8(tS + 8u * (uint32_t)part, pk);
+          }
+          sum = s0 + s1;
+        }
+        token_pass(grp, qd);
+        if (g > 0) wait(FPV_DONE + grp, (uint32_t)((g - 1) & 1));    // done long ago; keeps the barrier's phases in step
+        // A bf16 probability and an fp32 sum have room for 2^64 times the near tiles' exponent; a row beyond that (or the
+        // overflow it led to) moves its exponent, and with it this tile's P and the output so far.  Its scores are gone, so
+        // they are formed again, on the CUDA cores.
+        if (group_vote(grp, valid && sum > 1.8e19f)) {
+          const __nv_bfloat16* q = reinterpret_cast<const __nv_bfloat16*>(p.q) + (int64_t)item->bcoord * p.q_sb +
+                                   (valid ? tok : item->tok0) * p.q_st + (int64_t)h * p.q_sh;
+          const __nv_bfloat16* k = reinterpret_cast<const __nv_bfloat16*>(p.k) + (int64_t)item->bcoord * p.k_sb +
+                                   (item->tok0 + kt * BK + 64 * half) * p.k_st + (int64_t)h * p.k_sh;
+          const __nv_bfloat16* r = reinterpret_cast<const __nv_bfloat16*>(p.qr_exp) +
+                                   ((int64_t)h * p.exp_rows + (it < n_left ? p.exp_rows - 1 : 0)) * HD;
+          float mx = -CUDART_INF_F;
+#pragma unroll 1
+          for (int e = 0; e < 64 && e < nvalid; ++e) mx = fmaxf(mx, far_score<P2C>(q, k + e * p.k_st, r));
+          sts_f32(x_row + (uint32_t)half * (BQ * 4), mx);
+          group_sync(grp);
+          const float top = fmaf(fmaxf(lds_f32(x_row), lds_f32(x_row + BQ * 4)), sl2, c);
+          const bool redo = valid && top - m > 8.f;
+          if (__any_sync(0xffffffffu, redo)) {
+            const float m_new = redo ? top : m, alpha = redo ? ex2(m - top) : 1.f, bias = c - m_new;
+            tmem_st_wait();
+            sum = 0.f;
+#pragma unroll 1
+            for (int part = 0; part < 4; ++part) {
+              uint32_t pk[8];
+#pragma unroll
+              for (int e = 0; e < 8; ++e) {
+                const int j = 16 * part + 2 * e;
+                const float a = j < nvalid ? ex2(fmaf(far_score<P2C>(q, k + j * p.k_st, r), sl2, bias)) : 0.f;
+                const float b = j + 1 < nvalid ? ex2(fmaf(far_score<P2C>(q, k + (j + 1) * p.k_st, r), sl2, bias)) : 0.f;
+                sum += a + b;
+                pk[e] = pack_bf16x2(a, b);
+              }
+              __syncwarp();
+              tmem_st8(tS + 8u * (uint32_t)part, pk);
+            }
+            if (it > 0) {
+              uint32_t o[32];
+              tc_fence_after();
+              tmem_ld32(tO, o);
+              tmem_ld_wait32(o);
+#pragma unroll
+              for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * alpha);
+              tmem_st32(tO, o);
+            }
+            l *= alpha;
+            m = m_new;
+          }
+        }
+        l += sum;
+        if (it == 0 && gt == 0) mbar_arrive(bar(FQ_EMPTY + (n & 1)));      // behind the vote: the group has read its rows of Q
+        // Keys beyond the sequence have exact zeros as probabilities, but their rows of V may hold anything (0 x NaN): group A
+        // zeroes them in shared memory before it announces P, and the other group's product is issued after its own.
+        if (grp == 0 && nv_tile < BK) {
+          const int st = g % STAGES;
+          wait(FV_FULL + st, (uint32_t)((g / STAGES) & 1));
+          for (int i = gt; i < (BK - nv_tile) * 8; i += GT)
+            sts_128(sbase + F_OFF_V + st * TILE + (uint32_t)(nv_tile + (i >> 3)) * 128u + 16u * (uint32_t)(i & 7), 0u, 0u, 0u, 0u);
+          fence_proxy_async_smem();
+        }
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(FP_READY + grp));
+      }
+      // (far output + near output) / sum -> global; the near output is on its way while the last product runs
+      float nr[32];
+#pragma unroll
+      for (int i = 0; i < 32; ++i) nr[i] = valid ? __ldg(p.part_o + part * (BQ * HD) + (32 * half + i) * BQ + row_t) : 0.f;
+      group_sync(grp);                               // the last tile may have exchanged maxima in the same words
+      sts_f32(x_row + (uint32_t)half * (BQ * 4), l);
+      group_sync(grp);
+      const float beta = ex2(near.x - m);
+      const float l_tot = fmaf(near.y, beta, lds_f32(x_row) + lds_f32(x_row + BQ * 4));
+      wait(FPV_DONE + grp, (uint32_t)((g - 1) & 1));
+      tc_fence_after();
+      uint32_t r[32];
+      tmem_ld32(tO, r);
+      tmem_ld_wait32(r);
+      tc_fence_before();
+      if (row < item->rows) {
+        float inv;
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(l_tot));
+        uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.o) + (int64_t)item->bcoord * p.o_sb + tok * p.o_st +
+                                              (int64_t)h * p.o_sh + 32 * half);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float* v = nr + 8 * i;
+          uint32_t w[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            w[e] = valid ? pack_bf16x2(fmaf(v[2 * e], beta, __uint_as_float(r[8 * i + 2 * e])) * inv,
+                                       fmaf(v[2 * e + 1], beta, __uint_as_float(r[8 * i + 2 * e + 1])) * inv) : 0u;
+          dst[i] = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+        if (p.lse && half == 0)
+          p.lse[(int64_t)item->bcoord * p.lse_sb + (int64_t)h * p.lse_sh + tok] = valid ? m * 0.6931471805599453f + logf(l_tot) : 0.f;
+      }
+      group_sync(grp);                               // the exchange words are free again
+    }
+    if (grp == 0) token_wait(0, qd);                 // group B's last pass
+  }
+
+  // ---- teardown ------------------------------------------------------------------------------
+  if (*abort_flag) {                      // give copies that may still be in flight time to land
+    if (tid == 0 && p.gave_up != p.status) *reinterpret_cast<volatile int32_t*>(p.gave_up) = 1;
+    const uint64_t t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  if (warp == 2 * GW + 1) tmem_dealloc(tmem, F_TM_COLS);
+}
+
+template <bool C2P, bool P2C>
+int launch_far_variant(const AttnParams& p, dim3 grid, const CUtensorMap* maps, cudaStream_t s) {
+  auto kern = attn_far_kernel<C2P, P2C>;
+  const int rc = opt_in_smem(reinterpret_cast<const void*>(kern), (int)F_SMEM);
+  if (rc) return rc;
+  kern<<<grid, F_THREADS, F_SMEM, s>>>(p, p.counter + 2, maps[0], maps[1], maps[2], maps[3]);
+  return cuda_fail(cudaGetLastError(), "attn_far launch");
+}
+
+}  // namespace
+
+// `tiles`: query tiles of the whole problem (an upper bound in the packed form, whose list says how many there are).
+int launch_attn_far(const AttnParams& p, int64_t tiles, int sms, cudaStream_t s) {
+  CUtensorMap maps[4];
+  const int64_t tokens = p.varlen ? p.total_tokens : p.L;
+  const int B = p.varlen ? 1 : p.n_seqs;
+  int rc;
+  if ((rc = token_map(&maps[0], p.q, tokens, p.H, B, p.q_sb, p.q_st, p.q_sh, "q"))) return rc;
+  if ((rc = token_map(&maps[1], p.k, tokens, p.H, B, p.k_sb, p.k_st, p.k_sh, "k"))) return rc;
+  if ((rc = token_map(&maps[2], p.v, tokens, p.H, B, p.v_sb, p.v_st, p.v_sh, "v"))) return rc;
+  const bool c2p = p.flags & TDB_FLAG_C2P, p2c = p.flags & TDB_FLAG_P2C;
+  if (p2c) {
+    if ((rc = table_map(&maps[3], p.qr_exp, p.exp_rows, p.H, BQ, "qr_exp (far tiles)"))) return rc;
+  } else {
+    maps[3] = maps[0];
+  }
+  const int64_t items = tiles * p.H;
+  dim3 grid((unsigned)(items < sms ? items : sms), 1, 1);
+  if (c2p && p2c) return launch_far_variant<true, true>(p, grid, maps, s);
+  if (c2p) return launch_far_variant<true, false>(p, grid, maps, s);
+  return launch_far_variant<false, true>(p, grid, maps, s);
+}
+
+}  // namespace tdb

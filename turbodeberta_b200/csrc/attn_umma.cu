@@ -51,7 +51,7 @@
 //
 // Tensor-memory columns: [0,128) S, [128,192) O, [192,448) band buffer, [448,512) P (bf16).
 #include "tdb_internal.h"
-#include "ptx_sm100.cuh"
+#include "attn_common.cuh"
 #include <cudaTypedefs.h>
 #include <math_constants.h>
 #include <mutex>
@@ -61,7 +61,7 @@ using namespace ptx;
 
 namespace {
 
-constexpr int BQ = 128, BK = 128, HD = 64, BAND = 256;
+constexpr int BAND = 256;
 #ifndef TDB_GROUPS
 #define TDB_GROUPS 4
 #endif
@@ -178,24 +178,6 @@ __device__ __forceinline__ uint32_t lds_u32(uint32_t addr) {
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
   return v;
 }
-__device__ __forceinline__ float lds_f32(uint32_t addr) {
-  float v;
-  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
-  return v;
-}
-__device__ __forceinline__ void sts_f32(uint32_t addr, float v) {
-  asm volatile("st.shared.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
-}
-__device__ __forceinline__ uint4 lds_128(uint32_t addr) {
-  uint4 v;
-  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
-  return v;
-}
-__device__ __forceinline__ void sts_128(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
-}
-// Makes this thread's earlier shared-memory writes visible to the asynchronous proxy (the tensor cores' operand fetch).
-__device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void bar_all_cuda_warps() { asm volatile("bar.sync 1, %0;" ::"n"(NCT) : "memory"); }
 // The same barrier with an OR-reduction of one predicate per thread.
 __device__ __forceinline__ bool bar_all_cuda_warps_or(bool flag) {
@@ -265,10 +247,12 @@ constexpr int SATN = 128;                       // rows of the repeated-row boxe
 
 struct Work {
   int q0, len, rows, bcoord, h, n_kv;      // n_kv == 0: tile of padded query rows only (zeros, no tensor work)
+                                           // rows: that exist in the output; packed form: number of the sequence (all its rows do)
   int64_t tok0;
 };
 
 // perm: padded form only, sequences by decreasing length (null: natural order).
+template <bool SPLIT>
 __device__ __forceinline__ bool get_work(const AttnParams& p, int total_tiles, int w, const uint16_t* perm, Work& k) {
   const int tile = w / p.H;
   if (tile >= total_tiles) return false;
@@ -277,7 +261,7 @@ __device__ __forceinline__ bool get_work(const AttnParams& p, int total_tiles, i
     const int32_t* ws = reinterpret_cast<const int32_t*>(p.workspace);
     const int2 e = reinterpret_cast<const int2*>(ws + 4)[tile];
     const int c0 = p.cu_seqlens[e.x];
-    k.len = p.cu_seqlens[e.x + 1] - c0; k.rows = k.len; k.tok0 = c0; k.bcoord = 0; k.q0 = e.y;
+    k.len = p.cu_seqlens[e.x + 1] - c0; k.rows = e.x; k.tok0 = c0; k.bcoord = 0; k.q0 = e.y;
   } else {
     const int qtiles = (p.L + BQ - 1) / BQ;
     int seq = tile / qtiles;
@@ -288,11 +272,20 @@ __device__ __forceinline__ bool get_work(const AttnParams& p, int total_tiles, i
     k.rows = p.L; k.tok0 = 0; k.bcoord = seq;
   }
   k.n_kv = k.q0 < k.len ? (k.len + BK - 1) / BK : 0;
+  if (SPLIT && k.n_kv > 0) {               // the key tiles around the diagonal only (see near_first)
+    const int end = near_end(k.q0, p.split_sat);
+    k.n_kv = (end < k.n_kv ? end : k.n_kv) - near_first(k.q0, p.split_sat);
+  }
   return true;
 }
 
+// First key of an item's first key tile.
+template <bool SPLIT>
+__device__ __forceinline__ int first_key(const AttnParams& p, int q0) { return SPLIT ? near_first(q0, p.split_sat) * BK : 0; }
+
 // LONG: sequences can be long enough for saturated tiles (compiled out otherwise, which keeps the common kernel lean).
-template <bool C2P, bool P2C, bool LONG>
+// SPLIT: they are, and the kernel for far tiles takes those.
+template <bool C2P, bool P2C, bool LONG, bool SPLIT>
 __global__ void __launch_bounds__(NTHREADS, 1)
 attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                  const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_kr,
@@ -391,8 +384,9 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap tm_q, c
       Work k;
       int g = 0, n = 0;
       while (next_tensor_item(n, k)) {
+        const int kb = first_key<SPLIT>(p, k.q0);
         for (int it = 0; it < k.n_kv; ++it, ++g) {
-          const int k0 = it * BK;
+          const int k0 = kb + it * BK;
           const uint32_t pe = (uint32_t)((g - 1) & 1);
           int x0 = k.q0 - k0 - (BK - 1) + p.exp_delta_max;
           x0 = x0 < 0 ? 0 : (x0 > p.exp_rows - BAND ? p.exp_rows - BAND : x0);
@@ -425,11 +419,12 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap tm_q, c
       Work k;
       int g = 0, n = 0;
       while (next_tensor_item(n, k)) {
+        const int kb = first_key<SPLIT>(p, k.q0);
         for (int it = 0; it < k.n_kv; ++it, ++g) {
           if (g > 0) wait(V_EMPTY, (uint32_t)((g - 1) & 1));
           if (!*abort_flag) {
             mbar_expect_tx(bar(V_FULL), BK * HD * 2);
-            tma_load_4d(sV, &tm_v, bar(V_FULL), 0, (int)(k.tok0 + it * BK), k.h, k.bcoord);
+            tma_load_4d(sV, &tm_v, bar(V_FULL), 0, (int)(k.tok0 + kb + it * BK), k.h, k.bcoord);
           }
         }
         release(n);
@@ -472,7 +467,7 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap tm_q, c
       first = false;
       w = __shfl_sync(0xffffffffu, w, 0);
       Work k;
-      if (!get_work(p, total_tiles, w, perm, k)) k.n_kv = -1;
+      if (!get_work<SPLIT>(p, total_tiles, w, perm, k)) k.n_kv = -1;
       if (k.n_kv == 0) {
         for (int r = lane; r < BQ; r += 32) {
           if (k.q0 + r >= k.rows) break;
@@ -706,6 +701,7 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap tm_q, c
     auto finish_item = [&](int pn, int gl) {
       Work w;
       load_item(pn, w);
+      const int rows = p.varlen ? w.len : w.rows;
       const uint32_t par = (uint32_t)(pn & 1);
       float l_tot = 0.f;
 #pragma unroll
@@ -716,6 +712,21 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap tm_q, c
       uint32_t r[OPT];
       tmem_ld_cols<OPT>(tO, r);
       tc_fence_before();
+      if (SPLIT) {
+        const int all = (w.len + BK - 1) / BK;
+        if (near_first(w.q0, p.split_sat) > 0 || near_end(w.q0, p.split_sat) < all) {
+          // The far kernel carries on from here: unnormalised output, reference exponent and sum, fp32.
+          const int64_t part = partial_tile(p, w.tok0, w.rows, w.bcoord, w.q0) * p.H + w.h;
+          if (w.q0 + row_t < w.len) {
+            float* dst = p.part_o + part * (BQ * HD) + OPT * grp * BQ + row_t;
+#pragma unroll
+            for (int i = 0; i < OPT; ++i) dst[i * BQ] = __uint_as_float(r[i]);
+            if (grp == 0)
+              reinterpret_cast<float2*>(p.part_ml)[part * BQ + row_t] = make_float2(lds_f32(mx_row + par * (BQ * 4)), l_tot);
+          }
+          return;
+        }
+      }
       float inv;
       asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(l_tot));
       // The normalised rows go through shared memory (the quadrant's part of the p2c staging area, which nobody
@@ -740,11 +751,11 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap tm_q, c
           const int rq = 8 * grp + 4 * i + (lane >> 3);                        // row inside the quadrant
           const int row = w.q0 + 32 * qd + rq;
           const uint4 v = lds_128(obuf + (uint32_t)rq * 144u + 16u * (uint32_t)(lane & 7));
-          if (row < w.rows) *reinterpret_cast<uint4*>(obase + (w.tok0 + row) * p.o_st) = v;
+          if (row < rows) *reinterpret_cast<uint4*>(obase + (w.tok0 + row) * p.o_st) = v;
         }
         if (p.lse && grp == 0) {
           const int row = w.q0 + row_t;
-          if (row < w.rows)
+          if (row < rows)
             p.lse[(int64_t)w.bcoord * p.lse_sb + (int64_t)w.h * p.lse_sh + w.tok0 + row] =
                 valid ? (lds_f32(mx_row + par * (BQ * 4)) * 0.6931471805599453f + logf(l_tot)) : 0.f;
         }
@@ -754,10 +765,10 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap tm_q, c
 
     if (tid == 0) { leader_publish(0); leader_publish(1); }
     bar_all_cuda_warps();
-    struct { int q0, len, n_kv; } cur;
+    struct { int q0, len, n_kv; } cur;                                 // len: counted from the item's first key
     auto switch_item = [&](int n) {
       volatile Work* w = item_slots + (n & 3);
-      cur.q0 = w->q0; cur.len = w->len; cur.n_kv = w->n_kv;
+      cur.q0 = w->q0; cur.len = w->len - first_key<SPLIT>(p, w->q0); cur.n_kv = w->n_kv;
     };
     switch_item(0);
     if (cur.n_kv > 0) {
@@ -1010,7 +1021,9 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap tm_q, c
 }
 
 // ---------------------------------------------------------------------------------------------
-PFN_cuTensorMapEncodeTiled_v12000 get_encode_fn() {
+}  // namespace
+
+static PFN_cuTensorMapEncodeTiled_v12000 get_encode_fn() {
   // initialised once, by whichever thread comes first (function-local statics are thread-safe)
   static const PFN_cuTensorMapEncodeTiled_v12000 fn = [] {
     void* ptr = nullptr;
@@ -1023,7 +1036,7 @@ PFN_cuTensorMapEncodeTiled_v12000 get_encode_fn() {
   return fn;
 }
 
-int encode_map(CUtensorMap* m, const void* ptr, int rank, const uint64_t* dims, const uint64_t* strides_bytes,
+static int encode_map(CUtensorMap* m, const void* ptr, int rank, const uint64_t* dims, const uint64_t* strides_bytes,
                const uint32_t* box, const char* what) {
   auto fn = get_encode_fn();
   if (!fn) { set_error("cuTensorMapEncodeTiled entry point not found"); return TDB_ERR_CUDA; }
@@ -1051,9 +1064,11 @@ int table_map(CUtensorMap* m, const void* ptr, int rows, int H, int box_rows, co
   return encode_map(m, ptr, 3, dims, strides, box, what);
 }
 
-template <bool C2P, bool P2C, bool LONG>
+namespace {
+
+template <bool C2P, bool P2C, bool LONG, bool SPLIT = false>
 int launch_variant(const AttnParams& p, dim3 grid, const CUtensorMap* maps, cudaStream_t s) {
-  auto kern = attn_umma_kernel<C2P, P2C, LONG>;
+  auto kern = attn_umma_kernel<C2P, P2C, LONG, SPLIT>;
   const int rc = opt_in_smem(reinterpret_cast<const void*>(kern), (int)SMEM_BYTES);
   if (rc) return rc;
   kern<<<grid, NTHREADS, SMEM_BYTES, s>>>(p, maps[0], maps[1], maps[2], maps[3], maps[4], maps[5], maps[6]);
@@ -1093,6 +1108,10 @@ size_t umma_workspace_bytes(int n_seqs, int64_t total_tokens) {
   return sizeof(TileListHeader) + (size_t)cap * sizeof(int2);
 }
 
+bool has_far_tiles(const AttnParams& p) {
+  return p.flags && p.L >= 2 * (p.exp_delta_max - TDB_EXPAND_MARGIN) + BK;
+}
+
 int launch_attn_umma(const AttnParams& given, cudaStream_t s) {
   AttnParams p = given;
   if (!p.counter) { p.counter = p.status + 2; p.gave_up = p.status; }
@@ -1100,7 +1119,12 @@ int launch_attn_umma(const AttnParams& given, cudaStream_t s) {
   // them specially is a little slower on ordinary tiles, so it is used from twice that length on (p.L is the
   // padded length or the caller's max_seqlen).
   const bool c2p = p.flags & TDB_FLAG_C2P, p2c = p.flags & TDB_FLAG_P2C;
-  const bool lng = (c2p || p2c) && p.L >= 2 * (p.exp_delta_max - TDB_EXPAND_MARGIN) + BK;
+  const int sat = p.exp_delta_max - TDB_EXPAND_MARGIN;
+  bool lng = has_far_tiles(p);
+  // With room for the partial results the far tiles go to a kernel of their own, which has no bands to make room for.
+  const bool split = lng && p.part_o && p.part_ml && given.counter;
+  p.split_sat = split ? sat : 0;
+  lng = lng && !split;
   if (p.H > 65535) { set_error("more than 65535 heads"); return TDB_ERR_SHAPE; }
   CUtensorMap maps[7];
   memset(maps, 0, sizeof(maps));
@@ -1141,10 +1165,11 @@ int launch_attn_umma(const AttnParams& given, cudaStream_t s) {
   // status word 2 as the work counter: start it at zero even if the caller reuses the words
   if (p.counter == p.status + 2 &&
       (rc = cuda_fail(cudaMemsetAsync(p.counter, 0, sizeof(int32_t), s), "cudaMemsetAsync(work counter)"))) return rc;
-  if (c2p && p2c) return lng ? launch_variant<true, true, true>(p, grid, maps, s) : launch_variant<true, true, false>(p, grid, maps, s);
-  if (c2p) return lng ? launch_variant<true, false, true>(p, grid, maps, s) : launch_variant<true, false, false>(p, grid, maps, s);
-  if (p2c) return lng ? launch_variant<false, true, true>(p, grid, maps, s) : launch_variant<false, true, false>(p, grid, maps, s);
-  return launch_variant<false, false, false>(p, grid, maps, s);
+  if (c2p && p2c) rc = split ? launch_variant<true, true, false, true>(p, grid, maps, s) : lng ? launch_variant<true, true, true>(p, grid, maps, s) : launch_variant<true, true, false>(p, grid, maps, s);
+  else if (c2p) rc = split ? launch_variant<true, false, false, true>(p, grid, maps, s) : lng ? launch_variant<true, false, true>(p, grid, maps, s) : launch_variant<true, false, false>(p, grid, maps, s);
+  else if (p2c) rc = split ? launch_variant<false, true, false, true>(p, grid, maps, s) : lng ? launch_variant<false, true, true>(p, grid, maps, s) : launch_variant<false, true, false>(p, grid, maps, s);
+  else rc = launch_variant<false, false, false>(p, grid, maps, s);
+  return rc || !split ? rc : launch_attn_far(p, tiles, sms, s);
 }
 
 }  // namespace tdb

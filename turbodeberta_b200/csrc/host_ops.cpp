@@ -89,6 +89,21 @@ std::pair<int, int> collect(int dev, int slot, bool keep = false) {
   return r;
 }
 
+// Scratch for long sequences (see AttnParams::part_o), if the device has room for it; the call works without it too.
+Tensor partial_scratch(tdb::AttnParams& p, int dtype, int kernel, const Tensor& like) {
+  const int64_t n = tdb_partial_floats(&p, dtype, kernel);
+  if (n == 0) return {};
+  Tensor t;
+  try {
+    t = at::empty({n}, like.options().dtype(at::kFloat));
+  } catch (const c10::OutOfMemoryError&) {
+    return {};
+  }
+  p.part_o = t.data_ptr<float>();
+  p.part_ml = p.part_o + n / 66 * 64;
+  return t;
+}
+
 void release_unused(int dev, int slot) {
   if (slot < 0) return;
   std::lock_guard<std::mutex> lock(g_pools[dev].mu);
@@ -106,19 +121,21 @@ struct Status {
       p.counter = g_pools[dev].ctl + slot * SLOT_WORDS;
       p.gave_up = p.counter + 1;
     } else {
-      own = at::zeros({4}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, (c10::DeviceIndex)dev));
+      own = at::zeros({8}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, (c10::DeviceIndex)dev));
       p.status = own.data_ptr<int32_t>();
+      p.counter = p.status + 4;
+      p.gave_up = p.status + 5;
     }
   }
   // Leave the check to drain_pending(); words of the call's own go to `words`.  Needs no interpreter lock.
   void defer(cudaStream_t stream, std::vector<Tensor>& words) {
-    if (slot < 0) { words.push_back(own); return; }
+    if (slot < 0) { words.push_back(own.narrow(0, 0, SLOT_WORDS)); return; }
     std::lock_guard<std::mutex> lock(g_pools[dev].mu);
     g_pools[dev].pending.push_back({slot, stream, false});
   }
   // What the caller in Python gets to see: None (fine, or deferred into the pool), (word 0, word 1), or the tensor of words.
   py::object finish(bool check, cudaStream_t stream) {
-    if (slot < 0) return py::cast(own);
+    if (slot < 0) return py::cast(own.narrow(0, 0, SLOT_WORDS));
     if (!check) {
       std::lock_guard<std::mutex> lock(g_pools[dev].mu);
       g_pools[dev].pending.push_back({slot, stream, false});
@@ -255,6 +272,7 @@ using Result = std::tuple<Tensor, py::object, py::object>;      // o, lse or Non
 Result launch(tdb::AttnParams& p, int dtype, int kernel, int dev, Tensor o, const Tensor& lse, bool check) {
   cudaStream_t stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream();
   Status st(dev, p);
+  const Tensor partial = partial_scratch(p, dtype, kernel, o);
   const int rc = tdb_run_attn(&p, dtype, kernel, stream);
   py::object lse_out = lse.defined() ? py::cast(lse) : py::none();
   if (rc) {
@@ -629,6 +647,7 @@ class Encoder {
       Tensor out = every || i + 1 == layers_.size() ? at::empty_like(x) : s.z[i & 1];
       layer(layers_[i], in, out, s, cu_seqlens, length, linear, stream, i > 0, [&](tdb::AttnParams& p) {
         Status st(dev, p);
+        const Tensor partial = partial_scratch(p, dtype_code(x), TDB_KERNEL_AUTO, x);
         const int rc = tdb_run_attn(&p, dtype_code(x), TDB_KERNEL_AUTO, stream);
         if (rc) release_unused(dev, st.slot);
         ok(rc);
@@ -704,11 +723,11 @@ class Encoder {
   // Small passes are bound by the host: eight launches per layer of some 4 us each, for kernels of 2 to 8 us.  A shape that
   // comes a second time on a stream is recorded into a CUDA graph, which belongs to that stream (its buffers are in use until
   // the replay is over), as long as the weights stay where they are.  At most GRAPHS of them, the longest unused one goes first.
-  static constexpr int GRAPHS = 8;
+  static constexpr int GRAPHS = 8, BLOCK = 128;
   static constexpr int64_t GRAPH_MAX_ELEMENTS = 2048 * 1024;      // T * hidden: beyond it the GPU needs longer than the host
   struct Graph {
     int dev = 0, slot = -1;
-    Tensor x, out, cu, lt_ws;
+    Tensor x, out, cu, lt_ws, partial;
     std::unique_ptr<Scratch> scratch;
     std::vector<const void*> weights;
     cudaGraphExec_t exec = nullptr;
@@ -794,6 +813,10 @@ class Encoder {
     if (!ws.defined()) ws = at::empty({(int64_t)Linear::WORKSPACE}, x.options().dtype(at::kByte));
     g.lt_ws = ws;
     g.weights = weight_pointers();
+    if (length > 2 * BLOCK) {                                     // long enough for far key tiles
+      const int64_t n = cu_seqlens ? cu_seqlens->numel() - 1 : x.size(0) / length;
+      g.partial = at::empty({(x.size(0) / BLOCK + 2 * n + 1) * BLOCK * heads_ * 66}, x.options().dtype(at::kFloat));
+    }
     cudaStream_t side = nullptr;
     cudaGraph_t graph = nullptr;
     if (cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking) != cudaSuccess) return false;
@@ -808,6 +831,11 @@ class Encoder {
             p.status = g_pools[g.dev].host + g.slot * SLOT_WORDS;
             p.counter = g_pools[g.dev].ctl + g.slot * SLOT_WORDS;
             p.gave_up = p.counter + 1;
+            const int64_t n = tdb_partial_floats(&p, dtype_code(x), TDB_KERNEL_AUTO);
+            if (n > 0 && g.partial.defined() && n <= g.partial.numel()) {
+              p.part_o = g.partial.data_ptr<float>();
+              p.part_ml = p.part_o + n / 66 * 64;
+            }
             ok(tdb_run_attn(&p, dtype_code(x), TDB_KERNEL_AUTO, side));
           });
           in = out;

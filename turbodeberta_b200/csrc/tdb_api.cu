@@ -341,6 +341,12 @@ int tdb_run_attn(const tdb::AttnParams* p, int dtype, int kernel, void* stream) 
   return run_attn(*p, dtype, kernel, (cudaStream_t)stream);
 }
 
+int64_t tdb_partial_floats(const tdb::AttnParams* p, int dtype, int kernel) {
+  if (pick_kernel(dtype, kernel) != TDB_KERNEL_UMMA || dtype != TDB_DTYPE_BF16 || p->D != 64 || !has_far_tiles(*p)) return 0;
+  const int64_t tiles = p->varlen ? p->total_tokens / 128 + p->n_seqs + 1 : (int64_t)p->n_seqs * ((p->L + 127) / 128);
+  return tiles * p->H * 128 * (64 + 2);
+}
+
 int tdb_expand_pair(const void* kr, const void* qr, const int16_t* idx, int idx_delta_max, int H, int two_span,
                     int exp_delta_max, int exp_rows, void* kr_out, void* qr_out, void* stream) {
   return launch_relpos_expand_pair(kr, qr, idx, idx_delta_max, H, two_span, exp_delta_max, exp_rows, kr_out, qr_out,

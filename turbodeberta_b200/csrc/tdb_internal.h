@@ -38,8 +38,12 @@ struct AttnParams {
   int32_t* status;                                        // device-visible words: 0 = gave-up code, 1 = malformed offsets
   // Tensor-core kernel: the device-wide work counter (zero on entry, and zero again once the launch has finished) and the
   // flag that makes CTAs starting after a wait gave up hand out no work.  Null: status words 2 (reset by the launch) and 0.
+  // counter[2] is a second counter, of the kernel for far tiles.
   int32_t* counter; int32_t* gave_up;
   void* workspace; size_t workspace_bytes;
+  // Long sequences on the tensor cores: scratch for the softmax state that the kernel for near key tiles hands to the one for
+  // far tiles, tdb_partial_floats() of fp32, part_ml behind part_o's tiles (null: one kernel does both).  split_sat is the launcher's own.
+  float* part_o; float* part_ml; int split_sat;
   int tiles_listed;                                       // packed form: the workspace already holds this batch's tile list
 };
 
@@ -60,6 +64,7 @@ int launch_relpos_expand(const void* table, const int16_t* idx, int idx_delta_ma
 int launch_bounded_wait_selftest(int32_t* status, int code, uint64_t limit_ns, cudaStream_t s);
 int launch_attn_simt(const AttnParams& p, int dtype, cudaStream_t s);
 int launch_attn_umma(const AttnParams& p, cudaStream_t s);
+bool has_far_tiles(const AttnParams& p);
 size_t umma_workspace_bytes(int n_seqs, int64_t total_tokens);
 int launch_relpos_expand_pair(const void* kr, const void* qr, const int16_t* idx, int idx_delta_max, int H, int two_span,
                               int exp_delta_max, int exp_rows, void* kr_out, void* qr_out, cudaStream_t s);
@@ -72,6 +77,9 @@ int static_tile_scratch(void** ptr);   // device address of the library's fixed 
 #define TDB_HOST_API __attribute__((visibility("default")))
 extern "C" {
 TDB_HOST_API int tdb_run_attn(const tdb::AttnParams* p, int dtype, int kernel, void* stream);
+// Floats of part_o and part_ml together that the call could use (0: none), for p as it will be passed to tdb_run_attn; part_ml
+// starts at 64 / 66 of them.
+TDB_HOST_API int64_t tdb_partial_floats(const tdb::AttnParams* p, int dtype, int kernel);
 TDB_HOST_API int tdb_expand_pair(const void* kr, const void* qr, const int16_t* idx, int idx_delta_max, int H, int two_span,
                                  int exp_delta_max, int exp_rows, void* kr_out, void* qr_out, void* stream);
 TDB_HOST_API int tdb_add_layernorm(const void* x, const void* res, const void* w, const void* b, float eps, int64_t rows, int hidden,
