@@ -15,13 +15,15 @@
 //
 // Bound: the special-function unit, 16384 exponentials per tile = 1024 clocks, beside 768 clocks of tensor work.  What matters
 // is that neither waits for the other: three score buffers go round the two groups, so a group's next scores are complete
-// before it has finished with the last ones, and only P.V follows its hand-off.  (With one buffer per group a pair of tiles
-// took 4300 clocks, of which 1400 were spent waiting for scores; in the one kernel for all tiles, with one accumulator and all
-// sixteen warps in step, a saturated tile took 3700.)
+// before it has finished with the last ones, and only P.V follows its hand-off; and the two kinds of product are issued by two
+// warps, because issuing blocks while the tensor pipe is busy and a lone issuing warp then adds its waits and commits (some
+// 100 clocks each) to every batch.  A pair of tiles takes 2500 clocks (4 x 4096 tokens: 242 us for the kernel).  With one
+// buffer per group and one issuing lane it took 4300, with three buffers and one issuing warp 3300; in the one kernel for all
+// tiles, with one accumulator and all sixteen warps in step, 7400.  A quarter of the exponentials as polynomials on the FMA
+// pipe, and tokens that let one group at a time take exponentials, were slower (254 us and 266 us).
 //
 // Half-step t is group t & 1 at its tile t / 2.  Tensor-memory columns: three buffers of 128, S(t) in buffer t % 3 and P(t) (bf16)
-// over the columns of S(t) that its own thread has read; O of the two groups at [384,448) [448,512).  The MMA lane runs
-// S(0) S(1) S(2) | PV(0) S(3) | PV(1) S(4) | ...: S(t + 3) goes into the buffer that PV(t) reads, right behind it in the pipe.
+// over the columns of S(t) that its own thread has read; O of the two groups at [384,448) [448,512).
 // All hand-offs are mbarriers with bounded waits; a wait that gives up sets the CTA's abort flag, after which every role runs
 // out its loops (the groups take their trip counts from one copy of the work item, so their named barriers still match), tensor
 // memory is freed and the host reports it.
@@ -34,7 +36,7 @@ using namespace ptx;
 namespace {
 
 constexpr int GW = 8, GT = GW * 32;                  // warps, threads of a group
-constexpr int F_THREADS = 2 * GT + 4 * 32;           // + Q and K warp, MMA warp, scheduler warp, V warp
+constexpr int F_THREADS = 2 * GT + 3 * 32;           // + a warp of single lanes (Q and K; V; scheduler), two MMA warps
 constexpr int F_RING = 3, STAGES = 2, BUFS = 3;
 constexpr uint32_t TILE = BQ * HD * 2;               // bytes of a 128 x 64 bf16 tile
 // Q buffer b: query tile A, query tile B, left row of Qr, right row of Qr
@@ -47,8 +49,8 @@ constexpr uint32_t F_TM_S = 0, F_TM_O = 384, F_TM_COLS = 512;
 constexpr uint64_t F_WAIT_NS = 1000ull * 1000ull * 1000ull;
 
 enum FBar { FQ_FULL = 0, FQ_EMPTY = 2, FK_FULL = 4, FK_EMPTY = 6, FV_FULL = 8, FV_EMPTY = 10, FS_FULL = 12 /* per buffer */,
-            FP_READY = 15 /* per group */, FPV_DONE = 17, FWORK_FULL = 19, FWORK_EMPTY = 22, FDONE = 25, F_NBARS };
-constexpr int F_READERS = 3 + 1;                     // K lane, V lane, MMA lane, the groups' leader
+            FP_READY = 15 /* per group */, FPV_DONE = 17, FWORK_FULL = 19, FWORK_EMPTY = 22, FDONE = 25 /* two */, FBUF_FREE = 27, F_NBARS = 30 };
+constexpr int F_READERS = 4 + 1;                     // K lane, V lane, two MMA warps, the groups' leader
 
 // A pair of query tiles of one head and its far key tiles: [0, n_left) and [right, right + n_far - n_left).
 struct FarWork {
@@ -98,10 +100,6 @@ __device__ __forceinline__ bool group_vote(int grp, bool flag) {
       : "=r"(r) : "r"((uint32_t)flag), "r"(1 + grp), "n"(GT) : "memory");
   return r != 0;
 }
-// The right to take exponentials, one token per scheduler (both groups have two warps on each): side by side the groups would
-// each get half of the special-function unit and then leave it idle together.
-__device__ __forceinline__ void token_wait(int grp, int qd) { asm volatile("bar.sync %0, 128;" ::"r"(3 + 4 * grp + qd) : "memory"); }
-__device__ __forceinline__ void token_pass(int grp, int qd) { asm volatile("bar.arrive %0, 128;" ::"r"(3 + 4 * (grp ^ 1) + qd) : "memory"); }
 __device__ __forceinline__ void groups_sync() { asm volatile("bar.sync 11, %0;" ::"n"(2 * GT) : "memory"); }
 __device__ __forceinline__ void group_sync(int grp) { asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "n"(GT) : "memory"); }
 
@@ -134,7 +132,7 @@ attn_far_kernel(const AttnParams p, int32_t* counter, const __grid_constant__ CU
   auto bar = [&](int i) { return bars + 8u * (uint32_t)i; };
   auto wait = [&](int i, uint32_t parity) { return mbar_wait(bar(i), parity, abort_flag, p.status, 201 + i, F_WAIT_NS); };
   int32_t gave_up_before = 0;
-  if (warp == 2 * GW + 2 && lane == 0) gave_up_before = *reinterpret_cast<volatile int32_t*>(p.gave_up);
+  if (warp == 2 * GW && lane == 2) gave_up_before = *reinterpret_cast<volatile int32_t*>(p.gave_up);
 
   if (tid == 0) {
     *abort_flag = 0;
@@ -168,7 +166,7 @@ attn_far_kernel(const AttnParams p, int32_t* counter, const __grid_constant__ CU
   auto release = [&](int n) { mbar_arrive(bar(FWORK_EMPTY + (n % F_RING))); };
 
   if (warp == 2 * GW) {
-    // ================================ TMA producers ==========================================
+    // ================================ TMA producers and scheduler ============================
     if (lane == 0) {                                 // per item both query tiles and both saturated rows, then K
       FarWork k;
       int g = 0, n = 0;
@@ -195,9 +193,7 @@ attn_far_kernel(const AttnParams p, int32_t* counter, const __grid_constant__ CU
         }
       }
       release(n);
-    }
-  } else if (warp == 2 * GW + 3) {
-    if (lane == 0) {                                 // V
+    } else if (lane == 1) {                          // V
       FarWork k;
       int g = 0, n = 0;
       for (; fetch(n, k); release(n), ++n)
@@ -210,12 +206,9 @@ attn_far_kernel(const AttnParams p, int32_t* counter, const __grid_constant__ CU
           }
         }
       release(n);
-    }
-  } else if (warp == 2 * GW + 2) {
-    // ================================ scheduler ==============================================
-    // Every CTA with an index of its own draws until its first draw past the end: as many draws as indices, and the counter
-    // wraps back to zero (see attn_umma.cu).
-    if (lane == 0) {
+    } else if (lane == 2) {
+      // Scheduler.  Every CTA with an index of its own draws until its first draw past the end: as many draws as indices, and
+      // the counter wraps back to zero (see attn_umma.cu).
       const unsigned int last_item = (unsigned int)(total_tiles * p.H - 1);
       int n = 0;
       bool first = true;
@@ -234,9 +227,9 @@ attn_far_kernel(const AttnParams p, int32_t* counter, const __grid_constant__ CU
         if (k.n_far < 0) break;
       }
     }
-  } else if (warp == 2 * GW + 1) {
+  } else if (warp >= 2 * GW + 1) {
     // ================================ MMA issuer ============================================
-    // The whole warp walks the loop and one elected lane issues: 6 % of the kernel's time against a single-lane branch.
+    // First warp: scores; second: P.V.  The whole warp walks its loop and one elected lane issues.
     constexpr uint32_t ID_S = make_idesc_bf16(128, BK, 0), ID_PV = make_idesc_bf16(128, HD, 1);
     const uint64_t dQ = smem_desc_sw128(sbase + F_OFF_Q), dK = smem_desc_sw128(sbase + F_OFF_K), dV = smem_desc_sw128(sbase + F_OFF_V);
     constexpr uint64_t STEP = TILE >> 4;
@@ -249,66 +242,67 @@ attn_far_kernel(const AttnParams p, int32_t* counter, const __grid_constant__ CU
       c.n_far = __shfl_sync(0xffffffffu, k.n_far, 0);
       c.n_left = __shfl_sync(0xffffffffu, k.n_left, 0);
     };
-    Cur cs{0, 0, 0, 0}, cv;                            // scores, three half-steps ahead of P.V
-    load_item(cs);
-    cv = cs;
-    int ts = 0;
-    auto issue_s = [&]() {
-      if (cs.n_far <= 0) return;
-      const int grp = ts & 1, g = ts >> 1, buf = ts % BUFS;
-      if (grp == 0) {
-        if (cs.it == 0) wait(FQ_FULL + (cs.n & 1), (uint32_t)((cs.n >> 1) & 1));
-        wait(FK_FULL + (g % STAGES), (uint32_t)((g / STAGES) & 1));
+    Cur c{0, 0, 0, 0};
+    load_item(c);
+    if (warp == 2 * GW + 1) {
+#pragma unroll 1
+      for (int t = 0; c.n_far > 0; ++t) {
+        const int grp = t & 1, g = t >> 1, buf = t % BUFS;
+        if (grp == 0) {
+          if (c.it == 0) wait(FQ_FULL + (c.n & 1), (uint32_t)((c.n >> 1) & 1));
+          wait(FK_FULL + (g % STAGES), (uint32_t)((g / STAGES) & 1));
+        }
+        if (t >= BUFS) wait(FBUF_FREE + buf, (uint32_t)((t / BUFS - 1) & 1));
         tc_fence_after();
-      }
-      const uint32_t tS = tm + F_TM_S + 128u * (uint32_t)buf;
-      const uint64_t q = dQ + (uint64_t)((cs.n & 1) * 4) * STEP, kd = dK + (uint64_t)(g % STAGES) * STEP;
+        const uint32_t tS = tm + F_TM_S + 128u * (uint32_t)buf;
+        const uint64_t q = dQ + (uint64_t)((c.n & 1) * 4) * STEP, kd = dK + (uint64_t)(g % STAGES) * STEP;
 #pragma unroll
-      for (int i = 0; i < HD / 16; ++i) mma_ss_warp(tS, q + (uint64_t)grp * STEP + 2 * i, kd + 2 * i, ID_S, i > 0);
-      if (P2C) {
-        const uint64_t r = q + (cs.it < cs.n_left ? 2 : 3) * STEP;
+        for (int i = 0; i < HD / 16; ++i) mma_ss_warp(tS, q + (uint64_t)grp * STEP + 2 * i, kd + 2 * i, ID_S, i > 0);
+        if (P2C) {
+          const uint64_t r = q + (c.it < c.n_left ? 2 : 3) * STEP;
 #pragma unroll
-        for (int i = 0; i < HD / 16; ++i) mma_ss_warp(tS, r + 2 * i, kd + 2 * i, ID_S, 1u);
-      }
-      tc_commit_warp(bar(FS_FULL + buf));
-      ++ts;
-      if (grp == 1) {
-        tc_commit_warp(bar(FK_EMPTY + (g % STAGES)));
-        if (++cs.it == cs.n_far) {
-          tc_commit_warp(bar(FQ_EMPTY + (cs.n & 1)));
-          ++cs.n; cs.it = 0;
-          load_item(cs);
+          for (int i = 0; i < HD / 16; ++i) mma_ss_warp(tS, r + 2 * i, kd + 2 * i, ID_S, 1u);
+        }
+        tc_commit_warp(bar(FS_FULL + buf));
+        if (grp == 1) {
+          tc_commit_warp(bar(FK_EMPTY + (g % STAGES)));
+          if (++c.it == c.n_far) {
+            tc_commit_warp(bar(FQ_EMPTY + (c.n & 1)));
+            if (lane == 0) release(c.n);
+            ++c.n; c.it = 0;
+            load_item(c);
+          }
         }
       }
-    };
+    } else {
 #pragma unroll 1
-    for (int i = 0; i < BUFS; ++i) issue_s();
-#pragma unroll 1
-    for (int t = 0; cv.n_far > 0; ++t) {
-      const int grp = t & 1, g = t >> 1;
-      if (grp == 0) wait(FV_FULL + (g % STAGES), (uint32_t)((g / STAGES) & 1));
-      wait(FP_READY + grp, (uint32_t)(g & 1));
-      tc_fence_after();
-      const uint64_t vd = dV + (uint64_t)(g % STAGES) * STEP;
-      const uint32_t tP = tm + F_TM_S + 128u * (uint32_t)(t % BUFS), tO = tm + F_TM_O + 64u * (uint32_t)grp;
+      for (int t = 0; c.n_far > 0; ++t) {
+        const int grp = t & 1, g = t >> 1, buf = t % BUFS;
+        if (grp == 0) wait(FV_FULL + (g % STAGES), (uint32_t)((g / STAGES) & 1));
+        wait(FP_READY + grp, (uint32_t)(g & 1));
+        tc_fence_after();
+        const uint64_t vd = dV + (uint64_t)(g % STAGES) * STEP;
+        const uint32_t tP = tm + F_TM_S + 128u * (uint32_t)buf, tO = tm + F_TM_O + 64u * (uint32_t)grp;
 #pragma unroll
-      for (int i = 0; i < BK / 16; ++i)                // keys 64.. of P lie over columns 64.. of the scores
-        mma_ts_warp(tO, tP + 8u * (uint32_t)(i & 3) + 64u * (uint32_t)(i >> 2), vd + (uint64_t)(128 * i), ID_PV, (cv.it > 0 || i > 0) ? 1u : 0u);
-      tc_commit_warp(bar(FPV_DONE + grp));
-      if (grp == 1) {
-        tc_commit_warp(bar(FV_EMPTY + (g % STAGES)));
-        if (++cv.it == cv.n_far) {
-          if (lane == 0) release(cv.n);
-          ++cv.n; cv.it = 0;
-          load_item(cv);
+        for (int i = 0; i < BK / 16; ++i)                // keys 64.. of P lie over columns 64.. of the scores
+          mma_ts_warp(tO, tP + 8u * (uint32_t)(i & 3) + 64u * (uint32_t)(i >> 2), vd + (uint64_t)(128 * i), ID_PV, (c.it > 0 || i > 0) ? 1u : 0u);
+        tc_commit_warp(bar(FBUF_FREE + buf));
+        tc_commit_warp(bar(FPV_DONE + grp));
+        if (grp == 1) {
+          tc_commit_warp(bar(FV_EMPTY + (g % STAGES)));
+          if (++c.it == c.n_far) {
+            if (lane == 0) release(c.n);
+            ++c.n; c.it = 0;
+            load_item(c);
+          }
         }
       }
-      issue_s();
     }
-    if (lane == 0) release(cv.n);                      // the end-of-stream marker
-    tc_commit_warp(bar(FDONE));
+    if (lane == 0) release(c.n);                       // the end-of-stream marker
+    const int done = FDONE + (warp - 2 * GW - 1);
+    tc_commit_warp(bar(done));
     int never = 0;                                     // this wait runs even after an abort, with its own limit
-    mbar_wait(bar(FDONE), 0, &never, p.status, 201 + FDONE, F_WAIT_NS);
+    mbar_wait(bar(done), 0, &never, p.status, 201 + FDONE, F_WAIT_NS);
   } else {
     // ================================ softmax groups ========================================
     const int grp = warp / GW, gw = warp % GW, gt = tid - grp * GT;
@@ -332,7 +326,6 @@ attn_far_kernel(const AttnParams p, int32_t* counter, const __grid_constant__ CU
     };
     if (tid == 0) publish(0);
     groups_sync();
-    if (grp == 1) token_pass(1, qd);                 // group A goes first
     int g = 0;
     for (int n = 0;; ++n) {
       const FarWork* const item = items + (n & 3);
@@ -376,28 +369,27 @@ attn_far_kernel(const AttnParams p, int32_t* counter, const __grid_constant__ CU
         wait(FS_FULL + buf, (uint32_t)((t / BUFS) & 1));
         tc_fence_after();
         if (it == 0 && tid == 0) publish(n + 1);
-        token_wait(grp, qd);
-        // P of the thread's 64 keys, sixteen at a time: the next sixteen scores are on their way from tensor memory while the
-        // exponentials (against the row's reference exponent) of these are taken.  P goes over scores that have been read.
+        // P of the thread's 64 keys: all scores first, so that nothing but the special-function unit paces the exponentials
+        // (against the row's reference exponent); P goes over scores that have been read, sixteen keys at a time.
         float sum;
         {
-          float s[2][16];
+          float x[64];
           const float bias = c - m;
           float s0 = 0.f, s1 = 0.f;
-          tmem_ld16(tS, reinterpret_cast<uint32_t*>(s[0]));
+          tmem_ld32(tS, reinterpret_cast<uint32_t*>(x));
+          tmem_ld32(tS + 32u, reinterpret_cast<uint32_t*>(x + 32));
+          tmem_ld_wait32(reinterpret_cast<uint32_t*>(x));
+          tmem_ld_wait32(reinterpret_cast<uint32_t*>(x + 32));
+          if (nvalid < 64) {
+#pragma unroll
+            for (int e = 0; e < 64; ++e) x[e] = e < nvalid ? x[e] : -CUDART_INF_F;
+          }
 #pragma unroll
           for (int part = 0; part < 4; ++part) {
-            float* x = s[part & 1];
-            tmem_ld_wait16(reinterpret_cast<uint32_t*>(x));
-            if (part < 3) tmem_ld16(tS + 16u * (uint32_t)(part + 1), reinterpret_cast<uint32_t*>(s[(part + 1) & 1]));
-            if (nvalid < 64) {
-#pragma unroll
-              for (int e = 0; e < 16; ++e) x[e] = 16 * part + e < nvalid ? x[e] : -CUDART_INF_F;
-            }
             uint32_t pk[8];
 #pragma unroll
             for (int e = 0; e < 16; e += 2) {
-              const float a = ex2(fmaf(x[e], sl2, bias)), b = ex2(fmaf(x[e + 1], sl2, bias));
+              const float a = ex2(fmaf(x[16 * part + e], sl2, bias)), b = ex2(fmaf(x[16 * part + e + 1], sl2, bias));
               s0 += a; s1 += b;
               pk[e / 2] = pack_bf16x2(a, b);
             }
@@ -405,7 +397,6 @@ attn_far_kernel(const AttnParams p, int32_t* counter, const __grid_constant__ CU
           }
           sum = s0 + s1;
         }
-        token_pass(grp, qd);
         if (g > 0) wait(FPV_DONE + grp, (uint32_t)((g - 1) & 1));    // done long ago; keeps the barrier's phases in step
         // A bf16 probability and an fp32 sum have room for 2^64 times the near tiles' exponent; a row beyond that (or the
         // overflow it led to) moves its exponent, and with it this tile's P and the output so far.  Its scores are gone, so
@@ -506,7 +497,6 @@ attn_far_kernel(const AttnParams p, int32_t* counter, const __grid_constant__ CU
       }
       group_sync(grp);                               // the exchange words are free again
     }
-    if (grp == 0) token_wait(0, qd);                 // group B's last pass
   }
 
   // ---- teardown ------------------------------------------------------------------------------
