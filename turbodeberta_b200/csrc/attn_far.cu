@@ -41,7 +41,7 @@ constexpr int F_RING = 3, STAGES = 2, BUFS = 3;
 constexpr uint32_t TILE = BQ * HD * 2;               // bytes of a 128 x 64 bf16 tile
 // Q buffer b: query tile A, query tile B, left row of Qr, right row of Qr
 constexpr uint32_t F_OFF_Q = 0, F_OFF_K = 2 * 4 * TILE, F_OFF_V = F_OFF_K + STAGES * TILE, F_OFF_BAR = F_OFF_V + STAGES * TILE;
-constexpr uint32_t F_OFF_WORK = F_OFF_BAR + 256, F_OFF_ITEM = F_OFF_WORK + F_RING * 64, F_OFF_X = F_OFF_ITEM + 4 * 64;
+constexpr uint32_t F_OFF_WORK = F_OFF_BAR + 256, F_OFF_ITEM = F_OFF_WORK + F_RING * 64, F_OFF_X = F_OFF_ITEM + 8 * 64;
 constexpr uint32_t F_OFF_FLAG = F_OFF_X + 2 * 2 * BQ * 4;    // exchange: [group][half][row]
 constexpr uint32_t F_SMEM = F_OFF_FLAG + 64 + 1024;
 static_assert(F_SMEM <= 227 * 1024, "shared memory budget");
@@ -312,8 +312,9 @@ attn_far_kernel(const AttnParams p, int32_t* counter, const __grid_constant__ CU
     const uint32_t tO = tmem + lane_base + F_TM_O + 64u * (uint32_t)grp + 32u * (uint32_t)half;
     const uint32_t x_row = sbase + F_OFF_X + 4u * (uint32_t)(grp * 2 * BQ + row_t);             // + half * BQ * 4
     const float sl2 = p.sm_scale * 1.4426950408889634f;
-    // All threads take their trip counts from one copy of the items, which thread 0 keeps one item ahead of the stream: it is
-    // written before thread 0 passes its token in an item's first tile, and read after that tile's vote at the earliest.
+    // Thread 0 takes the items from the ring one ahead of the stream (in an item's first tile it fetches the next); each
+    // group's leader copies an item for its group before the barrier that ends the item before, so that all threads of a group
+    // have the same trip count, also after an abort.
     FarWork* const items = reinterpret_cast<FarWork*>(gbase + F_OFF_ITEM);
     auto publish = [&](int n) {
       FarWork k;
@@ -324,11 +325,14 @@ attn_far_kernel(const AttnParams p, int32_t* counter, const __grid_constant__ CU
       }
       items[n & 3] = k;
     };
+    FarWork* const mine = items + 4 + 2 * grp;
     if (tid == 0) publish(0);
     groups_sync();
+    if (gt == 0) mine[0] = items[0];
+    group_sync(grp);
     int g = 0;
     for (int n = 0;; ++n) {
-      const FarWork* const item = items + (n & 3);
+      const FarWork* const item = mine + (n & 1);
       const int n_far = item->n_far, n_left = item->n_left, right = item->right, len = item->len, h = item->h;
       const int row = item->q0 + BQ * grp + row_t;
       if (n_far <= 0) break;
@@ -495,6 +499,7 @@ attn_far_kernel(const AttnParams p, int32_t* counter, const __grid_constant__ CU
         if (p.lse && half == 0)
           p.lse[(int64_t)item->bcoord * p.lse_sb + (int64_t)h * p.lse_sh + tok] = valid ? m * 0.6931471805599453f + logf(l_tot) : 0.f;
       }
+      if (gt == 0) mine[(n + 1) & 1] = items[(n + 1) & 3];
       group_sync(grp);                               // the exchange words are free again
     }
   }
