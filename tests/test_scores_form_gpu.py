@@ -84,3 +84,27 @@ def test_scores_form_argument_errors():
         flash_attention_with_disentangled(qh, kh, vh, pos_key, None, False, None, 16, 64)
     with pytest.raises(ValueError):                   # the mirrored index exists for score tensors only
         flash_attention_with_disentangled(qh, kh, vh, tables.kr, tables.qr, False, None, 32, 64, p2c_mirrored=True)
+
+
+@pytest.mark.parametrize("lengths,L", [([1], 1), ([64, 63], 64), ([65, 0, 128], 129), ([300, 17], 300)])
+@pytest.mark.parametrize("terms,mirrored", [("both", False), ("c2p", False), ("p2c", True)])
+def test_bf16_scores_kernel_at_tile_edges(lengths, L, terms, mirrored):
+    """The tensor-core kernel for materialised scores around its 64-row tiles, padded rows holding NaN, against the f32
+    kernel on the same bf16 values."""
+    from turbodeberta_b200.ops.flash_attention import flash_attention_with_disentangled
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    B = len(lengths)
+    q, k, v = (torch.randn(B, 2, L, 64, generator=gen, device="cuda").bfloat16() for _ in range(3))
+    pos = [torch.randn(B, 2, L, 128, generator=gen, device="cuda").bfloat16() if terms in ("both", n) else None for n in ("c2p", "p2c")]
+    lens = torch.tensor(lengths, dtype=torch.int32, device="cuda")
+    for b, n in enumerate(lengths):
+        for t in (k, v, *[x for x in pos if x is not None]):
+            t[b, :, n:] = float("nan")
+    run = lambda dt: flash_attention_with_disentangled(
+        *(t.to(dt) for t in (q, k, v)), *(None if t is None else t.to(dt) for t in pos), False, 0.0722, 64, 128, seqlens=lens,
+        p2c_mirrored=mirrored, return_lse=True)
+    (o, lse), (o2, lse2) = run(torch.bfloat16), run(torch.float32)
+    assert (o.float() - o2).abs().max().item() < 1e-2
+    for b, n in enumerate(lengths):
+        assert torch.count_nonzero(o[b, :, n:]).item() == 0
+        assert n == 0 or (lse[b, :, :n] - lse2[b, :, :n]).abs().max().item() < 1e-3

@@ -1,0 +1,209 @@
+// Attention with materialised position scores (the legacy operator form), bf16: the two position products arrive as tensors
+// c2p_scores[q, r] = Q[q].Kr[r] and p2c_scores[k, r] = K[k].Qr[r] and are gathered,
+//
+//   score[q,k] = (Q[q].K[k] + c2p_scores[q, idx(q-k)] + p2c_scores[k, idx(q-k)]) * sm_scale
+//
+// (p2c at idx(k-q) with TDB_FLAG_P2C_MIRRORED).  Bound by the score tensors: 8 x 256 tokens of 12 heads bring 50 MB of them,
+// against 1.6 GFLOP; so the products run on the warp-level tensor instruction, whose fragment layout is what the gather wants:
+// a fragment register's 32 lanes are 8 rows x 4 pairs of keys, i.e. 8 short runs of a c2p row and 4 of a p2c row, where one
+// row per lane (the layout tensor memory would give) touches 32 lines per load.  One block of four warps owns 64 query rows and
+// walks key tiles of 64, K and V double-buffered by asynchronous copies.  P keeps two bf16 terms (value and remainder) for
+// P.V, so nothing but the output is rounded to bf16.
+// 8 x 256 tokens, 12 heads: 46 us per call, 1.4 TB/s of scores (CUDA-core kernel: 142 us).
+#include "attn_blocks.cuh"
+#include <math_constants.h>
+
+namespace tdb {
+
+namespace {
+
+constexpr int ST = 64, SP = 72, S_THREADS = 128;     // tile rows, row pitch in elements (144 bytes: conflict-free ldmatrix)
+
+__device__ __forceinline__ uint32_t saddr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+// 64 rows of 64 bf16; rows at or beyond `rows` become zeros (the caller's padding may hold anything).
+__device__ __forceinline__ void stage(__nv_bfloat16* dst, const __nv_bfloat16* src, int64_t pitch, int rows) {
+#pragma unroll
+  for (int i = 0; i < ST * 8 / S_THREADS; ++i) {
+    const int e = threadIdx.x + i * S_THREADS, row = e >> 3, c = e & 7;
+    const bool real = row < rows;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(saddr(dst + row * SP + c * 8)),
+                 "l"(src + (real ? (int64_t)row * pitch + c * 8 : 0)), "r"(real ? 16 : 0) : "memory");
+  }
+}
+__device__ __forceinline__ void ldsm4(uint32_t* r, const __nv_bfloat16* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(saddr(p)) : "memory");
+}
+__device__ __forceinline__ void ldsm4t(uint32_t* r, const __nv_bfloat16* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(saddr(p)) : "memory");
+}
+__device__ __forceinline__ void mma(float* d, const uint32_t* a, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
+  const __nv_bfloat162 t = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&t);
+}
+__device__ __forceinline__ float bf(unsigned short h) { return __uint_as_float((uint32_t)h << 16); }
+
+template <bool C2P, bool P2C>
+__global__ void __launch_bounds__(S_THREADS, 3) attn_scores_kernel(const AttnParams p) {
+  __shared__ __align__(16) __nv_bfloat16 sQ[ST * SP], sK[2][ST * SP], sV[2][ST * SP];
+  __shared__ int16_t sIdx[2][2 * ST];                // table row of distance q0 - k0 - 63 + x, and of its negative
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int s = longest_first(p, blockIdx.z), h = blockIdx.y, q0 = blockIdx.x * ST;
+  int len, rows;
+  int64_t tok0;
+  int b;
+  if (!sequence_of(p, s, len, rows, tok0, b) || q0 >= rows) return;
+  __nv_bfloat16* const ob = reinterpret_cast<__nv_bfloat16*>(p.o) + b * p.o_sb + tok0 * p.o_st + h * p.o_sh;
+  float* const lse = p.lse ? p.lse + b * p.lse_sb + h * p.lse_sh + tok0 : nullptr;
+  using bf16 = __nv_bfloat16;
+  const bf16* const qb = reinterpret_cast<const bf16*>(p.q) + b * p.q_sb + tok0 * p.q_st + h * p.q_sh;
+  const bf16* const kb = reinterpret_cast<const bf16*>(p.k) + b * p.k_sb + tok0 * p.k_st + h * p.k_sh;
+  const bf16* const vb = reinterpret_cast<const bf16*>(p.v) + b * p.v_sb + tok0 * p.v_st + h * p.v_sh;
+  const unsigned short* const c2p = C2P ? reinterpret_cast<const unsigned short*>(p.c2p_scores) + b * p.c2p_sb + tok0 * p.c2p_st + h * p.c2p_sh : nullptr;
+  const unsigned short* const p2c = P2C ? reinterpret_cast<const unsigned short*>(p.p2c_scores) + b * p.p2c_sb + tok0 * p.p2c_st + h * p.p2c_sh : nullptr;
+  const int dm = p.idx_delta_max;
+  auto row_of = [&](int delta) { return p.idx[delta < -dm ? 0 : (delta > dm ? 2 * dm : delta + dm)]; };
+
+  // this thread's rows r0 and r0 + 8 of the block, its keys 2 (lane % 4) + {0, 1} of every group of eight
+  const int r0 = warp * 16 + lane / 4, kc = 2 * (lane % 4);
+  float o[8][4], m[2] = {-CUDART_INF_F, -CUDART_INF_F}, l[2] = {0.f, 0.f};
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) o[i][e] = 0.f;
+  const float sl2 = p.sm_scale * 1.4426950408889634f;
+
+  if (q0 < len) {
+    stage(sQ, qb + (int64_t)q0 * p.q_st, p.q_st, len - q0);
+    auto load_tile = [&](int k0, int buf) {
+      stage(sK[buf], kb + (int64_t)k0 * p.k_st, p.k_st, len - k0);
+      stage(sV[buf], vb + (int64_t)k0 * p.v_st, p.v_st, len - k0);
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      const int delta = q0 - k0 - (ST - 1) + (int)threadIdx.x;
+      if (C2P || P2C) sIdx[buf][threadIdx.x] = row_of(delta);
+    };
+    load_tile(0, 0);
+    uint32_t qf[4][4];
+    // rows beyond the sequence read the last row's scores: in bounds, and their results are dropped
+    const int qr[2] = {min(q0 + r0, len - 1), min(q0 + r0 + 8, len - 1)};
+    for (int k0 = 0, buf = 0; k0 < len; k0 += ST, buf ^= 1) {
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      __syncthreads();
+      if (k0 + ST < len) load_tile(k0 + ST, buf ^ 1);
+      if (k0 == 0) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) ldsm4(qf[i], sQ + (warp * 16 + (lane & 15)) * SP + 16 * i + 8 * (lane >> 4));
+      }
+      float sc[8][4];
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        // gathers first: 32 loads in flight behind the products
+        unsigned short gc[4][4], gp[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int kl = 8 * (4 * half + i) + kc + (e & 1), rl = r0 + 8 * (e >> 1);
+            const int x = rl - kl + ST - 1;
+            const int r = sIdx[buf][x];
+            if (C2P) gc[i][e] = __ldg(c2p + (int64_t)qr[e >> 1] * p.c2p_st + r);
+            if (P2C) {
+              const int rm = (p.flags & TDB_FLAG_P2C_MIRRORED) ? row_of(k0 + kl - q0 - rl) : r;
+              gp[i][e] = __ldg(p2c + (int64_t)min(k0 + kl, len - 1) * p.p2c_st + rm);
+            }
+          }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) sc[4 * half + i][e] = 0.f;
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            uint32_t kf[4];                          // keys 8j..8j+15, columns 16kk..+15
+            const int j = 4 * half + 2 * i;
+            ldsm4(kf, sK[buf] + (8 * j + (lane & 7) + 8 * (lane >> 4)) * SP + 16 * kk + 8 * ((lane >> 3) & 1));
+            mma(sc[j], qf[kk], kf[0], kf[1]);
+            mma(sc[j + 1], qf[kk], kf[2], kf[3]);
+          }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            float x = sc[4 * half + i][e];
+            if (C2P) x += bf(gc[i][e]);
+            if (P2C) x += bf(gp[i][e]);
+            sc[4 * half + i][e] = k0 + 8 * (4 * half + i) + kc + (e & 1) < len ? x * sl2 : -CUDART_INF_F;
+          }
+      }
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        float mx = m[r];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) mx = fmaxf(mx, fmaxf(sc[i][2 * r], sc[i][2 * r + 1]));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));     // finite: every key tile has a valid key
+        const float corr = exp2f(m[r] - mx);
+        m[r] = mx;
+        float sum = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+          for (int e = 2 * r; e < 2 * r + 2; ++e) { sc[i][e] = exp2f(sc[i][e] - mx); sum += sc[i][e]; }
+        l[r] = l[r] * corr + sum;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) { o[i][2 * r] *= corr; o[i][2 * r + 1] *= corr; }
+      }
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk) {               // keys 16kk..+15
+        const float *a = sc[2 * kk], *c = sc[2 * kk + 1];
+        uint32_t hi[4] = {pack2(a[0], a[1]), pack2(a[2], a[3]), pack2(c[0], c[1]), pack2(c[2], c[3])}, lo[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float* v = (e < 2 ? a : c) + 2 * (e & 1);
+          lo[e] = pack2(v[0] - __uint_as_float(hi[e] << 16), v[1] - __uint_as_float(hi[e] & 0xffff0000u));
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          uint32_t vf[4];                            // keys 16kk..+15, columns 16i..+15
+          ldsm4t(vf, sV[buf] + (16 * kk + (lane & 15)) * SP + 16 * i + 8 * (lane >> 4));
+          mma(o[2 * i], hi, vf[0], vf[1]);
+          mma(o[2 * i + 1], hi, vf[2], vf[3]);
+          mma(o[2 * i], lo, vf[0], vf[1]);
+          mma(o[2 * i + 1], lo, vf[2], vf[3]);
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const int row = q0 + r0 + 8 * r;
+    float sum = l[r];
+    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+    if (row >= rows) continue;
+    const bool valid = row < len;                    // padded query rows of the padded form: zeros
+    const float inv = valid ? 1.f / sum : 0.f;
+    uint32_t* const dst = reinterpret_cast<uint32_t*>(ob + (int64_t)row * p.o_st + kc);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) dst[4 * i] = valid ? pack2(o[i][2 * r] * inv, o[i][2 * r + 1] * inv) : 0u;
+    if (lse && lane % 4 == 0) lse[row] = valid ? m[r] * 0.6931471805599453f + logf(sum) : 0.f;
+  }
+}
+
+}  // namespace
+
+int launch_attn_scores(const AttnParams& p, cudaStream_t s) {
+  dim3 grid((p.L + ST - 1) / ST, p.H, p.n_seqs);
+  const bool c2p = p.flags & TDB_FLAG_C2P, p2c = p.flags & TDB_FLAG_P2C;
+  if (c2p && p2c) attn_scores_kernel<true, true><<<grid, S_THREADS, 0, s>>>(p);
+  else if (c2p) attn_scores_kernel<true, false><<<grid, S_THREADS, 0, s>>>(p);
+  else attn_scores_kernel<false, true><<<grid, S_THREADS, 0, s>>>(p);
+  return cuda_fail(cudaGetLastError(), "attn_scores launch");
+}
+
+}  // namespace tdb

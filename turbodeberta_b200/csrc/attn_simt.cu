@@ -1,7 +1,7 @@
 // CUDA-core disentangled attention: exact fp32 arithmetic on f32 or bf16 inputs.
 //
 // This is the full-precision path (fp32 inputs must land within 1e-4 of the eager module, which the bf16 tensor-core
-// pipeline cannot do), the path of materialised position scores, and the cross-check for the tensor-core kernel.
+// pipeline cannot do), the path of materialised position scores in f32, and the cross-check for the tensor-core kernel.
 //
 //   score[q,k] = (Q[q].K[k] + Q[q].Kr[r] + K[k].Qr[r]) * sm_scale,  r = idx[clamp(q-k)]
 //
@@ -17,7 +17,7 @@
 // each other's loads.  The rows of one query tile stay inside one warp, so the softmax needs shuffles only.
 // One call of 8 x (48..387) fp32 tokens with 12 heads and both terms: 245 us, 23 TFLOP/s (one warp per query row, keys spread
 // over its lanes, every operand read row by row through L1: 1852 us).
-#include "tdb_internal.h"
+#include "attn_blocks.cuh"
 #include <math_constants.h>
 
 namespace tdb {
@@ -73,23 +73,6 @@ __device__ __forceinline__ void store4(__nv_bfloat16* d, float a, float b, float
   *reinterpret_cast<uint2*>(d) = v;
 }
 
-// The sequence that block row z works on.  Blocks start in grid order, and those of a long sequence last longest: with the
-// sequences taken by decreasing length (up to 64 of them, one per thread) the last blocks to start are the cheapest.
-__device__ __forceinline__ int longest_first(const AttnParams& p, int z) {
-  __shared__ int lens[THREADS], mine;
-  if (p.n_seqs == 1 || p.n_seqs > THREADS || !(p.varlen || p.seqlens)) return z;
-  const int t = threadIdx.x;
-  int len = -1;
-  if (t < p.n_seqs) len = p.varlen ? p.cu_seqlens[t + 1] - p.cu_seqlens[t] : p.seqlens[t];
-  lens[t] = len;
-  __syncthreads();
-  int rank = 0;
-  for (int j = 0; j < p.n_seqs; ++j) rank += lens[j] > len || (lens[j] == len && j < t);
-  if (t < p.n_seqs && rank == z) mine = t;
-  __syncthreads();
-  return mine;
-}
-
 template <int R> constexpr int smem_floats(bool tables) {
   const int half = (KT + (tables ? 2 * (8 * R + KT) : 0)) * HP;
   const int values = KT * DP;
@@ -111,25 +94,10 @@ __global__ void __launch_bounds__(THREADS, 4) attn_simt_kernel(const AttnParams 
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int ti = warp * 4 + lane / 8, tj = lane % 8;
   const int s = longest_first(p, blockIdx.z), h = blockIdx.y, q0 = blockIdx.x * QT;
-  int len, rows;                 // valid length; rows that exist in the output
-  int64_t tok0; int b;
-  if (p.varlen) {
-    int c0 = p.cu_seqlens[s];
-    len = p.cu_seqlens[s + 1] - c0; rows = len; tok0 = c0; b = 0;
-    if (c0 < 0 || len < 0 || (int64_t)c0 + len > p.total_tokens) {   // malformed offsets: report, touch nothing
-      if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0) *reinterpret_cast<volatile int32_t*>(p.status + 1) = 1;
-      return;
-    }
-    // The grid covers max_seqlen rows per sequence: a longer sequence would leave rows unwritten, and offsets that
-    // do not end at the token count leave tokens outside every sequence.  Both are reported, not guessed around.
-    if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0 &&
-        (len > p.L || (s == p.n_seqs - 1 && (int64_t)c0 + len != p.total_tokens)))
-      *reinterpret_cast<volatile int32_t*>(p.status + 1) = 1;
-  } else {
-    len = p.seqlens ? p.seqlens[s] : p.L; rows = p.L; tok0 = 0; b = s;
-    len = len < 0 ? 0 : (len > p.L ? p.L : len);
-  }
-  if (q0 >= rows) return;
+  int len, rows;
+  int64_t tok0;
+  int b;
+  if (!sequence_of(p, s, len, rows, tok0, b) || q0 >= rows) return;
   T* const ob = reinterpret_cast<T*>(p.o) + b * p.o_sb + tok0 * p.o_st + h * p.o_sh;
   float* const lse = p.lse ? p.lse + b * p.lse_sb + h * p.lse_sh + tok0 : nullptr;
 
@@ -318,6 +286,7 @@ int launch_dtype(const AttnParams& p, cudaStream_t s) {
 int launch_attn_simt(const AttnParams& p, int dtype, cudaStream_t s) {
   if (p.n_seqs == 0 || p.L == 0) return TDB_OK;
   if (p.n_seqs > 65535 || p.H > 65535) { set_error("attn_simt: more than 65535 sequences or heads"); return TDB_ERR_SHAPE; }
+  if (dtype == TDB_DTYPE_BF16 && (p.c2p_scores || p.p2c_scores)) return launch_attn_scores(p, s);
   return dtype == TDB_DTYPE_F32 ? launch_dtype<float>(p, s) : launch_dtype<__nv_bfloat16>(p, s);
 }
 
