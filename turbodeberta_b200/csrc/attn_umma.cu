@@ -87,6 +87,11 @@ constexpr int PERM_MAX = 256;
 #define TDB_FCB 9
 #endif
 constexpr int FCB = TDB_FCB;                    // step of the exponential loop at which the fused c2p drain starts
+#ifndef TDB_FPB
+#define TDB_FPB 4
+#endif
+constexpr int FPB = TDB_FPB;                    // step of the c2p loop at which the fused p2c drain starts
+static_assert(FPB >= 0 && FPB + STG_COLS / GROUPS / 8 <= KPT / 2 - 1, "the fused drain's last step must lie inside the loop");
 static_assert(FCB >= 0 && FCB + STG_COLS / GROUPS / 8 <= KPT / 2 - 1, "the fused drain's last step must lie inside the loop");
 constexpr uint32_t SMEM_BYTES = OFF_PERM + PERM_MAX * 2 + 1024;   // + slack for the 1024-byte alignment of the base
 static_assert(OFF_STP % 16 == 0 && OFF_XCH % 16 == 0 && OFF_BAR % 16 == 0 && OFF_LX % 16 == 0, "offsets must stay 16-byte aligned");
@@ -822,7 +827,6 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap tm_q, c
         const uint32_t dc_dst = c_row + 2u * (uint32_t)((STG_COLS / GROUPS) * grp);
         const uint32_t dp_src = tmem + lane_base + TM_RING + (uint32_t)(96 - 32 * qd + (STG_COLS / GROUPS) * grp);
         const uint32_t dp_dst = p_row + 2u * (uint32_t)((STG_COLS / GROUPS) * grp);
-        if (fuse_p) drain_begin(dp_src);
         wait(S_FULL, (uint32_t)(g & 1));
         tc_fence_after();
         float s[KPT];
@@ -852,7 +856,8 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap tm_q, c
               asm("mov.b32 {%0, %1}, %2;" : "=h"(lo), "=h"(hi) : "r"(v));
               s[KPT - 1 - 2 * k] = add_bf16(s[KPT - 1 - 2 * k], lo);
               s[KPT - 2 - 2 * k] = add_bf16(s[KPT - 2 - 2 * k], hi);
-              if ((k & 1) && k / 2 < STG_COLS / GROUPS / 8 && fuse_p) drain_step(k / 2, dp_src, dp_dst);
+              if (fuse_p && k == FPB) drain_begin(dp_src);
+              if (fuse_p && k > FPB && k <= FPB + STG_COLS / GROUPS / 8) drain_step(k - FPB - 1, dp_src, dp_dst);
             }
           }
         }
