@@ -17,7 +17,7 @@
 // over their saturated ends, so both position terms become two more products into the score accumulator itself
 // (operands = 128-row boxes of identical rows): such tiles have no band, no drain and no gather.
 //
-// Warp roles (608 threads): warps 0-15 do the CUDA-core work; warp w owns tensor-memory lanes 32*(w%4)..+31
+// Warp roles (608 threads, 640 with SPLIT): warps 0-15 do the CUDA-core work; warp w owns tensor-memory lanes 32*(w%4)..+31
 // (query rows, or key rows of P2) and column group w/4, i.e. four threads share a query row and each handles 32
 // of the 128 keys, which puts four warps on every scheduler to hide latency.  Warp 16 = TMA producers (lane 0:
 // tables and K, lane 1: V, lane 2: Q), warp 17 = tensor-memory allocation + MMA issue (one lane), warp 18 =
@@ -71,7 +71,8 @@ constexpr int KPT = BK / GROUPS;                // keys per thread in the softma
 constexpr int OPT = HD / GROUPS;                // output columns per thread
 constexpr int NCW = 4 * GROUPS;                 // CUDA-core warps
 constexpr int NCT = NCW * 32;                   // CUDA-core threads
-constexpr int NTHREADS = (NCW + 3) * 32;       // + TMA producer warp, MMA warp, scheduler warp
+// + TMA producer warp, MMA warp, scheduler warp, and for long sequences a second MMA warp
+template <bool SPLIT> constexpr int threads_of = (NCW + 3 + (SPLIT ? 1 : 0)) * 32;
 constexpr int STG_STRIDE = 336;                 // bytes per staging row: 160 bf16 + 16 pad (odd multiple of 16)
 constexpr int STG_COLS = 160;
 constexpr uint32_t OFF_Q = 0 /* two buffers */, OFF_K = 32768, OFF_V = 49152, OFF_KR = 65536, OFF_QR = 98304;
@@ -106,7 +107,7 @@ enum Bar { Q_FULL = 0 /* Q_FULL + buffer */, Q_FULL1, Q_EMPTY /* Q_EMPTY + buffe
            WORK_EMPTY0, WORK_EMPTY1, WORK_EMPTY2, WORK_EMPTY3, NBARS };
 constexpr int WORK_RING = 3;                     // the item in progress and the two after it: what the roles look ahead, and
                                                 // no more (every item claimed early is taken from a CTA that may be free sooner)
-constexpr int WORK_READERS = 3 + 1 + 1;         // three producer lanes, the MMA lane, the CUDA-core warps' leader
+constexpr int WORK_READERS = 3 + 1 + 1;         // three producer lanes, the MMA lane (one more if there are two), the CUDA-core warps' leader
 static_assert(NBARS * 8 <= 256, "barrier block");
 
 struct TileListHeader { int32_t n_tiles; int32_t pad[3]; };
@@ -291,7 +292,7 @@ __device__ __forceinline__ int first_key(const AttnParams& p, int q0) { return S
 // LONG: sequences can be long enough for saturated tiles (compiled out otherwise, which keeps the common kernel lean).
 // SPLIT: they are, and the kernel for far tiles takes those.
 template <bool C2P, bool P2C, bool LONG, bool SPLIT>
-__global__ void __launch_bounds__(NTHREADS, 1)
+__global__ void __launch_bounds__(threads_of<SPLIT>, 1)
 attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                  const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_kr,
                  const __grid_constant__ CUtensorMap tm_qr, const __grid_constant__ CUtensorMap tm_kr16,
@@ -325,7 +326,9 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap tm_q, c
     for (int i = 0; i < NBARS; ++i) {
       const bool by_warps = (i == S_TAKEN || i == BAND_FREE || i == P_READY);
       const bool by_readers = (i >= WORK_EMPTY0 && i <= WORK_EMPTY3);
-      mbar_init(bar(i), by_readers ? (uint32_t)WORK_READERS : (by_warps ? (uint32_t)NCW : 1u));
+      // what both MMA lanes read is free when both have said so
+      const bool by_lanes = SPLIT && ((i == K_EMPTY && P2C) || ((i == Q_EMPTY || i == Q_EMPTY1) && C2P) || i == DONE);
+      mbar_init(bar(i), by_readers ? (uint32_t)(WORK_READERS + (SPLIT ? 1 : 0)) : by_warps ? (uint32_t)NCW : by_lanes ? 2u : 1u);
     }
     fence_mbar_init();
   }
@@ -495,7 +498,7 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap tm_q, c
       ++n;
       if (k.n_kv < 0) break;
     }
-  } else if (warp == NCW + 1) {
+  } else if (warp == NCW + 1 || (SPLIT && warp == NCW + 3)) {
     // ================================ MMA issuer ============================================
     if (lane == 0) {
       constexpr uint32_t ID_S = make_idesc_bf16(128, BK, 0);
@@ -541,6 +544,7 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap tm_q, c
         for (int k = 0; k < HD / 16; ++k) mma_ss(tBand, dQc + 2 * k, dKr + 2 * k, ID_BAND, k > 0);
         ring_filled();
         tc_commit(bar(KR_EMPTY));
+        if (SPLIT && c.it + 1 == c.n_kv) tc_commit(bar(Q_EMPTY + (c.n & 1)));
       };
       // content score of key tile g; the last one of an item releases the item's Q buffer
       auto issue_s = [&](const TileCur& c, int g) {
@@ -567,11 +571,13 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap tm_q, c
           }
         }
         tc_commit(bar(S_FULL));
+        if (SPLIT) tc_commit(bar(K_EMPTY));
         if (c.it + 1 == c.n_kv) tc_commit(bar(Q_EMPTY + (c.n & 1)));
       };
       // position->content band of key tile g (rows = keys), once the c2p band has been drained; releases K
       auto issue_p2 = [&](const TileCur& c, int g) {
         if (P2C && !(LONG && tile_saturated(p, c.q0, c.it * BK))) {
+          if (SPLIT) wait(K_FULL, (uint32_t)(g & 1));
           wait(QR_FULL, (uint32_t)(g & 1));
           wait_ring_free();
           tc_fence_after();
@@ -579,8 +585,9 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap tm_q, c
           for (int k = 0; k < HD / 16; ++k) mma_ss(tBand, dK + 2 * k, dQr + 2 * k, ID_BAND, k > 0);
           ring_filled();
           tc_commit(bar(QR_EMPTY));
+          if (SPLIT) tc_commit(bar(K_EMPTY));
         }
-        tc_commit(bar(K_EMPTY));
+        if (!SPLIT) tc_commit(bar(K_EMPTY));
       };
       // O += P . V of key tile g.  The first one of an item overwrites O: the CUDA warps read the previous item's O
       // before they announce the P of this tile, so P_READY covers that as well.
@@ -595,40 +602,78 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap tm_q, c
         tc_commit(bar(V_EMPTY));
       };
 
-      // Issue order, by rounds r = -1, 0, 1, ...:  S(r) P2(r) PV(r-1) C(r+1), i.e.
-      //   C(0) | S(0) P2(0) C(1) | S(1) P2(1) PV(0) C(2) | S(2) P2(2) PV(1) C(3) | ...
-      // While the CUDA warps work on tile g they enable, in this order: C(g+1) (the p2c band of tile g leaves the band
-      // buffer during the c2p phase), P2(g+1) (the c2p band of tile g+1 leaves it during the exponentials) and
-      // P.V(g); the lane waits idle at the two band products, which are the tile's critical chain, and fits S(g+1) -
-      // enabled long before - between them.  One loop with every product issued from a single place keeps the lane's
-      // code small (it runs once per tile and should not fall out of the instruction cache in between).
-      TileCur cc, cs, cv;                  // c2p stream (two tiles ahead), score/p2c stream (one ahead), P.V stream
-      cc.n = 0; cc.it = 0; cur_fetch(cc);
-      cs = cc; cv = cc;
-      int gc = 0, gs = 0, gv = 0;
-      if (cv.ok) {
+      int last = 0;                        // ring index of the end-of-stream marker
+      if constexpr (!SPLIT) {
+        // Issue order, by rounds r = -1, 0, 1, ...:  S(r) P2(r) PV(r-1) C(r+1), i.e.
+        //   C(0) | S(0) P2(0) C(1) | S(1) P2(1) PV(0) C(2) | S(2) P2(2) PV(1) C(3) | ...
+        // While the CUDA warps work on tile g they enable, in this order: C(g+1) (the p2c band of tile g leaves the band
+        // buffer during the c2p phase), P2(g+1) (the c2p band of tile g+1 leaves it during the exponentials) and
+        // P.V(g); the lane waits idle at the two band products, which are the tile's critical chain, and fits S(g+1) -
+        // enabled long before - between them.  One loop with every product issued from a single place keeps the lane's
+        // code small (it runs once per tile and should not fall out of the instruction cache in between).
+        TileCur cc, cs, cv;                  // c2p stream (two tiles ahead), score/p2c stream (one ahead), P.V stream
+        cc.n = 0; cc.it = 0; cur_fetch(cc);
+        cs = cc; cv = cc;
+        int gc = 0, gs = 0, gv = 0;
+        if (cv.ok) {
 #pragma unroll 1
-        for (int r = -1; ; ++r) {
-          if (r >= 0 && cs.ok) {
-            issue_s(cs, gs); issue_p2(cs, gs); ++gs;
-            cur_next(cs);
+          for (int r = -1; ; ++r) {
+            if (r >= 0 && cs.ok) {
+              issue_s(cs, gs); issue_p2(cs, gs); ++gs;
+              cur_next(cs);
+            }
+            if (r > 0) {
+              issue_pv(cv, gv++);
+              if (cv.it + 1 == cv.n_kv) release(cv.n);
+              cur_next(cv);
+              if (!cv.ok) break;
+            }
+            if (C2P && cc.ok) { issue_c(cc, gc++); cur_next(cc); }
           }
-          if (r > 0) {
+        }
+        last = cv.n;
+      } else {
+        // Long sequences, some nine key tiles per item: two lanes, since issuing blocks while the tensor pipe is busy and
+        // the scores then stand in the bands' way (4 x 4096 tokens: 227 -> 218 us).  With one to four tiles per item a second
+        // lane that follows the items costs more than that (32 x 64..512: 70 -> 73 us).
+        TileCur c;
+        c.n = 0; c.it = 0; cur_fetch(c);
+        int g = 0;
+        if (warp == NCW + 1) {
+          // bands: C(0) P2(0) C(1) P2(1) ..., each as soon as the one before has left the band buffer
+#pragma unroll 1
+          while ((C2P || P2C) && c.ok) {
+            if (C2P) issue_c(c, g);
+            issue_p2(c, g);
+            ++g;
+            if (c.it + 1 == c.n_kv) release(c.n);
+            cur_next(c);
+          }
+          if (!(C2P || P2C))
+            while (c.ok) { release(c.n); ++c.n; cur_fetch(c); }
+        } else {
+          // S(0) | S(1) PV(0) | S(2) PV(1) | ...
+          TileCur cv = c;
+          int gv = 0;
+          if (c.ok) { issue_s(c, g++); cur_next(c); }
+#pragma unroll 1
+          while (cv.ok) {
+            if (c.ok) { issue_s(c, g++); cur_next(c); }
             issue_pv(cv, gv++);
             if (cv.it + 1 == cv.n_kv) release(cv.n);
             cur_next(cv);
-            if (!cv.ok) break;
           }
-          if (C2P && cc.ok) { issue_c(cc, gc++); cur_next(cc); }
+          c = cv;
         }
+        last = c.n;
       }
-      release(cv.n);                       // the end-of-stream marker
+      release(last);
       // Everything issued above must have retired before tensor memory is released.
       tc_commit(bar(DONE));
       int never = 0;                       // this wait runs even after an abort, with its own limit
       mbar_wait(bar(DONE), 0, &never, p.status, 1 + DONE, WAIT_LIMIT_NS);
     }
-  } else {
+  } else if (warp < NCW) {
     // ================================ drain + softmax + epilogue ============================
     const int qd = warp & 3, grp = warp >> 2;
     const int row_t = qd * 32 + lane;                                  // tensor-memory lane = query row (or key row of P2)
@@ -1076,7 +1121,7 @@ int launch_variant(const AttnParams& p, dim3 grid, const CUtensorMap* maps, cuda
   auto kern = attn_umma_kernel<C2P, P2C, LONG, SPLIT>;
   const int rc = opt_in_smem(reinterpret_cast<const void*>(kern), (int)SMEM_BYTES);
   if (rc) return rc;
-  kern<<<grid, NTHREADS, SMEM_BYTES, s>>>(p, maps[0], maps[1], maps[2], maps[3], maps[4], maps[5], maps[6]);
+  kern<<<grid, threads_of<SPLIT>, SMEM_BYTES, s>>>(p, maps[0], maps[1], maps[2], maps[3], maps[4], maps[5], maps[6]);
   return cuda_fail(cudaGetLastError(), "attn_umma launch");
 }
 

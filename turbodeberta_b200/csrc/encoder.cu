@@ -54,6 +54,12 @@ __global__ void __launch_bounds__(128) add_layernorm_kernel(const T* __restrict_
   const uint4* rr = reinterpret_cast<const uint4*>(res + row * hidden);
   float f[NV][N];
   float sum = 0.f;
+  uint4 wv[NV], bv[NV];                              // all loads at once: for a few rows their latency is the kernel's time
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int c = lane + 32 * i;
+    if (c < nv) { wv[i] = __ldg(reinterpret_cast<const uint4*>(w) + c); bv[i] = __ldg(reinterpret_cast<const uint4*>(b) + c); }
+  }
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
     const int c = lane + 32 * i;
@@ -79,8 +85,8 @@ __global__ void __launch_bounds__(128) add_layernorm_kernel(const T* __restrict_
     const int c = lane + 32 * i;
     if (c < nv) {
       float g[N], a[N];
-      Vec<T>::unpack(__ldg(reinterpret_cast<const uint4*>(w) + c), g);
-      Vec<T>::unpack(__ldg(reinterpret_cast<const uint4*>(b) + c), a);
+      Vec<T>::unpack(wv[i], g);
+      Vec<T>::unpack(bv[i], a);
 #pragma unroll
       for (int e = 0; e < N; ++e) f[i][e] = fmaf((f[i][e] - mean) * inv, g[e], a[e]);
       reinterpret_cast<uint4*>(out + row * hidden)[c] = Vec<T>::pack(f[i]);

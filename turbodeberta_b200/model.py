@@ -379,9 +379,10 @@ class FlashDebertaV2Encoder(DebertaV2Encoder):
         return host.Watch([m for m in self.layer.modules()]), native, attns
 
     def _native_plan(self, hidden_states, rel_embeddings):
-        """The native encoder with every layer's derived tensors up to date, or None where it does not apply."""
+        """The native encoder with every layer's derived tensors up to date, or None where it does not apply.  Whether a
+        kept plan still matches the modules is for the caller to ask (``holds()`` of its first entry), once the GPU is busy."""
         plan = _PLANS.get(self)
-        if plan is None or not plan[0].holds():
+        if plan is None:
             made = self._native_layers()
             if made is None or not made[0].holds():
                 return None
@@ -424,6 +425,7 @@ class FlashDebertaV2Encoder(DebertaV2Encoder):
         native = self._native_plan(hidden_states, self.get_rel_embedding())
         if native is None:
             return None
+        watch = _PLANS[self][0]
         every = output_hidden_states and _WANTED.hidden_states
         if info.all_ones:
             outs, words = native.run(hidden_states.reshape(B * L, hid), None, L, every)
@@ -436,6 +438,11 @@ class FlashDebertaV2Encoder(DebertaV2Encoder):
             padded = keep + [host.unpack_rows(outs[-1], pos, B, L)]
         for w in words:
             _PENDING_STATUS.append(w)
+        # The look at some two hundred modules takes the host 90 us, so it runs behind the launches, beside the GPU; the
+        # result has no side effects and is simply dropped when somebody has changed the modules since the last forward.
+        if not watch.holds():
+            del _PLANS[self]
+            return self._forward_native(hidden_states, attention_mask, output_hidden_states, return_dict)
         all_hidden = None
         if output_hidden_states:
             all_hidden = (hidden_states, *padded) if every else (padded[-1],)
