@@ -364,3 +364,41 @@ def test_repeated_shapes_replay_a_recorded_graph(lengths, L):
         a = model(**kw).last_hidden_state
         assert torch.equal(a, fresh(kw))
     check_pending_status()
+
+
+def test_plans_do_not_keep_models_alive():
+    """A model that is dropped takes its native plan, recorded graphs and weights along."""
+    import gc
+    from turbodeberta_b200 import model as M
+    model = M.FlashDebertaV2Model(_cfg(num_hidden_layers=2)).eval().to("cuda", torch.bfloat16)
+    ids = torch.randint(1, 500, (2, 40), device="cuda")
+    gc.collect()
+    before = len(M._PLANS)
+    with torch.no_grad():
+        for _ in range(3):
+            model(input_ids=ids, attention_mask=torch.ones_like(ids))
+    assert len(M._PLANS) == before + 2                   # the model's and its encoder's
+    del model
+    gc.collect()
+    assert len(M._PLANS) == before
+
+
+def test_replaced_embeddings_and_hooks_on_them_are_seen():
+    from turbodeberta_b200.model import FlashDebertaV2Model
+    torch.manual_seed(15)
+    model = FlashDebertaV2Model(_cfg(num_hidden_layers=2)).eval().to("cuda", torch.bfloat16)
+    ids = torch.randint(1, 500, (2, 40), device="cuda")
+    mask = torch.ones_like(ids)
+    mask[1, 20:] = 0
+    with torch.no_grad():
+        a = model(input_ids=ids, attention_mask=mask).last_hidden_state
+        assert torch.equal(a, model(ids, mask).last_hidden_state)          # positional arguments: the HF model's own forward
+        assert torch.equal(a, model(input_ids=ids, attention_mask=mask, return_dict=False)[0])
+        called = []
+        handle = model.embeddings.LayerNorm.register_forward_hook(lambda *x: called.append(1))
+        assert torch.equal(a, model(input_ids=ids, attention_mask=mask).last_hidden_state) and called
+        handle.remove()
+        model.embeddings.word_embeddings = torch.nn.Embedding(500, 128).to("cuda", torch.bfloat16)
+        b = model(input_ids=ids, attention_mask=mask).last_hidden_state
+        assert not torch.equal(a, b)
+        assert torch.equal(b, model(ids, mask).last_hidden_state)

@@ -122,6 +122,7 @@ attn_far_kernel(const AttnParams p, int32_t* counter, const __grid_constant__ CU
                 const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_qr) {
   extern __shared__ uint8_t smem_raw[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  wait_for_stream();                                 // behind the near kernel, which lets nothing start early
   const int total_tiles = p.varlen ? reinterpret_cast<const int32_t*>(p.workspace)[0] : p.n_seqs * ((p.L + BQ - 1) / BQ);
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gbase = smem_raw + (sbase - smem_u32(smem_raw));

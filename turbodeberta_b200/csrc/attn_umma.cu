@@ -303,12 +303,6 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap tm_q, c
   // Persistent CTA.  Work items (query tile x head) are handed out by a device-wide counter (status word 2), so a
   // CTA that drew short sequences simply draws more of them; a scheduler lane publishes each item in a small
   // shared-memory ring that every role reads in the same order.
-  const int total_tiles = p.varlen ? reinterpret_cast<const int32_t*>(p.workspace)[0]
-                                   : p.n_seqs * ((p.L + BQ - 1) / BQ);
-  // An earlier CTA gave up: the scheduler lane (which reads the word while the CTA sets itself up) hands out no work.
-  int32_t status_at_start = 0;
-  if (warp == NCW + 2 && lane == 0) status_at_start = *reinterpret_cast<volatile int32_t*>(p.gave_up);
-
   // ---- shared memory carve-up ----------------------------------------------------------------
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gbase = smem_raw + (sbase - smem_u32(smem_raw));
@@ -347,7 +341,13 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap tm_q, c
   // while the other warps set the CTA up: it needs nothing but the lengths in global memory and its own corner of
   // shared memory.
   const uint16_t* perm = nullptr;
+  int total_tiles = 0;
+  int32_t status_at_start = 0;
   if (warp == NCW + 2) {
+    wait_for_stream();
+    total_tiles = p.varlen ? reinterpret_cast<const int32_t*>(p.workspace)[0] : p.n_seqs * ((p.L + BQ - 1) / BQ);
+    // An earlier CTA gave up: no work is handed out.
+    if (lane == 0) status_at_start = *reinterpret_cast<volatile int32_t*>(p.gave_up);
     const int qtiles = (p.L + BQ - 1) / BQ;
     if (!p.varlen && p.seqlens && p.n_seqs > 1 && p.n_seqs <= PERM_MAX && p.n_seqs * (qtiles + 1) <= 2048) {
       uint16_t* pw = reinterpret_cast<uint16_t*>(gbase + OFF_PERM);
@@ -374,6 +374,7 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap tm_q, c
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  wait_for_stream();                       // all of the above ran beside the end of the kernel in front
 
   // Item n of this CTA's stream; n_kv < 0 marks the end of the stream.  (Tiles that consist of padded query rows
   // only never enter the ring: the scheduler warp zeroes them itself.)
@@ -1121,8 +1122,8 @@ int launch_variant(const AttnParams& p, dim3 grid, const CUtensorMap* maps, cuda
   auto kern = attn_umma_kernel<C2P, P2C, LONG, SPLIT>;
   const int rc = opt_in_smem(reinterpret_cast<const void*>(kern), (int)SMEM_BYTES);
   if (rc) return rc;
-  kern<<<grid, threads_of<SPLIT>, SMEM_BYTES, s>>>(p, maps[0], maps[1], maps[2], maps[3], maps[4], maps[5], maps[6]);
-  return cuda_fail(cudaGetLastError(), "attn_umma launch");
+  return cuda_fail(launch_early(kern, grid, threads_of<SPLIT>, SMEM_BYTES, s, p, maps[0], maps[1], maps[2], maps[3], maps[4], maps[5],
+                                maps[6]), "attn_umma launch");
 }
 
 }  // namespace

@@ -50,6 +50,7 @@ __global__ void __launch_bounds__(128) add_layernorm_kernel(const T* __restrict_
   const int64_t row = (int64_t)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
   const int lane = threadIdx.x % 32, nv = hidden / N;
   if (row >= rows) return;
+  wait_for_stream();
   const uint4* xr = reinterpret_cast<const uint4*>(x + row * hidden);
   const uint4* rr = reinterpret_cast<const uint4*>(res + row * hidden);
   float f[NV][N];
@@ -103,8 +104,8 @@ int launch_add_layernorm_t(const void* x, const void* res, const void* w, const 
   const unsigned blocks = (unsigned)((rows + warps - 1) / warps);
 #define TDB_LN(NV)                                                                                                              \
   if (nv <= NV) {                                                                                                               \
-    add_layernorm_kernel<T, NV><<<blocks, 32 * warps, 0, s>>>((const T*)x, (const T*)res, (const T*)w, (const T*)b, eps, rows, hidden, (T*)out); \
-    return cuda_fail(cudaGetLastError(), "add_layernorm launch");                                                               \
+    return cuda_fail(launch_early(add_layernorm_kernel<T, NV>, dim3(blocks), 32 * warps, 0, s, (const T*)x, (const T*)res,           \
+                                  (const T*)w, (const T*)b, eps, rows, hidden, (T*)out), "add_layernorm launch");                  \
   }
   TDB_LN(1) TDB_LN(3) TDB_LN(4) TDB_LN(6) TDB_LN(8)
 #undef TDB_LN
@@ -132,6 +133,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) gelu_kernel(uint4* __restrict__ x, int64_t n) {
   const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (i >= n) return;
+  wait_for_stream();
   float f[Vec<T>::N];
   Vec<T>::unpack(x[i], f);
 #pragma unroll
@@ -239,9 +241,8 @@ int tdb_gelu(void* x, int64_t elements, int dtype, void* stream) {
   const int64_t n = elements / (dtype == TDB_DTYPE_F32 ? 4 : 8);
   if (n == 0) return TDB_OK;
   const unsigned blocks = (unsigned)((n + 255) / 256);
-  if (dtype == TDB_DTYPE_F32) gelu_kernel<float><<<blocks, 256, 0, (cudaStream_t)stream>>>((uint4*)x, n);
-  else gelu_kernel<__nv_bfloat16><<<blocks, 256, 0, (cudaStream_t)stream>>>((uint4*)x, n);
-  return cuda_fail(cudaGetLastError(), "gelu launch");
+  return cuda_fail(launch_early(dtype == TDB_DTYPE_F32 ? gelu_kernel<float> : gelu_kernel<__nv_bfloat16>, dim3(blocks), 256, 0,
+                                (cudaStream_t)stream, (uint4*)x, n), "gelu launch");
 }
 
 int tdb_mask_rows(const void* mask, int elem_bytes, int B, int L, int32_t* seqlens, int32_t* cu, int32_t* ticket, int32_t* out, void* stream) {

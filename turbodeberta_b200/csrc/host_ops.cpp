@@ -928,6 +928,20 @@ Tensor unpack_rows(const Tensor& x, const Tensor& pos, int64_t B, int64_t L) {
   return out;
 }
 
+// The tables of one call from its projected tables (rows of 64): in the call's dtype, and expanded for bf16.
+Tables* call_tables(const OptTensor& kr, const OptTensor& qr, const Tensor& q, const Tensor& idx, int64_t exp_delta_max) {
+  auto fit = [&](const OptTensor& t) -> OptTensor {
+    if (!t) return std::nullopt;
+    device_of({&q, &*t});
+    return t->to(q.scalar_type()).contiguous();
+  };
+  const OptTensor k = fit(kr), r = fit(qr);
+  OptTensor ke, re;
+  if (q.scalar_type() == at::kBFloat16) std::tie(ke, re) = expand_pair(k, r, idx, exp_delta_max);
+  return new Tables{k, r, idx, ke, re, (int)(k ? *k : *r).size(1), (int)((idx.numel() - 1) / 2), (int)exp_delta_max,
+                    (int)((2 * exp_delta_max + 1 + 7) / 8 * 8)};
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
@@ -941,6 +955,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("attn_fixed_scores", &attn_fixed_scores);
   m.def("attn_packed_scores", &attn_packed_scores);
   m.def("expand_pair", &expand_pair);
+  m.def("call_tables", &call_tables);
   m.def("drain_pending", &drain_pending);
   py::class_<Watch>(m, "Watch").def(py::init<const py::list&>()).def("holds", &Watch::holds);
   py::class_<Encoder>(m, "Encoder")

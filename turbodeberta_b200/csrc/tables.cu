@@ -163,6 +163,7 @@ __global__ void __launch_bounds__(256) relpos_expand_pair_kernel(const uint4* __
                                                                  const int16_t* __restrict__ idx, int idx_delta_max, int H,
                                                                  int two_span, int exp_delta_max, int exp_rows,
                                                                  uint4* __restrict__ kr_out, uint4* __restrict__ qr_out) {
+  let_next_start();                        // the attention kernel sets itself up meanwhile
   const uint4* table = blockIdx.y == 0 ? kr : qr;
   uint4* out = blockIdx.y == 0 ? kr_out : qr_out;
   if (!table) return;

@@ -47,6 +47,25 @@ struct AttnParams {
   int tiles_listed;                                       // packed form: the workspace already holds this batch's tile list
 };
 
+// Launches a kernel that may start while the kernel in front of it on the stream is still running: its set-up (barriers,
+// tensor memory, descriptors) then costs nothing.  The kernel calls wait_for_stream() before it touches anything that earlier
+// work may have written or may still read.
+template <typename... K, typename... A>
+inline cudaError_t launch_early(void (*kernel)(K...), dim3 grid, unsigned block, size_t smem, cudaStream_t s, A&&... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid; cfg.blockDim = dim3(block); cfg.dynamicSmemBytes = smem; cfg.stream = s;
+  cfg.attrs = &attr; cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<K>(args)...);
+}
+#ifdef __CUDACC__
+__device__ __forceinline__ void wait_for_stream() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// From here on the next kernel may start (it waits by itself for what this one writes).
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+#endif
+
 void set_error(const char* fmt, ...);
 int cuda_fail(cudaError_t e, const char* what);
 

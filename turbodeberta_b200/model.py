@@ -24,7 +24,7 @@ import weakref
 import torch
 from torch import nn
 from transformers.models.deberta_v2.modeling_deberta_v2 import (
-    DebertaV2Attention, DebertaV2Encoder, DebertaV2ForMaskedLM, DebertaV2ForMultipleChoice,
+    DebertaV2Attention, DebertaV2Embeddings, DebertaV2Encoder, DebertaV2ForMaskedLM, DebertaV2ForMultipleChoice,
     DebertaV2ForQuestionAnswering, DebertaV2ForSequenceClassification, DebertaV2ForTokenClassification,
     DebertaV2Intermediate, DebertaV2Layer, DebertaV2Model, DebertaV2Output, DebertaV2SelfOutput,
     DisentangledSelfAttention)
@@ -275,7 +275,8 @@ class FlashDebertaV2Layer(DebertaV2Layer):
         self.attention = FlashDebertaV2Attention(config)
 
 
-# Native plans of live encoders; kept outside the modules, which stay plain data to copy and pickle.
+# Native plans of live encoders and models; kept outside the modules, which stay plain data to copy and pickle.  A plan
+# holds modules below its key, never the key itself, so it goes when the key goes.
 _PLANS: "weakref.WeakKeyDictionary" = weakref.WeakKeyDictionary()
 
 
@@ -500,6 +501,7 @@ class _Wanted(threading.local):
 
 
 _WANTED = _Wanted()
+_PLAIN_ARGUMENTS = frozenset(("input_ids", "attention_mask", "output_hidden_states", "output_attentions", "return_dict"))
 
 
 class FlashDebertaV2Model(DebertaV2Model):
@@ -515,9 +517,46 @@ class FlashDebertaV2Model(DebertaV2Model):
         before = _WANTED.hidden_states
         _WANTED.hidden_states = bool(wanted) or getattr(self, "z_steps", 0) != 0
         try:
+            if not args and not wanted and _PLAIN_ARGUMENTS.issuperset(kwargs):
+                out = self._forward_plain(kwargs.get("input_ids"), kwargs.get("attention_mask"), kwargs)
+                if out is not None:
+                    return out
             return super().forward(*args, **kwargs)
         finally:
             _WANTED.hidden_states = before
+
+    def _forward_plain(self, input_ids, attention_mask, kwargs):
+        """Ids and a 2-D mask in, last hidden states out, for inference with the stock embeddings (words and LayerNorm
+        only): the same operations as the HF model's forward without its argument handling, which takes the host as long as
+        a short text takes the GPU.  None where that forward has to run."""
+        if (self.training or torch.is_grad_enabled() or getattr(self, "z_steps", 0) != 0 or not isinstance(input_ids, torch.Tensor)
+                or not input_ids.is_cuda or input_ids.dim() != 2 or kwargs.get("output_attentions")
+                or kwargs.get("return_dict", True) is False or not getattr(self.config, "use_return_dict", True)
+                or getattr(self.config, "output_attentions", False) or torch.is_autocast_enabled()
+                or torch.nn.modules.module._has_any_global_hook()):
+            return None
+        if attention_mask is not None and (attention_mask.dim() != 2 or attention_mask.shape != input_ids.shape
+                                           or attention_mask.device != input_ids.device):
+            return None
+        emb = self.embeddings
+        watch, of = _PLANS.get(self, (None, None))
+        if watch is None or of is not emb:
+            if (type(emb) is not DebertaV2Embeddings or type(emb.word_embeddings) is not nn.Embedding
+                    or type(emb.LayerNorm) is not nn.LayerNorm or emb.word_embeddings.max_norm is not None
+                    or any(getattr(emb, n, None) is not None for n in ("position_embeddings", "token_type_embeddings", "embed_proj"))):
+                return None
+            watch = host.Watch(list(emb.modules()))
+            _PLANS[self] = (watch, emb)
+        if not watch.holds():
+            _PLANS.pop(self, None)
+            return None
+        if attention_mask is None:
+            attention_mask = torch.ones(input_ids.shape, dtype=torch.long, device=input_ids.device)
+        x = nn.functional.embedding(input_ids, emb.word_embeddings.weight)
+        norm = emb.LayerNorm
+        x = nn.functional.layer_norm(x, norm.normalized_shape, norm.weight, norm.bias, norm.eps)
+        x.mul_(attention_mask.to(x.dtype)[..., None])
+        return self.encoder(x, attention_mask, output_hidden_states=False, output_attentions=False, return_dict=True)
 
 
 def patch_model(model: nn.Module) -> nn.Module:

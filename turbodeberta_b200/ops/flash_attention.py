@@ -30,7 +30,7 @@ from .. import status as _status
 
 
 def _tables_from_args(q_pos, k_pos, q, position_buckets, max_relative_distance, tables):
-    """Normalise the position arguments into a RelPosTables (or None when no term is requested)."""
+    """Normalise the position arguments into something with a ``native()`` table object (None: no term is requested)."""
     if tables is not None:
         return tables
     if q_pos is None and k_pos is None:
@@ -46,7 +46,7 @@ def _tables_from_args(q_pos, k_pos, q, position_buckets, max_relative_distance, 
             raise ValueError(
                 f"{name} must be the projected relative table of shape (H, 2*span, D) = ({H}, 2*span, {D}) or the "
                 f"materialised score tensor of q's leading shape with 2*span columns; got {tuple(t.shape)}.")
-        return t.to(q.dtype).contiguous()
+        return t
 
     kr, qr = norm(q_pos, "q_pos"), norm(k_pos, "k_pos")
     two_span = (kr if kr is not None else qr).shape[1]
@@ -60,24 +60,34 @@ def _tables_from_args(q_pos, k_pos, q, position_buckets, max_relative_distance, 
             max_relative_distance = two_span // 2
         if two_span != 2 * max_relative_distance:
             raise ValueError(f"table has {two_span} rows but max_relative_distance={max_relative_distance}")
-    idx, idm, exp_dm, exp_rows = _geometry(position_buckets, max_relative_distance, q.device)
-    kr_exp, qr_exp = _relpos.expand_pair(kr, qr, idx, exp_dm) if q.dtype == torch.bfloat16 else (None, None)
-    return _relpos.RelPosTables(position_buckets, max_relative_distance, two_span, idx, idm, kr, qr, kr_exp, qr_exp,
-                                exp_dm, exp_rows)
+    if D != 64:
+        raise ValueError(f"head_dim {D}: only 64 is supported")
+    idx, exp_dm = _geometry(position_buckets, max_relative_distance, q.device)
+    return _CallTables(cabi.host.call_tables(kr, qr, q, idx, exp_dm))
+
+
+class _CallTables:
+    """Tables made for one call."""
+    __slots__ = ("_native",)
+
+    def __init__(self, native):
+        self._native = native
+
+    def native(self):
+        return self._native
 
 
 _GEOMETRY: dict = {}
 
 
 def _geometry(position_buckets, max_relative_distance, device):
-    """(index table, its delta_max, delta_max and rows of the expanded tables), kept per geometry and device."""
+    """(index table, delta_max of the expanded tables), kept per geometry and device."""
     key = (position_buckets, max_relative_distance, device)
     g = _GEOMETRY.get(key)
     if g is None:
         sat = _relpos.saturation_distance(position_buckets, max_relative_distance)
         idx = _relpos.bucket_index_table(position_buckets, max_relative_distance, sat + 1, device)
-        exp_dm = sat + cabi.TDB_EXPAND_MARGIN
-        g = _GEOMETRY[key] = (idx, sat + 1, exp_dm, (2 * exp_dm + 1 + 7) // 8 * 8)
+        g = _GEOMETRY[key] = (idx, sat + cabi.TDB_EXPAND_MARGIN)
     return g
 
 
