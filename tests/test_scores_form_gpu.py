@@ -87,15 +87,16 @@ def test_scores_form_argument_errors():
 
 
 @pytest.mark.parametrize("lengths,L", [([1], 1), ([64, 63], 64), ([65, 0, 128], 129), ([300, 17], 300)])
-@pytest.mark.parametrize("terms,mirrored", [("both", False), ("c2p", False), ("p2c", True)])
-def test_bf16_scores_kernel_at_tile_edges(lengths, L, terms, mirrored):
+@pytest.mark.parametrize("terms,mirrored", [("both", False), ("c2p", False), ("p2c", True), ("both", True)])
+@pytest.mark.parametrize("width", [128, 131])                              # 131: rows that are not 16-byte aligned
+def test_bf16_scores_kernel_at_tile_edges(lengths, L, terms, mirrored, width):
     """The tensor-core kernel for materialised scores around its 64-row tiles, padded rows holding NaN, against the f32
     kernel on the same bf16 values."""
     from turbodeberta_b200.ops.flash_attention import flash_attention_with_disentangled
     gen = torch.Generator(device="cuda").manual_seed(7)
     B = len(lengths)
     q, k, v = (torch.randn(B, 2, L, 64, generator=gen, device="cuda").bfloat16() for _ in range(3))
-    pos = [torch.randn(B, 2, L, 128, generator=gen, device="cuda").bfloat16() if terms in ("both", n) else None for n in ("c2p", "p2c")]
+    pos = [torch.randn(B, 2, L, width, generator=gen, device="cuda").bfloat16()[..., width - 128:] if terms in ("both", n) else None for n in ("c2p", "p2c")]
     lens = torch.tensor(lengths, dtype=torch.int32, device="cuda")
     for b, n in enumerate(lengths):
         for t in (k, v, *[x for x in pos if x is not None]):

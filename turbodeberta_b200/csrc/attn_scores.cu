@@ -4,12 +4,13 @@
 //   score[q,k] = (Q[q].K[k] + c2p_scores[q, idx(q-k)] + p2c_scores[k, idx(q-k)]) * sm_scale
 //
 // (p2c at idx(k-q) with TDB_FLAG_P2C_MIRRORED).  Bound by the score tensors: 8 x 256 tokens of 12 heads bring 50 MB of them,
-// against 1.6 GFLOP; so the products run on the warp-level tensor instruction, whose fragment layout is what the gather wants:
-// a fragment register's 32 lanes are 8 rows x 4 pairs of keys, i.e. 8 short runs of a c2p row and 4 of a p2c row, where one
-// row per lane (the layout tensor memory would give) touches 32 lines per load.  One block of four warps owns 64 query rows and
-// walks key tiles of 64, K and V double-buffered by asynchronous copies.  P keeps two bf16 terms (value and remainder) for
-// P.V, so nothing but the output is rounded to bf16.
-// 8 x 256 tokens, 12 heads: 46 us per call, 1.4 TB/s of scores (CUDA-core kernel: 142 us).
+// against 1.6 GFLOP; so the products run on the warp-level tensor instruction, and the work is in the gather.  The distances of
+// a 64 x 64 tile reach at most 127 neighbouring columns, so each of its c2p and p2c rows is one short run: the runs are copied
+// to shared memory in 16-byte pieces and gathered there (WINDOW).  Rows that are not 16-byte aligned are gathered from global
+// memory, where a fragment register's 32 lanes are 8 short runs of c2p rows, or 4 of p2c rows, which the first-level cache
+// takes one line at a time.  One block of four warps owns 64 query rows and walks key tiles of 64; three blocks per SM cover
+// each other's copies.  P keeps two bf16 terms (value and remainder) for P.V, so nothing but the output is rounded to bf16.
+// 8 x 256 tokens, 12 heads: CUDA-core kernel 142 us per call, gathered from global memory 46 us, with windows 41 us (23 us of them the kernel: 2.2 TB/s of scores).
 #include "attn_blocks.cuh"
 #include <math_constants.h>
 
@@ -18,6 +19,7 @@ namespace tdb {
 namespace {
 
 constexpr int ST = 64, SP = 72, S_THREADS = 128;     // tile rows, row pitch in elements (144 bytes: conflict-free ldmatrix)
+constexpr int WCH = 17, WP = 152;                    // 16-byte pieces of a score row's window, its pitch in elements (conflict-free)
 
 __device__ __forceinline__ uint32_t saddr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -47,10 +49,24 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
 }
 __device__ __forceinline__ float bf(unsigned short h) { return __uint_as_float((uint32_t)h << 16); }
 
-template <bool C2P, bool P2C>
+// The columns [lo, lo + 8 * pieces) of 64 rows to shared memory.
+__device__ __forceinline__ void stage_window(unsigned short* dst, const unsigned short* src, int64_t pitch, int rows, int lo, int pieces) {
+  for (int e = threadIdx.x; e < ST * WCH; e += S_THREADS) {
+    const int row = e / WCH, c = e - row * WCH;
+    if (row < rows && c < pieces)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(saddr(dst + row * WP + c * 8)), "l"(src + (int64_t)row * pitch + lo + c * 8) : "memory");
+  }
+}
+
+template <bool C2P, bool P2C, bool WINDOW>
 __global__ void __launch_bounds__(S_THREADS, 3) attn_scores_kernel(const AttnParams p) {
-  __shared__ __align__(16) __nv_bfloat16 sQ[ST * SP], sK[2][ST * SP], sV[2][ST * SP];
-  __shared__ int16_t sIdx[2][2 * ST];                // table row of distance q0 - k0 - 63 + x, and of its negative
+  constexpr int BUFS = WINDOW ? 1 : 2;               // with windows there is room for one tile; otherwise the next is on its way
+  extern __shared__ __align__(16) unsigned char smem[];
+  __nv_bfloat16* const sQ = reinterpret_cast<__nv_bfloat16*>(smem);
+  __nv_bfloat16 *const sK = sQ + ST * SP, *const sV = sK + BUFS * ST * SP;
+  unsigned short* const wC = reinterpret_cast<unsigned short*>(sV + BUFS * ST * SP);
+  unsigned short* const wP = wC + (C2P ? ST * WP : 0);
+  __shared__ int16_t sIdx[2][2 * ST];                // table row of distance q0 - k0 - 63 + x
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int s = longest_first(p, blockIdx.z), h = blockIdx.y, q0 = blockIdx.x * ST;
   int len, rows;
@@ -79,21 +95,38 @@ __global__ void __launch_bounds__(S_THREADS, 3) attn_scores_kernel(const AttnPar
 
   if (q0 < len) {
     stage(sQ, qb + (int64_t)q0 * p.q_st, p.q_st, len - q0);
+    const bool mirrored = p.flags & TDB_FLAG_P2C_MIRRORED;
     auto load_tile = [&](int k0, int buf) {
-      stage(sK[buf], kb + (int64_t)k0 * p.k_st, p.k_st, len - k0);
-      stage(sV[buf], vb + (int64_t)k0 * p.v_st, p.v_st, len - k0);
+      stage(sK + buf * ST * SP, kb + (int64_t)k0 * p.k_st, p.k_st, len - k0);
+      stage(sV + buf * ST * SP, vb + (int64_t)k0 * p.v_st, p.v_st, len - k0);
+      if (WINDOW) {                                  // the index grows with the distance: the ends of its range are the window's
+        if (C2P) {
+          const int lo = row_of(q0 - k0 - (ST - 1)) & ~7, hi = row_of(q0 - k0 + ST - 1);
+          stage_window(wC, c2p + (int64_t)q0 * p.c2p_st, p.c2p_st, len - q0, lo, (hi - lo) / 8 + 1);
+        }
+        if (P2C) {
+          const int d = mirrored ? k0 - q0 : q0 - k0;
+          const int lo = row_of(d - (ST - 1)) & ~7, hi = row_of(d + ST - 1);
+          stage_window(wP, p2c + (int64_t)k0 * p.p2c_st, p.p2c_st, len - k0, lo, (hi - lo) / 8 + 1);
+        }
+      }
       asm volatile("cp.async.commit_group;" ::: "memory");
       const int delta = q0 - k0 - (ST - 1) + (int)threadIdx.x;
-      if (C2P || P2C) sIdx[buf][threadIdx.x] = row_of(delta);
+      sIdx[buf][threadIdx.x] = row_of(delta);
     };
     load_tile(0, 0);
     uint32_t qf[4][4];
     // rows beyond the sequence read the last row's scores: in bounds, and their results are dropped
     const int qr[2] = {min(q0 + r0, len - 1), min(q0 + r0 + 8, len - 1)};
-    for (int k0 = 0, buf = 0; k0 < len; k0 += ST, buf ^= 1) {
+    for (int k0 = 0, buf = 0; k0 < len; k0 += ST, buf ^= (WINDOW ? 0 : 1)) {
+      if (WINDOW && k0 > 0) {
+        __syncthreads();                             // everybody is done with the tile before
+        load_tile(k0, 0);
+      }
       asm volatile("cp.async.wait_all;" ::: "memory");
       __syncthreads();
-      if (k0 + ST < len) load_tile(k0 + ST, buf ^ 1);
+      if (!WINDOW && k0 + ST < len) load_tile(k0 + ST, buf ^ 1);
+      const int lo_c = row_of(q0 - k0 - (ST - 1)) & ~7, lo_p = row_of((mirrored ? k0 - q0 : q0 - k0) - (ST - 1)) & ~7;
       if (k0 == 0) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) ldsm4(qf[i], sQ + (warp * 16 + (lane & 15)) * SP + 16 * i + 8 * (lane >> 4));
@@ -110,10 +143,10 @@ __global__ void __launch_bounds__(S_THREADS, 3) attn_scores_kernel(const AttnPar
             const int kl = 8 * (4 * half + i) + kc + (e & 1), rl = r0 + 8 * (e >> 1);
             const int x = rl - kl + ST - 1;
             const int r = sIdx[buf][x];
-            if (C2P) gc[i][e] = __ldg(c2p + (int64_t)qr[e >> 1] * p.c2p_st + r);
+            if (C2P) gc[i][e] = WINDOW ? wC[rl * WP + r - lo_c] : __ldg(c2p + (int64_t)qr[e >> 1] * p.c2p_st + r);
             if (P2C) {
-              const int rm = (p.flags & TDB_FLAG_P2C_MIRRORED) ? row_of(k0 + kl - q0 - rl) : r;
-              gp[i][e] = __ldg(p2c + (int64_t)min(k0 + kl, len - 1) * p.p2c_st + rm);
+              const int rm = mirrored ? row_of(k0 + kl - q0 - rl) : r;
+              gp[i][e] = WINDOW ? wP[kl * WP + rm - lo_p] : __ldg(p2c + (int64_t)min(k0 + kl, len - 1) * p.p2c_st + rm);
             }
           }
 #pragma unroll
@@ -126,7 +159,7 @@ __global__ void __launch_bounds__(S_THREADS, 3) attn_scores_kernel(const AttnPar
           for (int i = 0; i < 2; ++i) {
             uint32_t kf[4];                          // keys 8j..8j+15, columns 16kk..+15
             const int j = 4 * half + 2 * i;
-            ldsm4(kf, sK[buf] + (8 * j + (lane & 7) + 8 * (lane >> 4)) * SP + 16 * kk + 8 * ((lane >> 3) & 1));
+            ldsm4(kf, sK + buf * ST * SP + (8 * j + (lane & 7) + 8 * (lane >> 4)) * SP + 16 * kk + 8 * ((lane >> 3) & 1));
             mma(sc[j], qf[kk], kf[0], kf[1]);
             mma(sc[j + 1], qf[kk], kf[2], kf[3]);
           }
@@ -170,7 +203,7 @@ __global__ void __launch_bounds__(S_THREADS, 3) attn_scores_kernel(const AttnPar
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           uint32_t vf[4];                            // keys 16kk..+15, columns 16i..+15
-          ldsm4t(vf, sV[buf] + (16 * kk + (lane & 15)) * SP + 16 * i + 8 * (lane >> 4));
+          ldsm4t(vf, sV + buf * ST * SP + (16 * kk + (lane & 15)) * SP + 16 * i + 8 * (lane >> 4));
           mma(o[2 * i], hi, vf[0], vf[1]);
           mma(o[2 * i + 1], hi, vf[2], vf[3]);
           mma(o[2 * i], lo, vf[0], vf[1]);
@@ -197,13 +230,29 @@ __global__ void __launch_bounds__(S_THREADS, 3) attn_scores_kernel(const AttnPar
 
 }  // namespace
 
+template <bool C2P, bool P2C, bool WINDOW>
+static int launch_scores(const AttnParams& p, dim3 grid, cudaStream_t s) {
+  constexpr int SMEM = (ST * SP * (1 + 2 * (WINDOW ? 1 : 2)) + (WINDOW ? ((C2P ? 1 : 0) + (P2C ? 1 : 0)) * ST * WP : 0)) * 2;
+  auto kern = attn_scores_kernel<C2P, P2C, WINDOW>;
+  if (SMEM > 48 * 1024) {
+    const int rc = opt_in_smem(reinterpret_cast<const void*>(kern), SMEM);
+    if (rc) return rc;
+  }
+  kern<<<grid, S_THREADS, SMEM, s>>>(p);
+  return cuda_fail(cudaGetLastError(), "attn_scores launch");
+}
+
 int launch_attn_scores(const AttnParams& p, cudaStream_t s) {
   dim3 grid((p.L + ST - 1) / ST, p.H, p.n_seqs);
   const bool c2p = p.flags & TDB_FLAG_C2P, p2c = p.flags & TDB_FLAG_P2C;
-  if (c2p && p2c) attn_scores_kernel<true, true><<<grid, S_THREADS, 0, s>>>(p);
-  else if (c2p) attn_scores_kernel<true, false><<<grid, S_THREADS, 0, s>>>(p);
-  else attn_scores_kernel<false, true><<<grid, S_THREADS, 0, s>>>(p);
-  return cuda_fail(cudaGetLastError(), "attn_scores launch");
+  // 16-byte pieces of every row: aligned bases, strides and row length
+  auto pieces = [&](const void* x, int64_t sb, int64_t st, int64_t sh) {
+    return (reinterpret_cast<uintptr_t>(x) & 15) == 0 && ((sb | st | sh | p.two_span) & 7) == 0;
+  };
+  const bool window = (!c2p || pieces(p.c2p_scores, p.c2p_sb, p.c2p_st, p.c2p_sh)) && (!p2c || pieces(p.p2c_scores, p.p2c_sb, p.p2c_st, p.p2c_sh));
+  if (c2p && p2c) return window ? launch_scores<true, true, true>(p, grid, s) : launch_scores<true, true, false>(p, grid, s);
+  if (c2p) return window ? launch_scores<true, false, true>(p, grid, s) : launch_scores<true, false, false>(p, grid, s);
+  return window ? launch_scores<false, true, true>(p, grid, s) : launch_scores<false, true, false>(p, grid, s);
 }
 
 }  // namespace tdb

@@ -95,10 +95,13 @@ def _is_materialised(t, q, position_buckets=0, max_relative_distance=0) -> bool:
     """True when ``t`` is a per-token score tensor (``q.shape[:-1] + (2*span,)``) rather than a projected table
     (``(H, 2*span, D)``, optionally with a leading 1).  Where both readings fit the shape, the geometry arguments
     decide (a table has 2*span rows, a score tensor 2*span columns); if they do not, it is taken as a table."""
-    if t is None or t.dim() != q.dim() or tuple(t.shape[:-1]) != tuple(q.shape[:-1]):
+    if t is None or t.dim() != q.dim():
         return False
-    H, D = q.shape[-3] if q.dim() == 4 else q.shape[-2], q.shape[-1]
-    table = t.shape[0] == 1 and t.shape[1] == H and t.shape[3] == D if t.dim() == 4 else (t.shape[0] == H and t.shape[2] == D)
+    shape, qs = t.shape, q.shape
+    if shape[:-1] != qs[:-1]:
+        return False
+    H, D = qs[-3] if len(qs) == 4 else qs[-2], qs[-1]
+    table = shape[0] == 1 and shape[1] == H and shape[3] == D if len(shape) == 4 else (shape[0] == H and shape[2] == D)
     if not table:
         return True
     want = 2 * position_buckets if position_buckets > 0 else 2 * max_relative_distance
@@ -131,10 +134,11 @@ def refuse_gradients(*tensors) -> None:
 def _scores_fixed(q, k, v, c2p_scores, p2c_scores, seqlens, sm_scale, position_buckets, max_relative_distance,
                   p2c_mirrored, return_lse, check_status):
     """Legacy form of the fixed-length op: gather from materialised ``(B, H, L, 2*span)`` score tensors."""
-    dev = cabi.require_cuda(q, k, v, seqlens)
     refuse_gradients(q, k, v, c2p_scores, p2c_scores)
+    if not q.is_cuda:
+        cabi.require_cuda(q, k, v, seqlens)
     some = c2p_scores if c2p_scores is not None else p2c_scores
-    idx = _index_table_for_scores(some.shape[-1], position_buckets, max_relative_distance, dev)
+    idx = _index_table_for_scores(some.shape[-1], position_buckets, max_relative_distance, q.device)
     o, lse, st = cabi.host.attn_fixed_scores(q, k, v, c2p_scores, p2c_scores, idx, p2c_mirrored, seqlens, sm_scale,
                                              return_lse, check_status)
     if st is not None:
@@ -228,13 +232,14 @@ def flash_attention_with_disentangled(q, k, v, q_pos, k_pos, causal=False, sm_sc
         raise NotImplementedError("causal masking is not part of the DeBERTa encoder path")
     if sm_scale is None:
         sm_scale = 1.0 / math.sqrt(q.shape[-1])
-    mat = lambda t: _is_materialised(t, q, position_buckets, max_relative_distance)
-    if tables is None and (mat(q_pos) or mat(k_pos)):
-        if (q_pos is not None and not mat(q_pos)) or (k_pos is not None and not mat(k_pos)):
-            raise ValueError("q_pos and k_pos must both be tables (H, 2*span, D) or both be score tensors (B, H, L, 2*span)")
-        o, lse = _scores_fixed(q, k, v, q_pos, k_pos, seqlens, sm_scale, position_buckets, max_relative_distance,
-                               p2c_mirrored, return_lse, check_status)
-        return (o, lse) if return_lse else o
+    if tables is None and (q_pos is not None or k_pos is not None):
+        mat = [t is not None and _is_materialised(t, q, position_buckets, max_relative_distance) for t in (q_pos, k_pos)]
+        if any(mat):
+            if (q_pos is not None and not mat[0]) or (k_pos is not None and not mat[1]):
+                raise ValueError("q_pos and k_pos must both be tables (H, 2*span, D) or both be score tensors (B, H, L, 2*span)")
+            o, lse = _scores_fixed(q, k, v, q_pos, k_pos, seqlens, sm_scale, position_buckets, max_relative_distance,
+                                   p2c_mirrored, return_lse, check_status)
+            return (o, lse) if return_lse else o
     if p2c_mirrored:
         raise ValueError("p2c_mirrored applies to materialised score tensors only")
     tables = _tables_from_args(q_pos, k_pos, q, position_buckets, max_relative_distance, tables)

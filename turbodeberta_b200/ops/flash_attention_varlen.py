@@ -86,13 +86,14 @@ def flash_attention_with_disentangled_varlen(q, k, v, q_pos, k_pos, cu_seqlens_q
     T = q.shape[0]
     max_seqlen = max(int(max_seqlen_q), int(max_seqlen_k if max_seqlen_k is not None else max_seqlen_q))
     max_seqlen = max(1, min(max_seqlen, T)) if T > 0 else 1
-    mat = lambda t: _is_materialised(t, q, position_buckets, max_relative_distance)
-    if tables is None and (mat(q_pos) or mat(k_pos)):
-        if (q_pos is not None and not mat(q_pos)) or (k_pos is not None and not mat(k_pos)):
-            raise ValueError("q_pos and k_pos must both be tables (H, 2*span, D) or both be score tensors (T, H, 2*span)")
-        o, lse = _scores_varlen(q, k, v, q_pos, k_pos, cu_seqlens_q, max_seqlen, sm_scale, position_buckets,
-                                max_relative_distance, p2c_mirrored, return_lse, check_status, cu_seqlens_k)
-        return (o, lse) if return_lse else o
+    if tables is None and (q_pos is not None or k_pos is not None):
+        mat = [t is not None and _is_materialised(t, q, position_buckets, max_relative_distance) for t in (q_pos, k_pos)]
+        if any(mat):
+            if (q_pos is not None and not mat[0]) or (k_pos is not None and not mat[1]):
+                raise ValueError("q_pos and k_pos must both be tables (H, 2*span, D) or both be score tensors (T, H, 2*span)")
+            o, lse = _scores_varlen(q, k, v, q_pos, k_pos, cu_seqlens_q, max_seqlen, sm_scale, position_buckets,
+                                    max_relative_distance, p2c_mirrored, return_lse, check_status, cu_seqlens_k)
+            return (o, lse) if return_lse else o
     if p2c_mirrored:
         raise ValueError("p2c_mirrored applies to materialised score tensors only")
     tables = _tables_from_args(q_pos, k_pos, q, position_buckets, max_relative_distance, tables)
