@@ -344,3 +344,25 @@ def test_far_scores_far_above_the_near_ones(level):
     o2 = flash_attention_with_disentangled(*args, tables=tables, kernel=SIMT)
     assert torch.isfinite(o.float()).all()
     assert (o.float() - o2.float()).abs().max().item() < 2e-2
+
+
+@pytest.mark.parametrize("lengths,L", [([1], 1), ([16, 17, 1, 0], 17), ([33, 32, 48], 49), ([64, 63, 5], 64), ([65, 64], 65)])
+@pytest.mark.parametrize("c2p,p2c", [(True, True), (True, False), (False, True), (False, False)])
+def test_short_padded_batches(lengths, L, c2p, p2c):
+    """Up to 64 tokens run on a kernel of one block per sequence and head: lengths around its 16-row warps, empty rows,
+    NaN in the padding, against the exact kernel (and the next size up, on the other kernel)."""
+    from turbodeberta_b200.ops.flash_attention import flash_attention_with_disentangled
+    w = _wl(lengths, L, hidden=192, heads=3)
+    q, k, v, rel, P = util.device_inputs(w, DT)
+    tables = util.make_tables(w, rel, P, c2p, p2c) if (c2p or p2c) else None
+    lens = torch.tensor(lengths, dtype=torch.int32, device="cuda")
+    for b, n in enumerate(lengths):
+        k[b, n:] = float("nan")
+        v[b, n:] = float("nan")
+    args = [t.permute(0, 2, 1, 3) for t in (q, k, v)] + [None, None, False, 0.0722, 256, 512]
+    o, lse = flash_attention_with_disentangled(*args, seqlens=lens, tables=tables, kernel=UMMA, return_lse=True)
+    o2, lse2 = flash_attention_with_disentangled(*args, seqlens=lens, tables=tables, kernel=SIMT, return_lse=True)
+    assert (o.float() - o2.float()).abs().max().item() < 8e-3
+    for b, n in enumerate(lengths):
+        assert torch.count_nonzero(o[b, :, n:]).item() == 0 and torch.count_nonzero(lse[b, :, n:]).item() == 0
+        assert n == 0 or (lse[b, :, :n] - lse2[b, :, :n]).abs().max().item() < 1e-3

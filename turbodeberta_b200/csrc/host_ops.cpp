@@ -222,12 +222,20 @@ void* ptr(const OptTensor& t) { return t.has_value() && t->defined() ? t->data_p
 struct Tables {
   OptTensor kr, qr, idx, kr_exp, qr_exp;
   int two_span, idx_delta_max, exp_delta_max, exp_rows;
+  Tensor both;                                       // of a call's own tables: the expanded ones, c2p's in front
   void fill(tdb::AttnParams& p, const Tensor& q) const {
     for (const OptTensor* t : {&kr, &qr})
       if (t->has_value() && (*t)->scalar_type() != q.scalar_type()) throw py::value_error("relative tables must have the dtype of q");
     p.kr = ptr(kr); p.qr = ptr(qr); p.two_span = two_span;
     p.idx = static_cast<const int16_t*>(ptr(idx)); p.idx_delta_max = idx_delta_max;
-    p.kr_exp = ptr(kr_exp); p.qr_exp = ptr(qr_exp); p.exp_delta_max = exp_delta_max; p.exp_rows = exp_rows;
+    if (both.defined()) {
+      char* e = static_cast<char*>(both.data_ptr());
+      p.kr_exp = kr ? e : nullptr;
+      p.qr_exp = qr ? e + (kr ? both.nbytes() / 2 : 0) : nullptr;
+    } else {
+      p.kr_exp = ptr(kr_exp); p.qr_exp = ptr(qr_exp);
+    }
+    p.exp_delta_max = exp_delta_max; p.exp_rows = exp_rows;
     p.flags = (p.kr ? TDB_FLAG_C2P : 0) | (p.qr ? TDB_FLAG_P2C : 0);
   }
 };
@@ -404,19 +412,26 @@ Result attn_packed_scores(const Tensor& q, const Tensor& k, const Tensor& v, con
   return launch(p, code, TDB_KERNEL_SIMT, dev, o, lse, check);
 }
 
-// Distance-expanded copies of both tables (bf16, head_dim 64) with one allocation and one launch.
-std::pair<OptTensor, OptTensor> expand_pair(const OptTensor& kr, const OptTensor& qr, const Tensor& idx, int64_t exp_delta_max) {
+// Distance-expanded copies of both tables (bf16, head_dim 64) with one allocation and one launch: [1 or 2, H, rows, 64].
+Tensor expand_both(const OptTensor& kr, const OptTensor& qr, const Tensor& idx, int64_t exp_delta_max) {
   const Tensor& some = kr ? *kr : *qr;
   const int64_t H = some.size(0), two_span = some.size(1), exp_rows = (2 * exp_delta_max + 1 + 7) / 8 * 8;
   c10::cuda::CUDAGuard guard(some.device());
   const int n = (kr ? 1 : 0) + (qr ? 1 : 0);
   Tensor both = at::empty({n, H, exp_rows, 64}, some.options());
+  char* e = static_cast<char*>(both.data_ptr());
+  const int rc = tdb_expand_pair(ptr(kr), ptr(qr), idx.data_ptr<int16_t>(), (int)((idx.numel() - 1) / 2), (int)H, (int)two_span,
+                                 (int)exp_delta_max, (int)exp_rows, kr ? e : nullptr, qr ? e + (kr ? both.nbytes() / 2 : 0) : nullptr,
+                                 c10::cuda::getCurrentCUDAStream().stream());
+  if (rc) throw std::runtime_error(std::string("libtdb_b200: ") + tdb_last_error());
+  return both;
+}
+std::pair<OptTensor, OptTensor> expand_pair(const OptTensor& kr, const OptTensor& qr, const Tensor& idx, int64_t exp_delta_max) {
+  const OptTensor k = kr ? OptTensor(kr->contiguous()) : std::nullopt, r = qr ? OptTensor(qr->contiguous()) : std::nullopt;
+  const Tensor both = expand_both(k, r, idx, exp_delta_max);
   OptTensor ko, qo;
   if (kr) ko = both.select(0, 0);
-  if (qr) qo = both.select(0, n - 1);
-  const int rc = tdb_expand_pair(ptr(kr), ptr(qr), idx.data_ptr<int16_t>(), (int)((idx.numel() - 1) / 2), (int)H, (int)two_span,
-                                 (int)exp_delta_max, (int)exp_rows, ptr(ko), ptr(qo), c10::cuda::getCurrentCUDAStream().stream());
-  if (rc) throw std::runtime_error(std::string("libtdb_b200: ") + tdb_last_error());
+  if (qr) qo = both.select(0, both.size(0) - 1);
   return {ko, qo};
 }
 
@@ -933,13 +948,14 @@ Tables* call_tables(const OptTensor& kr, const OptTensor& qr, const Tensor& q, c
   auto fit = [&](const OptTensor& t) -> OptTensor {
     if (!t) return std::nullopt;
     device_of({&q, &*t});
+    if (t->scalar_type() == q.scalar_type() && t->is_contiguous()) return t;
     return t->to(q.scalar_type()).contiguous();
   };
   const OptTensor k = fit(kr), r = fit(qr);
-  OptTensor ke, re;
-  if (q.scalar_type() == at::kBFloat16) std::tie(ke, re) = expand_pair(k, r, idx, exp_delta_max);
-  return new Tables{k, r, idx, ke, re, (int)(k ? *k : *r).size(1), (int)((idx.numel() - 1) / 2), (int)exp_delta_max,
-                    (int)((2 * exp_delta_max + 1 + 7) / 8 * 8)};
+  Tensor both;
+  if (q.scalar_type() == at::kBFloat16) both = expand_both(k, r, idx, exp_delta_max);
+  return new Tables{k, r, idx, {}, {}, (int)(k ? *k : *r).size(1), (int)((idx.numel() - 1) / 2), (int)exp_delta_max,
+                    (int)((2 * exp_delta_max + 1 + 7) / 8 * 8), both};
 }
 
 }  // namespace
@@ -948,7 +964,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   py::class_<Tables>(m, "Tables")
       .def(py::init([](OptTensor kr, OptTensor qr, OptTensor idx, OptTensor kr_exp, OptTensor qr_exp, int two_span, int idx_delta_max,
                        int exp_delta_max, int exp_rows) {
-        return new Tables{kr, qr, idx, kr_exp, qr_exp, two_span, idx_delta_max, exp_delta_max, exp_rows};
+        return new Tables{kr, qr, idx, kr_exp, qr_exp, two_span, idx_delta_max, exp_delta_max, exp_rows, {}};
       }));
   m.def("attn_fixed", &attn_fixed);
   m.def("attn_packed", &attn_packed);

@@ -137,6 +137,7 @@ static int run_attn(const AttnParams& p, int dtype, int kernel, cudaStream_t str
     set_error("workspace of %zu bytes is smaller than the %zu required", p.workspace_bytes, umma_workspace_bytes(p.n_seqs, p.total_tokens));
     return TDB_ERR_WORKSPACE;
   }
+  if (small_applicable(p)) return launch_attn_small(p, stream);
   return launch_attn_umma(p, stream);
 }
 
