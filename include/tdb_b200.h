@@ -171,8 +171,8 @@ TDB_API int tdb_selftest_bounded_wait(int32_t* status, int code, int limit_us, v
  * its flag clear).  The kernel only gathers them: score[q,k] = (Q[q].K[k] + c2p_scores[q, idx(q-k)] + p2c_scores[k,
  * idx(q-k)]) * sm_scale, the eager module's convention (HF modeling_deberta_v2.py:315-343); with
  * TDB_FLAG_P2C_MIRRORED the p2c term is read at idx(k-q) instead, which is what the reference's own kernel does
- * (ops/flash_attention.py:126-132).  CUDA-core kernel, f32 or bf16; a compatibility path, not a throughput path --
- * the fused entry points above exist to avoid these tensors.  Strides in elements; other arguments as above. */
+ * (ops/flash_attention.py:126-132).  Tensor-core products in bf16, CUDA-core kernel in f32; bound by reading the score
+ * tensors, which the fused entry points above exist to avoid.  Strides in elements; other arguments as above. */
 TDB_API int tdb_attn_fwd_fixed_scores(const void* q, const void* k, const void* v, void* o,
                         int64_t q_sb, int64_t q_st, int64_t q_sh, int64_t k_sb, int64_t k_st, int64_t k_sh,
                         int64_t v_sb, int64_t v_st, int64_t v_sh, int64_t o_sb, int64_t o_st, int64_t o_sh,
