@@ -402,3 +402,22 @@ def test_replaced_embeddings_and_hooks_on_them_are_seen():
         b = model(input_ids=ids, attention_mask=mask).last_hidden_state
         assert not torch.equal(a, b)
         assert torch.equal(b, model(ids, mask).last_hidden_state)
+
+
+@pytest.mark.parametrize("tokens", [1, 16, 17, 32])
+@pytest.mark.parametrize("columns,features", [(32, 8), (768, 2304), (1024, 1000), (2080, 768), (3072, 776), (4096, 64)])
+@pytest.mark.parametrize("gelu", [False, True])
+def test_skinny_projection(tokens, columns, features, gelu):
+    """The projection kernel for few tokens at the edges of its token tiles, column blocks per warp and feature groups."""
+    from turbodeberta_b200 import _cabi as cabi
+    torch.manual_seed(16)
+    x = torch.randn(tokens, columns, device="cuda").bfloat16()
+    w = (torch.randn(features, columns, device="cuda") / columns ** 0.5).bfloat16()
+    b = torch.randn(features, device="cuda").bfloat16()
+    y = torch.full((tokens, features), float("nan"), device="cuda", dtype=torch.bfloat16)
+    cabi.check(cabi.host.skinny(x, w, b, gelu, y))
+    want = torch.nn.functional.linear(x.double(), w.double(), b.double())
+    want = torch.nn.functional.gelu(want) if gelu else want
+    assert ((y.double() - want).abs() <= 5e-3 * want.abs() + 1e-5).all()
+    big = torch.zeros(33, columns, device="cuda", dtype=torch.bfloat16)
+    assert cabi.host.skinny(big, w, b, gelu, y) == cabi.ERR_SHAPE

@@ -28,6 +28,7 @@ __global__ void __launch_bounds__(S_THREADS) attn_small_kernel(const AttnParams 
   float* const bP = bC + (C2P ? ST * BP : 0);
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, h = blockIdx.x, b = blockIdx.y;
   wait_for_stream();
+  let_next_start();
   int len = p.seqlens ? p.seqlens[b] : p.L;
   len = len < 0 ? 0 : (len > p.L ? p.L : len);
   const bf16* const qb = reinterpret_cast<const bf16*>(p.q) + b * p.q_sb + h * p.q_sh;

@@ -2,6 +2,7 @@
 // padded batches and the packed token stream.  All of them are bound by memory traffic (or, for a handful of tokens, by the
 // launch): each reads its inputs once and writes its output once.
 #include "tdb_internal.h"
+#include "gelu.cuh"
 
 namespace tdb {
 
@@ -41,16 +42,17 @@ __device__ __forceinline__ float warp_sum(float x) {
   return x;
 }
 
+// out may be x.  No __restrict__ on the activations: the kernel may have started beside the one that writes them, and the
+// non-coherent loads that it allows are not part of what wait_for_stream() makes visible.
 // out = LayerNorm(x + res) * w + b, one warp per row, the row held in registers (fp32 sum, mean and variance).  Per row three
 // row-sized transfers; 9.2k x 1024 bf16 (57 MB): 24 + 8 us as an addition and a LayerNorm kernel, about 10 us here.
 template <typename T, int NV>
-__global__ void __launch_bounds__(128) add_layernorm_kernel(const T* __restrict__ x, const T* __restrict__ res, const T* __restrict__ w,
-                                                            const T* __restrict__ b, float eps, int64_t rows, int hidden, T* __restrict__ out) {
+__global__ void __launch_bounds__(128) add_layernorm_kernel(const T* x, const T* res, const T* __restrict__ w,
+                                                            const T* __restrict__ b, float eps, int64_t rows, int hidden, T* out) {
   constexpr int N = Vec<T>::N;
   const int64_t row = (int64_t)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
   const int lane = threadIdx.x % 32, nv = hidden / N;
   if (row >= rows) return;
-  wait_for_stream();
   const uint4* xr = reinterpret_cast<const uint4*>(x + row * hidden);
   const uint4* rr = reinterpret_cast<const uint4*>(res + row * hidden);
   float f[NV][N];
@@ -61,6 +63,8 @@ __global__ void __launch_bounds__(128) add_layernorm_kernel(const T* __restrict_
     const int c = lane + 32 * i;
     if (c < nv) { wv[i] = __ldg(reinterpret_cast<const uint4*>(w) + c); bv[i] = __ldg(reinterpret_cast<const uint4*>(b) + c); }
   }
+  wait_for_stream();                                 // the weights, above, are older than the kernel in front
+  let_next_start();
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
     const int c = lane + 32 * i;
@@ -97,35 +101,20 @@ __global__ void __launch_bounds__(128) add_layernorm_kernel(const T* __restrict_
 
 template <typename T>
 int launch_add_layernorm_t(const void* x, const void* res, const void* w, const void* b, float eps, int64_t rows, int hidden, void* out,
-                           cudaStream_t s) {
+                           bool early, cudaStream_t s) {
   constexpr int PER = 32 * Vec<T>::N;
   const int nv = (hidden + PER - 1) / PER;
   const int warps = rows >= 148 * 16 ? 4 : 1;        // few rows: one per block, so that they spread over the SMs
   const unsigned blocks = (unsigned)((rows + warps - 1) / warps);
 #define TDB_LN(NV)                                                                                                              \
   if (nv <= NV) {                                                                                                               \
-    return cuda_fail(launch_early(add_layernorm_kernel<T, NV>, dim3(blocks), 32 * warps, 0, s, (const T*)x, (const T*)res,           \
+    return cuda_fail(launch_stream(add_layernorm_kernel<T, NV>, dim3(blocks), 32 * warps, 0, s, early, (const T*)x, (const T*)res,           \
                                   (const T*)w, (const T*)b, eps, rows, hidden, (T*)out), "add_layernorm launch");                  \
   }
   TDB_LN(1) TDB_LN(3) TDB_LN(4) TDB_LN(6) TDB_LN(8)
 #undef TDB_LN
   set_error("add_layernorm: hidden size %d is not supported", hidden);
   return TDB_ERR_SHAPE;
-}
-
-// Phi(-|x|) = erfc(|x| / sqrt 2) / 2 by formula 7.1.26 of Abramowitz and Stegun's handbook (absolute error below 1.5e-7;
-// relative to the value 5e-5 down to x = -3 and 2e-3 down to x = -5, where 1 + erf(x) in fp32 is off by 5e-2): for results that
-// are rounded to bf16.  One path for every x, two special-function operations; erff diverges into two branches of some forty instructions.
-__device__ __forceinline__ float phi_tail(float ax) {
-  const float z = ax * 0.70710678118654752f;
-  const float t = __fdividef(1.f, fmaf(0.3275911f, z, 1.f));
-  const float poly = t * fmaf(t, fmaf(t, fmaf(t, fmaf(t, 1.061405429f, -1.453152027f), 1.421413741f), -0.284496736f), 0.254829592f);
-  return 0.5f * poly * __expf(-z * z);
-}
-__device__ __forceinline__ float gelu(float x, float) { return 0.5f * x * (1.f + erff(x * 0.70710678118654752f)); }
-__device__ __forceinline__ float gelu(float x, __nv_bfloat16) {
-  const float tail = x * phi_tail(fabsf(x));
-  return x < 0.f ? tail : x - tail;
 }
 
 // x <- x * Phi(x) (the exact GELU), in place.  9.2k x 4096 bf16 (75 MB in, 75 MB out): 37 us with erff.
@@ -231,10 +220,10 @@ using namespace tdb;
 extern "C" {
 
 int tdb_add_layernorm(const void* x, const void* res, const void* w, const void* b, float eps, int64_t rows, int hidden, int dtype,
-                      void* out, void* stream) {
+                      void* out, int early, void* stream) {
   if (rows == 0) return TDB_OK;
-  return dtype == TDB_DTYPE_F32 ? launch_add_layernorm_t<float>(x, res, w, b, eps, rows, hidden, out, (cudaStream_t)stream)
-                                : launch_add_layernorm_t<__nv_bfloat16>(x, res, w, b, eps, rows, hidden, out, (cudaStream_t)stream);
+  return dtype == TDB_DTYPE_F32 ? launch_add_layernorm_t<float>(x, res, w, b, eps, rows, hidden, out, early, (cudaStream_t)stream)
+                                : launch_add_layernorm_t<__nv_bfloat16>(x, res, w, b, eps, rows, hidden, out, early, (cudaStream_t)stream);
 }
 
 int tdb_gelu(void* x, int64_t elements, int dtype, void* stream) {

@@ -545,14 +545,27 @@ class Linear {
                                   ws_.data_ptr(), WORKSPACE, stream_) == CUBLAS_STATUS_SUCCESS;
     return good;
   }
-  void operator()(Tensor& y, const Tensor& x, const Tensor& w, const Tensor& b) {
+  // gelu: y goes through it.  early: see tdb_skinny.
+  void operator()(Tensor& y, const Tensor& x, const Tensor& w, const Tensor& b, bool gelu = false, bool early = true) {
+    const int64_t T = x.size(0), k = x.size(1), n = w.size(0);
+    if (own_ && !(misaligned(x) | misaligned(w) | misaligned(b) | misaligned(y)) && tdb_skinny_applies(T, k, n)) {
+      check(tdb_skinny(x.data_ptr(), w.data_ptr(), b.data_ptr(), (int)T, (int)k, (int)n, gelu, early, y.data_ptr(), stream_));
+      return;
+    }
+    product(y, x, w, b);
+    if (gelu) check(tdb_gelu(y.data_ptr(), y.numel(), dtype_code(y), stream_));
+  }
+  static constexpr size_t WORKSPACE = 32u << 20;
+
+
+ private:
+  static bool misaligned(const Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) & 15; }
+  static void check(int rc) { TORCH_CHECK(rc == 0, "libtdb_b200: ", tdb_last_error(), " (code ", rc, ")"); }
+  void product(Tensor& y, const Tensor& x, const Tensor& w, const Tensor& b) {
     if (try_run(y, x, w, b)) return;
     TORCH_CHECK(!recording_, "not recordable");
     at::addmm_out(y, b, x, w.t());
   }
-  static constexpr size_t WORKSPACE = 32u << 20;
-
- private:
   struct Plan {
     bool usable = false;
     cublasLtMatmulDesc_t op = nullptr;
@@ -690,7 +703,7 @@ class Encoder {
   }
   static void ok(int rc) { TORCH_CHECK(rc == 0, "libtdb_b200: ", tdb_last_error(), " (code ", rc, ")"); }
   static void add_norm(Tensor& x, const Tensor& res, const Tensor& w, const Tensor& b, double eps, int code, cudaStream_t stream) {
-    ok(tdb_add_layernorm(x.data_ptr(), res.data_ptr(), w.data_ptr(), b.data_ptr(), (float)eps, x.size(0), (int)x.size(1), code, x.data_ptr(), stream));
+    ok(tdb_add_layernorm(x.data_ptr(), res.data_ptr(), w.data_ptr(), b.data_ptr(), (float)eps, x.size(0), (int)x.size(1), code, x.data_ptr(), 1, stream));
   }
   // The buffers of one pass: every layer writes over those of the layer before it.
   struct Scratch {
@@ -709,10 +722,10 @@ class Encoder {
 
   template <typename Attention>
   void layer(const Layer& l, const Tensor& x, Tensor& out, Scratch& s, const OptTensor& cu_seqlens, int64_t length, Linear& linear,
-             cudaStream_t stream, bool tiles_listed, Attention attention) {
+             cudaStream_t stream, bool not_first, Attention attention) {
     const int code = dtype_code(x);
     const int64_t T = x.size(0), hidden = x.size(1), e = x.element_size();
-    linear(s.qkv, x, l.qkv_w, l.qkv_b);
+    linear(s.qkv, x, l.qkv_w, l.qkv_b, false, not_first);      // a pass's first kernel starts behind all that came before
     tdb::AttnParams p{};
     char* base = static_cast<char*>(s.qkv.data_ptr());
     p.q = base; p.k = base + e * hidden; p.v = base + 2 * e * hidden; p.o = s.ctx.data_ptr();
@@ -721,7 +734,7 @@ class Encoder {
     p.H = heads_; p.D = (int)(hidden / heads_); p.sm_scale = (float)l.sm_scale; p.total_tokens = T;
     if (cu_seqlens) {
       p.varlen = 1; p.cu_seqlens = cu_seqlens->data_ptr<int32_t>(); p.n_seqs = (int)(cu_seqlens->numel() - 1); p.L = (int)length;
-      p.workspace = s.tiles.data_ptr(); p.workspace_bytes = s.tiles.numel(); p.tiles_listed = tiles_listed;
+      p.workspace = s.tiles.data_ptr(); p.workspace_bytes = s.tiles.numel(); p.tiles_listed = not_first;
     } else {
       p.n_seqs = (int)(T / length); p.L = (int)length;
       p.q_sb = p.k_sb = p.v_sb = 3 * hidden * length; p.o_sb = hidden * length;
@@ -729,8 +742,7 @@ class Encoder {
     attention(p);
     linear(s.y, s.ctx, l.out_w, l.out_b);
     add_norm(s.y, x, l.ln1_w, l.ln1_b, l.eps1, code, stream);
-    linear(s.u, s.y, l.up_w, l.up_b);
-    ok(tdb_gelu(s.u.data_ptr(), s.u.numel(), code, stream));
+    linear(s.u, s.y, l.up_w, l.up_b, true);
     linear(out, s.u, l.down_w, l.down_b);
     add_norm(out, s.y, l.ln2_w, l.ln2_b, l.eps2, code, stream);
   }
@@ -747,6 +759,7 @@ class Encoder {
     std::vector<const void*> weights;
     cudaGraphExec_t exec = nullptr;
     uint64_t used = 0;
+    bool refused = false;                                         // could not be recorded: stays eager until the weights move
     ~Graph() {
       if (!exec && slot < 0) return;
       int before = 0;
@@ -804,11 +817,15 @@ class Encoder {
       }
       it = graphs_.emplace(key, std::make_unique<Graph>()).first;
     }
-    Graph& g = *it->second;
-    if (!g.exec || g.weights != weight_pointers()) {
+    const bool same = it->second->weights == weight_pointers();
+    if (same && it->second->refused) return {};
+    if (!same || !it->second->exec) {
       it->second = std::make_unique<Graph>();
       if (!record(*it->second, x, cu_seqlens, length, stream)) {
-        graphs_.erase(key);
+        it->second = std::make_unique<Graph>();
+        it->second->refused = true;
+        it->second->weights = weight_pointers();
+        it->second->used = ++uses_;
         return {};
       }
     }
@@ -835,9 +852,9 @@ class Encoder {
     cudaStream_t side = nullptr;
     cudaGraph_t graph = nullptr;
     if (cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking) != cudaSuccess) return false;
+    Linear linear(x, side, g.lt_ws, true);                        // makes the library handle, which a capture would not allow
     bool good = cudaStreamBeginCapture(side, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
     if (good) {
-      Linear linear(x, side, g.lt_ws, true);
       try {
         Tensor in = g.x;
         for (size_t i = 0; good && i < layers_.size(); ++i) {
@@ -984,7 +1001,13 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("add_layernorm", [](const Tensor& x, const Tensor& res, const Tensor& w, const Tensor& b, double eps, const Tensor& out) {
     c10::cuda::CUDAGuard guard(x.device());
     return tdb_add_layernorm(x.data_ptr(), res.data_ptr(), w.data_ptr(), b.data_ptr(), (float)eps, x.size(0), (int)x.size(1), dtype_code(x),
-                             out.data_ptr(), c10::cuda::getCurrentCUDAStream().stream());
+                             out.data_ptr(), 0, c10::cuda::getCurrentCUDAStream().stream());
+  });
+  m.def("skinny", [](const Tensor& x, const Tensor& w, const Tensor& b, bool gelu, const Tensor& y) {
+    c10::cuda::CUDAGuard guard(x.device());
+    if (!tdb_skinny_applies(x.size(0), x.size(1), w.size(0))) return (int)TDB_ERR_SHAPE;
+    return tdb_skinny(x.data_ptr(), w.data_ptr(), b.data_ptr(), (int)x.size(0), (int)x.size(1), (int)w.size(0), gelu, 0, y.data_ptr(),
+                      c10::cuda::getCurrentCUDAStream().stream());
   });
   m.def("gelu_", [](const Tensor& x) {
     c10::cuda::CUDAGuard guard(x.device());

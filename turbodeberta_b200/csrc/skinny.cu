@@ -1,0 +1,129 @@
+// y = x W^T + b (optionally through GELU) in bf16 for a handful of tokens: the projections of a short request.
+//
+// Bound by the latency of one trip to memory for the weights (1.2 to 9.4 MB per projection) and by the launch in front of it,
+// so the weights do not wait for anything: a block owns 8 or 16 output features, its eight warps share the columns, and every
+// thread has its part of W in registers before it waits for the kernel in front, which may still be running (the launcher
+// says which launches may).  Then it reads x (L2), multiplies with the warp-level tensor instruction, and the warps' partial
+// sums are added up through shared memory.
+// The order of the columns inside a product is free as long as x and W share it, so a thread's fragments of two k16 steps are
+// one 16-byte load: lane % 4 takes eight consecutive columns of every 32.
+#include "attn_warp_mma.cuh"
+#include "gelu.cuh"
+
+namespace tdb {
+
+namespace {
+
+constexpr int WARPS = 8, KB = 32;                    // columns of one 16-byte load by four lanes
+
+// MT: tiles of 16 tokens; NF: groups of 8 features; NB: blocks of 32 columns per warp.
+template <int MT, int NF, int NB, bool GELU>
+__global__ void __launch_bounds__(WARPS * 32) skinny_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ w,
+                                                            const __nv_bfloat16* __restrict__ bias, int T, int K, int N,
+                                                            __nv_bfloat16* y) {     // x, y: no __restrict__, see encoder.cu
+  __shared__ float part[WARPS][MT * 16][NF * 8];
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, g = lane / 4, t = lane % 4;
+  const int n0 = blockIdx.x * NF * 8, blocks = K / KB;
+  uint4 wf[NB][NF];
+#pragma unroll
+  for (int i = 0; i < NB; ++i)
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+      const int b = warp + WARPS * i, n = n0 + 8 * f + g;
+      wf[i][f] = make_uint4(0, 0, 0, 0);
+      if (b < blocks && n < N) wf[i][f] = __ldg(reinterpret_cast<const uint4*>(w + (int64_t)n * K + b * KB) + t);
+    }
+  wait_for_stream();
+  let_next_start();
+  float acc[MT][NF][4];
+#pragma unroll
+  for (int m = 0; m < MT; ++m)
+#pragma unroll
+    for (int f = 0; f < NF; ++f)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[m][f][e] = 0.f;
+#pragma unroll
+  for (int i = 0; i < NB; ++i) {
+    const int b = warp + WARPS * i;
+    if (b >= blocks) break;
+    uint4 a[MT][2];                                  // rows beyond T repeat the last one; their results are dropped
+#pragma unroll
+    for (int m = 0; m < MT; ++m)
+#pragma unroll
+      for (int r = 0; r < 2; ++r)
+        a[m][r] = *(reinterpret_cast<const uint4*>(x + (int64_t)min(16 * m + g + 8 * r, T - 1) * K + b * KB) + t);
+#pragma unroll
+    for (int m = 0; m < MT; ++m) {
+      const uint32_t lo[4] = {a[m][0].x, a[m][1].x, a[m][0].y, a[m][1].y}, hi[4] = {a[m][0].z, a[m][1].z, a[m][0].w, a[m][1].w};
+#pragma unroll
+      for (int f = 0; f < NF; ++f) {
+        mma(acc[m][f], lo, wf[i][f].x, wf[i][f].y);
+        mma(acc[m][f], hi, wf[i][f].z, wf[i][f].w);
+      }
+    }
+  }
+#pragma unroll
+  for (int m = 0; m < MT; ++m)
+#pragma unroll
+    for (int f = 0; f < NF; ++f)
+#pragma unroll
+      for (int r = 0; r < 2; ++r)
+        *reinterpret_cast<float2*>(&part[warp][16 * m + g + 8 * r][8 * f + 2 * t]) = make_float2(acc[m][f][2 * r], acc[m][f][2 * r + 1]);
+  __syncthreads();
+  constexpr int PAIRS = NF * 4;
+  for (int e = threadIdx.x; e < MT * 16 * PAIRS; e += WARPS * 32) {
+    const int row = e / PAIRS, c = 2 * (e % PAIRS);
+    if (row >= T || n0 + c >= N) continue;
+    const __nv_bfloat162 bb = *reinterpret_cast<const __nv_bfloat162*>(bias + n0 + c);
+    float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+    for (int k = 0; k < WARPS; ++k) {
+      const float2 v = *reinterpret_cast<const float2*>(&part[k][row][c]);
+      s0 += v.x; s1 += v.y;
+    }
+    s0 += __low2float(bb); s1 += __high2float(bb);
+    if (GELU) { s0 = gelu(s0, __nv_bfloat16()); s1 = gelu(s1, __nv_bfloat16()); }
+    *reinterpret_cast<uint32_t*>(y + (int64_t)row * N + n0 + c) = pack2(s0, s1);
+  }
+}
+
+template <int MT, int NF, int NB>
+cudaError_t launch(const void* x, const void* w, const void* b, int T, int K, int N, bool gelu, bool early, void* y, cudaStream_t s) {
+  const dim3 grid((N + 8 * NF - 1) / (8 * NF));
+  using B = __nv_bfloat16;
+  return launch_stream(gelu ? skinny_kernel<MT, NF, NB, true> : skinny_kernel<MT, NF, NB, false>, grid, WARPS * 32, 0, s, early,
+                       (const B*)x, (const B*)w, (const B*)b, T, K, N, (B*)y);
+}
+
+template <int MT>
+cudaError_t launch_rows(const void* x, const void* w, const void* b, int T, int K, int N, bool gelu, bool early, void* y, cudaStream_t s) {
+  const int nb = (K / KB + WARPS - 1) / WARPS;
+  // 16 features per block read x half as often; 8 where 16 would leave SMs without a block or the registers without room.
+  if (nb <= 4) return N >= 148 * 16 - 64 ? launch<MT, 2, 4>(x, w, b, T, K, N, gelu, early, y, s) : launch<MT, 1, 4>(x, w, b, T, K, N, gelu, early, y, s);
+  if (nb <= 8) return launch<MT, 1, 8>(x, w, b, T, K, N, gelu, early, y, s);
+  if (nb <= 12) return launch<MT, 1, 12>(x, w, b, T, K, N, gelu, early, y, s);
+  return launch<MT, 1, 16>(x, w, b, T, K, N, gelu, early, y, s);
+}
+
+}  // namespace
+
+}  // namespace tdb
+
+using namespace tdb;
+
+extern "C" {
+
+// Every block reads all of x, so the line lies where that costs more than the library's tiles do.  One projection, weights from
+// memory, K 3072 and N 768, this kernel against the library's: 16 tokens 5.6 and 7.4 us, 32 tokens 6.3 and 6.7, 64 tokens 7.6
+// and 6.6; K 768 and N 2304: 3.0 and 3.6, 4.1 and 4.1, 5.1 and 4.1.  A pass of the base model, before and after: 8 tokens 531 and 445 us,
+// 16 tokens 512 and 449, 32 tokens 507 and 495; of the large one: 16 tokens 1057 and 884, 32 tokens 1000 and 999.  K up to what a warp's registers hold.
+int tdb_skinny_applies(int64_t T, int64_t K, int64_t N) { return T <= SKINNY_TOKENS && K % KB == 0 && K <= KB * WARPS * 16 && N % 8 == 0; }
+
+int tdb_skinny(const void* x, const void* w, const void* b, int T, int K, int N, int gelu, int early, void* y, void* stream) {
+  cudaStream_t s = (cudaStream_t)stream;
+  const cudaError_t e = T <= 16 ? launch_rows<1>(x, w, b, T, K, N, gelu, early, y, s)
+                                : launch_rows<2>(x, w, b, T, K, N, gelu, early, y, s);
+  return cuda_fail(e, "skinny projection launch");
+}
+
+}  // extern "C"
