@@ -15,8 +15,8 @@
 // twice as many), and nothing has to be skewed or gathered afterwards.  Operand rows are staged fp32, 36-word pitch, half a
 // head (32 columns) at a time: eight consecutive rows fall on different banks, and four blocks fit on an SM, which cover
 // each other's loads.  The rows of one query tile stay inside one warp, so the softmax needs shuffles only.
-// One call of 8 x (48..387) fp32 tokens with 12 heads and both terms: 245 us, 23 TFLOP/s (one warp per query row, keys spread
-// over its lanes, every operand read row by row through L1: 1852 us).
+// One call of 8 x (48..387) fp32 tokens with 12 heads and both terms: 217 us, 26 TFLOP/s (one warp per query row, keys spread
+// over its lanes, every operand read row by row through L1: 1852 us; with one multiply-add per instruction: 234 us).
 #include "attn_blocks.cuh"
 #include <math_constants.h>
 
@@ -61,9 +61,25 @@ __device__ __forceinline__ void staged() {
   __syncthreads();
 }
 
-__device__ __forceinline__ void fma4(float& acc, const float4& a, const float4& b) {
-  acc = fmaf(a.x, b.x, acc); acc = fmaf(a.y, b.y, acc); acc = fmaf(a.z, b.z, acc); acc = fmaf(a.w, b.w, acc);
+// Two fp32 multiply-adds per instruction, each rounded as fmaf rounds.  A pair holds the sums over even and odd columns.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pair(float a, float b) {
+  f32x2 v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
+  return v;
 }
+__device__ __forceinline__ float2 halves(f32x2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ void fma2(f32x2& acc, f32x2 a, f32x2 b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b)); }
+struct Four { f32x2 lo, hi; };                       // four columns
+__device__ __forceinline__ Four load4(const float* p) {
+  const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
+  return {v.x, v.y};
+}
+__device__ __forceinline__ void fma4(f32x2& acc, const Four& a, const Four& b) { fma2(acc, a.lo, b.lo); fma2(acc, a.hi, b.hi); }
 
 __device__ __forceinline__ void store4(float* d, float a, float b, float c, float e) { *reinterpret_cast<float4*>(d) = make_float4(a, b, c, e); }
 __device__ __forceinline__ void store4(__nv_bfloat16* d, float a, float b, float c, float e) {
@@ -114,22 +130,23 @@ __global__ void __launch_bounds__(THREADS, 4) attn_simt_kernel(const AttnParams 
   const int dm = p.idx_delta_max;
   auto clamped = [&](int delta) { return delta < -dm ? 0 : (delta > dm ? 2 * dm : delta + dm); };
 
-  float o[R][8], m[R], l[R];
+  f32x2 o[R][4];                                     // eight output columns
+  float m[R], l[R];
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     m[r] = -CUDART_INF_F; l[r] = 0.f;
 #pragma unroll
-    for (int c = 0; c < 8; ++c) o[r][c] = 0.f;
+    for (int c = 0; c < 4; ++c) o[r][c] = 0ull;
   }
 
   if (q0 < len) {
     stage_rows<T, 64, DP>(sQ, QT, qb, [&](int row) { return q0 + row < len ? qb + (int64_t)(q0 + row) * p.q_st : nullptr; });
     for (int k0 = 0; k0 < len; k0 += KT) {
-      float acc[R][8];
+      f32x2 acc2[R][8];
 #pragma unroll
       for (int r = 0; r < R; ++r)
 #pragma unroll
-        for (int c = 0; c < 8; ++c) acc[r][c] = 0.f;
+        for (int c = 0; c < 8; ++c) acc2[r][c] = 0ull;
 #pragma unroll 1
       for (int half = 0; half < 2; ++half) {
         const int d0 = half * HALF;
@@ -145,39 +162,44 @@ __global__ void __launch_bounds__(THREADS, 4) attn_simt_kernel(const AttnParams 
         const int x0 = ti - tj + (KT - 1) - 56;      // table row of (r, s) is x0 + 8 (r - s + 7)
 #pragma unroll 1
         for (int d = 0; d < HALF; d += 4) {
-          float4 kf[8];
+          Four kf[8];
 #pragma unroll
-          for (int c = 0; c < 8; ++c) kf[c] = *reinterpret_cast<const float4*>(kp + 8 * c * HP + d);
+          for (int c = 0; c < 8; ++c) kf[c] = load4(kp + 8 * c * HP + d);
           if (TABLES && krh) {
-            float4 t[R + 7];
+            Four t[R + 7];
 #pragma unroll
-            for (int x = 0; x < R + 7; ++x) t[x] = *reinterpret_cast<const float4*>(sKr + (x0 + 8 * x) * HP + d);
+            for (int x = 0; x < R + 7; ++x) t[x] = load4(sKr + (x0 + 8 * x) * HP + d);
 #pragma unroll
             for (int r = 0; r < R; ++r) {
-              const float4 qf = *reinterpret_cast<const float4*>(qp + 8 * r * DP + d);
+              const Four qf = load4(qp + 8 * r * DP + d);
 #pragma unroll
-              for (int c = 0; c < 8; ++c) { fma4(acc[r][c], qf, kf[c]); fma4(acc[r][c], qf, t[r - c + 7]); }
+              for (int c = 0; c < 8; ++c) { fma4(acc2[r][c], qf, kf[c]); fma4(acc2[r][c], qf, t[r - c + 7]); }
             }
           } else {
 #pragma unroll
             for (int r = 0; r < R; ++r) {
-              const float4 qf = *reinterpret_cast<const float4*>(qp + 8 * r * DP + d);
+              const Four qf = load4(qp + 8 * r * DP + d);
 #pragma unroll
-              for (int c = 0; c < 8; ++c) fma4(acc[r][c], qf, kf[c]);
+              for (int c = 0; c < 8; ++c) fma4(acc2[r][c], qf, kf[c]);
             }
           }
           if (TABLES && qrh) {
-            float4 t[R + 7];
+            Four t[R + 7];
 #pragma unroll
-            for (int x = 0; x < R + 7; ++x) t[x] = *reinterpret_cast<const float4*>(sQr + (x0 + 8 * x) * HP + d);
+            for (int x = 0; x < R + 7; ++x) t[x] = load4(sQr + (x0 + 8 * x) * HP + d);
 #pragma unroll
             for (int r = 0; r < R; ++r)
 #pragma unroll
-              for (int c = 0; c < 8; ++c) fma4(acc[r][c], kf[c], t[r - c + 7]);
+              for (int c = 0; c < 8; ++c) fma4(acc2[r][c], kf[c], t[r - c + 7]);
           }
         }
         __syncthreads();
       }
+      float acc[R][8];
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int c = 0; c < 8; ++c) { const float2 v = halves(acc2[r][c]); acc[r][c] = v.x + v.y; }
       // V replaces the operand rows while the softmax runs
       stage_rows<T, 64, DP>(sV, KT, vb, [&](int row) { return k0 + row < len ? vb + (int64_t)(k0 + row) * p.v_st : nullptr; });
 #pragma unroll
@@ -211,7 +233,7 @@ __global__ void __launch_bounds__(THREADS, 4) attn_simt_kernel(const AttnParams 
         }
         l[r] = l[r] * corr + sum;
 #pragma unroll
-        for (int c = 0; c < 8; ++c) o[r][c] *= corr;
+        for (int c = 0; c < 4; ++c) { const float2 v = halves(o[r][c]); o[r][c] = pair(v.x * corr, v.y * corr); }
       }
       staged();                                      // also makes the warp's own rows of P visible to its lanes
 #pragma unroll 1
@@ -221,15 +243,12 @@ __global__ void __launch_bounds__(THREADS, 4) attn_simt_kernel(const AttnParams 
         for (int r = 0; r < R; ++r) pf[r] = *reinterpret_cast<const float4*>(sP + (ti + 8 * r) * DP + j);
 #pragma unroll
         for (int jj = 0; jj < 4; ++jj) {
-          const float4 a = *reinterpret_cast<const float4*>(sV + (j + jj) * DP + 4 * tj);
-          const float4 c = *reinterpret_cast<const float4*>(sV + (j + jj) * DP + 32 + 4 * tj);
+          const Four a = load4(sV + (j + jj) * DP + 4 * tj), c = load4(sV + (j + jj) * DP + 32 + 4 * tj);
 #pragma unroll
           for (int r = 0; r < R; ++r) {
             const float w = jj == 0 ? pf[r].x : jj == 1 ? pf[r].y : jj == 2 ? pf[r].z : pf[r].w;
-            o[r][0] = fmaf(w, a.x, o[r][0]); o[r][1] = fmaf(w, a.y, o[r][1]);
-            o[r][2] = fmaf(w, a.z, o[r][2]); o[r][3] = fmaf(w, a.w, o[r][3]);
-            o[r][4] = fmaf(w, c.x, o[r][4]); o[r][5] = fmaf(w, c.y, o[r][5]);
-            o[r][6] = fmaf(w, c.z, o[r][6]); o[r][7] = fmaf(w, c.w, o[r][7]);
+            const f32x2 ww = pair(w, w);
+            fma2(o[r][0], ww, a.lo); fma2(o[r][1], ww, a.hi); fma2(o[r][2], ww, c.lo); fma2(o[r][3], ww, c.hi);
           }
         }
       }
@@ -247,8 +266,9 @@ __global__ void __launch_bounds__(THREADS, 4) attn_simt_kernel(const AttnParams 
     const float inv = valid ? 1.f / sum : 0.f;
     T* const orow = ob + (int64_t)qi * p.o_st;
     if (valid) {
-      store4(orow + 4 * tj, o[r][0] * inv, o[r][1] * inv, o[r][2] * inv, o[r][3] * inv);
-      store4(orow + 32 + 4 * tj, o[r][4] * inv, o[r][5] * inv, o[r][6] * inv, o[r][7] * inv);
+      const float2 a = halves(o[r][0]), b2 = halves(o[r][1]), c = halves(o[r][2]), d = halves(o[r][3]);
+      store4(orow + 4 * tj, a.x * inv, a.y * inv, b2.x * inv, b2.y * inv);
+      store4(orow + 32 + 4 * tj, c.x * inv, c.y * inv, d.x * inv, d.y * inv);
     } else {
       store4(orow + 4 * tj, 0.f, 0.f, 0.f, 0.f);
       store4(orow + 32 + 4 * tj, 0.f, 0.f, 0.f, 0.f);
