@@ -106,6 +106,7 @@ __global__ void __launch_bounds__(THREADS, 4) attn_simt_kernel(const AttnParams 
   float* const sKr = sK + KT * HP;                   // [XR][HP]
   float* const sQr = sKr + XR * HP;                  // [XR][HP]
   float* const sV = sK;                              // [KT][DP], over the three above
+  __shared__ int sRow[XR];                           // first element of the table row of distance q0 - k0 - 63 + x
 
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int ti = warp * 4 + lane / 8, tj = lane % 8;
@@ -141,6 +142,12 @@ __global__ void __launch_bounds__(THREADS, 4) attn_simt_kernel(const AttnParams 
 
   if (q0 < len) {
     stage_rows<T, 64, DP>(sQ, QT, qb, [&](int row) { return q0 + row < len ? qb + (int64_t)(q0 + row) * p.q_st : nullptr; });
+    auto table_rows = [&](int k0) {
+      if (TABLES)
+        for (int x = threadIdx.x; x < XR; x += THREADS) sRow[x] = p.idx[clamped(q0 - k0 - (KT - 1) + x)] * 64;
+    };
+    table_rows(0);
+    __syncthreads();
     for (int k0 = 0; k0 < len; k0 += KT) {
       f32x2 acc2[R][8];
 #pragma unroll
@@ -152,7 +159,7 @@ __global__ void __launch_bounds__(THREADS, 4) attn_simt_kernel(const AttnParams 
         const int d0 = half * HALF;
         stage_rows<T, HALF, HP>(sK, KT, kb, [&](int row) { return k0 + row < len ? kb + (int64_t)(k0 + row) * p.k_st + d0 : nullptr; });
         if (TABLES) {
-          auto table_row = [&](const T* t, int x) { return t + (int64_t)p.idx[clamped(q0 - k0 - (KT - 1) + x)] * 64 + d0; };
+          auto table_row = [&](const T* t, int x) { return t + sRow[x] + d0; };
           if (krh) stage_rows<T, HALF, HP>(sKr, XR, krh, [&](int x) { return table_row(krh, x); });
           if (qrh) stage_rows<T, HALF, HP>(sQr, XR, qrh, [&](int x) { return table_row(qrh, x); });
         }
@@ -200,7 +207,7 @@ __global__ void __launch_bounds__(THREADS, 4) attn_simt_kernel(const AttnParams 
       for (int r = 0; r < R; ++r)
 #pragma unroll
         for (int c = 0; c < 8; ++c) { const float2 v = halves(acc2[r][c]); acc[r][c] = v.x + v.y; }
-      // V replaces the operand rows while the softmax runs
+      table_rows(k0 + KT);                           // for the next tile; V replaces the operand rows while the softmax runs
       stage_rows<T, 64, DP>(sV, KT, vb, [&](int row) { return k0 + row < len ? vb + (int64_t)(k0 + row) * p.v_st : nullptr; });
 #pragma unroll
       for (int r = 0; r < R; ++r) {
