@@ -8,10 +8,12 @@ namespace tdb {
 // relative to the value 5e-5 down to x = -3 and 2e-3 down to x = -5, where 1 + erf(x) in fp32 is off by 5e-2): for results that
 // are rounded to bf16.  One path for every x, two special-function operations; erff diverges into two branches of some forty instructions.
 __device__ __forceinline__ float phi_tail(float ax) {
-  const float z = ax * 0.70710678118654752f;
-  const float t = __fdividef(1.f, fmaf(0.3275911f, z, 1.f));
-  const float poly = t * fmaf(t, fmaf(t, fmaf(t, fmaf(t, 1.061405429f, -1.453152027f), 1.421413741f), -0.284496736f), 0.254829592f);
-  return 0.5f * poly * __expf(-z * z);
+  float t, e;                                        // 1 / (1 + 0.3275911 z) and exp(-z^2), z = ax / sqrt 2, one instruction each
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t) : "f"(fmaf(0.3275911f * 0.70710678118654752f, ax, 1.f)));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(ax * ax * (-0.5f * 1.4426950408889634f)));
+  // the formula's coefficients with the half folded in
+  const float poly = t * fmaf(t, fmaf(t, fmaf(t, fmaf(t, 0.5307027145f, -0.7265760135f), 0.7107068705f), -0.142248368f), 0.127414796f);
+  return poly * e;
 }
 __device__ __forceinline__ float gelu(float x, float) { return 0.5f * x * (1.f + erff(x * 0.70710678118654752f)); }
 __device__ __forceinline__ float gelu(float x, __nv_bfloat16) {
