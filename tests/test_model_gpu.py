@@ -265,7 +265,7 @@ def _generic_route(model, **kw):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("lengths,L", [([1], 1), ([128, 128], 128), ([129, 1, 64], 129), ([33, 0, 7, 200], 200)])
+@pytest.mark.parametrize("lengths,L", [([1], 1), ([128, 128], 128), ([129, 1, 64], 129), ([33, 0, 7, 200], 200), ([64, 1, 0, 17], 64)])
 def test_native_layer_loop_matches_the_module_route(dtype, lengths, L):
     """The encoder's native loop against the modules it stands in for: one token, full rows, ragged rows, an empty row,
     holes in the mask; hooks and replaced parameters must be seen."""

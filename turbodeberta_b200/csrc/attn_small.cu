@@ -1,4 +1,4 @@
-// Sequences of at most 64 tokens (padded form), bf16, projected tables: one block of four warps per sequence and head.
+// Sequences of at most 64 tokens, bf16, projected tables: one block of four warps per sequence and head.
 //
 // Such a call is bound by latency, not by any unit: one score tile per head.  The persistent tensor-memory kernel takes 7.3 us
 // for it (scheduler ring, tensor-memory allocation and a chain of nine hand-offs between its roles); here the tile is four
@@ -29,18 +29,27 @@ __global__ void __launch_bounds__(S_THREADS) attn_small_kernel(const AttnParams 
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, h = blockIdx.x, b = blockIdx.y;
   wait_for_stream();
   let_next_start();
-  int len = p.seqlens ? p.seqlens[b] : p.L;
-  len = len < 0 ? 0 : (len > p.L ? p.L : len);
-  const bf16* const qb = reinterpret_cast<const bf16*>(p.q) + b * p.q_sb + h * p.q_sh;
-  const bf16* const kb = reinterpret_cast<const bf16*>(p.k) + b * p.k_sb + h * p.k_sh;
-  const bf16* const vb = reinterpret_cast<const bf16*>(p.v) + b * p.v_sb + h * p.v_sh;
-  bf16* const ob = reinterpret_cast<bf16*>(p.o) + b * p.o_sb + h * p.o_sh;
-  float* const lse = p.lse ? p.lse + b * p.lse_sb + h * p.lse_sh : nullptr;
-  if (len == 0) {                                    // nothing but padding: zeros
-    for (int e = threadIdx.x; e < p.L * 8; e += S_THREADS)
+  int len, rows_out;                                 // valid tokens, rows that exist in the output
+  int64_t tok0 = 0;
+  int64_t seq = b;
+  if (p.varlen) {
+    tok0 = p.cu_seqlens[b]; seq = 0;
+    rows_out = len = min(p.cu_seqlens[b + 1] - (int)tok0, ST);
+  } else {
+    len = p.seqlens ? p.seqlens[b] : p.L;
+    len = len < 0 ? 0 : (len > p.L ? p.L : len);
+    rows_out = p.L;
+  }
+  const bf16* const qb = reinterpret_cast<const bf16*>(p.q) + seq * p.q_sb + tok0 * p.q_st + h * p.q_sh;
+  const bf16* const kb = reinterpret_cast<const bf16*>(p.k) + seq * p.k_sb + tok0 * p.k_st + h * p.k_sh;
+  const bf16* const vb = reinterpret_cast<const bf16*>(p.v) + seq * p.v_sb + tok0 * p.v_st + h * p.v_sh;
+  bf16* const ob = reinterpret_cast<bf16*>(p.o) + seq * p.o_sb + tok0 * p.o_st + h * p.o_sh;
+  float* const lse = p.lse ? p.lse + seq * p.lse_sb + h * p.lse_sh + tok0 : nullptr;
+  if (len <= 0) {                                    // nothing but padding: zeros
+    for (int e = threadIdx.x; e < rows_out * 8; e += S_THREADS)
       *reinterpret_cast<uint4*>(ob + (e >> 3) * p.o_st + (e & 7) * 8) = make_uint4(0, 0, 0, 0);
     if (lse)
-      for (int e = threadIdx.x; e < p.L; e += S_THREADS) lse[e] = 0.f;
+      for (int e = threadIdx.x; e < rows_out; e += S_THREADS) lse[e] = 0.f;
     return;
   }
   stage(sQ, qb, p.q_st, len);
@@ -162,10 +171,10 @@ __global__ void __launch_bounds__(S_THREADS) attn_small_kernel(const AttnParams 
     }
   }
   // padded query rows: zeros
-  for (int e = threadIdx.x + len * 8; e < p.L * 8; e += S_THREADS)
+  for (int e = threadIdx.x + len * 8; e < rows_out * 8; e += S_THREADS)
     *reinterpret_cast<uint4*>(ob + (e >> 3) * p.o_st + (e & 7) * 8) = make_uint4(0, 0, 0, 0);
   if (lse)
-    for (int e = threadIdx.x + len; e < p.L; e += S_THREADS) lse[e] = 0.f;
+    for (int e = threadIdx.x + len; e < rows_out; e += S_THREADS) lse[e] = 0.f;
 }
 
 template <bool C2P, bool P2C>
@@ -181,9 +190,9 @@ int launch_small(const AttnParams& p, cudaStream_t s) {
 
 }  // namespace
 
-// The grid has one block per sequence and head; the packed form goes to the other kernel, which takes any lengths its offsets
-// may turn out to have.
-bool small_applicable(const AttnParams& p) { return !p.varlen && p.L <= ST && p.n_seqs <= 65535; }
+// The grid has one block per sequence and head.  Packed sequences only where the longest is known: with a caller's max_seqlen
+// they go to the other kernel, which takes any lengths the offsets may turn out to have.
+bool small_applicable(const AttnParams& p) { return (!p.varlen || p.lengths_known) && p.L <= ST && p.n_seqs <= 65535; }
 
 int launch_attn_small(const AttnParams& p, cudaStream_t s) {
   const bool c2p = p.flags & TDB_FLAG_C2P, p2c = p.flags & TDB_FLAG_P2C;

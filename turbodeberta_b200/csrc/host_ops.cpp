@@ -734,7 +734,7 @@ class Encoder {
     p.H = heads_; p.D = (int)(hidden / heads_); p.sm_scale = (float)l.sm_scale; p.total_tokens = T;
     if (cu_seqlens) {
       p.varlen = 1; p.cu_seqlens = cu_seqlens->data_ptr<int32_t>(); p.n_seqs = (int)(cu_seqlens->numel() - 1); p.L = (int)length;
-      p.workspace = s.tiles.data_ptr(); p.workspace_bytes = s.tiles.numel(); p.tiles_listed = not_first;
+      p.workspace = s.tiles.data_ptr(); p.workspace_bytes = s.tiles.numel(); p.tiles_listed = not_first; p.lengths_known = 1;
     } else {
       p.n_seqs = (int)(T / length); p.L = (int)length;
       p.q_sb = p.k_sb = p.v_sb = 3 * hidden * length; p.o_sb = hidden * length;

@@ -44,6 +44,7 @@ struct AttnParams {
   // Long sequences on the tensor cores: scratch for the softmax state that the kernel for near key tiles hands to the one for
   // far tiles, tdb_partial_floats() of fp32, part_ml behind part_o's tiles (null: one kernel does both).  split_sat is the launcher's own.
   float* part_o; float* part_ml; int split_sat;
+  int lengths_known;                                      // packed form: L is known to be the longest sequence's length
   int tiles_listed;                                       // packed form: the workspace already holds this batch's tile list
 };
 
