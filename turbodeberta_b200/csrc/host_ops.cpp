@@ -841,6 +841,8 @@ class Encoder {
     OptTensor cu;
     if (cu_seqlens) cu = g.cu = at::empty_like(*cu_seqlens);
     g.scratch = std::make_unique<Scratch>(*this, x, cu_seqlens);
+    for (auto w = lt_workspaces_.begin(); w != lt_workspaces_.end();)     // of streams whose last graph is gone
+      w = w->second.use_count() == 1 ? lt_workspaces_.erase(w) : std::next(w);
     Tensor& ws = lt_workspaces_[{g.dev, stream}];
     if (!ws.defined()) ws = at::empty({(int64_t)Linear::WORKSPACE}, x.options().dtype(at::kByte));
     g.lt_ws = ws;
