@@ -162,3 +162,29 @@ def test_mask_analysis_refresh_recomputes_lengths_without_changing_the_route():
     b = analyse_mask(m, 2, 6, refresh=True)
     assert b is not a and (b.all_ones, b.right_padded) == (False, True) and b.seqlens.tolist() == [6, 3]
     assert analyse_mask(m, 2, 6) is b                      # the refreshed analysis is what later calls see
+
+
+def _small_config(**kw):
+    from transformers import DebertaV2Config
+    return DebertaV2Config(**{**dict(vocab_size=50, hidden_size=128, num_hidden_layers=4, num_attention_heads=2,
+                                     intermediate_size=256, relative_attention=True, position_buckets=32,
+                                     max_relative_positions=64, norm_rel_ebd="layer_norm", share_att_key=True,
+                                     pos_att_type=["p2c", "c2p"], position_biased_input=False, type_vocab_size=0), **kw})
+
+
+@pytest.mark.parametrize("name,value", [("pos_att_type", ["c2p"]), ("pos_att_type", ["p2c"]), ("position_buckets", 16),
+                                        ("max_relative_positions", 128), ("num_attention_heads", 1)])
+def test_kept_tables_follow_the_modules_settings(name, value, monkeypatch):
+    """The tables that a layer keeps are those of its present settings, not of the ones it had when they were made."""
+    from turbodeberta_b200 import model as M
+    monkeypatch.setattr(M._relpos, "build_tables", lambda rel, **kw: {k: v for k, v in kw.items() if "weight" not in k and "bias" not in k})
+    sa = M.FlashDisentangledSelfAttention(_small_config()).eval()
+    rel = torch.randn(64, 128)
+    rel._tdb_stamp = (0, 1)
+    before = sa._relative_tables(rel, rel.dtype)
+    assert sa._relative_tables(rel, rel.dtype) is before and before["c2p"] and before["p2c"]
+    setattr(sa, name, value)
+    after = sa._relative_tables(rel, rel.dtype)
+    assert after == dict(before, **(dict(c2p="c2p" in value, p2c="p2c" in value) if name == "pos_att_type" else
+                                    {name.replace("num_attention_heads", "num_heads"): value}))
+    assert sa._relative_tables(rel, rel.dtype) is after

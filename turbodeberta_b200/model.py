@@ -198,7 +198,8 @@ class FlashDisentangledSelfAttention(DisentangledSelfAttention):
             qp = self.pos_query_proj if p2c else None
         stamp = getattr(rel_embeddings, "_tdb_stamp", None)
         params = [t for lin in (kp, qp) if lin is not None for t in (lin.weight, lin.bias) if t is not None]
-        key = (stamp, dtype, rel_embeddings.device, tuple((t.data_ptr(), t._version) for t in params))
+        key = (stamp, dtype, rel_embeddings.device, tuple((t.data_ptr(), t._version) for t in params), c2p, p2c,
+               self.share_att_key, self.num_attention_heads, self.position_buckets, self.max_relative_positions)
         if stamp is not None and self._tables is not None and self._tables_key == key:
             return self._tables
         rel = rel_embeddings.detach().to(dtype)
