@@ -188,3 +188,15 @@ def test_kept_tables_follow_the_modules_settings(name, value, monkeypatch):
     assert after == dict(before, **(dict(c2p="c2p" in value, p2c="p2c" in value) if name == "pos_att_type" else
                                     {name.replace("num_attention_heads", "num_heads"): value}))
     assert sa._relative_tables(rel, rel.dtype) is after
+
+
+def test_kept_relative_embeddings_follow_the_encoders_norm():
+    """eps alone changes no weight; without the norm in norm_rel_ebd the embeddings go as they are."""
+    from turbodeberta_b200 import model as M
+    enc = M.FlashDebertaV2Encoder(_small_config()).eval()
+    with torch.no_grad():
+        enc.get_rel_embedding()
+        enc.LayerNorm.eps = 0.5
+        assert torch.equal(enc.get_rel_embedding(), enc.LayerNorm(enc.rel_embeddings.weight))
+        enc.norm_rel_ebd = ["none"]
+        assert torch.equal(enc.get_rel_embedding(), enc.rel_embeddings.weight)

@@ -481,12 +481,13 @@ class FlashDebertaV2Encoder(DebertaV2Encoder):
     def get_rel_embedding(self):
         if not self.relative_attention:
             return None
-        params = [self.rel_embeddings.weight]
+        params, eps = [self.rel_embeddings.weight], None
         if "layer_norm" in self.norm_rel_ebd:
             params += [self.LayerNorm.weight, self.LayerNorm.bias]
+            eps = self.LayerNorm.eps
         if self.training or torch.is_grad_enabled():
             return super().get_rel_embedding()
-        key = tuple((t.data_ptr(), t._version, t.dtype, t.device) for t in params)
+        key = (eps, *((t.data_ptr(), t._version, t.dtype, t.device) for t in params))
         if self._rel_cache is None or key != self._rel_cache_key:
             rel = super().get_rel_embedding().detach()
             self._rel_stamp += 1
