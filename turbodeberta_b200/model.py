@@ -484,7 +484,7 @@ class FlashDebertaV2Encoder(DebertaV2Encoder):
         params, eps = [self.rel_embeddings.weight], None
         if "layer_norm" in self.norm_rel_ebd:
             params += [self.LayerNorm.weight, self.LayerNorm.bias]
-            eps = self.LayerNorm.eps
+            eps = getattr(self.LayerNorm, "eps", None)
         if self.training or torch.is_grad_enabled():
             return super().get_rel_embedding()
         key = (eps, *((t.data_ptr(), t._version, t.dtype, t.device) for t in params))
