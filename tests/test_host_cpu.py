@@ -200,3 +200,42 @@ def test_kept_relative_embeddings_follow_the_encoders_norm():
         assert torch.equal(enc.get_rel_embedding(), enc.LayerNorm(enc.rel_embeddings.weight))
         enc.norm_rel_ebd = ["none"]
         assert torch.equal(enc.get_rel_embedding(), enc.rel_embeddings.weight)
+
+
+def _set_eps(enc):
+    enc.layer[1].output.LayerNorm.eps = 0.25
+
+
+def _append_in_place(enc):
+    enc.layer[0].attention.self.pos_att_type.append("p2c")
+
+
+def _plain_gelu(enc):
+    act = enc.layer[3].intermediate.intermediate_act_fn
+    act.act = act._gelu_python
+
+
+@pytest.mark.parametrize("change,native_after", [
+    (lambda e: setattr(e, "layer", torch.nn.ModuleList(e.layer[:2])), True),          # pruned layers
+    (lambda e: setattr(e, "layer", torch.nn.ModuleList(list(e.layer)[::-1])), True),
+    (lambda e: e.layer.__delitem__(3), True),
+    (_set_eps, True), (_append_in_place, True), (_plain_gelu, False),
+    (lambda e: setattr(e.layer[0].attention.self, "share_att_key", False), True),
+    (lambda e: setattr(e.layer[2].attention.output, "dropout", torch.nn.ReLU().eval()), False)])
+def test_a_plan_is_of_the_encoders_present_layers(change, native_after):
+    """What the native loop was made from, and what it is made from after a change (on the CPU a stack without position
+    terms gets as far as that)."""
+    from turbodeberta_b200 import model as M
+    enc = M.FlashDebertaV2Encoder(_small_config(relative_attention=False, pos_att_type=[])).eval()
+    x = torch.zeros(1, 128)
+    with torch.no_grad():
+        first = enc._native_plan(x, None)
+        assert first.watch.holds() and enc._native_plan(x, None) is first and len(first.attns) == 4
+        change(enc)
+        kept = enc._native_plan(x, None)
+        assert kept is not first or not kept.watch.holds()       # the encoder's forward asks both
+        M._PLANS.pop(enc, None)
+        made = enc._native_plan(x, None)
+        assert (made is not None) == native_after
+        if native_after:
+            assert made.watch.holds() and made.attns == [layer.attention.self for layer in enc.layer]

@@ -421,3 +421,41 @@ def test_skinny_projection(tokens, columns, features, gelu):
     assert ((y.double() - want).abs() <= 5e-3 * want.abs() + 1e-5).all()
     big = torch.zeros(33, columns, device="cuda", dtype=torch.bfloat16)
     assert cabi.host.skinny(big, w, b, gelu, y) == cabi.ERR_SHAPE
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_changed_stacks_and_settings_are_seen(dtype):
+    """After a first pass: fewer layers in a new list, another eps, another set of position terms; each result is the
+    module route's for the model as it then is."""
+    from turbodeberta_b200.model import FlashDebertaV2Model
+    torch.manual_seed(17)
+    model = FlashDebertaV2Model(_cfg(num_hidden_layers=4)).eval().to("cuda", dtype)
+    ids = torch.randint(1, 500, (2, 40), device="cuda")
+    mask = torch.ones_like(ids)
+    mask[1, 20:] = 0
+    v = mask.bool()
+    enc = model.encoder
+
+    def prune():
+        enc.layer = torch.nn.ModuleList(enc.layer[:2])
+
+    def eps():
+        enc.layer[0].attention.output.LayerNorm.eps = 0.5
+
+    def terms():
+        for layer in enc.layer:
+            layer.attention.self.pos_att_type = ["c2p"]
+
+    tol = 1e-4 if dtype == torch.float32 else 4e-2
+    with torch.no_grad():
+        before = None
+        for change in (lambda: None, prune, eps, terms):
+            change()
+            for _ in range(3):                       # the last ones replay a recording in bf16
+                got = model(input_ids=ids, attention_mask=mask).last_hidden_state
+            want = _generic_route(model, input_ids=ids, attention_mask=mask).last_hidden_state
+            err = (got.float() - want.float())[v].abs().max().item()
+            assert err <= tol * want.float()[v].abs().max().item()
+            if before is not None:                   # and the change is no matter of rounding
+                assert (got.float() - before)[v].abs().max().item() > 4 * err
+            before = got.float()

@@ -444,15 +444,28 @@ Tensor mask_bytes(const Tensor& mask) {
 // A set of modules whose forward the native encoder stands in for, as it was when the plan was made.  The plan holds as long
 // as nobody has put a hook, a new child or parameter, or another forward on any of them, and all are in eval mode.  Checked
 // on every forward, so it follows pointers instead of looking names up: a module keeps its hook, child and parameter dicts.
+// settings: (module, attribute name) pairs of what else the plan was made from (a norm's eps, an attention's position terms).
 class Watch {
  public:
-  explicit Watch(const py::list& modules) {
+  Watch(const py::list& modules, const py::list& settings) {
     training_ = py::str("training");
     forward_ = py::str("forward");
+    const py::object list_type = py::module_::import("torch.nn").attr("ModuleList");
+    for (py::handle s : settings) {
+      auto [module, name] = s.cast<std::pair<py::object, py::str>>();
+      py::dict dict = module.attr("__dict__");
+      py::object value;                              // stays null where the attribute is absent
+      if (dict.contains(name)) {
+        value = dict[name];
+        if (py::isinstance<py::list>(value)) value = value.attr("copy")();       // may be changed in place
+      }
+      settings_.push_back({dict, name, value});
+    }
     for (py::handle m : modules) {
       Entry e;
       e.module = py::reinterpret_borrow<py::object>(m);
       e.type = Py_TYPE(m.ptr());
+      e.runs = (PyObject*)e.type != list_type.ptr();
       e.dict = m.attr("__dict__");
       for (const char* n : {"_forward_hooks", "_forward_pre_hooks"})       // no gradients here, so no backward hooks
         if (e.dict.contains(n)) e.hooks.push_back(e.dict[n]);
@@ -482,7 +495,7 @@ class Watch {
     for (const Entry& e : entries_) {
       if (Py_TYPE(e.module.ptr()) != e.type) return false;
       PyObject* d = e.dict.ptr();
-      if (PyDict_GetItem(d, training_.ptr()) != Py_False || PyDict_Contains(d, forward_.ptr())) return false;
+      if (e.runs && (PyDict_GetItem(d, training_.ptr()) != Py_False || PyDict_Contains(d, forward_.ptr()))) return false;
       for (const py::dict& h : e.hooks)
         if (PyDict_Size(h.ptr()) != 0) return false;
       for (const auto& [dict, values] : e.parts) {
@@ -492,6 +505,13 @@ class Watch {
         for (size_t i = 0; PyDict_Next(dict.ptr(), &pos, &k, &v); ++i)
           if (v != values[i].ptr()) return false;
       }
+    }
+    for (const Setting& s : settings_) {
+      PyObject* now = PyDict_GetItem(s.dict.ptr(), s.name.ptr());
+      if (now == s.value.ptr()) continue;
+      const int same = now && s.value ? PyObject_RichCompareBool(now, s.value.ptr(), Py_EQ) : 0;
+      if (same < 0) PyErr_Clear();                   // a value that does not compare is not the one of the plan
+      if (same != 1) return false;
     }
     return true;
   }
@@ -506,11 +526,17 @@ class Watch {
   struct Entry {
     py::object module;
     PyTypeObject* type;
+    bool runs;                                       // a list has no forward, and its mode means nothing (a new one trains)
     py::dict dict;
     std::vector<py::dict> hooks;
     std::vector<std::pair<py::dict, std::vector<py::object>>> parts;
   };
+  struct Setting {
+    py::dict dict;
+    py::object name, value;
+  };
   std::vector<Entry> entries_;
+  std::vector<Setting> settings_;
   py::object training_, forward_;
 };
 
@@ -992,7 +1018,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("expand_pair", &expand_pair);
   m.def("call_tables", &call_tables);
   m.def("drain_pending", &drain_pending);
-  py::class_<Watch>(m, "Watch").def(py::init<const py::list&>()).def("holds", &Watch::holds);
+  py::class_<Watch>(m, "Watch").def(py::init<const py::list&, const py::list&>(), py::arg("modules"), py::arg("settings") = py::list()).def("holds", &Watch::holds);
   py::class_<Encoder>(m, "Encoder")
       .def(py::init<int>())
       .def("add_layer", &Encoder::add_layer)

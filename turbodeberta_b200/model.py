@@ -280,6 +280,19 @@ class FlashDebertaV2Layer(DebertaV2Layer):
 # holds modules below its key, never the key itself, so it goes when the key goes.
 _PLANS: "weakref.WeakKeyDictionary" = weakref.WeakKeyDictionary()
 
+#: what the native loop takes over from an attention module besides its weights
+_ATTENTION_SETTINGS = ("num_attention_heads", "attention_head_size", "pos_att_type", "share_att_key", "relative_attention",
+                       "position_buckets", "max_relative_positions")
+
+
+class _EncoderPlan:
+    """The native form of an encoder's layer list, valid for that list object as long as ``watch`` holds."""
+    __slots__ = ("layers", "watch", "native", "attns", "stamp")
+
+    def __init__(self, layers, watch, native, attns):
+        self.layers, self.watch, self.native, self.attns = layers, watch, native, attns
+        self.stamp = None                    # of the relative embeddings behind the tables that ``native`` has
+
 
 class FlashDebertaV2Encoder(DebertaV2Encoder):
     """HF encoder whose layers use the fused attention.  Two host-side savings: the ``[L, L]`` relative
@@ -343,9 +356,9 @@ class FlashDebertaV2Encoder(DebertaV2Encoder):
 
     # -- the whole layer loop in one native call -------------------------------------------------------
     def _native_layers(self):
-        """(watched modules, native encoder, attention modules) for a stack made of the stock modules only, else None."""
+        """The plan of a stack made of the stock modules only, else None."""
         layers = list(self.layer)
-        native, attns = None, []
+        native, attns, settings = None, [], []
         for layer in layers:
             att, up, down = layer.attention, layer.intermediate, layer.output
             sa, so, act = att.self, att.output, layer.intermediate.intermediate_act_fn
@@ -365,6 +378,9 @@ class FlashDebertaV2Encoder(DebertaV2Encoder):
                 return None
             if any(type(m) is not nn.LayerNorm or m.weight is None or m.bias is None for m in norms):
                 return None
+            drops = [so.dropout, down.dropout] + ([sa.pos_dropout] if sa.relative_attention else [])
+            if any(type(m) not in (nn.Dropout, nn.Identity) for m in drops):         # in eval mode both do nothing
+                return None
             hidden = so.dense.out_features
             widest = 1024 if so.dense.weight.dtype == torch.float32 else 2048
             if hidden % 8 or hidden > widest or up.dense.out_features % 8 or hidden != 64 * sa.num_attention_heads:
@@ -376,25 +392,27 @@ class FlashDebertaV2Encoder(DebertaV2Encoder):
                               down.dense.weight, down.dense.bias, norms[1].weight, norms[1].bias], norms[0].eps,
                              norms[1].eps, 1.0 / math.sqrt(64 * terms), [t for m in lins[:3] + lins[6:] for t in (m.weight, m.bias)])
             attns.append(sa)
+            settings += [(sa, name) for name in _ATTENTION_SETTINGS]
+            settings += [(m, name) for m in norms for name in ("eps", "normalized_shape")] + [(act, "act"), (act, "approximate")]
         if native is None:
             return None
-        return host.Watch([m for m in self.layer.modules()]), native, attns
+        return _EncoderPlan(self.layer, host.Watch(list(self.layer.modules()), settings), native, attns)
 
     def _native_plan(self, hidden_states, rel_embeddings):
-        """The native encoder with every layer's derived tensors up to date, or None where it does not apply.  Whether a
-        kept plan still matches the modules is for the caller to ask (``holds()`` of its first entry), once the GPU is busy."""
+        """The plan with every layer's derived tensors up to date, or None where the native loop does not apply.  Whether a
+        kept plan still matches the modules in its list is for the caller to ask (``watch.holds()``), once the GPU is busy."""
         plan = _PLANS.get(self)
-        if plan is None:
-            made = self._native_layers()
-            if made is None or not made[0].holds():
+        if plan is None or plan.layers is not self.layer:
+            plan = self._native_layers()
+            if plan is None or not plan.watch.holds():
                 return None
-            plan = _PLANS[self] = [*made, None]      # the last entry: stamp of the relative embeddings behind its tables
-        _, native, attns, stamp = plan
+            _PLANS[self] = plan
+        native, attns = plan.native, plan.attns
         if not native.fits(hidden_states):
             return None
         dtype = hidden_states.dtype
         stamp_now = (getattr(rel_embeddings, "_tdb_stamp", None), dtype)
-        if stamp != stamp_now:
+        if plan.stamp != stamp_now:
             todo = range(len(attns))
             if rel_embeddings is not None and stamp_now[0] is None:
                 return None
@@ -406,8 +424,8 @@ class FlashDebertaV2Encoder(DebertaV2Encoder):
             if w.dtype != dtype or w.device != hidden_states.device:
                 return None
             native.set_derived(i, w, b, None if tables is None else tables.native())
-        plan[3] = stamp_now
-        return native
+        plan.stamp = stamp_now
+        return plan
 
     def _forward_native(self, hidden_states, attention_mask, output_hidden_states, return_dict):
         """The encoder as one native call on the token-major stream: packed (valid tokens only) for padded batches,
@@ -424,10 +442,10 @@ class FlashDebertaV2Encoder(DebertaV2Encoder):
             info = _analyse_2d(attention_mask, B, L)
             if info is None or (not info.all_ones and (not self.pack_padded_batches or info.packed[0] == 0)):
                 return None
-        native = self._native_plan(hidden_states, self.get_rel_embedding())
-        if native is None:
+        plan = self._native_plan(hidden_states, self.get_rel_embedding())
+        if plan is None:
             return None
-        watch = _PLANS[self][0]
+        native = plan.native
         every = output_hidden_states and _WANTED.hidden_states
         if info.all_ones:
             outs, words = native.run(hidden_states.reshape(B * L, hid), None, L, every)
@@ -442,7 +460,7 @@ class FlashDebertaV2Encoder(DebertaV2Encoder):
             _PENDING_STATUS.append(w)
         # The look at some two hundred modules takes the host 90 us, so it runs behind the launches, beside the GPU; the
         # result has no side effects and is simply dropped when somebody has changed the modules since the last forward.
-        if not watch.holds():
+        if not plan.watch.holds():
             del _PLANS[self]
             return self._forward_native(hidden_states, attention_mask, output_hidden_states, return_dict)
         all_hidden = None
@@ -547,7 +565,7 @@ class FlashDebertaV2Model(DebertaV2Model):
                     or type(emb.LayerNorm) is not nn.LayerNorm or emb.word_embeddings.max_norm is not None
                     or any(getattr(emb, n, None) is not None for n in ("position_embeddings", "token_type_embeddings", "embed_proj"))):
                 return None
-            watch = host.Watch(list(emb.modules()))
+            watch = host.Watch(list(emb.modules()), [(emb.word_embeddings, "max_norm")])
             _PLANS[self] = (watch, emb)
         if not watch.holds():
             _PLANS.pop(self, None)
