@@ -239,3 +239,85 @@ def test_a_plan_is_of_the_encoders_present_layers(change, native_after):
         assert (made is not None) == native_after
         if native_after:
             assert made.watch.holds() and made.attns == [layer.attention.self for layer in enc.layer]
+
+
+class _FakePlan:
+    """A plan that runs nothing; its watch fails the first time, after another thread has dropped the plan."""
+
+    def __init__(self):
+        self.native, self.watch, self.asked = self, self, 0
+
+    def run(self, x, *_):
+        return [x + 1], []
+
+    def holds(self):
+        self.asked += 1
+        return self.asked > 1
+
+
+def test_a_plan_that_another_thread_has_dropped(monkeypatch):
+    from turbodeberta_b200 import model as M
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    enc = M.FlashDebertaV2Encoder(_small_config()).eval()
+    plan = _FakePlan()
+    enc._native_plan = lambda *_: plan
+    with torch.no_grad():
+        out = enc._forward_native(torch.zeros(1, 3, 128), None, False, True)
+    assert plan.asked == 2 and torch.equal(out.last_hidden_state, torch.ones(1, 3, 128))
+
+
+def test_one_thread_at_a_time_brings_a_plan_up_to_date(monkeypatch):
+    import threading
+    import time
+    from turbodeberta_b200 import model as M
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    enc = M.FlashDebertaV2Encoder(_small_config()).eval()
+    inside, most, plan = [], [0], _FakePlan()
+    plan.asked = 1
+
+    def slow(*_):
+        inside.append(1)
+        most[0] = max(most[0], len(inside))
+        time.sleep(0.02)
+        inside.pop()
+        return plan
+    enc._native_plan = slow
+
+    def work():
+        with torch.no_grad():
+            enc._forward_native(torch.zeros(1, 3, 128), None, False, True)
+    threads = [threading.Thread(target=work) for _ in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert most[0] == 1
+
+
+def test_masks_of_several_threads():
+    """Masks that come and go in many threads: the cache of their analyses drops entries that others drop too."""
+    import sys
+    import threading
+    from turbodeberta_b200 import model as M
+    before, failed = sys.getswitchinterval(), []
+
+    def work():
+        try:
+            for i in range(400):
+                m = torch.ones(1, 2)
+                M._mask_cache_put(m, i)
+                keep = [torch.ones(1, 2) for _ in range(3)]
+                for t in keep:
+                    M._mask_cache_put(t, i)
+        except Exception as e:      # noqa: BLE001
+            failed.append(e)
+    sys.setswitchinterval(1e-6)
+    try:
+        threads = [threading.Thread(target=work) for _ in range(8)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+    finally:
+        sys.setswitchinterval(before)
+    assert not failed

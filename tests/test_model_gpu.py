@@ -459,3 +459,35 @@ def test_changed_stacks_and_settings_are_seen(dtype):
             if before is not None:                   # and the change is no matter of rounding
                 assert (got.float() - before)[v].abs().max().item() > 4 * err
             before = got.float()
+
+
+def test_first_passes_of_several_threads():
+    """Threads on streams of their own, all of them on a model without a plan and then on its recordings."""
+    import threading
+    from turbodeberta_b200.model import FlashDebertaV2Model
+    torch.manual_seed(18)
+    for _ in range(3):
+        model = FlashDebertaV2Model(_cfg(num_hidden_layers=3)).eval().to("cuda", torch.bfloat16)
+        ids = torch.randint(1, 500, (2, 60), device="cuda")
+        mask = torch.ones_like(ids)
+        torch.cuda.synchronize()
+        outs, failed = [], []
+
+        def work():
+            try:
+                with torch.no_grad(), torch.cuda.stream(torch.cuda.Stream()):
+                    for _ in range(4):
+                        out = model(input_ids=ids, attention_mask=mask).last_hidden_state
+                        torch.cuda.current_stream().synchronize()
+                        outs.append(out)
+            except Exception as e:      # noqa: BLE001
+                failed.append(e)
+        threads = [threading.Thread(target=work) for _ in range(4)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        assert not failed
+        with torch.no_grad():
+            want = model(input_ids=ids, attention_mask=mask).last_hidden_state
+        assert len(outs) == 16 and all(torch.equal(o, want) for o in outs)

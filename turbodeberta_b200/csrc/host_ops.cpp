@@ -638,14 +638,20 @@ class Linear {
   Tensor ws_;
 };
 
+// What is made from a layer's weights.  Never changed once made: a pass that runs without the interpreter lock works from the
+// ones it started with, whatever another thread replaces meanwhile.
+struct Derived {
+  Tensor qkv_w, qkv_b;
+  std::optional<Tables> tables;
+};
+using AllDerived = std::vector<std::shared_ptr<const Derived>>;
+
 struct Layer {
   Tensor out_w, out_b, ln1_w, ln1_b, up_w, up_b, down_w, down_b, ln2_w, ln2_b;
   double eps1, eps2, sm_scale;
-  std::vector<Tensor> sources;                       // what the derived tensors below were made from
+  std::vector<Tensor> sources;                       // what the derived tensors were made from
   std::vector<std::pair<void*, int64_t>> seen;
-  Tensor qkv_w, qkv_b;
-  py::object tables_ref;                             // keeps `tables` alive
-  const Tables* tables = nullptr;
+  std::shared_ptr<const Derived> derived;
 };
 
 // The encoder's layer loop on a token-major [T, hidden] stream: four library matrix products per layer, the fused attention,
@@ -655,7 +661,7 @@ class Encoder {
   Encoder(int heads) : heads_(heads) {}
   void add_layer(std::vector<Tensor> w, double eps1, double eps2, double sm_scale, std::vector<Tensor> sources) {
     TORCH_CHECK(w.size() == 10);
-    layers_.push_back(Layer{w[0], w[1], w[2], w[3], w[4], w[5], w[6], w[7], w[8], w[9], eps1, eps2, sm_scale, std::move(sources), {}, {}, {}, py::none(), nullptr});
+    layers_.push_back(Layer{w[0], w[1], w[2], w[3], w[4], w[5], w[6], w[7], w[8], w[9], eps1, eps2, sm_scale, std::move(sources), {}, {}});
   }
   // Layers whose derived tensors are missing, or older than what they were made from.
   std::vector<int> stale() const {
@@ -666,9 +672,9 @@ class Encoder {
   }
   void set_derived(int i, Tensor qkv_w, Tensor qkv_b, py::object tables) {
     Layer& l = layers_.at(i);
-    l.qkv_w = std::move(qkv_w); l.qkv_b = std::move(qkv_b);
-    l.tables_ref = tables;
-    l.tables = tables.is_none() ? nullptr : tables.cast<const Tables*>();
+    auto d = std::make_shared<Derived>(Derived{std::move(qkv_w), std::move(qkv_b), std::nullopt});
+    if (!tables.is_none()) d->tables = *tables.cast<const Tables*>();
+    l.derived = std::move(d);
     l.seen = stamp(l);
   }
   bool fits(const Tensor& x) const {
@@ -682,12 +688,15 @@ class Encoder {
   std::pair<std::vector<Tensor>, std::vector<Tensor>> run(const Tensor& x, const OptTensor& cu_seqlens, int64_t length, bool every) {
     std::pair<std::vector<Tensor>, std::vector<Tensor>> r;
     auto& [outs, words] = r;
+    AllDerived all;
+    all.reserve(layers_.size());
+    for (const Layer& l : layers_) all.push_back(l.derived);
     py::gil_scoped_release nogil;
     c10::cuda::CUDAGuard guard(x.device());
     at::AutoDispatchBelowAutograd below;
     cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
     if (!every) {
-      Tensor y = replay(x, cu_seqlens, length, stream);
+      Tensor y = replay(all, x, cu_seqlens, length, stream);
       if (y.defined()) {
         outs.push_back(y);
         return r;
@@ -699,7 +708,7 @@ class Encoder {
     Tensor in = x;
     for (size_t i = 0; i < layers_.size(); ++i) {
       Tensor out = every || i + 1 == layers_.size() ? at::empty_like(x) : s.z[i & 1];
-      layer(layers_[i], in, out, s, cu_seqlens, length, linear, stream, i > 0, [&](tdb::AttnParams& p) {
+      layer(layers_[i], *all[i], in, out, s, cu_seqlens, length, linear, stream, i > 0, [&](tdb::AttnParams& p) {
         Status st(dev, p);
         const Tensor partial = partial_scratch(p, dtype_code(x), TDB_KERNEL_AUTO, x);
         const int rc = tdb_run_attn(&p, dtype_code(x), TDB_KERNEL_AUTO, stream);
@@ -747,16 +756,16 @@ class Encoder {
   };
 
   template <typename Attention>
-  void layer(const Layer& l, const Tensor& x, Tensor& out, Scratch& s, const OptTensor& cu_seqlens, int64_t length, Linear& linear,
+  void layer(const Layer& l, const Derived& d, const Tensor& x, Tensor& out, Scratch& s, const OptTensor& cu_seqlens, int64_t length, Linear& linear,
              cudaStream_t stream, bool not_first, Attention attention) {
     const int code = dtype_code(x);
     const int64_t T = x.size(0), hidden = x.size(1), e = x.element_size();
-    linear(s.qkv, x, l.qkv_w, l.qkv_b, false, not_first);      // a pass's first kernel starts behind all that came before
+    linear(s.qkv, x, d.qkv_w, d.qkv_b, false, not_first);      // a pass's first kernel starts behind all that came before
     tdb::AttnParams p{};
     char* base = static_cast<char*>(s.qkv.data_ptr());
     p.q = base; p.k = base + e * hidden; p.v = base + 2 * e * hidden; p.o = s.ctx.data_ptr();
     p.q_st = p.k_st = p.v_st = 3 * hidden; p.q_sh = p.k_sh = p.v_sh = p.o_sh = hidden / heads_; p.o_st = hidden;
-    if (l.tables) l.tables->fill(p, x);
+    if (d.tables) d.tables->fill(p, x);
     p.H = heads_; p.D = (int)(hidden / heads_); p.sm_scale = (float)l.sm_scale; p.total_tokens = T;
     if (cu_seqlens) {
       p.varlen = 1; p.cu_seqlens = cu_seqlens->data_ptr<int32_t>(); p.n_seqs = (int)(cu_seqlens->numel() - 1); p.L = (int)length;
@@ -809,19 +818,21 @@ class Encoder {
   };
   using Key = std::tuple<int, cudaStream_t, int64_t, int64_t, int64_t>;   // device, stream, tokens, sequences (0: padded form), length
 
-  std::vector<const void*> weight_pointers() const {
+  std::vector<const void*> weight_pointers(const AllDerived& all) const {
     std::vector<const void*> w;
     w.reserve(layers_.size() * 14);
-    for (const Layer& l : layers_) {
-      for (const Tensor* t : {&l.qkv_w, &l.qkv_b, &l.out_w, &l.out_b, &l.ln1_w, &l.ln1_b, &l.up_w, &l.up_b, &l.down_w, &l.down_b, &l.ln2_w, &l.ln2_b})
+    for (size_t i = 0; i < layers_.size(); ++i) {
+      const Layer& l = layers_[i];
+      const Derived& d = *all[i];
+      for (const Tensor* t : {&d.qkv_w, &d.qkv_b, &l.out_w, &l.out_b, &l.ln1_w, &l.ln1_b, &l.up_w, &l.up_b, &l.down_w, &l.down_b, &l.ln2_w, &l.ln2_b})
         w.push_back(t->data_ptr());
-      w.push_back(l.tables ? ptr(l.tables->kr_exp) : nullptr);
-      w.push_back(l.tables ? ptr(l.tables->qr_exp) : nullptr);
+      w.push_back(d.tables ? ptr(d.tables->kr_exp) : nullptr);
+      w.push_back(d.tables ? ptr(d.tables->qr_exp) : nullptr);
     }
     return w;
   }
 
-  Tensor replay(const Tensor& x, const OptTensor& cu_seqlens, int64_t length, cudaStream_t stream) {
+  Tensor replay(const AllDerived& all, const Tensor& x, const OptTensor& cu_seqlens, int64_t length, cudaStream_t stream) {
     if (x.numel() > GRAPH_MAX_ELEMENTS || !Linear::applies(x) || !x.is_contiguous() ||
         at::cuda::currentStreamCaptureStatusMayInitCtx() != at::cuda::CaptureStatus::None)
       return {};
@@ -843,14 +854,14 @@ class Encoder {
       }
       it = graphs_.emplace(key, std::make_unique<Graph>()).first;
     }
-    const bool same = it->second->weights == weight_pointers();
+    const bool same = it->second->weights == weight_pointers(all);
     if (same && it->second->refused) return {};
     if (!same || !it->second->exec) {
       it->second = std::make_unique<Graph>();
-      if (!record(*it->second, x, cu_seqlens, length, stream)) {
+      if (!record(*it->second, all, x, cu_seqlens, length, stream)) {
         it->second = std::make_unique<Graph>();
         it->second->refused = true;
-        it->second->weights = weight_pointers();
+        it->second->weights = weight_pointers(all);
         it->second->used = ++uses_;
         return {};
       }
@@ -858,7 +869,7 @@ class Encoder {
     return launch_graph(*it->second, x, cu_seqlens, stream);
   }
 
-  bool record(Graph& g, const Tensor& x, const OptTensor& cu_seqlens, int64_t length, cudaStream_t stream) {
+  bool record(Graph& g, const AllDerived& all, const Tensor& x, const OptTensor& cu_seqlens, int64_t length, cudaStream_t stream) {
     g.dev = x.get_device();
     g.slot = acquire(g.dev);
     if (g.slot < 0) return false;
@@ -872,7 +883,7 @@ class Encoder {
     Tensor& ws = lt_workspaces_[{g.dev, stream}];
     if (!ws.defined()) ws = at::empty({(int64_t)Linear::WORKSPACE}, x.options().dtype(at::kByte));
     g.lt_ws = ws;
-    g.weights = weight_pointers();
+    g.weights = weight_pointers(all);
     if (length > 2 * BLOCK) {                                     // long enough for far key tiles
       const int64_t n = cu_seqlens ? cu_seqlens->numel() - 1 : x.size(0) / length;
       g.partial = at::empty({(x.size(0) / BLOCK + 2 * n + 1) * BLOCK * heads_ * 66}, x.options().dtype(at::kFloat));
@@ -887,7 +898,7 @@ class Encoder {
         Tensor in = g.x;
         for (size_t i = 0; good && i < layers_.size(); ++i) {
           Tensor out = i + 1 == layers_.size() ? g.out : g.scratch->z[i & 1];
-          layer(layers_[i], in, out, *g.scratch, cu, length, linear, side, i > 0, [&](tdb::AttnParams& p) {
+          layer(layers_[i], *all[i], in, out, *g.scratch, cu, length, linear, side, i > 0, [&](tdb::AttnParams& p) {
             p.status = g_pools[g.dev].host + g.slot * SLOT_WORDS;
             p.counter = g_pools[g.dev].ctl + g.slot * SLOT_WORDS;
             p.gave_up = p.counter + 1;

@@ -56,18 +56,20 @@ class MaskInfo:
 
 
 _MASK_CACHE: dict = {}
+_MASK_LOCK = threading.Lock()
 
 
 def _mask_cache_put(tensor: torch.Tensor, info) -> None:
     """Remember the analysis of a live mask tensor.  Entries of tensors that have been freed are dropped first; only
     if more than 64 live masks are tracked does the oldest entry go (so a mask that is passed again and again, e.g.
     the static input of a captured graph, is never re-analysed because other masks came and went)."""
-    dead = [k for k, (ref, _, _) in _MASK_CACHE.items() if ref() is None]
-    for k in dead:
-        del _MASK_CACHE[k]
-    while len(_MASK_CACHE) >= 64:
-        del _MASK_CACHE[next(iter(_MASK_CACHE))]
-    _MASK_CACHE[id(tensor)] = (weakref.ref(tensor), tensor._version, info)
+    with _MASK_LOCK:
+        dead = [k for k, (ref, _, _) in _MASK_CACHE.items() if ref() is None]
+        for k in dead:
+            del _MASK_CACHE[k]
+        while len(_MASK_CACHE) >= 64:
+            del _MASK_CACHE[next(iter(_MASK_CACHE))]
+        _MASK_CACHE[id(tensor)] = (weakref.ref(tensor), tensor._version, info)
 
 
 def analyse_mask(attention_mask: torch.Tensor | None, batch: int, length: int, refresh: bool = False) -> MaskInfo:
@@ -279,6 +281,8 @@ class FlashDebertaV2Layer(DebertaV2Layer):
 # Native plans of live encoders and models; kept outside the modules, which stay plain data to copy and pickle.  A plan
 # holds modules below its key, never the key itself, so it goes when the key goes.
 _PLANS: "weakref.WeakKeyDictionary" = weakref.WeakKeyDictionary()
+# Held while a plan is made or brought up to date: one thread does it, the others find it done.
+_PLAN_LOCK = threading.RLock()
 
 #: what the native loop takes over from an attention module besides its weights
 _ATTENTION_SETTINGS = ("num_attention_heads", "attention_head_size", "pos_att_type", "share_att_key", "relative_attention",
@@ -418,12 +422,17 @@ class FlashDebertaV2Encoder(DebertaV2Encoder):
                 return None
         else:
             todo = native.stale()
+        made = False
         for i in todo:
+            made = True
             w, b = attns[i]._qkv_weights()
             tables = attns[i]._relative_tables(rel_embeddings, dtype) if attns[i].relative_attention else None
             if w.dtype != dtype or w.device != hidden_states.device:
                 return None
             native.set_derived(i, w, b, None if tables is None else tables.native())
+        if made and hidden_states.is_cuda and not torch.cuda.is_current_stream_capturing():
+            # the next pass may come from another thread on another stream, which does not wait for this one
+            torch.cuda.current_stream(hidden_states.device).synchronize()
         plan.stamp = stamp_now
         return plan
 
@@ -442,7 +451,8 @@ class FlashDebertaV2Encoder(DebertaV2Encoder):
             info = _analyse_2d(attention_mask, B, L)
             if info is None or (not info.all_ones and (not self.pack_padded_batches or info.packed[0] == 0)):
                 return None
-        plan = self._native_plan(hidden_states, self.get_rel_embedding())
+        with _PLAN_LOCK:
+            plan = self._native_plan(hidden_states, self.get_rel_embedding())
         if plan is None:
             return None
         native = plan.native
@@ -461,7 +471,7 @@ class FlashDebertaV2Encoder(DebertaV2Encoder):
         # The look at some two hundred modules takes the host 90 us, so it runs behind the launches, beside the GPU; the
         # result has no side effects and is simply dropped when somebody has changed the modules since the last forward.
         if not plan.watch.holds():
-            del _PLANS[self]
+            _PLANS.pop(self, None)               # another thread may have been first
             return self._forward_native(hidden_states, attention_mask, output_hidden_states, return_dict)
         all_hidden = None
         if output_hidden_states:
