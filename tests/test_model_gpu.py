@@ -491,3 +491,21 @@ def test_first_passes_of_several_threads():
         with torch.no_grad():
             want = model(input_ids=ids, attention_mask=mask).last_hidden_state
         assert len(outs) == 16 and all(torch.equal(o, want) for o in outs)
+
+
+def test_status_slots_survive_calls_that_run_out_of_memory():
+    """More failing calls than there are slots: 32 MB of mask whose 256 MB of lengths and offsets do not fit."""
+    from turbodeberta_b200._cabi import host
+    mask = torch.ones(1 << 25, 1, dtype=torch.uint8, device="cuda")
+    small = torch.ones(2, 3, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (64 << 20)) / total)
+    try:
+        for _ in range(300):
+            with pytest.raises(torch.OutOfMemoryError):
+                host.mask_rows(mask)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert host.mask_rows(small)[:4] == (True, True, 6, 3)

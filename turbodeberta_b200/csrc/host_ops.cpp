@@ -20,6 +20,7 @@
 #include <algorithm>
 #include <map>
 #include <mutex>
+#include <utility>
 #include <vector>
 
 #include "tdb_internal.h"
@@ -110,7 +111,8 @@ void release_unused(int dev, int slot) {
   g_pools[dev].free.push_back(slot);
 }
 
-// Where one call reports: a pool slot, or words of its own.
+// Where one call reports: a pool slot, or words of its own.  The slot goes back by itself if the call ends (by an exception of
+// the allocator, say) before anything was launched with it.
 struct Status {
   int dev, slot = -1;
   Tensor own;
@@ -127,18 +129,28 @@ struct Status {
       p.gave_up = p.status + 5;
     }
   }
+  Status(const Status&) = delete;
+  Status& operator=(const Status&) = delete;
+  ~Status() { release_unused(dev, slot); }
+  // The launch failed.  One of its kernels may be running all the same, and then reports into the slot until it ends.
+  void failed(cudaStream_t stream) {
+    if (slot < 0) return;
+    cudaStreamSynchronize(stream);
+    (void)cudaGetLastError();
+    collect(dev, std::exchange(slot, -1));
+  }
   // Leave the check to drain_pending(); words of the call's own go to `words`.  Needs no interpreter lock.
   void defer(cudaStream_t stream, std::vector<Tensor>& words) {
     if (slot < 0) { words.push_back(own.narrow(0, 0, SLOT_WORDS)); return; }
     std::lock_guard<std::mutex> lock(g_pools[dev].mu);
-    g_pools[dev].pending.push_back({slot, stream, false});
+    g_pools[dev].pending.push_back({std::exchange(slot, -1), stream, false});
   }
   // What the caller in Python gets to see: None (fine, or deferred into the pool), (word 0, word 1), or the tensor of words.
   py::object finish(bool check, cudaStream_t stream) {
     if (slot < 0) return py::cast(own.narrow(0, 0, SLOT_WORDS));
     if (!check) {
       std::lock_guard<std::mutex> lock(g_pools[dev].mu);
-      g_pools[dev].pending.push_back({slot, stream, false});
+      g_pools[dev].pending.push_back({std::exchange(slot, -1), stream, false});
       return py::none();
     }
     cudaError_t e;
@@ -146,7 +158,7 @@ struct Status {
       py::gil_scoped_release nogil;
       e = cudaStreamSynchronize(stream);
     }
-    const auto r = collect(dev, slot);
+    const auto r = collect(dev, std::exchange(slot, -1));
     cuda_ok(e, "cudaStreamSynchronize");
     if (r.first || r.second) return py::make_tuple(r.first, r.second);
     return py::none();
@@ -284,7 +296,7 @@ Result launch(tdb::AttnParams& p, int dtype, int kernel, int dev, Tensor o, cons
   const int rc = tdb_run_attn(&p, dtype, kernel, stream);
   py::object lse_out = lse.defined() ? py::cast(lse) : py::none();
   if (rc) {
-    release_unused(dev, st.slot);
+    st.failed(stream);
     return {o, lse_out, py::int_(rc)};
   }
   return {o, lse_out, st.finish(check, stream)};
@@ -712,7 +724,7 @@ class Encoder {
         Status st(dev, p);
         const Tensor partial = partial_scratch(p, dtype_code(x), TDB_KERNEL_AUTO, x);
         const int rc = tdb_run_attn(&p, dtype_code(x), TDB_KERNEL_AUTO, stream);
-        if (rc) release_unused(dev, st.slot);
+        if (rc) st.failed(stream);
         ok(rc);
         st.defer(stream, words);
       });
@@ -955,9 +967,12 @@ py::object mask_rows(const Tensor& mask) {
   c10::cuda::CUDAGuard guard((c10::DeviceIndex)dev);
   cudaStream_t stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream();
   const int64_t B = m.size(0), L = m.size(1);
-  const int slot = acquire(dev);
-  if (slot < 0) return py::none();
-  int32_t* out = g_pools[dev].host + slot * SLOT_WORDS;
+  struct Slot {
+    int dev, i;
+    ~Slot() { release_unused(dev, i); }
+  } slot{dev, acquire(dev)};
+  if (slot.i < 0) return py::none();
+  int32_t* out = g_pools[dev].host + slot.i * SLOT_WORDS;
   Tensor both;
   int rc;
   cudaError_t e = cudaSuccess;
@@ -966,11 +981,10 @@ py::object mask_rows(const Tensor& mask) {
     py::gil_scoped_release nogil;
     both = at::empty({2 * B + 1}, m.options().dtype(at::kInt));
     int32_t* lens = both.data_ptr<int32_t>();
-    rc = tdb_mask_rows(m.data_ptr(), (int)m.element_size(), (int)B, (int)L, lens, lens + B, g_pools[dev].ctl + slot * SLOT_WORDS, out, stream);
+    rc = tdb_mask_rows(m.data_ptr(), (int)m.element_size(), (int)B, (int)L, lens, lens + B, g_pools[dev].ctl + slot.i * SLOT_WORDS, out, stream);
     if (!rc) e = cudaStreamSynchronize(stream);
     for (int i = 0; i < 4; ++i) { w[i] = reinterpret_cast<volatile int32_t*>(out)[i]; out[i] = 0; }
   }
-  release_unused(dev, slot);
   TORCH_CHECK(rc == 0, "libtdb_b200: ", tdb_last_error());
   cuda_ok(e, "cudaStreamSynchronize");
   return py::make_tuple((bool)w[0], (bool)w[1], w[2], w[3], both.narrow(0, 0, B), both.narrow(0, B, B + 1));
