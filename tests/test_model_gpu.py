@@ -509,3 +509,32 @@ def test_status_slots_survive_calls_that_run_out_of_memory():
     finally:
         torch.cuda.set_per_process_memory_fraction(1.0)
     assert host.mask_rows(small)[:4] == (True, True, 6, 3)
+
+
+def test_streams_that_their_owner_destroys():
+    """Deferred checks and recordings of a stream of the caller's that is gone when they are looked at, or whose handle has
+    passed to a new stream."""
+    import ctypes
+    from turbodeberta_b200.model import FlashDebertaV2Model
+    from turbodeberta_b200.ops.flash_attention import check_pending_status, flash_attention_with_disentangled
+    torch.manual_seed(19)
+    model = FlashDebertaV2Model(_cfg(num_hidden_layers=2)).eval().to("cuda", torch.bfloat16)
+    rt = torch.cuda.cudart()
+    q = torch.randn(1, 2, 40, 64, device="cuda").bfloat16()
+    want = flash_attention_with_disentangled(q, q, q, None, None)
+    for _ in range(4):
+        ids = torch.randint(1, 500, (2, 40), device="cuda")
+        with torch.no_grad():
+            ref = model(input_ids=ids, attention_mask=torch.ones_like(ids)).last_hidden_state
+        torch.cuda.synchronize()
+        handle = ctypes.c_void_p(0)
+        assert int(rt.cudaStreamCreate(ctypes.addressof(handle))) == 0
+        with torch.no_grad(), torch.cuda.stream(torch.cuda.ExternalStream(handle.value)):
+            outs = [model(input_ids=ids, attention_mask=torch.ones_like(ids)).last_hidden_state for _ in range(3)]
+            o = flash_attention_with_disentangled(q, q, q, None, None, check_status=False)
+            torch.cuda.current_stream().synchronize()
+            outs = [t.cpu() for t in outs]
+            same = torch.equal(o, want)
+        assert int(rt.cudaStreamDestroy(handle.value)) == 0
+        check_pending_status()
+        assert same and all(torch.equal(t, ref.cpu()) for t in outs)

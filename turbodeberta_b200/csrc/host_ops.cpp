@@ -33,12 +33,47 @@ namespace {
 
 constexpr int MAX_DEV = 64, SLOTS = 256, SLOT_WORDS = 4;
 
+// The end of what a stream holds now.  torch never destroys its own streams, so their handle stays good to wait for; one that a
+// caller made and handed to torch may be gone by then, and is marked with an event instead.
+class Mark {
+ public:
+  explicit Mark(c10::cuda::CUDAStream s) : stream_(s.stream()) {
+    if (!stream_ || c10::cuda::getStreamFromExternal(stream_, s.device_index()).id() != s.id()) return;
+    own_ = false;
+    if (cudaEventCreateWithFlags(&event_, cudaEventDisableTiming) != cudaSuccess) event_ = nullptr;
+    renew();
+  }
+  Mark(Mark&& o) noexcept : stream_(o.stream_), own_(o.own_), event_(std::exchange(o.event_, nullptr)) {}
+  Mark& operator=(Mark&& o) noexcept {
+    std::swap(stream_, o.stream_); std::swap(own_, o.own_); std::swap(event_, o.event_);
+    return *this;
+  }
+  ~Mark() {
+    if (event_) cudaEventDestroy(event_);
+  }
+  // Called while the stream is the current one: move the mark behind what it holds by now.
+  void renew() {
+    if (own_ || (event_ && cudaEventRecord(event_, stream_) == cudaSuccess)) return;
+    (void)cudaGetLastError();
+    cudaStreamSynchronize(stream_);                  // no event to be had: nothing left to wait for later
+    if (event_) cudaEventDestroy(std::exchange(event_, nullptr));
+  }
+  bool on(cudaStream_t s) const { return own_ && stream_ == s; }
+  cudaError_t wait() const { return own_ ? cudaStreamSynchronize(stream_) : event_ ? cudaEventSynchronize(event_) : cudaSuccess; }
+  cudaStream_t stream() const { return stream_; }    // to compare with, not to use
+
+ private:
+  cudaStream_t stream_;
+  bool own_ = true;                                  // torch's own, or the legacy stream
+  cudaEvent_t event_ = nullptr;
+};
+
 struct StatusPool {
   std::mutex mu;
   int32_t* host = nullptr;        // SLOTS x 4 words, pinned and mapped
   int32_t* ctl = nullptr;         // SLOTS x 4 words on the device: work counter, gave-up flag
   std::vector<int> free;
-  struct Pending { int slot; cudaStream_t stream; bool keep; };   // keep: the slot stays its owner's
+  struct Pending { int slot; Mark mark; bool keep; };             // keep: the slot stays its owner's
   std::vector<Pending> pending;   // launches whose check was deferred
 };
 StatusPool g_pools[MAX_DEV];
@@ -140,23 +175,25 @@ struct Status {
     collect(dev, std::exchange(slot, -1));
   }
   // Leave the check to drain_pending(); words of the call's own go to `words`.  Needs no interpreter lock.
-  void defer(cudaStream_t stream, std::vector<Tensor>& words) {
+  void defer(c10::cuda::CUDAStream stream, std::vector<Tensor>& words) {
     if (slot < 0) { words.push_back(own.narrow(0, 0, SLOT_WORDS)); return; }
+    Mark mark(stream);
     std::lock_guard<std::mutex> lock(g_pools[dev].mu);
-    g_pools[dev].pending.push_back({std::exchange(slot, -1), stream, false});
+    g_pools[dev].pending.push_back({std::exchange(slot, -1), std::move(mark), false});
   }
   // What the caller in Python gets to see: None (fine, or deferred into the pool), (word 0, word 1), or the tensor of words.
-  py::object finish(bool check, cudaStream_t stream) {
+  py::object finish(bool check, c10::cuda::CUDAStream stream) {
     if (slot < 0) return py::cast(own.narrow(0, 0, SLOT_WORDS));
     if (!check) {
+      Mark mark(stream);
       std::lock_guard<std::mutex> lock(g_pools[dev].mu);
-      g_pools[dev].pending.push_back({std::exchange(slot, -1), stream, false});
+      g_pools[dev].pending.push_back({std::exchange(slot, -1), std::move(mark), false});
       return py::none();
     }
     cudaError_t e;
     {
       py::gil_scoped_release nogil;
-      e = cudaStreamSynchronize(stream);
+      e = cudaStreamSynchronize(stream.stream());
     }
     const auto r = collect(dev, std::exchange(slot, -1));
     cuda_ok(e, "cudaStreamSynchronize");
@@ -180,14 +217,11 @@ py::object drain_pending() {
     cudaError_t e = cudaSuccess;
     {
       py::gil_scoped_release nogil;
-      cudaStream_t last = nullptr;
-      bool any = false;
+      const Mark* last = nullptr;
       for (const auto& t : take) {
-        if (any && t.stream == last) continue;
-        last = t.stream; any = true;
-        if (cudaStreamSynchronize(t.stream) == cudaSuccess) continue;
-        (void)cudaGetLastError();                       // e.g. a stream that its owner has destroyed
-        if ((e = cudaDeviceSynchronize()) != cudaSuccess) break;
+        if (last && t.mark.on(last->stream()) && last->on(t.mark.stream())) continue;
+        last = &t.mark;
+        if ((e = t.mark.wait()) != cudaSuccess) break;
       }
     }
     for (const auto& t : take) {
@@ -290,7 +324,7 @@ Tensor lens_on_device(const Tensor& seqlens, int64_t B, const Tensor& q) {
 using Result = std::tuple<Tensor, py::object, py::object>;      // o, lse or None, status (see Status::finish) or an error code
 
 Result launch(tdb::AttnParams& p, int dtype, int kernel, int dev, Tensor o, const Tensor& lse, bool check) {
-  cudaStream_t stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream();
+  const c10::cuda::CUDAStream stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev);
   Status st(dev, p);
   const Tensor partial = partial_scratch(p, dtype, kernel, o);
   const int rc = tdb_run_attn(&p, dtype, kernel, stream);
@@ -706,9 +740,10 @@ class Encoder {
     py::gil_scoped_release nogil;
     c10::cuda::CUDAGuard guard(x.device());
     at::AutoDispatchBelowAutograd below;
-    cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
+    const c10::cuda::CUDAStream torch_stream = c10::cuda::getCurrentCUDAStream();
+    const cudaStream_t stream = torch_stream.stream();
     if (!every) {
-      Tensor y = replay(all, x, cu_seqlens, length, stream);
+      Tensor y = replay(all, x, cu_seqlens, length, torch_stream);
       if (y.defined()) {
         outs.push_back(y);
         return r;
@@ -726,7 +761,7 @@ class Encoder {
         const int rc = tdb_run_attn(&p, dtype_code(x), TDB_KERNEL_AUTO, stream);
         if (rc) st.failed(stream);
         ok(rc);
-        st.defer(stream, words);
+        st.defer(torch_stream, words);
       });
       in = out;
       if (every) outs.push_back(out);
@@ -828,7 +863,8 @@ class Encoder {
       if (!listed) p.free.push_back(slot);
     }
   };
-  using Key = std::tuple<int, cudaStream_t, int64_t, int64_t, int64_t>;   // device, stream, tokens, sequences (0: padded form), length
+  // Device, id of the stream (no other gets it later, as it may get the handle), tokens, sequences (0: padded form), length.
+  using Key = std::tuple<int, unsigned long long, int64_t, int64_t, int64_t>;
 
   std::vector<const void*> weight_pointers(const AllDerived& all) const {
     std::vector<const void*> w;
@@ -844,12 +880,17 @@ class Encoder {
     return w;
   }
 
-  Tensor replay(const AllDerived& all, const Tensor& x, const OptTensor& cu_seqlens, int64_t length, cudaStream_t stream) {
+  Tensor replay(const AllDerived& all, const Tensor& x, const OptTensor& cu_seqlens, int64_t length, c10::cuda::CUDAStream stream) {
     if (x.numel() > GRAPH_MAX_ELEMENTS || !Linear::applies(x) || !x.is_contiguous() ||
         at::cuda::currentStreamCaptureStatusMayInitCtx() != at::cuda::CaptureStatus::None)
       return {};
     const int dev = x.get_device();
-    const Key key(dev, stream, x.size(0), cu_seqlens ? cu_seqlens->numel() - 1 : 0, length);
+    unsigned long long id = 0;
+    if (cudaStreamGetId(stream.stream(), &id) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return {};
+    }
+    const Key key(dev, id, x.size(0), cu_seqlens ? cu_seqlens->numel() - 1 : 0, length);
     std::lock_guard<std::mutex> lock(graph_mu_);
     auto it = graphs_.find(key);
     if (it == graphs_.end()) {
@@ -870,7 +911,7 @@ class Encoder {
     if (same && it->second->refused) return {};
     if (!same || !it->second->exec) {
       it->second = std::make_unique<Graph>();
-      if (!record(*it->second, all, x, cu_seqlens, length, stream)) {
+      if (!record(*it->second, all, x, cu_seqlens, length, id)) {
         it->second = std::make_unique<Graph>();
         it->second->refused = true;
         it->second->weights = weight_pointers(all);
@@ -881,7 +922,7 @@ class Encoder {
     return launch_graph(*it->second, x, cu_seqlens, stream);
   }
 
-  bool record(Graph& g, const AllDerived& all, const Tensor& x, const OptTensor& cu_seqlens, int64_t length, cudaStream_t stream) {
+  bool record(Graph& g, const AllDerived& all, const Tensor& x, const OptTensor& cu_seqlens, int64_t length, unsigned long long stream_id) {
     g.dev = x.get_device();
     g.slot = acquire(g.dev);
     if (g.slot < 0) return false;
@@ -892,7 +933,7 @@ class Encoder {
     g.scratch = std::make_unique<Scratch>(*this, x, cu_seqlens);
     for (auto w = lt_workspaces_.begin(); w != lt_workspaces_.end();)     // of streams whose last graph is gone
       w = w->second.use_count() == 1 ? lt_workspaces_.erase(w) : std::next(w);
-    Tensor& ws = lt_workspaces_[{g.dev, stream}];
+    Tensor& ws = lt_workspaces_[{g.dev, stream_id}];
     if (!ws.defined()) ws = at::empty({(int64_t)Linear::WORKSPACE}, x.options().dtype(at::kByte));
     g.lt_ws = ws;
     g.weights = weight_pointers(all);
@@ -935,7 +976,8 @@ class Encoder {
     return good;
   }
 
-  Tensor launch_graph(Graph& g, const Tensor& x, const OptTensor& cu_seqlens, cudaStream_t stream) {
+  Tensor launch_graph(Graph& g, const Tensor& x, const OptTensor& cu_seqlens, c10::cuda::CUDAStream torch_stream) {
+    const cudaStream_t stream = torch_stream.stream();
     g.used = ++uses_;
     Tensor y = at::empty_like(x);
     cuda_ok(cudaMemcpyAsync(g.x.data_ptr(), x.data_ptr(), x.nbytes(), cudaMemcpyDeviceToDevice, stream), "copy of the encoder's input");
@@ -945,8 +987,12 @@ class Encoder {
     StatusPool& p = g_pools[g.dev];
     std::lock_guard<std::mutex> lock(p.mu);
     bool listed = false;
-    for (const auto& t : p.pending) listed = listed || (t.slot == g.slot && t.keep && t.stream == stream);
-    if (!listed) p.pending.push_back({g.slot, stream, true});
+    for (auto& t : p.pending)
+      if (t.slot == g.slot && t.keep) {                           // the graph is one stream's, so there is one entry at most
+        t.mark.renew();
+        listed = true;
+      }
+    if (!listed) p.pending.push_back({g.slot, Mark(torch_stream), true});
     return y;
   }
 
@@ -955,7 +1001,7 @@ class Encoder {
   std::mutex graph_mu_;
   std::map<Key, std::unique_ptr<Graph>> graphs_;
   std::vector<Key> seen_;
-  std::map<std::pair<int, cudaStream_t>, Tensor> lt_workspaces_;
+  std::map<std::pair<int, unsigned long long>, Tensor> lt_workspaces_;       // by device and stream id
   uint64_t uses_ = 0;
 };
 
