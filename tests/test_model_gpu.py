@@ -538,3 +538,35 @@ def test_streams_that_their_owner_destroys():
         assert int(rt.cudaStreamDestroy(handle.value)) == 0
         check_pending_status()
         assert same and all(torch.equal(t, ref.cpu()) for t in outs)
+
+
+def _flatten_parameters(model, shift):
+    """All parameters as views of one buffer, each `shift` bytes behind a 256-byte boundary."""
+    params = list(model.parameters())
+    size = params[0].element_size()
+    step = 256 // size
+    flat = torch.empty(sum((p.numel() // step + 2) * step for p in params), dtype=params[0].dtype, device="cuda")
+    at = 0
+    for p in params:
+        view = flat[at + shift // size:][:p.numel()].view_as(p)
+        view.copy_(p.data)
+        p.data = view
+        at += (p.numel() // step + 2) * step
+    assert all(p.data_ptr() % 256 == shift for p in params)
+
+
+def test_parameters_in_one_flat_buffer():
+    """Weights, biases and norms that start on 16-byte boundaries only: the native loop takes them, with library products chosen
+    for that alignment (72 tokens) and with the projection kernels (24)."""
+    from turbodeberta_b200 import model as M
+    torch.manual_seed(20)
+    model = M.FlashDebertaV2Model(_cfg(num_hidden_layers=2)).eval().to("cuda", torch.bfloat16)
+    aligned = [torch.randint(1, 500, (2, n), device="cuda") for n in (36, 12)]
+    with torch.no_grad():
+        before = [model(input_ids=i, attention_mask=torch.ones_like(i)).last_hidden_state for i in aligned]
+        _flatten_parameters(model, 16)
+        for ids, want in zip(aligned, before):
+            for _ in range(3):
+                got = model(input_ids=ids, attention_mask=torch.ones_like(ids)).last_hidden_state
+                assert (got.float() - want.float()).abs().max().item() <= 4e-2 * want.float().abs().max().item()
+        assert M._PLANS.get(model.encoder) is not None

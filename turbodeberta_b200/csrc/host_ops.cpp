@@ -605,10 +605,11 @@ class Linear {
   }
   // False: the caller's torch has to do it.
   bool try_run(Tensor& y, const Tensor& x, const Tensor& w, const Tensor& b) {
-    if (!own_ || (reinterpret_cast<uintptr_t>(x.data_ptr()) | reinterpret_cast<uintptr_t>(w.data_ptr()) | reinterpret_cast<uintptr_t>(b.data_ptr())) & 15)
-      return false;
+    const uintptr_t addresses = reinterpret_cast<uintptr_t>(x.data_ptr()) | reinterpret_cast<uintptr_t>(w.data_ptr()) |
+                                reinterpret_cast<uintptr_t>(b.data_ptr()) | reinterpret_cast<uintptr_t>(y.data_ptr());
+    if (!own_ || addresses & 15) return false;
     const int64_t T = x.size(0), k = x.size(1), n = w.size(0);
-    Plan& p = plan(T, k, n);
+    Plan& p = plan(T, k, n, addresses & 255 ? 16 : 256);
     if (!p.usable) return false;
     const void* bias = b.data_ptr();
     const float one = 1.f, zero = 0.f;
@@ -629,7 +630,6 @@ class Linear {
   }
   static constexpr size_t WORKSPACE = 32u << 20;
 
-
  private:
   static bool misaligned(const Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) & 15; }
   static void check(int rc) { TORCH_CHECK(rc == 0, "libtdb_b200: ", tdb_last_error(), " (code ", rc, ")"); }
@@ -649,12 +649,14 @@ class Linear {
         if (l) cublasLtMatrixLayoutDestroy(l);
     }
   };
-  Plan& plan(int64_t T, int64_t k, int64_t n) {
+  // alignment: of all four addresses, 256 (what the library takes for granted unless told otherwise, and what an allocation of
+  // torch's has) or 16 (parameters that are views of one flat buffer).
+  Plan& plan(int64_t T, int64_t k, int64_t n, uint32_t alignment) {
     // per thread (a descriptor is written to before each launch), and bounded: a packed batch brings a new T each time
-    thread_local std::map<std::tuple<int, int64_t, int64_t, int64_t>, std::unique_ptr<Plan>> plans;
+    thread_local std::map<std::tuple<int, int64_t, int64_t, int64_t, uint32_t>, std::unique_ptr<Plan>> plans;
     int dev = 0;
     cudaGetDevice(&dev);
-    const auto key = std::make_tuple(dev, T, k, n);
+    const auto key = std::make_tuple(dev, T, k, n, alignment);
     auto it = plans.find(key);
     if (it != plans.end()) return *it->second;
     if (plans.size() >= 256) plans.clear();
@@ -671,8 +673,11 @@ class Linear {
                 cublasLtMatrixLayoutCreate(&p->x, CUDA_R_16BF, k, T, k) == CUBLAS_STATUS_SUCCESS &&
                 cublasLtMatrixLayoutCreate(&p->y, CUDA_R_16BF, n, T, n) == CUBLAS_STATUS_SUCCESS &&
                 cublasLtMatmulPreferenceCreate(&pref) == CUBLAS_STATUS_SUCCESS &&
-                cublasLtMatmulPreferenceSetAttribute(pref, CUBLASLT_MATMUL_PREF_MAX_WORKSPACE_BYTES, &WORKSPACE_BYTES, sizeof(WORKSPACE_BYTES)) == CUBLAS_STATUS_SUCCESS &&
-                cublasLtMatmulAlgoGetHeuristic(handle_, p->op, p->w, p->x, p->y, p->y, pref, 1, &found, &count) == CUBLAS_STATUS_SUCCESS && count == 1;
+                cublasLtMatmulPreferenceSetAttribute(pref, CUBLASLT_MATMUL_PREF_MAX_WORKSPACE_BYTES, &WORKSPACE_BYTES, sizeof(WORKSPACE_BYTES)) == CUBLAS_STATUS_SUCCESS;
+    for (auto which : {CUBLASLT_MATMUL_PREF_MIN_ALIGNMENT_A_BYTES, CUBLASLT_MATMUL_PREF_MIN_ALIGNMENT_B_BYTES,
+                       CUBLASLT_MATMUL_PREF_MIN_ALIGNMENT_C_BYTES, CUBLASLT_MATMUL_PREF_MIN_ALIGNMENT_D_BYTES})
+      good = good && cublasLtMatmulPreferenceSetAttribute(pref, which, &alignment, sizeof(alignment)) == CUBLAS_STATUS_SUCCESS;
+    good = good && cublasLtMatmulAlgoGetHeuristic(handle_, p->op, p->w, p->x, p->y, p->y, pref, 1, &found, &count) == CUBLAS_STATUS_SUCCESS && count == 1;
     if (pref) cublasLtMatmulPreferenceDestroy(pref);
     if (good) { p->algo = found.algo; p->usable = true; }
     return *(plans[key] = std::move(p));
