@@ -321,3 +321,34 @@ def test_masks_of_several_threads():
     finally:
         sys.setswitchinterval(before)
     assert not failed
+
+
+def _shift(p):
+    buf = torch.empty(p.numel() + 1)
+    p.data = buf[1:].view_as(p).copy_(p.data)
+
+
+@pytest.mark.parametrize("change,width,fits", [
+    (lambda layer: None, 128, True), (lambda layer: None, 64, False), (lambda layer: None, 192, False),
+    (lambda layer: _shift(layer.output.LayerNorm.weight), 128, False),
+    (lambda layer: _shift(layer.output.dense.weight), 128, True),           # products look at that themselves
+    (lambda layer: setattr(layer.output.dense.weight, "data", layer.output.dense.weight.data[:, :64].contiguous()), 128, False),
+    (lambda layer: setattr(layer.intermediate.dense.bias, "data", layer.intermediate.dense.bias.data[:64]), 128, False),
+    (lambda layer: setattr(layer.attention.self.key_proj.weight, "data", torch.zeros(64, 128)), 128, False)])
+def test_the_native_loop_takes_only_what_it_can_read(change, width, fits):
+    from turbodeberta_b200 import model as M
+    enc = M.FlashDebertaV2Encoder(_small_config(relative_attention=False, pos_att_type=[])).eval()
+    with torch.no_grad():
+        assert enc._native_plan(torch.zeros(1, 128), None) is not None
+        change(enc.layer[1])
+        assert (enc._native_plan(torch.zeros(1, width), None) is not None) == fits
+
+
+def test_a_mask_on_another_device_is_not_for_the_mask_kernel(monkeypatch):
+    from turbodeberta_b200 import model as M
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    monkeypatch.setattr(M, "analyse_mask", lambda *_, **__: M.MaskInfo(False, True, None, None))
+    monkeypatch.setattr(M, "_analyse_2d", lambda *_: pytest.fail("another device's mask"))
+    enc = M.FlashDebertaV2Encoder(_small_config()).eval()
+    with torch.no_grad():
+        assert enc._forward_native(torch.zeros(1, 3, 128), torch.ones(1, 3, device="meta"), False, True) is None

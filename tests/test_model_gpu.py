@@ -570,3 +570,36 @@ def test_parameters_in_one_flat_buffer():
                 got = model(input_ids=ids, attention_mask=torch.ones_like(ids)).last_hidden_state
                 assert (got.float() - want.float()).abs().max().item() <= 4e-2 * want.float().abs().max().item()
         assert M._PLANS.get(model.encoder) is not None
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("padded", [False, True])
+def test_encoder_inputs_of_any_layout(dtype, padded):
+    """Hidden states that are a slice of wider rows or start between two 16-byte pieces; rows of the wrong width are refused as
+    by the modules."""
+    from turbodeberta_b200.model import FlashDebertaV2Encoder
+    torch.manual_seed(21)
+    enc = FlashDebertaV2Encoder(_cfg(num_hidden_layers=2)).eval().to("cuda", dtype)
+    B, L = 2, 40
+    mask = torch.ones(B, L, dtype=torch.long, device="cuda")
+    if padded:
+        mask[1, 20:] = 0
+    x = torch.randn(B, L, 128, device="cuda").to(dtype)
+    wide = torch.randn(B, L, 256, device="cuda").to(dtype)
+    wide[..., :128] = x
+    flat = torch.empty(B * L * 128 + 1, device="cuda", dtype=dtype)
+    flat[1:] = x.flatten()
+    with torch.no_grad():
+        for every in (True, False, False, False):
+            want = enc(x, mask, output_hidden_states=every).last_hidden_state
+            for y in (wide[..., :128], flat[1:].view(B, L, 128), x.transpose(0, 1).contiguous().transpose(0, 1)):
+                assert torch.equal(enc(y, mask, output_hidden_states=every).last_hidden_state, want)
+        for width in (64, 192):
+            with pytest.raises(RuntimeError):
+                enc(torch.randn(B, L, width, device="cuda").to(dtype), mask)
+        norm = enc.layer[0].output.LayerNorm
+        shifted = torch.empty(129, device="cuda", dtype=dtype)[1:]
+        norm.weight.data = shifted.copy_(norm.weight.data)
+        got = enc(x, mask).last_hidden_state
+    tol = 1e-4 if dtype == torch.float32 else 4e-2
+    assert (got.float() - want.float()).abs().max().item() <= tol * want.float().abs().max().item()

@@ -586,6 +586,14 @@ class Watch {
   py::object training_, forward_;
 };
 
+bool misaligned(const Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) & 15; }
+
+// x itself where the kernels can read it as it is, a copy otherwise (a slice of wider rows, or one that starts anywhere).
+Tensor rows_of_16_bytes(const Tensor& x) {
+  const Tensor c = x.contiguous();
+  return misaligned(c) ? c.clone() : c;
+}
+
 int64_t version_of(const Tensor& t) { return t.is_inference() ? 0 : (int64_t)t._version(); }
 
 // y = x W^T + b for bf16, straight through cuBLASLt: the library picks the kernel as it does behind torch's linear, but the
@@ -631,7 +639,6 @@ class Linear {
   static constexpr size_t WORKSPACE = 32u << 20;
 
  private:
-  static bool misaligned(const Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) & 15; }
   static void check(int rc) { TORCH_CHECK(rc == 0, "libtdb_b200: ", tdb_last_error(), " (code ", rc, ")"); }
   void product(Tensor& y, const Tensor& x, const Tensor& w, const Tensor& b) {
     if (try_run(y, x, w, b)) return;
@@ -728,23 +735,37 @@ class Encoder {
     l.derived = std::move(d);
     l.seen = stamp(l);
   }
+  // Whether the loop can run on x ([.., hidden]) with the parameters as they are now: sizes are taken from x below, vectors of the
+  // norms are read 16 bytes at a time, and a parameter's data may have been replaced by another tensor's.
   bool fits(const Tensor& x) const {
-    for (const Layer& l : layers_)
+    const int64_t hidden = 64 * heads_;
+    if (x.size(-1) != hidden) return false;
+    for (const Layer& l : layers_) {
+      const int64_t inner = l.up_b.numel();
+      if (l.out_w.sizes() != at::IntArrayRef{hidden, hidden} || l.up_w.sizes() != at::IntArrayRef{inner, hidden} ||
+          l.down_w.sizes() != at::IntArrayRef{hidden, inner})
+        return false;
+      for (const Tensor* t : {&l.out_b, &l.ln1_w, &l.ln1_b, &l.down_b, &l.ln2_w, &l.ln2_b})
+        if (t->numel() != hidden) return false;
+      for (const Tensor* t : {&l.ln1_w, &l.ln1_b, &l.ln2_w, &l.ln2_b})
+        if (misaligned(*t)) return false;
       for (const Tensor* t : {&l.out_w, &l.out_b, &l.ln1_w, &l.ln1_b, &l.up_w, &l.up_b, &l.down_w, &l.down_b, &l.ln2_w, &l.ln2_b})
         if (t->scalar_type() != x.scalar_type() || t->device() != x.device() || !t->is_contiguous()) return false;
+    }
     return true;
   }
   // x: [T, hidden].  Packed form: cu_seqlens; padded form: batch rows of `length` tokens, all valid.  Returns the outputs of
   // all layers (or of the last one), and the status words that the caller has to look at (see Status).
-  std::pair<std::vector<Tensor>, std::vector<Tensor>> run(const Tensor& x, const OptTensor& cu_seqlens, int64_t length, bool every) {
+  std::pair<std::vector<Tensor>, std::vector<Tensor>> run(const Tensor& given, const OptTensor& cu_seqlens, int64_t length, bool every) {
     std::pair<std::vector<Tensor>, std::vector<Tensor>> r;
     auto& [outs, words] = r;
     AllDerived all;
     all.reserve(layers_.size());
     for (const Layer& l : layers_) all.push_back(l.derived);
     py::gil_scoped_release nogil;
-    c10::cuda::CUDAGuard guard(x.device());
+    c10::cuda::CUDAGuard guard(given.device());
     at::AutoDispatchBelowAutograd below;
+    const Tensor x = rows_of_16_bytes(given);
     const c10::cuda::CUDAStream torch_stream = c10::cuda::getCurrentCUDAStream();
     const cudaStream_t stream = torch_stream.stream();
     if (!every) {
@@ -873,12 +894,13 @@ class Encoder {
 
   std::vector<const void*> weight_pointers(const AllDerived& all) const {
     std::vector<const void*> w;
-    w.reserve(layers_.size() * 14);
+    w.reserve(layers_.size() * 15);
     for (size_t i = 0; i < layers_.size(); ++i) {
       const Layer& l = layers_[i];
       const Derived& d = *all[i];
       for (const Tensor* t : {&d.qkv_w, &d.qkv_b, &l.out_w, &l.out_b, &l.ln1_w, &l.ln1_b, &l.up_w, &l.up_b, &l.down_w, &l.down_b, &l.ln2_w, &l.ln2_b})
         w.push_back(t->data_ptr());
+      w.push_back(reinterpret_cast<const void*>(l.up_w.size(0)));        // with the addresses, all that can differ
       w.push_back(d.tables ? ptr(d.tables->kr_exp) : nullptr);
       w.push_back(d.tables ? ptr(d.tables->qr_exp) : nullptr);
     }
@@ -1045,7 +1067,7 @@ py::object mask_rows(const Tensor& mask) {
 std::pair<Tensor, Tensor> pack_rows(const Tensor& x, const Tensor& mask, const Tensor& cu, int64_t tokens) {
   c10::cuda::CUDAGuard guard(x.device());
   cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
-  const Tensor m = mask_bytes(mask), xc = x.contiguous();
+  const Tensor m = mask_bytes(mask), xc = rows_of_16_bytes(x);
   const int64_t B = x.size(0), L = x.size(1), hidden = x.size(2);
   Tensor pos = at::empty({B * L}, cu.options()), out = at::empty({tokens, hidden}, x.options());
   int rc = tdb_mask_positions(m.data_ptr(), (int)m.element_size(), cu.data_ptr<int32_t>(), (int)B, (int)L, pos.data_ptr<int32_t>(), stream);

@@ -427,7 +427,8 @@ class FlashDebertaV2Encoder(DebertaV2Encoder):
             made = True
             w, b = attns[i]._qkv_weights()
             tables = attns[i]._relative_tables(rel_embeddings, dtype) if attns[i].relative_attention else None
-            if w.dtype != dtype or w.device != hidden_states.device:
+            hid = hidden_states.shape[-1]
+            if w.dtype != dtype or w.device != hidden_states.device or w.shape != (3 * hid, hid) or b.shape != (3 * hid,):
                 return None
             native.set_derived(i, w, b, None if tables is None else tables.native())
         if made and hidden_states.is_cuda and not torch.cuda.is_current_stream_capturing():
@@ -443,7 +444,8 @@ class FlashDebertaV2Encoder(DebertaV2Encoder):
                 or torch.nn.modules.module._has_any_global_hook() or hidden_states.numel() == 0):
             return None
         B, L, hid = hidden_states.shape
-        if torch.cuda.is_current_stream_capturing() or attention_mask is None or attention_mask.dim() != 2:
+        if (torch.cuda.is_current_stream_capturing() or attention_mask is None or attention_mask.dim() != 2
+                or attention_mask.device != hidden_states.device):
             info = analyse_mask(attention_mask, B, L, refresh=True)
             if not info.all_ones:
                 return None
