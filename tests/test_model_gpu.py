@@ -603,3 +603,34 @@ def test_encoder_inputs_of_any_layout(dtype, padded):
         got = enc(x, mask).last_hidden_state
     tol = 1e-4 if dtype == torch.float32 else 4e-2
     assert (got.float() - want.float()).abs().max().item() <= tol * want.float().abs().max().item()
+
+
+def test_recordings_are_kept_for_shapes_that_come_back():
+    """Eight recordings.  More shapes than that in turn push none of them out; a shape that keeps coming while another stays
+    away takes its place; weights that change with every pass are not recorded for.  Every pass gives the first one's result."""
+    from turbodeberta_b200 import model as M
+    torch.manual_seed(22)
+    model = M.FlashDebertaV2Model(_cfg(num_hidden_layers=2)).eval().to("cuda", torch.bfloat16)
+    ids = [torch.randint(1, 500, (1, n), device="cuda") for n in range(20, 32)]
+
+    @torch.no_grad()
+    def run(x):
+        out = model(input_ids=x, attention_mask=torch.ones_like(x)).last_hidden_state
+        return out, M._PLANS[model.encoder].native.recordings
+
+    want = [run(x)[0] for x in ids]
+    assert run(ids[0])[1] == 1                       # the second appearance
+    for _ in range(20):
+        for x, w in zip(ids, want):
+            out, made = run(x)
+            assert torch.equal(out, w)
+    assert made == 8
+    for i in range(12):
+        out, made = run(ids[11])                     # one of the four without a recording
+        assert torch.equal(out, want[11])
+    assert made == 9
+    made = run(ids[0])[1]
+    with torch.no_grad():
+        for _ in range(6):
+            model.encoder.layer[0].attention.self.key_proj.bias.add_(0.01)
+            assert run(ids[1])[1] == made

@@ -754,6 +754,7 @@ class Encoder {
     }
     return true;
   }
+  int64_t recordings() const { return recordings_; }
   // x: [T, hidden].  Packed form: cu_seqlens; padded form: batch rows of `length` tokens, all valid.  Returns the outputs of
   // all layers (or of the last one), and the status words that the caller has to look at (see Status).
   std::pair<std::vector<Tensor>, std::vector<Tensor>> run(const Tensor& given, const OptTensor& cu_seqlens, int64_t length, bool every) {
@@ -857,8 +858,10 @@ class Encoder {
 
   // Small passes are bound by the host: eight launches per layer of some 4 us each, for kernels of 2 to 8 us.  A shape that
   // comes a second time on a stream is recorded into a CUDA graph, which belongs to that stream (its buffers are in use until
-  // the replay is over), as long as the weights stay where they are.  At most GRAPHS of them, the longest unused one goes first.
-  static constexpr int GRAPHS = 8, BLOCK = 128;
+  // the replay is over), as long as the weights stay where they are.  At most GRAPHS of them.  A shape then has to come COMEBACKS
+  // times while the longest unused recording does not come once: only then does it take that one's place.  With any number of
+  // shapes in turn the first GRAPHS stay recorded and the others stay eager.
+  static constexpr int GRAPHS = 8, COMEBACKS = 8, SEEN = 64, BLOCK = 128;
   static constexpr int64_t GRAPH_MAX_ELEMENTS = 2048 * 1024;      // T * hidden: beyond it the GPU needs longer than the host
   struct Graph {
     int dev = 0, slot = -1;
@@ -892,6 +895,47 @@ class Encoder {
   // Device, id of the stream (no other gets it later, as it may get the handle), tokens, sequences (0: padded form), length.
   using Key = std::tuple<int, unsigned long long, int64_t, int64_t, int64_t>;
 
+  // A shape without a recording: when it last came with these weights, in passes, the latest at (n - 1) % COMEBACKS.
+  struct Seen {
+    std::vector<const void*> weights;
+    uint64_t at[COMEBACKS] = {}, n = 0;
+    void came(uint64_t pass, const std::vector<const void*>& with) {
+      if (weights != with) { weights = with; n = 0; }
+      at[n++ % COMEBACKS] = pass;
+    }
+    uint64_t last() const { return at[(n - 1) % COMEBACKS]; }
+    bool came_often_since(uint64_t pass) const { return n >= COMEBACKS && at[n % COMEBACKS] > pass; }
+  };
+
+  // The recording of this shape for these weights (one to be made, if it has none yet), or null if it is not worth one so far.
+  // What has to make room goes to `gone`.
+  Graph* recording_of(const Key& key, const std::vector<const void*>& weights, std::vector<std::unique_ptr<Graph>>& gone) {
+    const auto it = graphs_.find(key);
+    if (it != graphs_.end()) {
+      if (it->second->weights == weights) return it->second.get();
+      gone.push_back(std::move(it->second));                      // weights that change with every pass are not worth another
+      graphs_.erase(it);
+    }
+    Seen& s = seen_[key];
+    s.came(++uses_, weights);
+    auto older = [](const auto& a, const auto& b) { return a.second->used < b.second->used; };
+    const auto oldest = std::min_element(graphs_.begin(), graphs_.end(), older);
+    const bool room = graphs_.size() < GRAPHS;
+    if (room ? s.n < 2 : !s.came_often_since(oldest->second->used)) {
+      if (seen_.size() > SEEN)
+        seen_.erase(std::min_element(seen_.begin(), seen_.end(), [](const auto& a, const auto& b) { return a.second.last() < b.second.last(); }));
+      return nullptr;
+    }
+    seen_.erase(key);
+    if (!room) {
+      gone.push_back(std::move(oldest->second));
+      graphs_.erase(oldest);
+    }
+    Graph& g = *graphs_.emplace(key, std::make_unique<Graph>()).first->second;
+    g.weights = weights;
+    return &g;
+  }
+
   std::vector<const void*> weight_pointers(const AllDerived& all) const {
     std::vector<const void*> w;
     w.reserve(layers_.size() * 15);
@@ -918,35 +962,22 @@ class Encoder {
       return {};
     }
     const Key key(dev, id, x.size(0), cu_seqlens ? cu_seqlens->numel() - 1 : 0, length);
+    std::vector<std::unique_ptr<Graph>> gone;                     // destroyed, which waits for the GPU, without the lock
     std::lock_guard<std::mutex> lock(graph_mu_);
-    auto it = graphs_.find(key);
-    if (it == graphs_.end()) {
-      if (std::find(seen_.begin(), seen_.end(), key) == seen_.end()) {      // first time: not worth recording yet
-        seen_.push_back(key);
-        if (seen_.size() > 64) seen_.erase(seen_.begin());
+    Graph* g = recording_of(key, weight_pointers(all), gone);
+    if (!g || g->refused) return {};
+    if (!g->exec) {
+      if (!record(*g, all, x, cu_seqlens, length, id)) {
+        auto note = std::make_unique<Graph>();                    // without the buffers
+        note->refused = true;
+        note->weights = g->weights;
+        note->used = ++uses_;
+        gone.push_back(std::exchange(graphs_.at(key), std::move(note)));
         return {};
       }
-      if (graphs_.size() >= GRAPHS) {
-        auto oldest = graphs_.begin();
-        for (auto g = graphs_.begin(); g != graphs_.end(); ++g)
-          if (g->second->used < oldest->second->used) oldest = g;
-        graphs_.erase(oldest);
-      }
-      it = graphs_.emplace(key, std::make_unique<Graph>()).first;
+      ++recordings_;
     }
-    const bool same = it->second->weights == weight_pointers(all);
-    if (same && it->second->refused) return {};
-    if (!same || !it->second->exec) {
-      it->second = std::make_unique<Graph>();
-      if (!record(*it->second, all, x, cu_seqlens, length, id)) {
-        it->second = std::make_unique<Graph>();
-        it->second->refused = true;
-        it->second->weights = weight_pointers(all);
-        it->second->used = ++uses_;
-        return {};
-      }
-    }
-    return launch_graph(*it->second, x, cu_seqlens, stream);
+    return launch_graph(*g, x, cu_seqlens, stream);
   }
 
   bool record(Graph& g, const AllDerived& all, const Tensor& x, const OptTensor& cu_seqlens, int64_t length, unsigned long long stream_id) {
@@ -963,7 +994,6 @@ class Encoder {
     Tensor& ws = lt_workspaces_[{g.dev, stream_id}];
     if (!ws.defined()) ws = at::empty({(int64_t)Linear::WORKSPACE}, x.options().dtype(at::kByte));
     g.lt_ws = ws;
-    g.weights = weight_pointers(all);
     if (length > 2 * BLOCK) {                                     // long enough for far key tiles
       const int64_t n = cu_seqlens ? cu_seqlens->numel() - 1 : x.size(0) / length;
       g.partial = at::empty({(x.size(0) / BLOCK + 2 * n + 1) * BLOCK * heads_ * 66}, x.options().dtype(at::kFloat));
@@ -1027,9 +1057,10 @@ class Encoder {
   std::vector<Layer> layers_;
   std::mutex graph_mu_;
   std::map<Key, std::unique_ptr<Graph>> graphs_;
-  std::vector<Key> seen_;
+  std::map<Key, Seen> seen_;                                      // the last SEEN of them
   std::map<std::pair<int, unsigned long long>, Tensor> lt_workspaces_;       // by device and stream id
-  uint64_t uses_ = 0;
+  uint64_t uses_ = 0;                                             // passes that looked for a recording
+  int64_t recordings_ = 0;
 };
 
 
@@ -1123,6 +1154,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("stale", &Encoder::stale)
       .def("set_derived", &Encoder::set_derived)
       .def("fits", &Encoder::fits)
+      .def_property_readonly("recordings", &Encoder::recordings)
       .def("run", &Encoder::run);
   m.def("add_layernorm", [](const Tensor& x, const Tensor& res, const Tensor& w, const Tensor& b, double eps, const Tensor& out) {
     c10::cuda::CUDAGuard guard(x.device());
