@@ -435,12 +435,17 @@ def test_changed_stacks_and_settings_are_seen(dtype):
     mask[1, 20:] = 0
     v = mask.bool()
     enc = model.encoder
+    with torch.no_grad():                            # scores of some size, so that the position terms matter
+        for layer in enc.layer:
+            layer.attention.self.query_proj.weight.mul_(10)
+            layer.attention.self.key_proj.weight.mul_(10)
+            layer.attention.self.value_proj.weight.mul_(10)
 
     def prune():
         enc.layer = torch.nn.ModuleList(enc.layer[:2])
 
     def eps():
-        enc.layer[0].attention.output.LayerNorm.eps = 0.5
+        enc.layer[-1].output.LayerNorm.eps = 0.5
 
     def terms():
         for layer in enc.layer:
