@@ -702,7 +702,11 @@ struct Derived {
   Tensor qkv_w, qkv_b;
   std::optional<Tables> tables;
 };
-using AllDerived = std::vector<std::shared_ptr<const Derived>>;
+struct AllDerived {
+  std::vector<std::shared_ptr<const Derived>> layers;
+  uint64_t version = 0;                              // goes up whenever one of them is made anew
+  const Derived& operator[](size_t i) const { return *layers[i]; }
+};
 
 struct Layer {
   Tensor out_w, out_b, ln1_w, ln1_b, up_w, up_b, down_w, down_b, ln2_w, ln2_b;
@@ -734,6 +738,7 @@ class Encoder {
     if (!tables.is_none()) d->tables = *tables.cast<const Tables*>();
     l.derived = std::move(d);
     l.seen = stamp(l);
+    ++derived_version_;
   }
   // Whether the loop can run on x ([.., hidden]) with the parameters as they are now: sizes are taken from x below, vectors of the
   // norms are read 16 bytes at a time, and a parameter's data may have been replaced by another tensor's.
@@ -761,8 +766,9 @@ class Encoder {
     std::pair<std::vector<Tensor>, std::vector<Tensor>> r;
     auto& [outs, words] = r;
     AllDerived all;
-    all.reserve(layers_.size());
-    for (const Layer& l : layers_) all.push_back(l.derived);
+    all.version = derived_version_;
+    all.layers.reserve(layers_.size());
+    for (const Layer& l : layers_) all.layers.push_back(l.derived);
     py::gil_scoped_release nogil;
     c10::cuda::CUDAGuard guard(given.device());
     at::AutoDispatchBelowAutograd below;
@@ -782,7 +788,7 @@ class Encoder {
     Tensor in = x;
     for (size_t i = 0; i < layers_.size(); ++i) {
       Tensor out = every || i + 1 == layers_.size() ? at::empty_like(x) : s.z[i & 1];
-      layer(layers_[i], *all[i], in, out, s, cu_seqlens, length, linear, stream, i > 0, [&](tdb::AttnParams& p) {
+      layer(layers_[i], all[i], in, out, s, cu_seqlens, length, linear, stream, i > 0, [&](tdb::AttnParams& p) {
         Status st(dev, p);
         const Tensor partial = partial_scratch(p, dtype_code(x), TDB_KERNEL_AUTO, x);
         const int rc = tdb_run_attn(&p, dtype_code(x), TDB_KERNEL_AUTO, stream);
@@ -895,12 +901,11 @@ class Encoder {
   // Device, id of the stream (no other gets it later, as it may get the handle), tokens, sequences (0: padded form), length.
   using Key = std::tuple<int, unsigned long long, int64_t, int64_t, int64_t>;
 
-  // A shape without a recording: when it last came with these weights, in passes, the latest at (n - 1) % COMEBACKS.
+  // A shape without a recording: when it last came with these derived tensors, in passes, the latest at (n - 1) % COMEBACKS.
   struct Seen {
-    std::vector<const void*> weights;
-    uint64_t at[COMEBACKS] = {}, n = 0;
-    void came(uint64_t pass, const std::vector<const void*>& with) {
-      if (weights != with) { weights = with; n = 0; }
+    uint64_t at[COMEBACKS] = {}, n = 0, derived = 0;
+    void came(uint64_t pass, uint64_t with) {
+      if (std::exchange(derived, with) != with) n = 0;
       at[n++ % COMEBACKS] = pass;
     }
     uint64_t last() const { return at[(n - 1) % COMEBACKS]; }
@@ -909,15 +914,15 @@ class Encoder {
 
   // The recording of this shape for these weights (one to be made, if it has none yet), or null if it is not worth one so far.
   // What has to make room goes to `gone`.
-  Graph* recording_of(const Key& key, const std::vector<const void*>& weights, std::vector<std::unique_ptr<Graph>>& gone) {
+  Graph* recording_of(const Key& key, const AllDerived& all, std::vector<std::unique_ptr<Graph>>& gone) {
     const auto it = graphs_.find(key);
     if (it != graphs_.end()) {
-      if (it->second->weights == weights) return it->second.get();
+      if (it->second->weights == weight_pointers(all)) return it->second.get();
       gone.push_back(std::move(it->second));                      // weights that change with every pass are not worth another
       graphs_.erase(it);
     }
     Seen& s = seen_[key];
-    s.came(++uses_, weights);
+    s.came(++uses_, all.version);
     auto older = [](const auto& a, const auto& b) { return a.second->used < b.second->used; };
     const auto oldest = std::min_element(graphs_.begin(), graphs_.end(), older);
     const bool room = graphs_.size() < GRAPHS;
@@ -932,7 +937,7 @@ class Encoder {
       graphs_.erase(oldest);
     }
     Graph& g = *graphs_.emplace(key, std::make_unique<Graph>()).first->second;
-    g.weights = weights;
+    g.weights = weight_pointers(all);
     return &g;
   }
 
@@ -941,7 +946,7 @@ class Encoder {
     w.reserve(layers_.size() * 15);
     for (size_t i = 0; i < layers_.size(); ++i) {
       const Layer& l = layers_[i];
-      const Derived& d = *all[i];
+      const Derived& d = all[i];
       for (const Tensor* t : {&d.qkv_w, &d.qkv_b, &l.out_w, &l.out_b, &l.ln1_w, &l.ln1_b, &l.up_w, &l.up_b, &l.down_w, &l.down_b, &l.ln2_w, &l.ln2_b})
         w.push_back(t->data_ptr());
       w.push_back(reinterpret_cast<const void*>(l.up_w.size(0)));        // with the addresses, all that can differ
@@ -964,7 +969,7 @@ class Encoder {
     const Key key(dev, id, x.size(0), cu_seqlens ? cu_seqlens->numel() - 1 : 0, length);
     std::vector<std::unique_ptr<Graph>> gone;                     // destroyed, which waits for the GPU, without the lock
     std::lock_guard<std::mutex> lock(graph_mu_);
-    Graph* g = recording_of(key, weight_pointers(all), gone);
+    Graph* g = recording_of(key, all, gone);
     if (!g || g->refused) return {};
     if (!g->exec) {
       if (!record(*g, all, x, cu_seqlens, length, id)) {
@@ -1008,7 +1013,7 @@ class Encoder {
         Tensor in = g.x;
         for (size_t i = 0; good && i < layers_.size(); ++i) {
           Tensor out = i + 1 == layers_.size() ? g.out : g.scratch->z[i & 1];
-          layer(layers_[i], *all[i], in, out, *g.scratch, cu, length, linear, side, i > 0, [&](tdb::AttnParams& p) {
+          layer(layers_[i], all[i], in, out, *g.scratch, cu, length, linear, side, i > 0, [&](tdb::AttnParams& p) {
             p.status = g_pools[g.dev].host + g.slot * SLOT_WORDS;
             p.counter = g_pools[g.dev].ctl + g.slot * SLOT_WORDS;
             p.gave_up = p.counter + 1;
@@ -1061,6 +1066,7 @@ class Encoder {
   std::map<std::pair<int, unsigned long long>, Tensor> lt_workspaces_;       // by device and stream id
   uint64_t uses_ = 0;                                             // passes that looked for a recording
   int64_t recordings_ = 0;
+  uint64_t derived_version_ = 0;
 };
 
 
