@@ -498,21 +498,31 @@ def test_first_passes_of_several_threads():
         assert len(outs) == 16 and all(torch.equal(o, want) for o in outs)
 
 
+class _room:
+    """At most this many more bytes from the device while it lasts."""
+
+    def __init__(self, room):
+        self.room = room
+
+    def __enter__(self):
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        total = torch.cuda.get_device_properties(0).total_memory
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + self.room) / total)
+
+    def __exit__(self, *_):
+        torch.cuda.set_per_process_memory_fraction(1.0)
+
+
 def test_status_slots_survive_calls_that_run_out_of_memory():
     """More failing calls than there are slots: 32 MB of mask whose 256 MB of lengths and offsets do not fit."""
     from turbodeberta_b200._cabi import host
     mask = torch.ones(1 << 25, 1, dtype=torch.uint8, device="cuda")
     small = torch.ones(2, 3, dtype=torch.uint8, device="cuda")
-    torch.cuda.synchronize()
-    torch.cuda.empty_cache()
-    total = torch.cuda.get_device_properties(0).total_memory
-    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (64 << 20)) / total)
-    try:
+    with _room(64 << 20):
         for _ in range(300):
             with pytest.raises(torch.OutOfMemoryError):
                 host.mask_rows(mask)
-    finally:
-        torch.cuda.set_per_process_memory_fraction(1.0)
     assert host.mask_rows(small)[:4] == (True, True, 6, 3)
 
 
@@ -639,3 +649,52 @@ def test_recordings_are_kept_for_shapes_that_come_back():
         for _ in range(6):
             model.encoder.layer[0].attention.self.key_proj.bias.add_(0.01)
             assert run(ids[1])[1] == made
+
+
+def test_long_sequences_without_room_for_scratch_say_so():
+    """24 MB of output fit, 49 MB of scratch do not: a warning, and the same attention."""
+    import warnings
+    from turbodeberta_b200 import relpos
+    from turbodeberta_b200.ops.flash_attention import flash_attention_with_disentangled
+    torch.manual_seed(23)
+    q, k, v = (torch.randn(4, 4096, 12, 64, device="cuda").bfloat16().permute(0, 2, 1, 3) for _ in range(3))
+    w = [(torch.randn(768, 768, device="cuda") / 56).bfloat16() for _ in range(2)]
+    tables = relpos.build_tables(torch.randn(512, 768, device="cuda").bfloat16(), num_heads=12, position_buckets=256,
+                                 max_relative_positions=512, key_weight=w[0], query_weight=w[1])
+
+    def call():
+        return flash_attention_with_disentangled(q, k, v, None, None, False, 1 / 192 ** 0.5, 256, 512, tables=tables)
+    with warnings.catch_warnings():
+        warnings.simplefilter("error")
+        want = call()
+        with _room(40 << 20):
+            with pytest.raises(RuntimeWarning, match="49 MB of scratch"):
+                call()
+    with _room(40 << 20), pytest.warns(RuntimeWarning, match="49 MB of scratch"):
+        got = call()
+    # both round P to bf16 against reference exponents of their own: two roundings of half a unit, outputs below 1
+    assert (got.float() - want.float()).abs().max().item() < 8e-3
+
+
+def test_a_pass_that_fits_once_fits_again():
+    """The buffers of a recording may not fit where the pass itself does."""
+    from turbodeberta_b200.model import FlashDebertaV2Encoder
+    torch.manual_seed(24)
+    enc = FlashDebertaV2Encoder(_cfg(num_hidden_layers=2)).eval().to("cuda", torch.bfloat16)
+    x = torch.randn(32, 256, 128, device="cuda").bfloat16()          # 2 MB
+    mask = torch.ones(32, 256, dtype=torch.long, device="cuda")
+    fitted = 0
+    with torch.no_grad():
+        want = enc(x, mask, output_hidden_states=False).last_hidden_state
+        for room in range(32, 96, 4):
+            with torch.cuda.stream(torch.cuda.Stream()):
+                with _room(room << 20):
+                    try:
+                        first = enc(x, mask, output_hidden_states=False).last_hidden_state
+                    except torch.OutOfMemoryError:
+                        continue
+                    del first
+                    fitted += 1
+                    second = enc(x, mask, output_hidden_states=False).last_hidden_state
+                assert torch.equal(second, want)
+    assert fitted

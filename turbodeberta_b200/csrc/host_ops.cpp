@@ -125,7 +125,14 @@ std::pair<int, int> collect(int dev, int slot, bool keep = false) {
   return r;
 }
 
-// Scratch for long sequences (see AttnParams::part_o), if the device has room for it; the call works without it too.
+// A Python warning; as an error, where the caller's filters ask for that.
+void warn(const std::string& text) {
+  py::gil_scoped_acquire gil;
+  if (PyErr_WarnEx(PyExc_RuntimeWarning, text.c_str(), 1) < 0) throw py::error_already_set();
+}
+
+// Scratch for long sequences (see AttnParams::part_o), 264 bytes per query row and head, if the device has room for it.  The call
+// works without it too, on the kernel that takes near and far key tiles, and says so.
 Tensor partial_scratch(tdb::AttnParams& p, int dtype, int kernel, const Tensor& like) {
   const int64_t n = tdb_partial_floats(&p, dtype, kernel);
   if (n == 0) return {};
@@ -133,6 +140,8 @@ Tensor partial_scratch(tdb::AttnParams& p, int dtype, int kernel, const Tensor& 
   try {
     t = at::empty({n}, like.options().dtype(at::kFloat));
   } catch (const c10::OutOfMemoryError&) {
+    warn("turbodeberta_b200: no room for " + std::to_string(n * 4 >> 20) + " MB of scratch for long sequences; the call takes a kernel that "
+         "needs none and is up to 1.5 times slower (and torch's allocator has given its cached blocks back)");
     return {};
   }
   p.part_o = t.data_ptr<float>();
@@ -971,8 +980,17 @@ class Encoder {
     std::lock_guard<std::mutex> lock(graph_mu_);
     Graph* g = recording_of(key, all, gone);
     if (!g || g->refused) return {};
+    const Tensor y = at::empty_like(x);                           // before a recording takes its buffers
     if (!g->exec) {
-      if (!record(*g, all, x, cu_seqlens, length, id)) {
+      bool recorded;
+      try {
+        recorded = record(*g, all, x, cu_seqlens, length, id);
+      } catch (const c10::OutOfMemoryError&) {                    // a recording's buffers are its own: the pass may fit without
+        graphs_.erase(key);
+        drop_idle_workspaces();
+        return {};
+      }
+      if (!recorded) {
         auto note = std::make_unique<Graph>();                    // without the buffers
         note->refused = true;
         note->weights = g->weights;
@@ -982,7 +1000,14 @@ class Encoder {
       }
       ++recordings_;
     }
-    return launch_graph(*g, x, cu_seqlens, stream);
+    launch_graph(*g, x, cu_seqlens, y, stream);
+    return y;
+  }
+
+  // Those of streams whose last graph is gone.
+  void drop_idle_workspaces() {
+    for (auto w = lt_workspaces_.begin(); w != lt_workspaces_.end();)
+      w = w->second.use_count() == 1 ? lt_workspaces_.erase(w) : std::next(w);
   }
 
   bool record(Graph& g, const AllDerived& all, const Tensor& x, const OptTensor& cu_seqlens, int64_t length, unsigned long long stream_id) {
@@ -994,8 +1019,7 @@ class Encoder {
     OptTensor cu;
     if (cu_seqlens) cu = g.cu = at::empty_like(*cu_seqlens);
     g.scratch = std::make_unique<Scratch>(*this, x, cu_seqlens);
-    for (auto w = lt_workspaces_.begin(); w != lt_workspaces_.end();)     // of streams whose last graph is gone
-      w = w->second.use_count() == 1 ? lt_workspaces_.erase(w) : std::next(w);
+    drop_idle_workspaces();
     Tensor& ws = lt_workspaces_[{g.dev, stream_id}];
     if (!ws.defined()) ws = at::empty({(int64_t)Linear::WORKSPACE}, x.options().dtype(at::kByte));
     g.lt_ws = ws;
@@ -1038,10 +1062,9 @@ class Encoder {
     return good;
   }
 
-  Tensor launch_graph(Graph& g, const Tensor& x, const OptTensor& cu_seqlens, c10::cuda::CUDAStream torch_stream) {
+  void launch_graph(Graph& g, const Tensor& x, const OptTensor& cu_seqlens, const Tensor& y, c10::cuda::CUDAStream torch_stream) {
     const cudaStream_t stream = torch_stream.stream();
     g.used = ++uses_;
-    Tensor y = at::empty_like(x);
     cuda_ok(cudaMemcpyAsync(g.x.data_ptr(), x.data_ptr(), x.nbytes(), cudaMemcpyDeviceToDevice, stream), "copy of the encoder's input");
     if (cu_seqlens) cuda_ok(cudaMemcpyAsync(g.cu.data_ptr(), cu_seqlens->data_ptr(), cu_seqlens->nbytes(), cudaMemcpyDeviceToDevice, stream), "copy of the offsets");
     cuda_ok(cudaGraphLaunch(g.exec, stream), "cudaGraphLaunch");
@@ -1055,7 +1078,6 @@ class Encoder {
         listed = true;
       }
     if (!listed) p.pending.push_back({g.slot, Mark(torch_stream), true});
-    return y;
   }
 
   int heads_;
