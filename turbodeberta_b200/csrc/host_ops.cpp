@@ -506,16 +506,7 @@ class Watch {
     training_ = py::str("training");
     forward_ = py::str("forward");
     const py::object list_type = py::module_::import("torch.nn").attr("ModuleList");
-    for (py::handle s : settings) {
-      auto [module, name] = s.cast<std::pair<py::object, py::str>>();
-      py::dict dict = module.attr("__dict__");
-      py::object value;                              // stays null where the attribute is absent
-      if (dict.contains(name)) {
-        value = dict[name];
-        if (py::isinstance<py::list>(value)) value = value.attr("copy")();       // may be changed in place
-      }
-      settings_.push_back({dict, name, value});
-    }
+    std::map<PyObject*, size_t> at;
     for (py::handle m : modules) {
       Entry e;
       e.module = py::reinterpret_borrow<py::object>(m);
@@ -530,7 +521,20 @@ class Watch {
         for (auto kv : d) values.push_back(py::reinterpret_borrow<py::object>(kv.second));
         e.parts.emplace_back(d, std::move(values));
       }
+      at[m.ptr()] = entries_.size();
       entries_.push_back(std::move(e));
+    }
+    for (py::handle s : settings) {
+      auto [module, name] = s.cast<std::pair<py::object, py::str>>();
+      const auto found = at.find(module.ptr());
+      TORCH_CHECK(found != at.end(), "a setting of a module that is not watched");
+      Entry& e = entries_[found->second];
+      py::object value;                              // stays null where the attribute is absent
+      if (e.dict.contains(name)) {
+        value = e.dict[name];
+        if (py::isinstance<py::list>(value)) value = value.attr("copy")();       // may be changed in place
+      }
+      e.settings.emplace_back(name, value);
     }
   }
   bool holds() const {
@@ -551,6 +555,13 @@ class Watch {
       if (Py_TYPE(e.module.ptr()) != e.type) return false;
       PyObject* d = e.dict.ptr();
       if (e.runs && (PyDict_GetItem(d, training_.ptr()) != Py_False || PyDict_Contains(d, forward_.ptr()))) return false;
+      for (const auto& [name, value] : e.settings) {
+        PyObject* now = PyDict_GetItem(d, name.ptr());
+        if (now == value.ptr()) continue;
+        const int same = now && value ? PyObject_RichCompareBool(now, value.ptr(), Py_EQ) : 0;
+        if (same < 0) PyErr_Clear();                 // a value that does not compare is not the one of the plan
+        if (same != 1) return false;
+      }
       for (const py::dict& h : e.hooks)
         if (PyDict_Size(h.ptr()) != 0) return false;
       for (const auto& [dict, values] : e.parts) {
@@ -561,13 +572,6 @@ class Watch {
           if (v != values[i].ptr()) return false;
       }
     }
-    for (const Setting& s : settings_) {
-      PyObject* now = PyDict_GetItem(s.dict.ptr(), s.name.ptr());
-      if (now == s.value.ptr()) continue;
-      const int same = now && s.value ? PyObject_RichCompareBool(now, s.value.ptr(), Py_EQ) : 0;
-      if (same < 0) PyErr_Clear();                   // a value that does not compare is not the one of the plan
-      if (same != 1) return false;
-    }
     return true;
   }
 
@@ -576,22 +580,19 @@ class Watch {
   static void prefetch_keys(PyObject* d) {
     const char* k = reinterpret_cast<const char*>(reinterpret_cast<PyDictObject*>(d)->ma_keys);
     for (int i = 0; i < 8; ++i) __builtin_prefetch(k + 64 * i);
-    if (reinterpret_cast<PyDictObject*>(d)->ma_values) __builtin_prefetch(reinterpret_cast<PyDictObject*>(d)->ma_values);
+    const char* v = reinterpret_cast<const char*>(reinterpret_cast<PyDictObject*>(d)->ma_values);
+    for (int i = 0; v && i < 4; ++i) __builtin_prefetch(v + 64 * i);
   }
   struct Entry {
     py::object module;
     PyTypeObject* type;
     bool runs;                                       // a list has no forward, and its mode means nothing (a new one trains)
     py::dict dict;
+    std::vector<std::pair<py::object, py::object>> settings;     // name, value
     std::vector<py::dict> hooks;
     std::vector<std::pair<py::dict, std::vector<py::object>>> parts;
   };
-  struct Setting {
-    py::dict dict;
-    py::object name, value;
-  };
   std::vector<Entry> entries_;
-  std::vector<Setting> settings_;
   py::object training_, forward_;
 };
 

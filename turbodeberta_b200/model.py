@@ -406,7 +406,7 @@ class FlashDebertaV2Encoder(DebertaV2Encoder):
         """The plan with every layer's derived tensors up to date, or None where the native loop does not apply.  Whether a
         kept plan still matches the modules in its list is for the caller to ask (``watch.holds()``), once the GPU is busy."""
         plan = _PLANS.get(self)
-        if plan is None or plan.layers is not self.layer:
+        if plan is None or plan.layers is not self._modules["layer"]:
             plan = self._native_layers()
             if plan is None or not plan.watch.holds():
                 return None
