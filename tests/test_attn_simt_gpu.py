@@ -130,3 +130,27 @@ def test_backward_raises_like_the_reference():
     with torch.no_grad():
         o = flash_attention_with_disentangled(q, q, q, scores, None, position_buckets=256, max_relative_distance=512)
     assert not o.requires_grad
+
+
+@pytest.mark.parametrize("lengths,c2p,p2c", [([16], True, True), ([387, 300, 130, 65], True, True), ([512, 64], True, False), ([2048], True, True)])
+def test_fp32_error_does_not_grow_with_the_sequence(lengths, c2p, p2c):
+    """Relative 2-norm against float64 within four units of fp32 rounding (2^-24): the scores of unit variance bring about two, the
+    output's own rounding half of one, and sums over 16 keys, the tile and the tiles are short enough to stay below those."""
+    from turbodeberta_b200 import relpos
+    from turbodeberta_b200.ops.flash_attention import flash_attention_with_disentangled
+    from oracle import disentangled_oracle as orc
+    g = torch.Generator(device="cuda").manual_seed(31)
+    H, L = 4, max(lengths)
+    q, k, v = (torch.randn(len(lengths), L, H, 64, generator=g, device="cuda") for _ in range(3))
+    rel = torch.randn(512, H * 64, generator=g, device="cuda")
+    w = [torch.randn(H * 64, H * 64, generator=g, device="cuda") * (0.5 / (H * 64) ** 0.5) for _ in range(2)]
+    t = relpos.build_tables(rel, num_heads=H, position_buckets=256, max_relative_positions=512, key_weight=w[0], query_weight=w[1],
+                            c2p=c2p, p2c=p2c)
+    scale = 1 / (64 * (1 + c2p + p2c)) ** 0.5
+    got = flash_attention_with_disentangled(*(x.permute(0, 2, 1, 3) for x in (q, k, v)), None, None, False, scale, 256, 512, tables=t,
+                                            seqlens=torch.tensor(lengths, device="cuda", dtype=torch.int32))
+    f64 = lambda x: None if x is None else x.double().cpu().numpy()      # noqa: E731
+    want = orc.attention_fixed(f64(q), f64(k), f64(v), f64(t.kr), f64(t.qr), lengths, position_buckets=256, max_relative_positions=512,
+                               c2p=c2p, p2c=p2c, sm_scale=scale)
+    err = np.linalg.norm(got.permute(0, 2, 1, 3).double().cpu().numpy() - want) / np.linalg.norm(want)
+    assert err <= 4 * 2.0 ** -24, err
