@@ -5,8 +5,8 @@
 //
 //   score[q,k] = (Q[q].K[k] + Q[q].Kr[r] + K[k].Qr[r]) * sm_scale,  r = idx[clamp(q-k)]
 //
-// Legacy form: the two position products arrive materialised (c2p_scores[q, r], p2c_scores[k, r]) and are only
-// gathered; with TDB_FLAG_P2C_MIRRORED the p2c term is read at idx[clamp(k-q)], the reference kernel's convention.
+// Legacy form, f32: the two position products arrive materialised (c2p_scores[q, r], p2c_scores[k, r]) and are only
+// gathered (attn_scores.cu does so in bf16); with TDB_FLAG_P2C_MIRRORED the p2c term is read at idx[clamp(k-q)], the reference kernel's convention.
 //
 // Bound by the FMA pipes and, close behind, by shared-memory reads (256 fp32 multiply-adds per score with both terms).
 // A block of two warps owns 8R query rows and walks the keys in tiles of 64.  A thread owns R x 8 scores at rows ti + 8r and
@@ -31,9 +31,6 @@ namespace tdb {
 namespace {
 
 constexpr int KT = 64, HALF = 32, HP = HALF + 4, DP = 64 + 4, THREADS = 64, PV = 16;
-
-__device__ __forceinline__ float to_float(float x) { return x; }
-__device__ __forceinline__ float to_float(__nv_bfloat16 x) { return __bfloat162float(x); }
 
 __device__ __forceinline__ void cp_async16(float* dst, const void* src, bool real) {
   const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
@@ -102,9 +99,10 @@ template <int R> constexpr int smem_floats(bool tables) {
   return 2 * 8 * R * DP + (half > values ? half : values);
 }
 
-// TABLES: position terms from the projected tables (either may be absent); otherwise none, or gathered scores.
+// TABLES: position terms from the projected tables (either may be absent); otherwise none, or in f32 gathered scores.
 template <typename T, int R, bool TABLES>
 __global__ void __launch_bounds__(THREADS, 4) attn_simt_kernel(const AttnParams p) {
+  constexpr bool GATHER = !TABLES && sizeof(T) == 4;
   constexpr int QT = 8 * R, XR = QT + KT;           // XR: table rows a tile can touch (QT + KT - 1, padded)
   extern __shared__ __align__(16) float smem[];
   float* const sQ = smem;                            // [QT][DP]
@@ -131,9 +129,9 @@ __global__ void __launch_bounds__(THREADS, 4) attn_simt_kernel(const AttnParams 
   const T* const krh = (TABLES && (p.flags & TDB_FLAG_C2P)) ? reinterpret_cast<const T*>(p.kr) + (int64_t)h * p.two_span * 64 : nullptr;
   const T* const qrh = (TABLES && (p.flags & TDB_FLAG_P2C)) ? reinterpret_cast<const T*>(p.qr) + (int64_t)h * p.two_span * 64 : nullptr;
   // materialised scores: the base of this head's c2p rows (one per query) and p2c rows (one per key)
-  const T* const c2p_base = (!TABLES && (p.flags & TDB_FLAG_C2P))
+  const T* const c2p_base = (GATHER && (p.flags & TDB_FLAG_C2P))
       ? reinterpret_cast<const T*>(p.c2p_scores) + b * p.c2p_sb + tok0 * p.c2p_st + h * p.c2p_sh : nullptr;
-  const T* const p2c_base = (!TABLES && (p.flags & TDB_FLAG_P2C))
+  const T* const p2c_base = (GATHER && (p.flags & TDB_FLAG_P2C))
       ? reinterpret_cast<const T*>(p.p2c_scores) + b * p.p2c_sb + tok0 * p.p2c_st + h * p.p2c_sh : nullptr;
   const int dm = p.idx_delta_max;
   auto clamped = [&](int delta) { return delta < -dm ? 0 : (delta > dm ? 2 * dm : delta + dm); };
@@ -229,10 +227,10 @@ __global__ void __launch_bounds__(THREADS, 4) attn_simt_kernel(const AttnParams 
         for (int c = 0; c < 8; ++c) {
           const int kj = k0 + tj + 8 * c;
           float sc = acc[r][c];
-          if (!TABLES && kj < len && qi < len) {
+          if (GATHER && kj < len && qi < len) {
             const int x = clamped(qi - kj);
-            if (c2p_base) sc += to_float(c2p_base[(int64_t)qi * p.c2p_st + p.idx[x]]);
-            if (p2c_base) sc += to_float(p2c_base[(int64_t)kj * p.p2c_st + p.idx[(p.flags & TDB_FLAG_P2C_MIRRORED) ? 2 * dm - x : x]]);
+            if (c2p_base) sc += (float)c2p_base[(int64_t)qi * p.c2p_st + p.idx[x]];
+            if (p2c_base) sc += (float)p2c_base[(int64_t)kj * p.p2c_st + p.idx[(p.flags & TDB_FLAG_P2C_MIRRORED) ? 2 * dm - x : x]];
           }
           sc = kj < len ? sc * p.sm_scale : -CUDART_INF_F;
           acc[r][c] = sc;

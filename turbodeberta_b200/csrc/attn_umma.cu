@@ -62,11 +62,7 @@ using namespace ptx;
 namespace {
 
 constexpr int BAND = 256;
-#ifndef TDB_GROUPS
-#define TDB_GROUPS 4
-#endif
-constexpr int GROUPS = TDB_GROUPS;              // threads per query row (2 or 4)
-static_assert(GROUPS == 4, "four threads per query row (the drain split and the staging windows assume it)");
+constexpr int GROUPS = 4;                       // threads per query row (the drain split and the staging windows assume four)
 constexpr int KPT = BK / GROUPS;                // keys per thread in the softmax
 constexpr int OPT = HD / GROUPS;                // output columns per thread
 constexpr int NCW = 4 * GROUPS;                 // CUDA-core warps
@@ -84,14 +80,8 @@ constexpr uint32_t OFF_LX = OFF_CUR + 160;          // row-sum partials of a fin
 constexpr uint32_t OFF_MX = OFF_LX + 2 * GROUPS * BQ * 4;   // its reference exponents, [item parity][row]
 constexpr uint32_t OFF_PERM = OFF_MX + 2 * BQ * 4;          // padded form: sequences by decreasing length
 constexpr int PERM_MAX = 256;
-#ifndef TDB_FCB
-#define TDB_FCB 9
-#endif
-constexpr int FCB = TDB_FCB;                    // step of the exponential loop at which the fused c2p drain starts
-#ifndef TDB_FPB
-#define TDB_FPB 4
-#endif
-constexpr int FPB = TDB_FPB;                    // step of the c2p loop at which the fused p2c drain starts
+constexpr int FCB = 9;                          // step of the exponential loop at which the fused c2p drain starts
+constexpr int FPB = 4;                          // step of the c2p loop at which the fused p2c drain starts
 static_assert(FPB >= 0 && FPB + STG_COLS / GROUPS / 8 <= KPT / 2 - 1, "the fused drain's last step must lie inside the loop");
 static_assert(FCB >= 0 && FCB + STG_COLS / GROUPS / 8 <= KPT / 2 - 1, "the fused drain's last step must lie inside the loop");
 constexpr uint32_t SMEM_BYTES = OFF_PERM + PERM_MAX * 2 + 1024;   // + slack for the 1024-byte alignment of the base
