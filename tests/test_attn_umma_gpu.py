@@ -366,3 +366,28 @@ def test_short_padded_batches(lengths, L, c2p, p2c):
     for b, n in enumerate(lengths):
         assert torch.count_nonzero(o[b, :, n:]).item() == 0 and torch.count_nonzero(lse[b, :, n:]).item() == 0
         assert n == 0 or (lse[b, :, :n] - lse2[b, :, :n]).abs().max().item() < 1e-3
+
+
+@pytest.mark.parametrize("lengths,heads", [([40, 64, 9], 4), ([512, 200, 64], 4), ([2048, 1300], 2)])
+@pytest.mark.parametrize("c2p,p2c", [(True, True), (True, False), (False, True)])
+def test_error_against_float64_is_that_of_the_roundings(lengths, heads, c2p, p2c):
+    """Short, band and far kernels: relative 2-norm against the oracle.  Three roundings to bf16 at most (P, the output, the bands'
+    scores), each 0.86 * 2^-9 in that norm, in quadrature."""
+    from turbodeberta_b200 import relpos
+    from turbodeberta_b200.ops.flash_attention import flash_attention_with_disentangled
+    from oracle import disentangled_oracle as orc
+    g = torch.Generator(device="cuda").manual_seed(41)
+    L, hid = max(lengths), 64 * heads
+    q, k, v = (torch.randn(len(lengths), L, heads, 64, generator=g, device="cuda").bfloat16() for _ in range(3))
+    rel = torch.randn(512, hid, generator=g, device="cuda").bfloat16()
+    w = [(torch.randn(hid, hid, generator=g, device="cuda") * (0.5 / hid ** 0.5)).bfloat16() for _ in range(2)]
+    t = relpos.build_tables(rel, num_heads=heads, position_buckets=256, max_relative_positions=512, key_weight=w[0], query_weight=w[1],
+                            c2p=c2p, p2c=p2c)
+    scale = 1 / (64 * (1 + c2p + p2c)) ** 0.5
+    got = flash_attention_with_disentangled(*(x.permute(0, 2, 1, 3) for x in (q, k, v)), None, None, False, scale, 256, 512, tables=t,
+                                            seqlens=torch.tensor(lengths, device="cuda", dtype=torch.int32))
+    f64 = lambda x: None if x is None else util.f64(x)      # noqa: E731
+    want = orc.attention_fixed(f64(q), f64(k), f64(v), f64(t.kr), f64(t.qr), lengths, position_buckets=256, max_relative_positions=512,
+                               c2p=c2p, p2c=p2c, sm_scale=scale)
+    err = np.linalg.norm(util.f64(got.permute(0, 2, 1, 3)) - want) / np.linalg.norm(want)
+    assert err <= 3 ** 0.5 * 0.86 * 2.0 ** -9, err

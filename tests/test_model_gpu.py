@@ -700,3 +700,19 @@ def test_a_pass_that_fits_once_fits_again():
                     second = enc(x, mask, output_hidden_states=False).last_hidden_state
                 assert torch.equal(second, want)
     assert fitted
+
+
+@pytest.mark.parametrize("tokens,features", [(16, 3552), (16, 3560), (1, 4104), (17, 1184), (17, 1192), (32, 4096)])
+@pytest.mark.parametrize("columns", [32, 768, 1024])
+def test_skinny_projection_on_both_sides_of_its_rule(tokens, features, columns):
+    """8 features per block up to three (one token tile) or one (two) of them per SM, 16 beyond; also a last block that is half full."""
+    from turbodeberta_b200 import _cabi as cabi
+    torch.manual_seed(25)
+    x = torch.randn(tokens, columns, device="cuda").bfloat16()
+    w = (torch.randn(features, columns, device="cuda") / columns ** 0.5).bfloat16()
+    b = torch.randn(features, device="cuda").bfloat16()
+    y = torch.full((tokens + 1, features), float("nan"), device="cuda", dtype=torch.bfloat16)
+    cabi.check(cabi.host.skinny(x, w, b, False, y))
+    want = torch.nn.functional.linear(x.double(), w.double(), b.double())
+    assert ((y[:tokens].double() - want).abs() <= 5e-3 * want.abs() + 1e-5).all()
+    assert y[tokens].isnan().all()

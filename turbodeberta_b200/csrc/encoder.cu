@@ -45,7 +45,7 @@ __device__ __forceinline__ float warp_sum(float x) {
 // out may be x.  No __restrict__ on the activations: the kernel may have started beside the one that writes them, and the
 // non-coherent loads that it allows are not part of what wait_for_stream() makes visible.
 // out = LayerNorm(x + res) * w + b, one warp per row, the row held in registers (fp32 sum, mean and variance).  Per row three
-// row-sized transfers; 9.2k x 1024 bf16 (57 MB): 24 + 8 us as an addition and a LayerNorm kernel, about 10 us here.
+// row-sized transfers; 9.2k x 1024 bf16 (57 MB): 24 + 8 us as an addition and a LayerNorm kernel, 11.4 us here.
 // FEW: for a few rows the loads' latency is the kernel's time, so w and b come first; with many rows they are in the first-level
 // cache and better left out of the registers (9.2k x 1024: 13.8 us with, 11.4 without).
 template <typename T, int NV, bool FEW>
@@ -106,7 +106,9 @@ int launch_add_layernorm_t(const void* x, const void* res, const void* w, const 
                            bool early, cudaStream_t s) {
   constexpr int PER = 32 * Vec<T>::N;
   const int nv = (hidden + PER - 1) / PER;
-  const int warps = rows >= 148 * 16 ? 4 : 1;        // few rows: one per block, so that they spread over the SMs
+  int sms = 0;
+  if (const int rc = device_sms(&sms)) return rc;
+  const int warps = rows >= 16 * sms ? 4 : 1;        // few rows: one per block, so that they spread over the SMs
   const unsigned blocks = (unsigned)((rows + warps - 1) / warps);
 #define TDB_LN(NV)                                                                                                              \
   if (nv <= NV) {                                                                                                               \

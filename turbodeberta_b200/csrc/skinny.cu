@@ -96,10 +96,15 @@ cudaError_t launch(const void* x, const void* w, const void* b, int T, int K, in
 }
 
 template <int MT>
-cudaError_t launch_rows(const void* x, const void* w, const void* b, int T, int K, int N, bool gelu, bool early, void* y, cudaStream_t s) {
+cudaError_t launch_rows(const void* x, const void* w, const void* b, int T, int K, int N, bool gelu, bool early, void* y, int sms, cudaStream_t s) {
   const int nb = (K / KB + WARPS - 1) / WARPS;
-  // 16 features per block read x half as often; 8 where 16 would leave SMs without a block or the registers without room.
-  if (nb <= 4) return N >= 148 * 16 - 64 ? launch<MT, 2, 4>(x, w, b, T, K, N, gelu, early, y, s) : launch<MT, 1, 4>(x, w, b, T, K, N, gelu, early, y, s);
+  // 16 features per block read x half as often, 8 make more blocks.  What decides is how many blocks of 8 an SM would get: up to 16
+  // tokens three are no worse than two of 16, with two token tiles a second one already is.  us per projection, weights from memory,
+  // 8 against 16 features: 16 tokens, K 768, N 2304 2.58 and 2.62, N 3072 3.44 and 3.44, N 4096 4.28 and 3.61; 32 tokens, K 768, N 1024
+  // 2.68 and 2.63, N 1536 2.97 and 2.71, N 2560 4.30 and 3.54; K 1024, N 1024 2.85 and 2.93, N 3072 5.41 and 4.70.  More columns
+  // leave no registers for 16.
+  if (nb <= 4)
+    return N > 8 * sms * (MT == 1 ? 3 : 1) ? launch<MT, 2, 4>(x, w, b, T, K, N, gelu, early, y, s) : launch<MT, 1, 4>(x, w, b, T, K, N, gelu, early, y, s);
   if (nb <= 8) return launch<MT, 1, 8>(x, w, b, T, K, N, gelu, early, y, s);
   if (nb <= 12) return launch<MT, 1, 12>(x, w, b, T, K, N, gelu, early, y, s);
   return launch<MT, 1, 16>(x, w, b, T, K, N, gelu, early, y, s);
@@ -113,16 +118,21 @@ using namespace tdb;
 
 extern "C" {
 
-// Every block reads all of x, so the line lies where that costs more than the library's tiles do.  One projection, weights from
-// memory, K 3072 and N 768, this kernel against the library's: 16 tokens 5.6 and 7.4 us, 32 tokens 6.3 and 6.7, 64 tokens 7.6
-// and 6.6; K 768 and N 2304: 3.0 and 3.6, 4.1 and 4.1, 5.1 and 4.1.  A pass of the base model, before and after: 8 tokens 531 and 445 us,
-// 16 tokens 512 and 449, 32 tokens 507 and 495; of the large one: 16 tokens 1057 and 884, 32 tokens 1000 and 999.  K up to what a warp's registers hold.
+// Every block reads all of x, so the line lies where that costs more than the library's tiles do.  us per projection, weights from
+// memory, this kernel against the library's.  32 tokens: K 768 and N 768 2.5 and 3.3, N 2304 3.0 and 3.9, N 3072 4.1 and 4.2, K 3072
+// and N 768 5.8 and 6.6; K 1024 and N 3072 4.7 and 4.7, N 4096 5.5 and 5.0 (where GELU in the epilogue saves a launch).  With three token
+// tiles the narrow projections would still gain and the wide ones lose, 48 tokens: 3.2 and 3.3, 4.0 and 4.1, 4.8 and 4.4, 6.5 and
+// 6.7; K 1024 5.6 and 4.8, 5.9 and 5.1; with four all lose (64 tokens: 3.5 and 3.3, 4.2 and 4.0, 5.6 and 4.4, 7.0 and 6.8).  A pass of the
+// base model with and without: 8 tokens 445 and 531 us, 16 tokens 449 and 512, 32 tokens 495 and 507; of the large one: 16 tokens 884
+// and 1057, 32 tokens 999 and 1000.  K up to what a warp's registers hold.
 int tdb_skinny_applies(int64_t T, int64_t K, int64_t N) { return T <= SKINNY_TOKENS && K % KB == 0 && K <= KB * WARPS * 16 && N % 8 == 0; }
 
 int tdb_skinny(const void* x, const void* w, const void* b, int T, int K, int N, int gelu, int early, void* y, void* stream) {
   cudaStream_t s = (cudaStream_t)stream;
-  const cudaError_t e = T <= 16 ? launch_rows<1>(x, w, b, T, K, N, gelu, early, y, s)
-                                : launch_rows<2>(x, w, b, T, K, N, gelu, early, y, s);
+  int sms = 0;
+  if (const int rc = device_sms(&sms)) return rc;
+  const cudaError_t e = T <= 16 ? launch_rows<1>(x, w, b, T, K, N, gelu, early, y, sms, s)
+                                : launch_rows<2>(x, w, b, T, K, N, gelu, early, y, sms, s);
   return cuda_fail(e, "skinny projection launch");
 }
 
