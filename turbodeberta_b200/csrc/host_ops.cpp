@@ -731,6 +731,9 @@ struct Layer {
 class Encoder {
  public:
   Encoder(int heads) : heads_(heads) {}
+  ~Encoder() {
+    if (ready_) cudaEventDestroy(ready_);
+  }
   void add_layer(std::vector<Tensor> w, double eps1, double eps2, double sm_scale, std::vector<Tensor> sources) {
     TORCH_CHECK(w.size() == 10);
     layers_.push_back(Layer{w[0], w[1], w[2], w[3], w[4], w[5], w[6], w[7], w[8], w[9], eps1, eps2, sm_scale, std::move(sources), {}, {}});
@@ -749,6 +752,18 @@ class Encoder {
     l.derived = std::move(d);
     l.seen = stamp(l);
     ++derived_version_;
+  }
+  // The derived tensors were made on the current stream, which may not be done with that.
+  void set_ready() {
+    const cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
+    if (ready_) {                                                 // of others, made on another stream perhaps
+      cuda_ok(cudaStreamWaitEvent(stream, ready_, 0), "cudaStreamWaitEvent");
+      cudaEventDestroy(std::exchange(ready_, nullptr));
+    }
+    if (cudaEventCreateWithFlags(&ready_, cudaEventDisableTiming) == cudaSuccess && cudaEventRecord(ready_, stream) == cudaSuccess) return;
+    (void)cudaGetLastError();
+    if (ready_) cudaEventDestroy(std::exchange(ready_, nullptr));
+    cuda_ok(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
   }
   // Whether the loop can run on x ([.., hidden]) with the parameters as they are now: sizes are taken from x below, vectors of the
   // norms are read 16 bytes at a time, and a parameter's data may have been replaced by another tensor's.
@@ -779,8 +794,17 @@ class Encoder {
     all.version = derived_version_;
     all.layers.reserve(layers_.size());
     for (const Layer& l : layers_) all.layers.push_back(l.derived);
-    py::gil_scoped_release nogil;
     c10::cuda::CUDAGuard guard(given.device());
+    if (ready_ && at::cuda::currentStreamCaptureStatusMayInitCtx() == at::cuda::CaptureStatus::None) {       // this stream may be another
+      const cudaError_t e = cudaEventQuery(ready_);
+      if (e == cudaSuccess) {
+        cudaEventDestroy(std::exchange(ready_, nullptr));
+      } else {
+        (void)cudaGetLastError();
+        cuda_ok(cudaStreamWaitEvent(c10::cuda::getCurrentCUDAStream().stream(), ready_, 0), "cudaStreamWaitEvent");
+      }
+    }
+    py::gil_scoped_release nogil;
     at::AutoDispatchBelowAutograd below;
     const Tensor x = rows_of_16_bytes(given);
     const c10::cuda::CUDAStream torch_stream = c10::cuda::getCurrentCUDAStream();
@@ -1090,6 +1114,7 @@ class Encoder {
   uint64_t uses_ = 0;                                             // passes that looked for a recording
   int64_t recordings_ = 0;
   uint64_t derived_version_ = 0;
+  cudaEvent_t ready_ = nullptr;                                   // behind what made them; used with the interpreter lock held
 };
 
 
@@ -1182,6 +1207,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("add_layer", &Encoder::add_layer)
       .def("stale", &Encoder::stale)
       .def("set_derived", &Encoder::set_derived)
+      .def("set_ready", &Encoder::set_ready)
       .def("fits", &Encoder::fits)
       .def_property_readonly("recordings", &Encoder::recordings)
       .def("run", &Encoder::run);

@@ -432,8 +432,8 @@ class FlashDebertaV2Encoder(DebertaV2Encoder):
                 return None
             native.set_derived(i, w, b, None if tables is None else tables.native())
         if made and hidden_states.is_cuda and not torch.cuda.is_current_stream_capturing():
-            # the next pass may come from another thread on another stream, which does not wait for this one
-            torch.cuda.current_stream(hidden_states.device).synchronize()
+            with torch.cuda.device(hidden_states.device):
+                native.set_ready()               # passes on other streams wait for this
         plan.stamp = stamp_now
         return plan
 
