@@ -499,7 +499,7 @@ Tensor mask_bytes(const Tensor& mask) {
 // A set of modules whose forward the native encoder stands in for, as it was when the plan was made.  The plan holds as long
 // as nobody has put a hook, a new child or parameter, or another forward on any of them, and all are in eval mode.  Checked
 // on every forward, so it follows pointers instead of looking names up: a module keeps its hook, child and parameter dicts.
-// settings: (module, attribute name) pairs of what else the plan was made from (a norm's eps, an attention's position terms).
+// settings: (module, names of attributes) pairs of what else the plan was made from (a norm's eps, an attention's position terms).
 class Watch {
  public:
   Watch(const py::list& modules, const py::list& settings) {
@@ -525,16 +525,17 @@ class Watch {
       entries_.push_back(std::move(e));
     }
     for (py::handle s : settings) {
-      auto [module, name] = s.cast<std::pair<py::object, py::str>>();
-      const auto found = at.find(module.ptr());
-      TORCH_CHECK(found != at.end(), "a setting of a module that is not watched");
+      const py::tuple of = py::reinterpret_borrow<py::tuple>(s), names = of[1];
+      const auto found = at.find(of[0].ptr());
+      TORCH_CHECK(found != at.end(), "settings of a module that is not watched");
       Entry& e = entries_[found->second];
-      py::object value;                              // stays null where the attribute is absent
-      if (e.dict.contains(name)) {
-        value = e.dict[name];
-        if (py::isinstance<py::list>(value)) value = value.attr("copy")();       // may be changed in place
+      e.settings.reserve(names.size());
+      for (py::handle name : names) {
+        PyObject* now = PyDict_GetItem(e.dict.ptr(), name.ptr());               // null where the attribute is absent
+        py::object value = py::reinterpret_borrow<py::object>(now);
+        if (now && PyList_Check(now)) value = py::reinterpret_steal<py::object>(PyList_GetSlice(now, 0, PyList_Size(now)));       // may be changed in place
+        e.settings.emplace_back(py::reinterpret_borrow<py::object>(name), std::move(value));
       }
-      e.settings.emplace_back(name, value);
     }
   }
   bool holds() const {

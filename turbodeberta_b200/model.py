@@ -284,9 +284,11 @@ _PLANS: "weakref.WeakKeyDictionary" = weakref.WeakKeyDictionary()
 # Held while a plan is made or brought up to date: one thread does it, the others find it done.
 _PLAN_LOCK = threading.RLock()
 
-#: what the native loop takes over from an attention module besides its weights
+#: what the native loop takes over from the modules besides their weights
 _ATTENTION_SETTINGS = ("num_attention_heads", "attention_head_size", "pos_att_type", "share_att_key", "relative_attention",
                        "position_buckets", "max_relative_positions")
+_NORM_SETTINGS = ("eps", "normalized_shape")
+_GELU_SETTINGS = ("act", "approximate")
 
 
 class _EncoderPlan:
@@ -382,7 +384,8 @@ class FlashDebertaV2Encoder(DebertaV2Encoder):
                 return None
             if any(type(m) is not nn.LayerNorm or m.weight is None or m.bias is None for m in norms):
                 return None
-            drops = [so.dropout, down.dropout] + ([sa.pos_dropout] if sa.relative_attention else [])
+            drops = [so._modules.get("dropout"), down._modules.get("dropout")]
+            drops += [sa._modules.get("pos_dropout")] if sa.relative_attention else []
             if any(type(m) not in (nn.Dropout, nn.Identity) for m in drops):         # in eval mode both do nothing
                 return None
             hidden = so.dense.out_features
@@ -396,8 +399,7 @@ class FlashDebertaV2Encoder(DebertaV2Encoder):
                               down.dense.weight, down.dense.bias, norms[1].weight, norms[1].bias], norms[0].eps,
                              norms[1].eps, 1.0 / math.sqrt(64 * terms), [t for m in lins[:3] + lins[6:] for t in (m.weight, m.bias)])
             attns.append(sa)
-            settings += [(sa, name) for name in _ATTENTION_SETTINGS]
-            settings += [(m, name) for m in norms for name in ("eps", "normalized_shape")] + [(act, "act"), (act, "approximate")]
+            settings += [(sa, _ATTENTION_SETTINGS), (norms[0], _NORM_SETTINGS), (norms[1], _NORM_SETTINGS), (act, _GELU_SETTINGS)]
         if native is None:
             return None
         return _EncoderPlan(self.layer, host.Watch(list(self.layer.modules()), settings), native, attns)
@@ -577,7 +579,7 @@ class FlashDebertaV2Model(DebertaV2Model):
                     or type(emb.LayerNorm) is not nn.LayerNorm or emb.word_embeddings.max_norm is not None
                     or any(getattr(emb, n, None) is not None for n in ("position_embeddings", "token_type_embeddings", "embed_proj"))):
                 return None
-            watch = host.Watch(list(emb.modules()), [(emb.word_embeddings, "max_norm")])
+            watch = host.Watch(list(emb.modules()), [(emb.word_embeddings, ("max_norm",))])
             _PLANS[self] = (watch, emb)
         if not watch.holds():
             _PLANS.pop(self, None)
