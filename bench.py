@@ -28,10 +28,10 @@ sys.path.insert(0, ROOT)
 
 METRIC = "disentangled_attn_algorithmic_tflops"
 UNIT = "TFLOP/s"
-# dram__bytes_read.sum + dram__bytes_write.sum of ONE launch of the attention kernel, from an ncu capture of that
-# workload, as summarised in profiles/ (c2: 56.31 MB read + 3.54..3.96 MB written; c3: 420.3 + 106.9 MB; c5f: 80.3 + 11.2 MB).
+# dram__bytes_read.sum + dram__bytes_write.sum of ONE step's attention kernels, from an ncu capture of that workload, as summarised
+# in profiles/ (c2: 56.30 MB read + 4.03 MB written; c3: 422.2 + 104.4 MB; c5f: near 80.3 + 27.4 MB, far 130.8 + 17.9 MB).
 # Workloads without a capture report null.
-NCU_TRAFFIC_BYTES = {"c2": 60.06e6, "c3": 527.2e6, "c5f": 91.47e6}
+NCU_TRAFFIC_BYTES = {"c2": 60.34e6, "c3": 526.6e6, "c5f": 256.4e6}
 NO_TRAFFIC_REASON = "no ncu capture of this workload (a launch holds more than the capture-size rule allows or was not captured)"
 
 

@@ -103,7 +103,9 @@ TDB_API size_t tdb_attn_workspace_bytes(int n_seqs, int64_t total_tokens);
  * status: int32[4] device words, zero on entry; word 0 becomes non-zero if a bounded wait gave up, word 1 if
  * cu_seqlens was malformed (packed form: decreasing offsets, a sequence longer than max_seqlen, a last offset that
  * differs from total_tokens); word 2 is used by the tensor-core kernel as its work counter (the launch
- * resets it), word 3 is reserved.  Do not share one status block between launches that can overlap. */
+ * resets it), word 3 is reserved.  Do not share one status block between launches that can overlap.
+ * Sequences beyond twice the saturation distance: these entry points take no scratch, so one kernel works on near and
+ * far key tiles; the Python operators allocate 264 bytes per query row and head and run two, 1.5 times as fast. */
 TDB_API int tdb_attn_fwd_fixed(const void* q, const void* k, const void* v, void* o,
                        int64_t q_sb, int64_t q_st, int64_t q_sh,
                        int64_t k_sb, int64_t k_st, int64_t k_sh,

@@ -17,10 +17,14 @@
 // is that neither waits for the other: three score buffers go round the two groups, so a group's next scores are complete
 // before it has finished with the last ones, and only P.V follows its hand-off; and the two kinds of product are issued by two
 // warps, because issuing blocks while the tensor pipe is busy and a lone issuing warp then adds its waits and commits (some
-// 100 clocks each) to every batch.  A pair of tiles takes 2500 clocks (4 x 4096 tokens: 242 us for the kernel).  With one
+// 100 clocks each) to every batch.  A pair of tiles takes 2500 clocks (4 x 4096 tokens: 247 us for the kernel).  With one
 // buffer per group and one issuing lane it took 4300, with three buffers and one issuing warp 3300; in the one kernel for all
 // tiles, with one accumulator and all sixteen warps in step, 7400.  A quarter of the exponentials as polynomials on the FMA
-// pipe, and tokens that let one group at a time take exponentials, were slower (254 us and 266 us).
+// pipe, and tokens that let one group at a time take exponentials, were slower (254 us and 266 us against 242 of the version before).
+//
+// Error against float64: 2.392e-3 in the relative 2-norm at 1 x 4096, 2.379e-3 at 2 x 2048 with 64 buckets, against 2.389e-3 and
+// 2.373e-3 of the one kernel for all tiles.  A pair of query tiles has its far tiles in common, so a tile more per side of each
+// row is taken as a near one, whose bands are staged in bf16.
 //
 // Half-step t is group t & 1 at its tile t / 2.  Tensor-memory columns: three buffers of 128, S(t) in buffer t % 3 and P(t) (bf16)
 // over the columns of S(t) that its own thread has read; O of the two groups at [384,448) [448,512).

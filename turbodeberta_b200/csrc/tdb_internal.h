@@ -90,7 +90,7 @@ int launch_relpos_expand(const void* table, const int16_t* idx, int idx_delta_ma
 int launch_bounded_wait_selftest(int32_t* status, int code, uint64_t limit_ns, cudaStream_t s);
 int launch_attn_simt(const AttnParams& p, int dtype, cudaStream_t s);
 int launch_attn_scores(const AttnParams& p, cudaStream_t s);          // bf16, materialised position scores
-bool small_applicable(const AttnParams& p);                            // padded sequences of at most 64 tokens
+bool small_applicable(const AttnParams& p);                            // sequences of at most 64 tokens: padded, or packed with a known longest
 int launch_attn_small(const AttnParams& p, cudaStream_t s);
 int launch_attn_umma(const AttnParams& p, cudaStream_t s);
 bool has_far_tiles(const AttnParams& p);
