@@ -20,6 +20,7 @@
 #include <algorithm>
 #include <map>
 #include <mutex>
+#include <unordered_map>
 #include <utility>
 #include <vector>
 
@@ -33,12 +34,17 @@ namespace {
 
 constexpr int MAX_DEV = 64, SLOTS = 256, SLOT_WORDS = 4;
 
+// Whether the stream is a caller's (cudaStreamCreate, handed to torch) and not one of torch's or the legacy one.
+bool is_external(c10::cuda::CUDAStream s) {
+  return s.stream() && c10::cuda::getStreamFromExternal(s.stream(), s.device_index()).id() == s.id();
+}
+
 // The end of what a stream holds now.  torch never destroys its own streams, so their handle stays good to wait for; one that a
 // caller made and handed to torch may be gone by then, and is marked with an event instead.
 class Mark {
  public:
   explicit Mark(c10::cuda::CUDAStream s) : stream_(s.stream()) {
-    if (!stream_ || c10::cuda::getStreamFromExternal(stream_, s.device_index()).id() != s.id()) return;
+    if (!is_external(s)) return;
     own_ = false;
     if (cudaEventCreateWithFlags(&event_, cudaEventDisableTiming) != cudaSuccess) event_ = nullptr;
     renew();
@@ -506,7 +512,9 @@ class Watch {
     training_ = py::str("training");
     forward_ = py::str("forward");
     const py::object list_type = py::module_::import("torch.nn").attr("ModuleList");
-    std::map<PyObject*, size_t> at;
+    std::unordered_map<PyObject*, size_t> at;
+    at.reserve(modules.size());
+    entries_.reserve(modules.size());
     for (py::handle m : modules) {
       Entry e;
       e.module = py::reinterpret_borrow<py::object>(m);
@@ -549,6 +557,7 @@ class Watch {
     }
     for (const Entry& e : entries_) {
       prefetch_keys(e.dict.ptr());
+      if (!e.settings.empty()) prefetch_values(e.dict.ptr());
       for (const auto& part : e.parts)
         if (!part.second.empty()) prefetch_keys(part.first.ptr());
     }
@@ -581,8 +590,11 @@ class Watch {
   static void prefetch_keys(PyObject* d) {
     const char* k = reinterpret_cast<const char*>(reinterpret_cast<PyDictObject*>(d)->ma_keys);
     for (int i = 0; i < 8; ++i) __builtin_prefetch(k + 64 * i);
+    if (reinterpret_cast<PyDictObject*>(d)->ma_values) __builtin_prefetch(reinterpret_cast<PyDictObject*>(d)->ma_values);
+  }
+  static void prefetch_values(PyObject* d) {         // the first line: above
     const char* v = reinterpret_cast<const char*>(reinterpret_cast<PyDictObject*>(d)->ma_values);
-    for (int i = 0; v && i < 4; ++i) __builtin_prefetch(v + 64 * i);
+    for (int i = 1; v && i < 4; ++i) __builtin_prefetch(v + 64 * i);
   }
   struct Entry {
     py::object module;
@@ -746,16 +758,23 @@ class Encoder {
       if (!current(layers_[i])) r.push_back((int)i);
     return r;
   }
-  void set_derived(int i, Tensor qkv_w, Tensor qkv_b, py::object tables) {
+  // False: not tensors that the loop can take for inputs like x.
+  bool set_derived(int i, const Tensor& x, Tensor qkv_w, Tensor qkv_b, py::object tables) {
+    const int64_t hidden = 64 * heads_;
+    if (qkv_w.scalar_type() != x.scalar_type() || qkv_w.device() != x.device() || qkv_w.sizes() != at::IntArrayRef{3 * hidden, hidden} ||
+        qkv_b.numel() != 3 * hidden)
+      return false;
     Layer& l = layers_.at(i);
     auto d = std::make_shared<Derived>(Derived{std::move(qkv_w), std::move(qkv_b), std::nullopt});
     if (!tables.is_none()) d->tables = *tables.cast<const Tables*>();
     l.derived = std::move(d);
     l.seen = stamp(l);
     ++derived_version_;
+    return true;
   }
-  // The derived tensors were made on the current stream, which may not be done with that.
-  void set_ready() {
+  // The derived tensors for inputs like x were made on the current stream, which may not be done with that.
+  void set_ready(const Tensor& x) {
+    c10::cuda::CUDAGuard guard(x.device());
     const cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
     if (ready_) {                                                 // of others, made on another stream perhaps
       cuda_ok(cudaStreamWaitEvent(stream, ready_, 0), "cudaStreamWaitEvent");
@@ -939,8 +958,9 @@ class Encoder {
       if (!listed) p.free.push_back(slot);
     }
   };
-  // Device, id of the stream (no other gets it later, as it may get the handle), tokens, sequences (0: padded form), length.
-  using Key = std::tuple<int, unsigned long long, int64_t, int64_t, int64_t>;
+  // Of a stream, and of no other later (as a caller's handle may be): torch's own id, or CUDA's for a caller's stream.
+  using StreamId = std::pair<bool, uint64_t>;
+  using Key = std::tuple<int, StreamId, int64_t, int64_t, int64_t>;        // device, stream, tokens, sequences (0: padded form), length
 
   // A shape without a recording: when it last came with these derived tensors, in passes, the latest at (n - 1) % COMEBACKS.
   struct Seen {
@@ -1002,10 +1022,14 @@ class Encoder {
         at::cuda::currentStreamCaptureStatusMayInitCtx() != at::cuda::CaptureStatus::None)
       return {};
     const int dev = x.get_device();
-    unsigned long long id = 0;
-    if (cudaStreamGetId(stream.stream(), &id) != cudaSuccess) {
-      (void)cudaGetLastError();
-      return {};
+    StreamId id(is_external(stream), (uint64_t)stream.id());
+    if (id.first) {
+      unsigned long long unique = 0;
+      if (cudaStreamGetId(stream.stream(), &unique) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return {};
+      }
+      id.second = unique;
     }
     const Key key(dev, id, x.size(0), cu_seqlens ? cu_seqlens->numel() - 1 : 0, length);
     std::vector<std::unique_ptr<Graph>> gone;                     // destroyed, which waits for the GPU, without the lock
@@ -1042,7 +1066,7 @@ class Encoder {
       w = w->second.use_count() == 1 ? lt_workspaces_.erase(w) : std::next(w);
   }
 
-  bool record(Graph& g, const AllDerived& all, const Tensor& x, const OptTensor& cu_seqlens, int64_t length, unsigned long long stream_id) {
+  bool record(Graph& g, const AllDerived& all, const Tensor& x, const OptTensor& cu_seqlens, int64_t length, const StreamId& stream_id) {
     g.dev = x.get_device();
     g.slot = acquire(g.dev);
     if (g.slot < 0) return false;
@@ -1117,7 +1141,7 @@ class Encoder {
   std::mutex graph_mu_;
   std::map<Key, std::unique_ptr<Graph>> graphs_;
   std::map<Key, Seen> seen_;                                      // the last SEEN of them
-  std::map<std::pair<int, unsigned long long>, Tensor> lt_workspaces_;       // by device and stream id
+  std::map<std::pair<int, StreamId>, Tensor> lt_workspaces_;
   uint64_t uses_ = 0;                                             // passes that looked for a recording
   int64_t recordings_ = 0;
   uint64_t derived_version_ = 0;

@@ -429,13 +429,10 @@ class FlashDebertaV2Encoder(DebertaV2Encoder):
             made = True
             w, b = attns[i]._qkv_weights()
             tables = attns[i]._relative_tables(rel_embeddings, dtype) if attns[i].relative_attention else None
-            hid = hidden_states.shape[-1]
-            if w.dtype != dtype or w.device != hidden_states.device or w.shape != (3 * hid, hid) or b.shape != (3 * hid,):
+            if not native.set_derived(i, hidden_states, w, b, None if tables is None else tables.native()):
                 return None
-            native.set_derived(i, w, b, None if tables is None else tables.native())
         if made and hidden_states.is_cuda and not torch.cuda.is_current_stream_capturing():
-            with torch.cuda.device(hidden_states.device):
-                native.set_ready()               # passes on other streams wait for this
+            native.set_ready(hidden_states)      # passes on other streams wait for this
         plan.stamp = stamp_now
         return plan
 
