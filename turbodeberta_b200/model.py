@@ -232,8 +232,8 @@ class FlashDisentangledSelfAttention(DisentangledSelfAttention):
                        "reference's kernel) and no backward pass: attention_probs_dropout_prob is ignored")
         q, k, v = self._project_qkv(hidden_states, query_states)
         if q.dtype == torch.float32 and B * L >= 4096:
-            _warn_once("fp32", "float32 inputs run on the exact CUDA-core attention kernel (one warp per query row), "
-                       "which is a correctness mode and far slower than the bf16 tensor-core kernel; "
+            _warn_once("fp32", "float32 inputs run on the exact CUDA-core attention kernel, some ten times slower than the bf16 "
+                       "tensor-core kernel; "
                        "convert the model with .bfloat16() for throughput")
         scale_factor = 1 + int("c2p" in self.pos_att_type) + int("p2c" in self.pos_att_type)
         sm_scale = 1.0 / math.sqrt(D * scale_factor)

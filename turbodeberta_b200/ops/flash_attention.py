@@ -14,8 +14,8 @@ with q, k, v of logical shape ``(B, H, L, D)`` and arbitrary strides (a permuted
 which the reference kernel does not have.  Forward only, like the reference (``ops/flash_attention.py:341-343``).
 
 The reference's own calling convention still works: when ``q_pos`` / ``k_pos`` have the shape ``(B, H, L, 2*span)``
-they are taken as the materialised scores and only gathered (a CUDA-core compatibility path, far slower than the
-fused one).  The gather follows the eager module (same index for both terms) unless ``p2c_mirrored=True``, which
+they are taken as the materialised scores and only gathered (``attn_scores.cu`` in bf16, the CUDA-core kernel in
+fp32; both are bound by reading them).  The gather follows the eager module (same index for both terms) unless ``p2c_mirrored=True``, which
 reproduces the reference kernel's mirrored position->content index (``ops/flash_attention.py:126-132``).
 """
 from __future__ import annotations

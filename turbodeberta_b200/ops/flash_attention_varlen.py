@@ -10,7 +10,7 @@ q, k, v are ``(T, H, D)`` with the sequences back to back; ``cu_seqlens`` is int
 fixed-length op, ``q_pos``/``k_pos`` are the projected tables ``(H, 2*span, D)`` rather than the per-token score
 tensors ``(T, H, 2*span)`` of the reference.  Relative positions restart at every sequence.  The tile list is
 built on the device from ``cu_seqlens``; nothing is read back except the status words at the end of the call.
-Score tensors of shape ``(T, H, 2*span)`` are still accepted and gathered by a CUDA-core compatibility kernel
+Score tensors of shape ``(T, H, 2*span)`` are still accepted and only gathered, as in the padded form
 (``p2c_mirrored=True`` reproduces the reference kernel's index, ``ops/flash_attention_varlen.py:144-152``).
 """
 from __future__ import annotations
