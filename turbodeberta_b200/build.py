@@ -12,7 +12,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libtdb_b200.so")
 HOST = os.path.join(HERE, "_host.so")
 HOST_SOURCES = ["host_ops.cpp"]
-SOURCES = ["tdb_api.cu", "tables.cu", "attn_simt.cu", "attn_scores.cu", "attn_small.cu", "attn_umma.cu", "attn_far.cu", "relpos_umma.cu", "encoder.cu", "skinny.cu"]
+SOURCES = ["tdb_api.cu", "tables.cu", "attn_simt.cu", "attn_scores.cu", "attn_small.cu", "attn_umma.cu", "attn_far.cu", "relpos_umma.cu", "encoder.cu", "skinny.cu", "encoder_short.cu"]
 HEADERS = ["tdb_internal.h", "ptx_sm100.cuh", "attn_common.cuh", "gelu.cuh", "attn_blocks.cuh", "attn_warp_mma.cuh", os.path.join("..", "..", "include", "tdb_b200.h")]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden"]

@@ -24,9 +24,11 @@
 // score and over all keys: 3.6e-7, 4.5e-7, 8.3e-7, at the same speed; one warp per query row: 1.9e-7, 2.0e-7, 2.3e-7; without
 // the sum per tile: 1.8e-7, 1.9e-7, 2.6e-7).
 #include "attn_blocks.cuh"
+#include "ptx_sm100.cuh"
 #include <math_constants.h>
 
 namespace tdb {
+using namespace ptx;
 
 namespace {
 
@@ -64,20 +66,7 @@ __device__ __forceinline__ void staged() {
   __syncthreads();
 }
 
-// Two fp32 multiply-adds per instruction, each rounded as fmaf rounds.  A pair holds the sums over even and odd columns.
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pair(float a, float b) {
-  f32x2 v;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
-  return v;
-}
-__device__ __forceinline__ float2 halves(f32x2 v) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
-}
-__device__ __forceinline__ void fma2(f32x2& acc, f32x2 a, f32x2 b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b)); }
-__device__ __forceinline__ void add2(f32x2& acc, f32x2 a) { asm("add.rn.f32x2 %0, %0, %1;" : "+l"(acc) : "l"(a)); }
+// A pair (f32x2) holds the sums over even and odd columns.
 struct Four { f32x2 lo, hi; };                       // four columns
 __device__ __forceinline__ Four load4(const float* p) {
   const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);

@@ -830,7 +830,8 @@ class Encoder {
     const c10::cuda::CUDAStream torch_stream = c10::cuda::getCurrentCUDAStream();
     const cudaStream_t stream = torch_stream.stream();
     if (!every) {
-      Tensor y = replay(all, x, cu_seqlens, length, torch_stream);
+      Tensor y = short_stack(all, x, cu_seqlens, length, torch_stream, words);
+      if (!y.defined()) y = replay(all, x, cu_seqlens, length, torch_stream);
       if (y.defined()) {
         outs.push_back(y);
         return r;
@@ -916,16 +917,55 @@ class Encoder {
     add_norm(out, s.y, l.ln2_w, l.ln2_b, l.eps2, code, stream);
   }
 
-  // Small passes are bound by the host: eight launches per layer of some 4 us each, for kernels of 2 to 8 us.  A shape that
+  // All layers in one kernel (see encoder_short.cu), or nothing where it does not apply.  It needs no recording: it is one launch.
+  Tensor short_stack(const AllDerived& all, const Tensor& x, const OptTensor& cu_seqlens, int64_t length, c10::cuda::CUDAStream stream,
+                     std::vector<Tensor>& words) {
+    const int64_t T = x.size(0), hidden = x.size(1);
+    if (!Linear::applies(x) || !tdb_short_stack_applies(T, hidden, layers_[0].up_w.size(0), (int64_t)layers_.size())) return {};
+    tdb::ShortStack p{};
+    for (size_t i = 0; i < layers_.size(); ++i) {
+      const Layer& l = layers_[i];
+      const Derived& d = all[i];
+      if (l.up_w.size(0) != 4 * hidden) return {};
+      for (const Tensor* t : {&d.qkv_w, &d.qkv_b, &l.out_w, &l.out_b, &l.up_w, &l.up_b, &l.down_w, &l.down_b})      // the norms': see fits()
+        if (misaligned(*t) || !t->is_contiguous()) return {};
+      tdb::AttnParams a{};
+      if (d.tables) d.tables->fill(a, x);
+      auto b = [](const Tensor& t) { return reinterpret_cast<const __nv_bfloat16*>(t.data_ptr()); };
+      p.layer[i] = {b(d.qkv_w), b(d.qkv_b), b(l.out_w), b(l.out_b), b(l.ln1_w), b(l.ln1_b), b(l.up_w), b(l.up_b), b(l.down_w), b(l.down_b),
+                    b(l.ln2_w), b(l.ln2_b), static_cast<const __nv_bfloat16*>(a.kr_exp), static_cast<const __nv_bfloat16*>(a.qr_exp),
+                    (float)l.eps1, (float)l.eps2, (float)l.sm_scale, a.exp_delta_max, a.exp_rows};
+    }
+    const Tensor y = at::empty_like(x), scratch = at::empty({10 * T * hidden}, x.options());
+    __nv_bfloat16* at = reinterpret_cast<__nv_bfloat16*>(scratch.data_ptr());
+    auto take = [&](int64_t columns) { return std::exchange(at, at + T * columns); };
+    p.qkv = take(3 * hidden); p.ctx = take(hidden); p.y = take(hidden); p.u = take(4 * hidden); p.z = take(hidden);
+    p.x = reinterpret_cast<const __nv_bfloat16*>(x.data_ptr());
+    p.out = reinterpret_cast<__nv_bfloat16*>(y.data_ptr());
+    p.n_layers = (int)layers_.size(); p.tokens = (int)T;
+    p.n_seqs = (int)(cu_seqlens ? cu_seqlens->numel() - 1 : T / length); p.length = (int)length;
+    p.cu_seqlens = cu_seqlens ? cu_seqlens->data_ptr<int32_t>() : nullptr;
+    tdb::AttnParams reports{};
+    Status st(x.get_device(), reports);
+    p.status = reports.status; p.counter = reports.counter; p.gave_up = reports.gave_up;
+    if (tdb_short_stack(&p, (int)hidden, stream.stream())) {      // not all of its blocks can be resident here
+      st.failed(stream.stream());
+      return {};
+    }
+    st.defer(stream, words);
+    return y;
+  }
+
+  // Small passes that the one kernel does not take are bound by the host: eight launches per layer of some 4 us each, for kernels of
+  // 2 to 8 us.  A shape that
   // comes a second time on a stream is recorded into a CUDA graph, which belongs to that stream (its buffers are in use until
   // the replay is over), as long as the weights stay where they are.  At most GRAPHS of them.  A shape then has to come COMEBACKS
   // times while the longest unused recording does not come once: only then does it take that one's place.  With any number of
   // shapes in turn the first GRAPHS stay recorded and the others stay eager.
-  // us per pass, eager and replayed, and what the pass that records costs beyond an eager one: base model, 32 tokens 515, 498,
-  // 430; 128 tokens 659, 562, 730; 2048 tokens 1027, 899, 700; large model, 128 tokens 1271, 1086, 1150; 2048 tokens 2337, 2081,
+  // us per pass, eager and replayed, and what the pass that records costs beyond an eager one: base model, 128 tokens 659, 562, 730; 2048 tokens 1027, 899, 700; large model, 128 tokens 1271, 1086, 1150; 2048 tokens 2337, 2081,
   // 1040.  So a recording has paid for itself after six to eight replays (COMEBACKS), 25 where the projections are kernels of our
-  // own.  Twelve shapes in turn, one sentence each: 502 us per pass; 40 shapes 574; all new ones 632 (when every shape that came
-  // back pushed the oldest out: 1070 and 1277).  Beyond GRAPH_MAX_ELEMENTS the gain falls (6 M elements 5 %, 9 to 12 M 1 to 2 %) and the
+  // own.  Twelve shapes in turn of some 30 tokens each, before the one kernel took those: 502 us per pass; 40 shapes 574; all new ones
+  // 632 (when every shape that came back pushed the oldest out: 1070 and 1277).  Beyond GRAPH_MAX_ELEMENTS the gain falls (6 M elements 5 %, 9 to 12 M 1 to 2 %) and the
   // buffers grow: a recording at the limit holds 52 MB, and each stream with one 32 MB of workspace.
   static constexpr int GRAPHS = 8, COMEBACKS = 8, SEEN = 64, BLOCK = 128;
   static constexpr int64_t GRAPH_MAX_ELEMENTS = 2048 * 1024;      // T * hidden, see above

@@ -247,5 +247,22 @@ __device__ __forceinline__ float ex2(float x) {
   return y;
 }
 
+
+// Two fp32 operations per instruction, each rounded as the single one is.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pair(float a, float b) {
+  f32x2 v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
+  return v;
+}
+__device__ __forceinline__ float2 halves(f32x2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ void fma2(f32x2& acc, f32x2 a, f32x2 b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b)); }
+__device__ __forceinline__ void add2(f32x2& acc, f32x2 a) { asm("add.rn.f32x2 %0, %0, %1;" : "+l"(acc) : "l"(a)); }
+__device__ __forceinline__ void mul2(f32x2& acc, f32x2 a) { asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(acc) : "l"(a)); }
+
 }  // namespace ptx
 }  // namespace tdb

@@ -101,9 +101,27 @@ int static_tile_scratch(void** ptr);   // device address of the library's fixed 
 
 }  // namespace tdb
 
+constexpr int SKINNY_TOKENS = 32;
+namespace tdb {
+// The encoder's layers as encoder_short.cu takes them, all of them bf16: weights [features, columns], tables as in AttnParams (null: absent).
+constexpr int SHORT_LAYERS = 48;
+struct ShortLayer {
+  const __nv_bfloat16 *qkv_w, *qkv_b, *out_w, *out_b, *ln1_w, *ln1_b, *up_w, *up_b, *down_w, *down_b, *ln2_w, *ln2_b, *kr, *qr;
+  float eps1, eps2, sm_scale;
+  int exp_delta_max, exp_rows;
+};
+struct ShortStack {
+  ShortLayer layer[SHORT_LAYERS];
+  int n_layers, tokens, n_seqs, length;               // length: of every sequence, where there are no offsets
+  const __nv_bfloat16* x;                             // [tokens, hidden], like out, ctx, y and z; qkv: three times, u: four times as wide
+  __nv_bfloat16 *out, *qkv, *ctx, *y, *u, *z;
+  const int32_t* cu_seqlens;
+  int32_t *status, *counter, *gave_up;                // as in AttnParams; counter[0] and counter[3] are zero on entry and again at the end
+};
+}  // namespace tdb
+
 // What the host extension calls (the checks and the launch behind the tdb_attn_fwd_* entry points on a filled AttnParams,
 // and kernels that have no C entry point of their own).
-constexpr int SKINNY_TOKENS = 32;
 #define TDB_HOST_API __attribute__((visibility("default")))
 extern "C" {
 TDB_HOST_API int tdb_run_attn(const tdb::AttnParams* p, int dtype, int kernel, void* stream);
@@ -120,6 +138,9 @@ TDB_HOST_API int tdb_gelu(void* x, int64_t elements, int dtype, void* stream);
 // then must not be what wrote W (W is read before the wait for it).
 TDB_HOST_API int tdb_skinny_applies(int64_t T, int64_t K, int64_t N);
 TDB_HOST_API int tdb_skinny(const void* x, const void* w, const void* b, int T, int K, int N, int gelu, int early, void* y, void* stream);
+// All layers for at most SKINNY_TOKENS tokens in one kernel whose blocks wait for one another.
+TDB_HOST_API int tdb_short_stack_applies(int64_t tokens, int64_t hidden, int64_t inner, int64_t layers);
+TDB_HOST_API int tdb_short_stack(const tdb::ShortStack* p, int hidden, void* stream);
 TDB_HOST_API int tdb_mask_rows(const void* mask, int elem_bytes, int B, int L, int32_t* seqlens, int32_t* cu, int32_t* ticket,
                                int32_t* out, void* stream);
 TDB_HOST_API int tdb_mask_positions(const void* mask, int elem_bytes, const int32_t* cu, int B, int L, int32_t* pos, void* stream);
