@@ -1,0 +1,53 @@
+"""The model's input in one kernel: gather, LayerNorm, padding mask."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("shape,hidden", [((1, 1), 8), ((3, 7), 264), ((2, 33), 768), ((40, 61), 1024)])
+@pytest.mark.parametrize("ids_type,mask_type", [(torch.long, torch.long), (torch.int32, torch.bool), (torch.long, torch.uint8)])
+def test_embeddings(shape, hidden, dtype, ids_type, mask_type):
+    """Against the four operations that it stands for, in float64.  Errors are relative to the two terms that are added, which may
+    cancel: bf16 rounds the sum once (2^-9 of it), fp32 carries some ten roundings (2^-24 each) of mean, variance and products."""
+    from turbodeberta_b200._cabi import host
+    torch.manual_seed(41)
+    table = torch.randn(97, hidden, device="cuda").to(dtype)
+    w, b = (torch.randn(hidden, device="cuda").to(dtype) for _ in range(2))
+    ids = torch.randint(0, 97, shape, device="cuda")
+    ids.view(-1)[:1] = 96
+    mask = torch.rand(shape, device="cuda") < 0.7
+    out, words = host.embed(ids.to(ids_type), table, w, b, 1e-7, mask.to(mask_type))
+    product = torch.nn.functional.layer_norm(table.double()[ids], (hidden,), w.double(), None, 1e-7)
+    want = (product + b.double()) * mask[..., None]
+    bound = 2.0 ** -8 if dtype == torch.bfloat16 else 1e-6
+    assert ((out.double() - want).abs() <= bound * (product.abs() + b.double().abs()) + 1e-7).all()
+    assert words is None and host.drain_pending() is None
+
+
+def test_embeddings_leave_other_tensors_to_torch():
+    from turbodeberta_b200._cabi import host
+    table, v = torch.randn(9, 16, device="cuda"), torch.ones(16, device="cuda")
+    ids, mask = torch.zeros(2, 4, dtype=torch.long, device="cuda"), torch.ones(2, 4, dtype=torch.long, device="cuda")
+    assert host.embed(ids, table, v, v, 1e-7, mask) is not None
+    wide = torch.randn(9, 32, device="cuda")
+    for bad in ((ids.t(), table, v, v, mask.t()), (ids, wide[:, :16], v, v, mask), (ids, wide.view(-1)[1:145].view(9, 16), v, v, mask), (ids, table, v, v.bfloat16(), mask),
+                (ids, table, v, v, mask.float()), (ids, table.half(), v.half(), v.half(), mask), (ids[:0], table, v, v, mask[:0])):
+        assert host.embed(*bad[:4], 1e-7, bad[4]) is None
+    host.drain_pending()
+
+
+def test_ids_outside_the_vocabulary_are_reported():
+    from tests.test_model_gpu import _cfg
+    from turbodeberta_b200.model import FlashDebertaV2Model
+    model = FlashDebertaV2Model(_cfg()).eval().to("cuda", torch.bfloat16)
+    ids = torch.randint(0, 500, (2, 20), device="cuda")
+    with torch.no_grad():
+        want = model(input_ids=ids).last_hidden_state
+        for bad in (500, -1, 1 << 40):
+            wrong = ids.clone()
+            wrong[1, 3] = bad
+            with pytest.raises(IndexError):
+                model(input_ids=wrong)
+        assert torch.equal(model(input_ids=ids).last_hidden_state, want)

@@ -1,4 +1,4 @@
-// The encoder's kernels between its matrix products and the attention: residual + LayerNorm, GELU, and the passage between
+// The encoder's kernels around its matrix products and the attention: the embeddings, residual + LayerNorm, GELU, and the passage between
 // padded batches and the packed token stream.  All of them are bound by memory traffic (or, for a handful of tokens, by the
 // launch): each reads its inputs once and writes its output once.
 #include "tdb_internal.h"
@@ -35,6 +35,9 @@ template <> struct Vec<__nv_bfloat16> {
     return make_uint4(w[0], w[1], w[2], w[3]);
   }
 };
+
+__device__ __forceinline__ float rounded(float x, float) { return x; }
+__device__ __forceinline__ float rounded(float x, __nv_bfloat16) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
 __device__ __forceinline__ float warp_sum(float x) {
 #pragma unroll
@@ -118,6 +121,76 @@ int launch_add_layernorm_t(const void* x, const void* res, const void* w, const 
   TDB_LN(1) TDB_LN(3) TDB_LN(4) TDB_LN(6) TDB_LN(8)
 #undef TDB_LN
   set_error("add_layernorm: hidden size %d is not supported", hidden);
+  return TDB_ERR_SHAPE;
+}
+
+// out = LayerNorm(table[ids]) * w + b, times the padding mask: a model's input, one warp per token.  Bound by the rows that come and go
+// (32 x 512 tokens of 1024 bf16: 33 MB each way, the padding's row from L2); as a gather, a LayerNorm, the mask's conversion and a
+// multiplication they took 96 us there, and for one short text some 60 us of launches.  The roundings are those of these four.
+template <typename T, int NV, typename I>
+__global__ void __launch_bounds__(128) embed_kernel(const I* __restrict__ ids, const T* __restrict__ table, int64_t vocabulary, const T* __restrict__ w,
+                                                    const T* __restrict__ b, float eps, const void* __restrict__ mask, int mask_bytes,
+                                                    int64_t rows, int hidden, T* __restrict__ out, int32_t* status) {
+  constexpr int N = Vec<T>::N;
+  const int64_t row = (int64_t)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
+  const int lane = threadIdx.x % 32, nv = hidden / N;
+  if (row >= rows) return;
+  int64_t id = ids[row];
+  if (id < 0 || id >= vocabulary) {
+    if (lane == 0 && *reinterpret_cast<volatile int32_t*>(status) == 0) *reinterpret_cast<volatile int32_t*>(status) = TDB_BAD_TOKEN;
+    id = 0;
+  }
+  const float keep = mask_bytes == 8 ? (float)static_cast<const int64_t*>(mask)[row] : (float)static_cast<const uint8_t*>(mask)[row];
+  const uint4* src = reinterpret_cast<const uint4*>(table + id * hidden);
+  float f[NV][N], sum = 0.f;
+#pragma unroll
+  for (int i = 0; i < NV; ++i)
+    if (lane + 32 * i < nv) {
+      Vec<T>::unpack(__ldg(src + lane + 32 * i), f[i]);
+#pragma unroll
+      for (int e = 0; e < N; ++e) sum += f[i][e];
+    }
+  const float mean = warp_sum(sum) / (float)hidden;
+  float sq = 0.f;
+#pragma unroll
+  for (int i = 0; i < NV; ++i)
+    if (lane + 32 * i < nv) {
+#pragma unroll
+      for (int e = 0; e < N; ++e) { const float d = f[i][e] - mean; sq = fmaf(d, d, sq); }
+    }
+  const float inv = rsqrtf(warp_sum(sq) / (float)hidden + eps);
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int c = lane + 32 * i;
+    if (c < nv) {
+      float g[N], a[N];
+      Vec<T>::unpack(__ldg(reinterpret_cast<const uint4*>(w) + c), g);
+      Vec<T>::unpack(__ldg(reinterpret_cast<const uint4*>(b) + c), a);
+#pragma unroll
+      for (int e = 0; e < N; ++e) f[i][e] = rounded(fmaf((f[i][e] - mean) * inv, g[e], a[e]), T()) * rounded(keep, T());
+      reinterpret_cast<uint4*>(out + row * hidden)[c] = Vec<T>::pack(f[i]);
+    }
+  }
+}
+
+template <typename T, typename I>
+int launch_embed_t(const void* ids, const void* table, int64_t vocabulary, const void* w, const void* b, float eps, const void* mask, int mask_bytes,
+                   int64_t rows, int hidden, void* out, int32_t* status, cudaStream_t s) {
+  constexpr int PER = 32 * Vec<T>::N;
+  const int nv = (hidden + PER - 1) / PER;
+  int sms = 0;
+  if (const int rc = device_sms(&sms)) return rc;
+  const int warps = rows >= 16 * sms ? 4 : 1;        // few rows: one per block, so that they spread over the SMs
+  const unsigned blocks = (unsigned)((rows + warps - 1) / warps);
+#define TDB_EMBED(NV)                                                                                                           \
+  if (nv <= NV) {                                                                                                               \
+    embed_kernel<T, NV, I><<<blocks, 32 * warps, 0, s>>>((const I*)ids, (const T*)table, vocabulary, (const T*)w, (const T*)b, eps, mask, mask_bytes, rows, \
+                                                         hidden, (T*)out, status);                                              \
+    return cuda_fail(cudaGetLastError(), "embed launch");                                                                       \
+  }
+  TDB_EMBED(1) TDB_EMBED(3) TDB_EMBED(4) TDB_EMBED(6) TDB_EMBED(8)
+#undef TDB_EMBED
+  set_error("embed: hidden size %d is not supported", hidden);
   return TDB_ERR_SHAPE;
 }
 
@@ -228,6 +301,14 @@ int tdb_add_layernorm(const void* x, const void* res, const void* w, const void*
   if (rows == 0) return TDB_OK;
   return dtype == TDB_DTYPE_F32 ? launch_add_layernorm_t<float>(x, res, w, b, eps, rows, hidden, out, early, (cudaStream_t)stream)
                                 : launch_add_layernorm_t<__nv_bfloat16>(x, res, w, b, eps, rows, hidden, out, early, (cudaStream_t)stream);
+}
+
+int tdb_embed(const void* ids, int id_bytes, const void* table, int64_t vocabulary, const void* w, const void* b, float eps, const void* mask,
+              int mask_bytes, int64_t rows, int hidden, int dtype, void* out, int32_t* status, void* stream) {
+  if (rows == 0) return TDB_OK;
+  auto run = id_bytes == 8 ? (dtype == TDB_DTYPE_F32 ? launch_embed_t<float, int64_t> : launch_embed_t<__nv_bfloat16, int64_t>)
+                           : (dtype == TDB_DTYPE_F32 ? launch_embed_t<float, int32_t> : launch_embed_t<__nv_bfloat16, int32_t>);
+  return run(ids, table, vocabulary, w, b, eps, mask, mask_bytes, rows, hidden, out, status, (cudaStream_t)stream);
 }
 
 int tdb_gelu(void* x, int64_t elements, int dtype, void* stream) {

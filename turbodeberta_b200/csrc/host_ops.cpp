@@ -1219,6 +1219,32 @@ py::object mask_rows(const Tensor& mask) {
   return py::make_tuple((bool)w[0], (bool)w[1], w[2], w[3], both.narrow(0, 0, B), both.narrow(0, B, B + 1));
 }
 
+// A model's input from ids [B, L]: LayerNorm of their embeddings, times the padding mask.  (output, words that somebody has to look at
+// or None), or None where the kernel does not take the tensors as they are.
+py::object embed(const Tensor& ids, const Tensor& table, const Tensor& w, const Tensor& b, double eps, const Tensor& mask) {
+  const at::ScalarType t = table.scalar_type();
+  const int64_t hidden = table.size(1);
+  const bool types = (t == at::kFloat || t == at::kBFloat16) && w.scalar_type() == t && b.scalar_type() == t &&
+                     (ids.scalar_type() == at::kLong || ids.scalar_type() == at::kInt) &&
+                     (mask.scalar_type() == at::kLong || mask.scalar_type() == at::kBool || mask.scalar_type() == at::kByte);
+  if (!types || hidden % 8 || hidden > (t == at::kFloat ? 1024 : 2048) || w.numel() != hidden || b.numel() != hidden || ids.numel() == 0 || mask.sizes() != ids.sizes())
+    return py::none();
+  for (const Tensor* x : {&ids, &table, &w, &b, &mask})
+    if (!x->is_cuda() || x->get_device() != ids.get_device() || !x->is_contiguous()) return py::none();
+  if (misaligned(table) | misaligned(w) | misaligned(b)) return py::none();
+  c10::cuda::CUDAGuard guard(ids.device());
+  at::AutoDispatchBelowAutograd below;
+  const c10::cuda::CUDAStream stream = c10::cuda::getCurrentCUDAStream();
+  Tensor out = at::empty({ids.size(0), ids.size(1), hidden}, table.options());
+  tdb::AttnParams reports{};
+  Status st(ids.get_device(), reports);
+  const int rc = tdb_embed(ids.data_ptr(), (int)ids.element_size(), table.data_ptr(), table.size(0), w.data_ptr(), b.data_ptr(), (float)eps,
+                           mask.data_ptr(), (int)mask.element_size(), ids.numel(), (int)hidden, dtype_code(table), out.data_ptr(), reports.status, stream);
+  if (rc) st.failed(stream);
+  TORCH_CHECK(rc == 0, "libtdb_b200: ", tdb_last_error());
+  return py::make_tuple(out, st.finish(false, stream));
+}
+
 // The valid rows of x [B, L, hidden] back to back, and each token's place in that stream (-1: padding).
 std::pair<Tensor, Tensor> pack_rows(const Tensor& x, const Tensor& mask, const Tensor& cu, int64_t tokens) {
   c10::cuda::CUDAGuard guard(x.device());
@@ -1297,6 +1323,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     c10::cuda::CUDAGuard guard(x.device());
     return tdb_gelu(x.data_ptr(), x.numel(), dtype_code(x), c10::cuda::getCurrentCUDAStream().stream());
   });
+  m.def("embed", &embed);
+  m.attr("BAD_TOKEN") = TDB_BAD_TOKEN;
   m.def("mask_rows", &mask_rows);
   m.def("pack_rows", &pack_rows);
   m.def("unpack_rows", &unpack_rows);

@@ -133,6 +133,11 @@ TDB_HOST_API int tdb_expand_pair(const void* kr, const void* qr, const int16_t* 
 // early: as for tdb_skinny, of w and b.
 TDB_HOST_API int tdb_add_layernorm(const void* x, const void* res, const void* w, const void* b, float eps, int64_t rows, int hidden,
                                    int dtype, void* out, int early, void* stream);
+// Embeddings of `rows` tokens (ids of 4 or 8 bytes, a mask of 1 or 8): see embed_kernel.  An id outside the vocabulary is reported
+// in status word 0 as TDB_BAD_TOKEN.
+constexpr int TDB_BAD_TOKEN = 401;
+TDB_HOST_API int tdb_embed(const void* ids, int id_bytes, const void* table, int64_t vocabulary, const void* w, const void* b, float eps, const void* mask,
+                           int mask_bytes, int64_t rows, int hidden, int dtype, void* out, int32_t* status, void* stream);
 TDB_HOST_API int tdb_gelu(void* x, int64_t elements, int dtype, void* stream);
 // bf16 projection of a few tokens, y = x W^T + b, through GELU if asked.  early: may start beside the kernel in front, which
 // then must not be what wrote W (W is read before the wait for it).

@@ -137,7 +137,7 @@ def _analyse_2d(attention_mask: torch.Tensor, batch: int, length: int) -> MaskIn
     if rows is None:
         return None
     all_ones, right, tokens, longest, seqlens, cu = rows
-    info = MaskInfo(all_ones, right, seqlens, attention_mask != 0 if all_ones else None, (tokens, longest, cu))
+    info = MaskInfo(all_ones, right, seqlens, None, (tokens, longest, cu))      # who needs the validity itself asks analyse_mask
     if all_ones and not attention_mask.is_inference():
         _mask_cache_put(attention_mask, info)
     return info
@@ -583,10 +583,18 @@ class FlashDebertaV2Model(DebertaV2Model):
             return None
         if attention_mask is None:
             attention_mask = torch.ones(input_ids.shape, dtype=torch.long, device=input_ids.device)
-        x = nn.functional.embedding(input_ids, emb.word_embeddings.weight)
-        norm = emb.LayerNorm
-        x = nn.functional.layer_norm(x, norm.normalized_shape, norm.weight, norm.bias, norm.eps)
-        x.mul_(attention_mask.to(x.dtype)[..., None])
+        table, norm = emb.word_embeddings.weight, emb.LayerNorm
+        embedded = None
+        if norm.weight is not None and norm.bias is not None and tuple(norm.normalized_shape) == table.shape[1:]:
+            embedded = host.embed(input_ids, table, norm.weight, norm.bias, norm.eps, attention_mask)
+        if embedded is not None:
+            x, words = embedded
+            if words is not None:
+                _PENDING_STATUS.append(words)
+        else:
+            x = nn.functional.embedding(input_ids, table)
+            x = nn.functional.layer_norm(x, norm.normalized_shape, norm.weight, norm.bias, norm.eps)
+            x.mul_(attention_mask.to(x.dtype)[..., None])
         return self.encoder(x, attention_mask, output_hidden_states=False, output_attentions=False, return_dict=True)
 
 

@@ -169,6 +169,8 @@ def _check_status(status: torch.Tensor):
 
 
 def _raise_for(st):
+    if st[0] == cabi.host.BAD_TOKEN:
+        raise IndexError("a token id lies outside the vocabulary")
     if st[0]:
         raise cabi.TdbError(cabi.ERR_TIMEOUT, f"a device-side wait gave up (barrier code {st[0]})")
     if st[1]:
