@@ -328,6 +328,25 @@ def test_far_tiles_take_over_from_near_tiles(lengths, geometry, heads):
     assert torch.equal(packed, o.permute(0, 2, 1, 3)[keep])
 
 
+@pytest.mark.parametrize("c2p,p2c", [(True, True), (True, False), (False, True)])
+def test_far_items_in_a_row(c2p, p2c):
+    """More items than SMs, so that an item's operands and the near kernel's state come in while the one before is at work: one far
+    tile and many, pairs without a second tile, rows of different lengths, against the exact kernel.  Both round the output (half a unit
+    each: 2^-8 of it), one rounds P (2^-9 of values up to 4, averaged over the keys)."""
+    from turbodeberta_b200.ops.flash_attention import flash_attention_with_disentangled
+    lengths = [1025, 1024, 512, 400, 897, 640, 0, 1]
+    w = _wl(lengths, 1025, hidden=64 * 24, heads=24, buckets=64, maxpos=128)
+    q, k, v, rel, P = util.device_inputs(w, DT)
+    tables = util.make_tables(w, rel, P, c2p, p2c)
+    lens = torch.tensor(lengths, dtype=torch.int32, device="cuda")
+    args = [t.permute(0, 2, 1, 3) for t in (q, k, v)] + [None, None, False, 0.0722, 64, 128]
+    o = flash_attention_with_disentangled(*args, seqlens=lens, tables=tables, kernel=UMMA)
+    o2 = flash_attention_with_disentangled(*args, seqlens=lens, tables=tables, kernel=SIMT)
+    assert ((o.float() - o2.float()).abs() <= 2.0 ** -7 * o2.float().abs() + 4e-3).all()
+    for _ in range(3):
+        assert torch.equal(flash_attention_with_disentangled(*args, seqlens=lens, tables=tables, kernel=UMMA), o)
+
+
 @pytest.mark.parametrize("level", [4.0, 16.0, 60.0])
 def test_far_scores_far_above_the_near_ones(level):
     """Far keys whose scores lie up to hundreds of powers of two above the near tiles': within what the near tiles'

@@ -11,13 +11,18 @@
 // tile each, two threads per row; while one group takes exponentials the tensor cores form the other's scores.
 //
 // The kernel for near key tiles (attn_umma.cu) has left each row's unnormalised output, reference exponent and sum in fp32;
-// a group starts from that exponent, adds the near output at the end and writes the finished rows.
+// a group starts from that exponent, adds the near output at the end and writes the finished rows.  That state comes in as bulk
+// copies while the item is at work (64 KB of outputs per pair of tiles, for which Q has one buffer and not two: the products run
+// ahead of the exponentials by more than Q's way from memory), and the constants are formed one side per thread: read and formed by
+// the groups at the item's ends, they took 6 of the 9.5 thousand clocks between two items.  Padded batches take the outer pairs
+// first, which have most far tiles.  us per call before and after: 4 x 4096 tokens 512 and 502 (this kernel 252 and 237), 1 x 4096
+// 212 and 170 (the order), 8 x 2048 350 and 337, 13 x 1200 286 and 270; 64 packed sequences of 2048 to 8192 the same, under the power cap.
 //
 // Bound: the special-function unit, 16384 exponentials per tile = 1024 clocks, beside 768 clocks of tensor work.  What matters
 // is that neither waits for the other: three score buffers go round the two groups, so a group's next scores are complete
 // before it has finished with the last ones, and only P.V follows its hand-off; and the two kinds of product are issued by two
 // warps, because issuing blocks while the tensor pipe is busy and a lone issuing warp then adds its waits and commits (some
-// 100 clocks each) to every batch.  A pair of tiles takes 2500 clocks (4 x 4096 tokens: 247 us for the kernel).  With one
+// 100 clocks each) to every batch.  A pair of tiles takes 2500 to 2800 clocks.  With one
 // buffer per group and one issuing lane it took 4300, with three buffers and one issuing warp 3300; in the one kernel for all
 // tiles, with one accumulator and all sixteen warps in step, 7400.  A quarter of the exponentials as polynomials on the FMA
 // pipe, and tokens that let one group at a time take exponentials, were slower (254 us and 266 us against 242 of the version before).
@@ -43,8 +48,10 @@ constexpr int GW = 8, GT = GW * 32;                  // warps, threads of a grou
 constexpr int F_THREADS = 2 * GT + 3 * 32;           // + a warp of single lanes (Q and K; V; scheduler), two MMA warps
 constexpr int F_RING = 3, STAGES = 2, BUFS = 3;
 constexpr uint32_t TILE = BQ * HD * 2;               // bytes of a 128 x 64 bf16 tile
-// Q buffer b: query tile A, query tile B, left row of Qr, right row of Qr
-constexpr uint32_t F_OFF_Q = 0, F_OFF_K = 2 * 4 * TILE, F_OFF_V = F_OFF_K + STAGES * TILE, F_OFF_BAR = F_OFF_V + STAGES * TILE;
+// of an item: query tiles A and B, left and right row of Qr; the near kernel's outputs of both tiles, its exponents and sums; both rows of Kr
+constexpr uint32_t NEAR = BQ * HD * 4;
+constexpr uint32_t F_OFF_Q = 0, F_OFF_K = 4 * TILE, F_OFF_V = F_OFF_K + STAGES * TILE, F_OFF_N = F_OFF_V + STAGES * TILE;
+constexpr uint32_t F_OFF_ML = F_OFF_N + 2 * NEAR, F_OFF_KR = F_OFF_ML + 2 * BQ * 8, F_OFF_BAR = F_OFF_KR + 2 * HD * 2;
 constexpr uint32_t F_OFF_WORK = F_OFF_BAR + 256, F_OFF_ITEM = F_OFF_WORK + F_RING * 64, F_OFF_X = F_OFF_ITEM + 8 * 64;
 constexpr uint32_t F_OFF_FLAG = F_OFF_X + 2 * 2 * BQ * 4;    // exchange: [group][half][row]
 constexpr uint32_t F_SMEM = F_OFF_FLAG + 64 + 1024;
@@ -52,7 +59,7 @@ static_assert(F_SMEM <= 227 * 1024, "shared memory budget");
 constexpr uint32_t F_TM_S = 0, F_TM_O = 384, F_TM_COLS = 512;
 constexpr uint64_t F_WAIT_NS = 1000ull * 1000ull * 1000ull;
 
-enum FBar { FQ_FULL = 0, FQ_EMPTY = 2, FK_FULL = 4, FK_EMPTY = 6, FV_FULL = 8, FV_EMPTY = 10, FS_FULL = 12 /* per buffer */,
+enum FBar { FQ_FULL = 0, FQ_EMPTY, FN_FULL, FN_EMPTY, FK_FULL = 4, FK_EMPTY = 6, FV_FULL = 8, FV_EMPTY = 10, FS_FULL = 12 /* per buffer */,
             FP_READY = 15 /* per group */, FPV_DONE = 17, FWORK_FULL = 19, FWORK_EMPTY = 22, FDONE = 25 /* two */, FBUF_FREE = 27, F_NBARS = 30 };
 constexpr int F_READERS = 4 + 1;                     // K lane, V lane, two MMA warps, the groups' leader
 
@@ -64,19 +71,23 @@ struct FarWork {
 };
 static_assert(sizeof(FarWork) == 64, "a ring slot");
 
+// Index space: packed form, the listed tiles (of which every second one of a sequence has nothing to do); padded form, pairs of
+// tiles, from the ends of the sequences inwards: the outer pairs have most far tiles, and the cheapest come last.
+__device__ __forceinline__ int far_rows(const AttnParams& p) {
+  return p.varlen ? reinterpret_cast<const int32_t*>(p.workspace)[0] : p.n_seqs * ((p.L + 2 * BQ - 1) / (2 * BQ));
+}
 // False: past the last index.  n_far == 0: nothing to do at this index.
-__device__ __forceinline__ bool far_work(const AttnParams& p, int total_tiles, int w, FarWork& k) {
+__device__ __forceinline__ bool far_work(const AttnParams& p, int total, int w, FarWork& k) {
   const int tile = w / p.H;
-  if (tile >= total_tiles) return false;
+  if (tile >= total) return false;
   k.h = w - tile * p.H;
   if (p.varlen) {
     const int2 e = reinterpret_cast<const int2*>(reinterpret_cast<const int32_t*>(p.workspace) + 4)[tile];
     const int c0 = p.cu_seqlens[e.x];
     k.len = p.cu_seqlens[e.x + 1] - c0; k.rows = k.len; k.tok0 = c0; k.bcoord = 0; k.q0 = e.y; k.seq = e.x;
   } else {
-    const int qtiles = (p.L + BQ - 1) / BQ;
-    const int seq = tile / qtiles;
-    k.q0 = (tile - seq * qtiles) * BQ;
+    const int pairs = (p.L + 2 * BQ - 1) / (2 * BQ), rank = tile / p.n_seqs, seq = tile - rank * p.n_seqs;
+    k.q0 = ((rank & 1) ? pairs - 1 - rank / 2 : rank / 2) * (2 * BQ);
     const int len = p.seqlens ? p.seqlens[seq] : p.L;
     k.len = len < 0 ? 0 : (len > p.L ? p.L : len);
     k.rows = p.L; k.tok0 = 0; k.bcoord = seq; k.seq = seq;
@@ -127,7 +138,7 @@ attn_far_kernel(const AttnParams p, int32_t* counter, const __grid_constant__ CU
   extern __shared__ uint8_t smem_raw[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   wait_for_stream();                                 // behind the near kernel, which lets nothing start early
-  const int total_tiles = p.varlen ? reinterpret_cast<const int32_t*>(p.workspace)[0] : p.n_seqs * ((p.L + BQ - 1) / BQ);
+  const int total = far_rows(p);
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gbase = smem_raw + (sbase - smem_u32(smem_raw));
   const uint32_t bars = sbase + F_OFF_BAR;
@@ -143,9 +154,8 @@ attn_far_kernel(const AttnParams p, int32_t* counter, const __grid_constant__ CU
     *abort_flag = 0;
     for (int i = 0; i < F_NBARS; ++i) {
       const bool by_warps = i >= FP_READY && i < FP_READY + 2, by_readers = i >= FWORK_EMPTY && i < FWORK_EMPTY + F_RING;
-      // a Q buffer is free when its products are done and both groups have taken their rows' constants from it
-      const bool q_empty = i >= FQ_EMPTY && i < FQ_EMPTY + 2;
-      mbar_init(bar(i), by_readers ? (uint32_t)F_READERS : by_warps ? (uint32_t)GW : q_empty ? 3u : 1u);
+      // Q is free when its products are done and both groups have taken their rows' constants; what the near kernel left, when both have read it
+      mbar_init(bar(i), by_readers ? (uint32_t)F_READERS : by_warps ? (uint32_t)GW : i == FQ_EMPTY ? 3u : i == FN_EMPTY ? 2u : 1u);
     }
     fence_mbar_init();
   }
@@ -169,24 +179,33 @@ attn_far_kernel(const AttnParams p, int32_t* counter, const __grid_constant__ CU
     return k.n_far > 0;
   };
   auto release = [&](int n) { mbar_arrive(bar(FWORK_EMPTY + (n % F_RING))); };
+  // where the near kernel has left the state of an item's tile
+  auto state_of = [&](const FarWork& k, int tile) { return partial_tile(p, k.tok0, k.seq, k.bcoord, k.q0 + BQ * tile) * p.H + k.h; };
 
   if (warp == 2 * GW) {
     // ================================ TMA producers and scheduler ============================
-    if (lane == 0) {                                 // per item both query tiles and both saturated rows, then K
+    if (lane == 0) {                                 // per item what its products and its rows' constants need, then K
       FarWork k;
       int g = 0, n = 0;
       for (; fetch(n, k); release(n), ++n) {
-        const int b = n & 1;
-        const uint32_t q = sbase + F_OFF_Q + (uint32_t)b * 4 * TILE;
-        if (n >= 2) wait(FQ_EMPTY + b, (uint32_t)(((n >> 1) - 1) & 1));
+        const uint32_t q = sbase + F_OFF_Q;
+        const bool both = k.q0 + BQ < k.len;         // the near kernel has left something of the second tile too
+        if (n >= 1) wait(FQ_EMPTY, (uint32_t)((n - 1) & 1));
         if (!*abort_flag) {
-          mbar_expect_tx(bar(FQ_FULL + b), (P2C ? 4 : 2) * TILE);
-          tma_load_4d(q, &tm_q, bar(FQ_FULL + b), 0, (int)k.tok0 + k.q0, k.h, k.bcoord);
-          tma_load_4d(q + TILE, &tm_q, bar(FQ_FULL + b), 0, (int)k.tok0 + k.q0 + BQ, k.h, k.bcoord);
+          mbar_expect_tx(bar(FQ_FULL), (P2C ? 4 : 2) * TILE + (C2P ? 2 * HD * 2 : 0) + (both ? 2 : 1) * BQ * 8);
+          tma_load_4d(q, &tm_q, bar(FQ_FULL), 0, (int)k.tok0 + k.q0, k.h, k.bcoord);
           if (P2C) {
-            tma_load_3d(q + 2 * TILE, &tm_qr, bar(FQ_FULL + b), 0, p.exp_rows - BQ, k.h);     // distances far above zero
-            tma_load_3d(q + 3 * TILE, &tm_qr, bar(FQ_FULL + b), 0, 0, k.h);                    // far below
+            tma_load_3d(q + 2 * TILE, &tm_qr, bar(FQ_FULL), 0, p.exp_rows - BQ, k.h);     // distances far above zero
+            tma_load_3d(q + 3 * TILE, &tm_qr, bar(FQ_FULL), 0, 0, k.h);                    // far below
           }
+          tma_load_4d(q + TILE, &tm_q, bar(FQ_FULL), 0, (int)k.tok0 + k.q0 + BQ, k.h, k.bcoord);
+          if (C2P) {
+            const __nv_bfloat16* kr = reinterpret_cast<const __nv_bfloat16*>(p.kr_exp) + (int64_t)k.h * p.exp_rows * HD;
+            bulk_load(sbase + F_OFF_KR, kr + (int64_t)(p.exp_rows - 1) * HD, HD * 2, bar(FQ_FULL));
+            bulk_load(sbase + F_OFF_KR + HD * 2, kr, HD * 2, bar(FQ_FULL));
+          }
+          for (int i = 0; i < (both ? 2 : 1); ++i)
+            bulk_load(sbase + F_OFF_ML + (uint32_t)i * BQ * 8, p.part_ml + state_of(k, i) * (2 * BQ), BQ * 8, bar(FQ_FULL));
         }
         for (int it = 0; it < k.n_far; ++it, ++g) {
           const int st = g % STAGES;
@@ -209,12 +228,20 @@ attn_far_kernel(const AttnParams p, int32_t* counter, const __grid_constant__ CU
             mbar_expect_tx(bar(FV_FULL + st), TILE);
             tma_load_4d(sbase + F_OFF_V + st * TILE, &tm_v, bar(FV_FULL + st), 0, (int)k.tok0 + far_tile(k, it) * BK, k.h, k.bcoord);
           }
+          if (it != (k.n_far > 1 ? 1 : 0)) continue;
+          // the near kernel's outputs: needed at the item's end, the buffer is free since the end of the one before
+          if (n >= 1) wait(FN_EMPTY, (uint32_t)((n - 1) & 1));
+          if (*abort_flag) continue;
+          const bool both = k.q0 + BQ < k.len;
+          mbar_expect_tx(bar(FN_FULL), (both ? 2 : 1) * NEAR);
+          for (int i = 0; i < (both ? 2 : 1); ++i)
+            bulk_load(sbase + F_OFF_N + (uint32_t)i * NEAR, p.part_o + state_of(k, i) * (BQ * HD), NEAR, bar(FN_FULL));
         }
       release(n);
     } else if (lane == 2) {
       // Scheduler.  Every CTA with an index of its own draws until its first draw past the end: as many draws as indices, and
       // the counter wraps back to zero (see attn_umma.cu).
-      const unsigned int last_item = (unsigned int)(total_tiles * p.H - 1);
+      const unsigned int last_item = (unsigned int)(total * p.H - 1);
       int n = 0;
       bool first = true;
       while (true) {
@@ -223,7 +250,7 @@ attn_far_kernel(const AttnParams p, int32_t* counter, const __grid_constant__ CU
                               : (int)gridDim.x + (int)atomicInc(reinterpret_cast<unsigned int*>(counter), last_item);
         first = false;
         FarWork k;
-        if (!far_work(p, total_tiles, w, k)) k.n_far = -1;
+        if (!far_work(p, total, w, k)) k.n_far = -1;
         if (k.n_far == 0) continue;
         if (n >= F_RING) wait(FWORK_EMPTY + (n % F_RING), (uint32_t)(((n / F_RING) - 1) & 1));
         ring[n % F_RING] = k;
@@ -254,13 +281,13 @@ attn_far_kernel(const AttnParams p, int32_t* counter, const __grid_constant__ CU
       for (int t = 0; c.n_far > 0; ++t) {
         const int grp = t & 1, g = t >> 1, buf = t % BUFS;
         if (grp == 0) {
-          if (c.it == 0) wait(FQ_FULL + (c.n & 1), (uint32_t)((c.n >> 1) & 1));
+          if (c.it == 0) wait(FQ_FULL, (uint32_t)(c.n & 1));
           wait(FK_FULL + (g % STAGES), (uint32_t)((g / STAGES) & 1));
         }
         if (t >= BUFS) wait(FBUF_FREE + buf, (uint32_t)((t / BUFS - 1) & 1));
         tc_fence_after();
         const uint32_t tS = tm + F_TM_S + 128u * (uint32_t)buf;
-        const uint64_t q = dQ + (uint64_t)((c.n & 1) * 4) * STEP, kd = dK + (uint64_t)(g % STAGES) * STEP;
+        const uint64_t q = dQ, kd = dK + (uint64_t)(g % STAGES) * STEP;
 #pragma unroll
         for (int i = 0; i < HD / 16; ++i) mma_ss_warp(tS, q + (uint64_t)grp * STEP + 2 * i, kd + 2 * i, ID_S, i > 0);
         if (P2C) {
@@ -272,7 +299,7 @@ attn_far_kernel(const AttnParams p, int32_t* counter, const __grid_constant__ CU
         if (grp == 1) {
           tc_commit_warp(bar(FK_EMPTY + (g % STAGES)));
           if (++c.it == c.n_far) {
-            tc_commit_warp(bar(FQ_EMPTY + (c.n & 1)));
+            tc_commit_warp(bar(FQ_EMPTY));
             if (lane == 0) release(c.n);
             ++c.n; c.it = 0;
             load_item(c);
@@ -342,31 +369,30 @@ attn_far_kernel(const AttnParams p, int32_t* counter, const __grid_constant__ CU
       const int row = item->q0 + BQ * grp + row_t;
       if (n_far <= 0) break;
       const int64_t tok = item->tok0 + row;                          // of the packed stream, or of its batch row
-      const int64_t part = partial_tile(p, item->tok0, item->seq, item->bcoord, item->q0 + BQ * grp) * p.H + h;
       const bool valid = row < len;
+      wait(FQ_FULL, (uint32_t)(n & 1));
       float2 near = make_float2(0.f, 0.f);                           // the near tiles' exponent and sum
-      if (valid) near = __ldg(reinterpret_cast<const float2*>(p.part_ml) + part * BQ + row_t);
+      if (valid) near = make_float2(lds_f32(sbase + F_OFF_ML + 8u * (uint32_t)(grp * BQ + row_t)), lds_f32(sbase + F_OFF_ML + 8u * (uint32_t)(grp * BQ + row_t) + 4u));
       float c_left = 0.f, c_right = 0.f;
-      wait(FQ_FULL + (n & 1), (uint32_t)((n >> 1) & 1));
-      if (C2P) {                                                     // Q[i].Kr[r] of both sides
-        const uint4* kl = reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(p.kr_exp) +
-                                                         ((int64_t)h * p.exp_rows + p.exp_rows - 1) * HD);
-        const uint4* kr = reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(p.kr_exp) + (int64_t)h * p.exp_rows * HD);
-        const uint32_t qrow = sbase + F_OFF_Q + (uint32_t)((n & 1) * 4 + grp) * TILE + 128u * (uint32_t)row_t;
+      if (C2P) {                                                     // Q[i].Kr[r], a side by each of the row's two threads
+        float c0 = 0.f, c1 = 0.f;
+        if (half == 0 ? n_left > 0 : n_far > n_left) {
+          const uint32_t qrow = sbase + F_OFF_Q + (uint32_t)grp * TILE + 128u * (uint32_t)row_t, kr = sbase + F_OFF_KR + (uint32_t)half * (HD * 2);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const uint4 a = lds_128(qrow + 16u * (uint32_t)(i ^ (row_t & 7))), b = __ldg(kl + i), c = __ldg(kr + i);
-          const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w}, cw[4] = {c.x, c.y, c.z, c.w};
+          for (int i = 0; i < 8; ++i) {
+            const uint4 a = lds_128(qrow + 16u * (uint32_t)(i ^ (row_t & 7))), b = lds_128(kr + 16u * (uint32_t)i);
+            const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float a0 = __uint_as_float(aw[e] << 16), a1 = __uint_as_float(aw[e] & 0xffff0000u);
-            c_left = fmaf(a0, __uint_as_float(bw[e] << 16), c_left);
-            c_left = fmaf(a1, __uint_as_float(bw[e] & 0xffff0000u), c_left);
-            c_right = fmaf(a0, __uint_as_float(cw[e] << 16), c_right);
-            c_right = fmaf(a1, __uint_as_float(cw[e] & 0xffff0000u), c_right);
+            for (int e = 0; e < 4; ++e) {
+              c0 = fmaf(__uint_as_float(aw[e] << 16), __uint_as_float(bw[e] << 16), c0);
+              c1 = fmaf(__uint_as_float(aw[e] & 0xffff0000u), __uint_as_float(bw[e] & 0xffff0000u), c1);
+            }
           }
         }
-        c_left *= sl2; c_right *= sl2;
+        sts_f32(x_row + (uint32_t)half * (BQ * 4), (c0 + c1) * sl2);
+        group_sync(grp);                                             // written again behind the first tile's vote at the earliest
+        c_left = lds_f32(x_row);
+        c_right = lds_f32(x_row + BQ * 4);
       }
       float m = near.x, l = 0.f;
       for (int it = 0; it < n_far; ++it, ++g) {
@@ -456,7 +482,7 @@ attn_far_kernel(const AttnParams p, int32_t* counter, const __grid_constant__ CU
           }
         }
         l += sum;
-        if (it == 0 && gt == 0) mbar_arrive(bar(FQ_EMPTY + (n & 1)));      // behind the vote: the group has read its rows of Q
+        if (it == 0 && gt == 0) mbar_arrive(bar(FQ_EMPTY));                // behind the vote: the group has read its rows of Q
         // Keys beyond the sequence have exact zeros as probabilities, but their rows of V may hold anything (0 x NaN): group A
         // zeroes them in shared memory before it announces P, and the other group's product is issued after its own.
         if (grp == 0 && nv_tile < BK) {
@@ -471,15 +497,16 @@ attn_far_kernel(const AttnParams p, int32_t* counter, const __grid_constant__ CU
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(FP_READY + grp));
       }
-      // (far output + near output) / sum -> global; the near output is on its way while the last product runs
-      float nr[32];
-#pragma unroll
-      for (int i = 0; i < 32; ++i) nr[i] = valid ? __ldg(p.part_o + part * (BQ * HD) + (32 * half + i) * BQ + row_t) : 0.f;
+      // (far output + near output) / sum -> global
       group_sync(grp);                               // the last tile may have exchanged maxima in the same words
       sts_f32(x_row + (uint32_t)half * (BQ * 4), l);
       group_sync(grp);
       const float beta = ex2(near.x - m);
       const float l_tot = fmaf(near.y, beta, lds_f32(x_row) + lds_f32(x_row + BQ * 4));
+      wait(FN_FULL, (uint32_t)(n & 1));
+      float nr[32];
+#pragma unroll
+      for (int i = 0; i < 32; ++i) nr[i] = valid ? lds_f32(sbase + F_OFF_N + (uint32_t)grp * NEAR + 4u * (uint32_t)((32 * half + i) * BQ + row_t)) : 0.f;
       wait(FPV_DONE + grp, (uint32_t)((g - 1) & 1));
       tc_fence_after();
       uint32_t r[32];
@@ -505,7 +532,8 @@ attn_far_kernel(const AttnParams p, int32_t* counter, const __grid_constant__ CU
           p.lse[(int64_t)item->bcoord * p.lse_sb + (int64_t)h * p.lse_sh + tok] = valid ? m * 0.6931471805599453f + logf(l_tot) : 0.f;
       }
       if (gt == 0) mine[(n + 1) & 1] = items[(n + 1) & 3];
-      group_sync(grp);                               // the exchange words are free again
+      group_sync(grp);                               // the exchange words are free again, and the near outputs have been read
+      if (gt == 0) mbar_arrive(bar(FN_EMPTY));
     }
   }
 
@@ -532,7 +560,8 @@ int launch_far_variant(const AttnParams& p, dim3 grid, const CUtensorMap* maps, 
 
 }  // namespace
 
-// `tiles`: query tiles of the whole problem (an upper bound in the packed form, whose list says how many there are).
+// `tiles`: query tiles of the whole problem (an upper bound in the packed form, whose list says how many there are); at least as many as
+// the kernel's indices.
 int launch_attn_far(const AttnParams& p, int64_t tiles, int sms, cudaStream_t s) {
   CUtensorMap maps[4];
   const int64_t tokens = p.varlen ? p.total_tokens : p.L;

@@ -81,11 +81,6 @@ __device__ __forceinline__ void warp_sums(float* x) {          // of two values
     x[0] += a; x[1] += b;
   }
 }
-__device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
-}
-
 // Out of line, like the LayerNorm: the kernel's code runs once per layer, so what is not in it need not be fetched again.
 __device__ __noinline__ void wait_longer(uint32_t bar, uint32_t phase, volatile int* abort_flag, int32_t* status) {
   mbar_wait(bar, phase, abort_flag, status, 301, MEET_NS);
@@ -323,7 +318,7 @@ __global__ void __launch_bounds__(MT * KS * 32, 1) short_stack_kernel(const __gr
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     if (lane == 0) mbar_expect_tx(bar, (uint32_t)rows * bytes);
     __syncwarp();
-    if (lane < rows) bulk_copy(dst + (uint32_t)lane * pitch, mine, bytes, bar);
+    if (lane < rows) bulk_load(dst + (uint32_t)lane * pitch, mine, bytes, bar);
   };
   auto bring_qkv = [&](const ShortLayer& l) {
     bring(sA, P::PITCH, barA, 24, 2 * H, l.qkv_w + ((int64_t)(lane >> 3) * H + 8 * block + (lane & 7)) * H);
