@@ -387,6 +387,51 @@ def test_short_padded_batches(lengths, L, c2p, p2c):
         assert n == 0 or (lse[b, :, :n] - lse2[b, :, :n]).abs().max().item() < 1e-3
 
 
+@pytest.mark.parametrize("lengths,L", [([65], 65), ([128, 64, 1, 0], 128), ([127, 97, 96, 33], 127), ([80, 65, 16], 112)])
+@pytest.mark.parametrize("c2p,p2c", [(True, True), (True, False), (False, True), (False, False)])
+def test_padded_batches_of_two_tiles(lengths, L, c2p, p2c):
+    """65 to 128 tokens as long as every block of 64 query rows has an SM: lengths around its tiles and its warps' 32 keys, empty rows, NaN
+    in the padding, against the exact kernel and the next size up; tables that belong to the call, by index and expanded."""
+    from turbodeberta_b200.ops.flash_attention import flash_attention_with_disentangled
+    w = _wl(lengths, L, hidden=192, heads=3)
+    q, k, v, rel, P = util.device_inputs(w, DT)
+    tables = util.make_tables(w, rel, P, c2p, p2c) if (c2p or p2c) else None
+    lens = torch.tensor(lengths, dtype=torch.int32, device="cuda")
+    for b, n in enumerate(lengths):
+        k[b, n:] = float("nan")
+        v[b, n:] = float("nan")
+    args = [t.permute(0, 2, 1, 3) for t in (q, k, v)] + [None, None, False, 0.0722, 256, 512]
+    o, lse = flash_attention_with_disentangled(*args, seqlens=lens, tables=tables, return_lse=True)
+    o2, lse2 = flash_attention_with_disentangled(*args, seqlens=lens, tables=tables, kernel=SIMT, return_lse=True)
+    many = [t.repeat(20, 1, 1, 1) for t in args[:3]]
+    o3 = flash_attention_with_disentangled(*many, *args[3:], seqlens=lens.repeat(20), tables=tables)[:len(lengths)]
+    for other in (o2, o3):
+        assert ((o.float() - other.float()).abs() <= 2.0 ** -7 * other.float().abs() + 4e-3).all()
+    for b, n in enumerate(lengths):
+        assert torch.count_nonzero(o[b, :, n:]).item() == 0 and torch.count_nonzero(lse[b, :, n:]).item() == 0
+        assert n == 0 or (lse[b, :, :n] - lse2[b, :, :n]).abs().max().item() < 1e-3
+    if tables is not None:
+        args[3:5] = tables.kr, tables.qr
+        assert torch.equal(flash_attention_with_disentangled(*args, seqlens=lens), o)
+        assert torch.equal(flash_attention_with_disentangled(*many, *args[3:], seqlens=lens.repeat(20))[:len(lengths)], o3)
+
+
+@pytest.mark.parametrize("L", [1, 33, 64])
+@pytest.mark.parametrize("buckets,maxpos", [(256, 512), (8, 16), (0, 32)])
+def test_tables_of_one_call_are_read_by_index(L, buckets, maxpos):
+    """The same rows as from expanded tables, so the same bits: also where most distances of a tile are saturated."""
+    from turbodeberta_b200.ops.flash_attention import flash_attention_with_disentangled
+    w = _wl([L, max(1, L // 2)], L, hidden=128, heads=2, buckets=buckets, maxpos=maxpos)
+    q, k, v, rel, P = util.device_inputs(w, DT)
+    t = util.make_tables(w, rel, P)
+    qkv = [x.permute(0, 2, 1, 3) for x in (q, k, v)]
+    for kr, qr in ((t.kr, t.qr), (t.kr, None), (None, t.qr)):
+        kept = util.make_tables(w, rel, P, kr is not None, qr is not None)
+        want = flash_attention_with_disentangled(*qkv, None, None, False, 0.0722, buckets, maxpos, tables=kept)
+        got = flash_attention_with_disentangled(*qkv, kr, qr, False, 0.0722, buckets, maxpos)
+        assert torch.equal(got, want)
+
+
 @pytest.mark.parametrize("lengths,heads", [([40, 64, 9], 4), ([512, 200, 64], 4), ([2048, 1300], 2)])
 @pytest.mark.parametrize("c2p,p2c", [(True, True), (True, False), (False, True)])
 def test_error_against_float64_is_that_of_the_roundings(lengths, heads, c2p, p2c):

@@ -9,16 +9,15 @@ constexpr int ST = 64, SP = 72, S_THREADS = 128;     // tile rows, row pitch in 
 
 __device__ __forceinline__ uint32_t saddr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-// 64 rows of 64 bf16; rows at or beyond `rows` become zeros (the caller's padding may hold anything).
+// 64 rows of 64 bf16, by THREADS threads; rows at or beyond `rows` become zeros (the caller's padding may hold anything).
+template <int THREADS = S_THREADS>
 __device__ __forceinline__ void stage(__nv_bfloat16* dst, const __nv_bfloat16* src, int64_t pitch, int rows) {
-  const int c = threadIdx.x & 7, row = threadIdx.x >> 3;
-  constexpr int STEP = S_THREADS / 8;
-  const __nv_bfloat16* from = src + row * pitch + c * 8;
-  const uint32_t to = saddr(dst + row * SP + c * 8);
 #pragma unroll
-  for (int i = 0; i < ST / STEP; ++i, from += STEP * pitch) {
-    const bool real = row + i * STEP < rows;
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to + 2u * i * STEP * SP), "l"(real ? from : src), "r"(real ? 16 : 0) : "memory");
+  for (int i = 0; i < ST * 8 / THREADS; ++i) {
+    const int e = threadIdx.x + i * THREADS, row = e >> 3, c = e & 7;
+    const bool real = row < rows;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(saddr(dst + row * SP + c * 8)),
+                 "l"(src + (real ? (int64_t)row * pitch + c * 8 : 0)), "r"(real ? 16 : 0) : "memory");
   }
 }
 __device__ __forceinline__ void ldsm4(uint32_t* r, const __nv_bfloat16* p) {

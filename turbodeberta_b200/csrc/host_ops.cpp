@@ -283,19 +283,13 @@ void* ptr(const OptTensor& t) { return t.has_value() && t->defined() ? t->data_p
 struct Tables {
   OptTensor kr, qr, idx, kr_exp, qr_exp;
   int two_span, idx_delta_max, exp_delta_max, exp_rows;
-  Tensor both;                                       // of a call's own tables: the expanded ones, c2p's in front
+  bool one_call = false;                             // made for one call, whose kernel decides whether they have to be expanded
   void fill(tdb::AttnParams& p, const Tensor& q) const {
     for (const OptTensor* t : {&kr, &qr})
       if (t->has_value() && (*t)->scalar_type() != q.scalar_type()) throw py::value_error("relative tables must have the dtype of q");
     p.kr = ptr(kr); p.qr = ptr(qr); p.two_span = two_span;
     p.idx = static_cast<const int16_t*>(ptr(idx)); p.idx_delta_max = idx_delta_max;
-    if (both.defined()) {
-      char* e = static_cast<char*>(both.data_ptr());
-      p.kr_exp = kr ? e : nullptr;
-      p.qr_exp = qr ? e + (kr ? both.nbytes() / 2 : 0) : nullptr;
-    } else {
-      p.kr_exp = ptr(kr_exp); p.qr_exp = ptr(qr_exp);
-    }
+    p.kr_exp = ptr(kr_exp); p.qr_exp = ptr(qr_exp);
     p.exp_delta_max = exp_delta_max; p.exp_rows = exp_rows;
     p.flags = (p.kr ? TDB_FLAG_C2P : 0) | (p.qr ? TDB_FLAG_P2C : 0);
   }
@@ -351,6 +345,32 @@ Result launch(tdb::AttnParams& p, int dtype, int kernel, int dev, Tensor o, cons
   return {o, lse_out, st.finish(check, stream)};
 }
 
+// Distance-expanded copies of both tables (bf16, head_dim 64) with one allocation and one launch: [1 or 2, H, rows, 64].
+Tensor expand_both(const OptTensor& kr, const OptTensor& qr, const Tensor& idx, int64_t exp_delta_max) {
+  const Tensor& some = kr ? *kr : *qr;
+  const int64_t H = some.size(0), two_span = some.size(1), exp_rows = (2 * exp_delta_max + 1 + 7) / 8 * 8;
+  c10::cuda::CUDAGuard guard(some.device());
+  const int n = (kr ? 1 : 0) + (qr ? 1 : 0);
+  Tensor both = at::empty({n, H, exp_rows, 64}, some.options());
+  char* e = static_cast<char*>(both.data_ptr());
+  const int rc = tdb_expand_pair(ptr(kr), ptr(qr), idx.data_ptr<int16_t>(), (int)((idx.numel() - 1) / 2), (int)H, (int)two_span,
+                                 (int)exp_delta_max, (int)exp_rows, kr ? e : nullptr, qr ? e + (kr ? both.nbytes() / 2 : 0) : nullptr,
+                                 c10::cuda::getCurrentCUDAStream().stream());
+  if (rc) throw std::runtime_error(std::string("libtdb_b200: ") + tdb_last_error());
+  return both;
+}
+// Tables of one call are expanded only for a kernel that reads them so.  Returns the expanded ones, for p to point into.
+Tensor expand_for(tdb::AttnParams& p, const Tables* tables, int dtype, int kernel) {
+  if (!tables || !tables->one_call || dtype != TDB_DTYPE_BF16) return {};
+  p.direct_tables = tdb_takes_direct_tables(&p, dtype, kernel);
+  if (p.direct_tables) return {};
+  const Tensor both = expand_both(tables->kr, tables->qr, *tables->idx, tables->exp_delta_max);
+  char* e = static_cast<char*>(both.data_ptr());
+  p.kr_exp = tables->kr ? e : nullptr;
+  p.qr_exp = tables->qr ? e + (tables->kr ? both.nbytes() / 2 : 0) : nullptr;
+  return both;
+}
+
 Result attn_fixed(const Tensor& q, const Tensor& k, const Tensor& v, const Tables* tables, const OptTensor& seqlens,
                   double sm_scale, int kernel, bool return_lse, bool check) {
   const int dev = device_of({&q, &k, &v, seqlens ? &*seqlens : nullptr});
@@ -371,6 +391,7 @@ Result attn_fixed(const Tensor& q, const Tensor& k, const Tensor& v, const Table
   p.n_seqs = int_size(B); p.L = int_size(L); p.total_tokens = B * L; p.H = int_size(H); p.D = int_size(q.size(3));
   p.sm_scale = (float)sm_scale;
   if (return_lse) { p.lse = lse.data_ptr<float>(); p.lse_sb = H * L; p.lse_sh = L; }
+  const Tensor expanded = expand_for(p, tables, code, kernel);
   return launch(p, code, kernel, dev, o, lse, check);
 }
 
@@ -402,6 +423,7 @@ Result attn_packed(const Tensor& q, const Tensor& k, const Tensor& v, const Tabl
   p.workspace_bytes = tdb_attn_workspace_bytes(p.n_seqs, T);
   const Tensor ws = at::empty({(int64_t)std::max<size_t>(p.workspace_bytes, 16)}, q.options().dtype(at::kByte));
   p.workspace = ws.data_ptr();
+  const Tensor expanded = expand_for(p, tables, code, kernel);
   return launch(p, code, kernel, dev, o, lse, check);
 }
 
@@ -473,20 +495,6 @@ Result attn_packed_scores(const Tensor& q, const Tensor& k, const Tensor& v, con
   return launch(p, code, TDB_KERNEL_SIMT, dev, o, lse, check);
 }
 
-// Distance-expanded copies of both tables (bf16, head_dim 64) with one allocation and one launch: [1 or 2, H, rows, 64].
-Tensor expand_both(const OptTensor& kr, const OptTensor& qr, const Tensor& idx, int64_t exp_delta_max) {
-  const Tensor& some = kr ? *kr : *qr;
-  const int64_t H = some.size(0), two_span = some.size(1), exp_rows = (2 * exp_delta_max + 1 + 7) / 8 * 8;
-  c10::cuda::CUDAGuard guard(some.device());
-  const int n = (kr ? 1 : 0) + (qr ? 1 : 0);
-  Tensor both = at::empty({n, H, exp_rows, 64}, some.options());
-  char* e = static_cast<char*>(both.data_ptr());
-  const int rc = tdb_expand_pair(ptr(kr), ptr(qr), idx.data_ptr<int16_t>(), (int)((idx.numel() - 1) / 2), (int)H, (int)two_span,
-                                 (int)exp_delta_max, (int)exp_rows, kr ? e : nullptr, qr ? e + (kr ? both.nbytes() / 2 : 0) : nullptr,
-                                 c10::cuda::getCurrentCUDAStream().stream());
-  if (rc) throw std::runtime_error(std::string("libtdb_b200: ") + tdb_last_error());
-  return both;
-}
 std::pair<OptTensor, OptTensor> expand_pair(const OptTensor& kr, const OptTensor& qr, const Tensor& idx, int64_t exp_delta_max) {
   const OptTensor k = kr ? OptTensor(kr->contiguous()) : std::nullopt, r = qr ? OptTensor(qr->contiguous()) : std::nullopt;
   const Tensor both = expand_both(k, r, idx, exp_delta_max);
@@ -1268,7 +1276,7 @@ Tensor unpack_rows(const Tensor& x, const Tensor& pos, int64_t B, int64_t L) {
   return out;
 }
 
-// The tables of one call from its projected tables (rows of 64): in the call's dtype, and expanded for bf16.
+// The tables of one call from its projected tables (rows of 64), in the call's dtype.
 Tables* call_tables(const OptTensor& kr, const OptTensor& qr, const Tensor& q, const Tensor& idx, int64_t exp_delta_max) {
   auto fit = [&](const OptTensor& t) -> OptTensor {
     if (!t) return std::nullopt;
@@ -1277,10 +1285,8 @@ Tables* call_tables(const OptTensor& kr, const OptTensor& qr, const Tensor& q, c
     return t->to(q.scalar_type()).contiguous();
   };
   const OptTensor k = fit(kr), r = fit(qr);
-  Tensor both;
-  if (q.scalar_type() == at::kBFloat16) both = expand_both(k, r, idx, exp_delta_max);
   return new Tables{k, r, idx, {}, {}, (int)(k ? *k : *r).size(1), (int)((idx.numel() - 1) / 2), (int)exp_delta_max,
-                    (int)((2 * exp_delta_max + 1 + 7) / 8 * 8), both};
+                    (int)((2 * exp_delta_max + 1 + 7) / 8 * 8), true};
 }
 
 }  // namespace
@@ -1289,7 +1295,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   py::class_<Tables>(m, "Tables")
       .def(py::init([](OptTensor kr, OptTensor qr, OptTensor idx, OptTensor kr_exp, OptTensor qr_exp, int two_span, int idx_delta_max,
                        int exp_delta_max, int exp_rows) {
-        return new Tables{kr, qr, idx, kr_exp, qr_exp, two_span, idx_delta_max, exp_delta_max, exp_rows, {}};
+        return new Tables{kr, qr, idx, kr_exp, qr_exp, two_span, idx_delta_max, exp_delta_max, exp_rows, false};
       }));
   m.def("attn_fixed", &attn_fixed);
   m.def("attn_packed", &attn_packed);

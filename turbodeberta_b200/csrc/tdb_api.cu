@@ -132,6 +132,7 @@ static int run_attn(const AttnParams& p, int dtype, int kernel, cudaStream_t str
     return TDB_ERR_ARG;
   }
   if (pick_kernel(dtype, kernel) == TDB_KERNEL_SIMT) return launch_attn_simt(p, dtype, stream);
+  if (p.direct_tables && dtype == TDB_DTYPE_BF16 && small_applicable(p)) return launch_attn_small(p, stream);
   if ((rc = check_umma(p, dtype))) return rc;
   if (p.varlen && (!p.workspace || p.workspace_bytes < umma_workspace_bytes(p.n_seqs, p.total_tokens))) {
     set_error("workspace of %zu bytes is smaller than the %zu required", p.workspace_bytes, umma_workspace_bytes(p.n_seqs, p.total_tokens));
@@ -346,6 +347,13 @@ int64_t tdb_partial_floats(const tdb::AttnParams* p, int dtype, int kernel) {
   if (pick_kernel(dtype, kernel) != TDB_KERNEL_UMMA || dtype != TDB_DTYPE_BF16 || p->D != 64 || !has_far_tiles(*p)) return 0;
   const int64_t tiles = p->varlen ? p->total_tokens / 128 + p->n_seqs + 1 : (int64_t)p->n_seqs * ((p->L + 127) / 128);
   return tiles * p->H * 128 * (64 + 2);
+}
+
+int tdb_takes_direct_tables(const tdb::AttnParams* p, int dtype, int kernel) {
+  tdb::AttnParams direct = *p;
+  direct.direct_tables = 1;
+  return pick_kernel(dtype, kernel) == TDB_KERNEL_UMMA && dtype == TDB_DTYPE_BF16 && p->D == 64 && small_applicable(direct) &&
+         aligned16(p->kr) && aligned16(p->qr);
 }
 
 int tdb_expand_pair(const void* kr, const void* qr, const int16_t* idx, int idx_delta_max, int H, int two_span,

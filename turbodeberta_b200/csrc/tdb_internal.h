@@ -45,6 +45,7 @@ struct AttnParams {
   // far tiles, tdb_partial_floats() of fp32, part_ml behind part_o's tiles (null: one kernel does both).  split_sat is the launcher's own.
   float* part_o; float* part_ml; int split_sat;
   int lengths_known;                                      // packed form: L is known to be the longest sequence's length
+  int direct_tables;                                      // kr and qr are read by index; kr_exp and qr_exp do not exist (kernel for short sequences only)
   int tiles_listed;                                       // packed form: the workspace already holds this batch's tile list
 };
 
@@ -90,7 +91,7 @@ int launch_relpos_expand(const void* table, const int16_t* idx, int idx_delta_ma
 int launch_bounded_wait_selftest(int32_t* status, int code, uint64_t limit_ns, cudaStream_t s);
 int launch_attn_simt(const AttnParams& p, int dtype, cudaStream_t s);
 int launch_attn_scores(const AttnParams& p, cudaStream_t s);          // bf16, materialised position scores
-bool small_applicable(const AttnParams& p);                            // sequences of at most 64 tokens: padded, or packed with a known longest
+bool small_applicable(const AttnParams& p);                            // short sequences: padded, or packed with a known longest
 int launch_attn_small(const AttnParams& p, cudaStream_t s);
 int launch_attn_umma(const AttnParams& p, cudaStream_t s);
 bool has_far_tiles(const AttnParams& p);
@@ -128,6 +129,8 @@ TDB_HOST_API int tdb_run_attn(const tdb::AttnParams* p, int dtype, int kernel, v
 // Floats of part_o and part_ml together that the call could use (0: none), for p as it will be passed to tdb_run_attn; part_ml
 // starts at 64 / 66 of them.
 TDB_HOST_API int64_t tdb_partial_floats(const tdb::AttnParams* p, int dtype, int kernel);
+// Whether the call runs on the kernel that can do without expanded tables (AttnParams::direct_tables).
+TDB_HOST_API int tdb_takes_direct_tables(const tdb::AttnParams* p, int dtype, int kernel);
 TDB_HOST_API int tdb_expand_pair(const void* kr, const void* qr, const int16_t* idx, int idx_delta_max, int H, int two_span,
                                  int exp_delta_max, int exp_rows, void* kr_out, void* qr_out, void* stream);
 // early: as for tdb_skinny, of w and b.
