@@ -32,7 +32,7 @@ using namespace ptx;
 
 namespace {
 
-constexpr int KT = 64, HALF = 32, HP = HALF + 4, DP = 64 + 4, THREADS = 64, PV = 16;
+constexpr int KT = 64, HALF = 32, HP = HALF + 4, DP = 64 + 4, THREADS = 64 /* of a group */, PV = 16;
 
 __device__ __forceinline__ void cp_async16(float* dst, const void* src, bool real) {
   const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
@@ -41,9 +41,9 @@ __device__ __forceinline__ void cp_async16(float* dst, const void* src, bool rea
 
 // COLS columns of ROWS rows to shared memory as fp32; src(row) is the row's first element, or null for a row of zeros.
 template <typename T, int COLS, int PITCH, typename F>
-__device__ __forceinline__ void stage_rows(float* dst, int rows, const T* any, F src) {
+__device__ __forceinline__ void stage_rows(float* dst, int rows, const T* any, F src, int tid, int threads = THREADS) {
   constexpr int PER = 16 / sizeof(T), CH = COLS / PER;
-  for (int e = threadIdx.x; e < rows * CH; e += THREADS) {
+  for (int e = tid; e < rows * CH; e += threads) {
     const int row = e / CH, c = e % CH;
     const T* s = src(row);
     float* d = dst + row * PITCH + c * PER;
@@ -61,9 +61,14 @@ __device__ __forceinline__ void stage_rows(float* dst, int rows, const T* any, F
     }
   }
 }
-__device__ __forceinline__ void staged() {
+// The threads of one group (a whole block where there is only one).
+template <int GROUPS> __device__ __forceinline__ void group_sync(int group) {
+  if (GROUPS == 1) __syncthreads();
+  else asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(THREADS) : "memory");
+}
+template <int GROUPS> __device__ __forceinline__ void staged(int group) {
   asm volatile("cp.async.wait_all;" ::: "memory");
-  __syncthreads();
+  group_sync<GROUPS>(group);
 }
 
 // A pair (f32x2) holds the sums over even and odd columns.
@@ -82,27 +87,29 @@ __device__ __forceinline__ void store4(__nv_bfloat16* d, float a, float b, float
   *reinterpret_cast<uint2*>(d) = v;
 }
 
-template <int R> constexpr int smem_floats(bool tables) {
-  const int half = (KT + (tables ? 2 * (8 * R + KT) : 0)) * HP;
-  const int values = KT * DP;
-  return 2 * 8 * R * DP + (half > values ? half : values);
-}
+// Of a group: P, and the operand rows of half a head, over which V comes.
+template <int R, bool TABLES> constexpr int operand_floats = (KT + (TABLES ? 2 * (8 * R + KT) : 0)) * HP;
+template <int R, bool TABLES> constexpr int group_floats = 8 * R * DP + (operand_floats<R, TABLES> > KT * DP ? operand_floats<R, TABLES> : KT * DP);
+template <int R, bool TABLES, int GROUPS> constexpr int smem_floats = 8 * R * DP + GROUPS * group_floats<R, TABLES>;
 
 // TABLES: position terms from the projected tables (either may be absent); otherwise none, or in f32 gathered scores.
-template <typename T, int R, bool TABLES>
-__global__ void __launch_bounds__(THREADS, 4) attn_simt_kernel(const AttnParams p) {
+// GROUPS: pairs of warps that share the query rows and take every GROUPS-th key tile each; the first adds the others' states up.
+template <typename T, int R, bool TABLES, int GROUPS>
+__global__ void __launch_bounds__(THREADS * GROUPS, 4 / GROUPS) attn_simt_kernel(const AttnParams p) {
   constexpr bool GATHER = !TABLES && sizeof(T) == 4;
   constexpr int QT = 8 * R, XR = QT + KT;           // XR: table rows a tile can touch (QT + KT - 1, padded)
   extern __shared__ __align__(16) float smem[];
   float* const sQ = smem;                            // [QT][DP]
-  float* const sP = sQ + QT * DP;                    // [QT][DP]
+  const int group = GROUPS == 1 ? 0 : (int)threadIdx.x / THREADS, tid = (int)threadIdx.x - group * THREADS;
+  float* const sP = sQ + QT * DP + group * group_floats<R, TABLES>;        // [QT][DP]
   float* const sK = sP + QT * DP;                    // [KT][HP], half a head
   float* const sKr = sK + KT * HP;                   // [XR][HP]
   float* const sQr = sKr + XR * HP;                  // [XR][HP]
   float* const sV = sK;                              // [KT][DP], over the three above
-  __shared__ int sRow[XR];                           // first element of the table row of distance q0 - k0 - 63 + x
+  __shared__ int rows_of[GROUPS][XR];                // first element of the table row of distance q0 - k0 - 63 + x
+  int* const sRow = rows_of[group];
 
-  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int warp = tid / 32, lane = tid % 32;
   const int ti = warp * 4 + lane / 8, tj = lane % 8;
   const int s = longest_first(p, blockIdx.z), h = blockIdx.y, q0 = blockIdx.x * QT;
   int len, rows;
@@ -135,14 +142,15 @@ __global__ void __launch_bounds__(THREADS, 4) attn_simt_kernel(const AttnParams 
   }
 
   if (q0 < len) {
-    stage_rows<T, 64, DP>(sQ, QT, qb, [&](int row) { return q0 + row < len ? qb + (int64_t)(q0 + row) * p.q_st : nullptr; });
+    stage_rows<T, 64, DP>(sQ, QT, qb, [&](int row) { return q0 + row < len ? qb + (int64_t)(q0 + row) * p.q_st : nullptr; }, threadIdx.x, THREADS * GROUPS);
     auto table_rows = [&](int k0) {
       if (TABLES)
-        for (int x = threadIdx.x; x < XR; x += THREADS) sRow[x] = p.idx[clamped(q0 - k0 - (KT - 1) + x)] * 64;
+        for (int x = tid; x < XR; x += THREADS) sRow[x] = p.idx[clamped(q0 - k0 - (KT - 1) + x)] * 64;
     };
-    table_rows(0);
+    table_rows(group * KT);
+    if (GROUPS > 1) asm volatile("cp.async.wait_all;" ::: "memory");        // Q is everybody's
     __syncthreads();
-    for (int k0 = 0; k0 < len; k0 += KT) {
+    for (int k0 = group * KT; k0 < len; k0 += GROUPS * KT) {
       float acc[R][8];
 #pragma unroll
       for (int r = 0; r < R; ++r)
@@ -156,13 +164,13 @@ __global__ void __launch_bounds__(THREADS, 4) attn_simt_kernel(const AttnParams 
         for (int r = 0; r < R; ++r)
 #pragma unroll
           for (int c = 0; c < 8; ++c) acc2[r][c] = 0ull;
-        stage_rows<T, HALF, HP>(sK, KT, kb, [&](int row) { return k0 + row < len ? kb + (int64_t)(k0 + row) * p.k_st + d0 : nullptr; });
+        stage_rows<T, HALF, HP>(sK, KT, kb, [&](int row) { return k0 + row < len ? kb + (int64_t)(k0 + row) * p.k_st + d0 : nullptr; }, tid);
         if (TABLES) {
           auto table_row = [&](const T* t, int x) { return t + sRow[x] + d0; };
-          if (krh) stage_rows<T, HALF, HP>(sKr, XR, krh, [&](int x) { return table_row(krh, x); });
-          if (qrh) stage_rows<T, HALF, HP>(sQr, XR, qrh, [&](int x) { return table_row(qrh, x); });
+          if (krh) stage_rows<T, HALF, HP>(sKr, XR, krh, [&](int x) { return table_row(krh, x); }, tid);
+          if (qrh) stage_rows<T, HALF, HP>(sQr, XR, qrh, [&](int x) { return table_row(qrh, x); }, tid);
         }
-        staged();
+        staged<GROUPS>(group);
         const float* const kp = sK + tj * HP;
         const float* const qp = sQ + ti * DP + d0;
         const int x0 = ti - tj + (KT - 1) - 56;      // table row of (r, s) is x0 + 8 (r - s + 7)
@@ -203,10 +211,10 @@ __global__ void __launch_bounds__(THREADS, 4) attn_simt_kernel(const AttnParams 
         for (int r = 0; r < R; ++r)
 #pragma unroll
           for (int c = 0; c < 8; ++c) { const float2 v = halves(acc2[r][c]); acc[r][c] += v.x + v.y; }
-        __syncthreads();
+        group_sync<GROUPS>(group);
       }
-      table_rows(k0 + KT);                           // for the next tile; V replaces the operand rows while the softmax runs
-      stage_rows<T, 64, DP>(sV, KT, vb, [&](int row) { return k0 + row < len ? vb + (int64_t)(k0 + row) * p.v_st : nullptr; });
+      table_rows(k0 + GROUPS * KT);                  // for the next tile; V replaces the operand rows while the softmax runs
+      stage_rows<T, 64, DP>(sV, KT, vb, [&](int row) { return k0 + row < len ? vb + (int64_t)(k0 + row) * p.v_st : nullptr; }, tid);
       float corr[R];
 #pragma unroll
       for (int r = 0; r < R; ++r) {
@@ -239,7 +247,7 @@ __global__ void __launch_bounds__(THREADS, 4) attn_simt_kernel(const AttnParams 
         }
         l[r] = l[r] * corr[r] + sum;
       }
-      staged();                                      // also makes the warp's own rows of P visible to its lanes
+      staged<GROUPS>(group);                         // also makes the warp's own rows of P visible to its lanes
       f32x2 tile[R][4];
 #pragma unroll
       for (int r = 0; r < R; ++r)
@@ -281,7 +289,38 @@ __global__ void __launch_bounds__(THREADS, 4) attn_simt_kernel(const AttnParams 
           fma2(sum, o[r][c], pair(corr[r], corr[r]));
           o[r][c] = sum;
         }
-      __syncthreads();                               // the next tile's operand rows go where V is
+      group_sync<GROUPS>(group);                     // the next tile's operand rows go where V is
+    }
+  }
+  if constexpr (GROUPS > 1) {
+    // A group's state of a thread's rows: maximum, sum and eight outputs, to where its P was; a group without a key tile has none.
+    constexpr int STATE = R * 10;
+    static_assert(STATE * THREADS <= group_floats<R, TABLES>, "the state fits");
+    if (group > 0) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        float* const d = sP + r * 10 * THREADS + tid;
+        d[0] = m[r]; d[THREADS] = l[r];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) { const float2 v = halves(o[r][c]); d[(2 + 2 * c) * THREADS] = v.x; d[(3 + 2 * c) * THREADS] = v.y; }
+      }
+    }
+    __syncthreads();
+    if (group > 0) return;
+    for (int g = 1; g < GROUPS && g * KT < len; ++g) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const float* const d = sP + g * group_floats<R, TABLES> + r * 10 * THREADS + tid;
+        const float mn = fmaxf(m[r], d[0]), mine = expf(m[r] - mn), theirs = expf(d[0] - mn);
+        m[r] = mn;
+        l[r] = l[r] * mine + d[THREADS] * theirs;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          f32x2 sum = pair(d[(2 + 2 * c) * THREADS] * theirs, d[(3 + 2 * c) * THREADS] * theirs);
+          fma2(sum, o[r][c], pair(mine, mine));
+          o[r][c] = sum;
+        }
+      }
     }
   }
 #pragma unroll
@@ -306,28 +345,37 @@ __global__ void __launch_bounds__(THREADS, 4) attn_simt_kernel(const AttnParams 
   }
 }
 
-template <typename T, int R, bool TABLES>
+template <typename T, int R, bool TABLES, int GROUPS = 1>
 int launch_variant(const AttnParams& p, cudaStream_t s) {
-  constexpr int SMEM = smem_floats<R>(TABLES) * 4;
-  auto kern = attn_simt_kernel<T, R, TABLES>;
-  if (SMEM > 48 * 1024) {
+  constexpr int SMEM = smem_floats<R, TABLES, GROUPS> * 4;
+  auto kern = attn_simt_kernel<T, R, TABLES, GROUPS>;
+  if (SMEM > 47 * 1024) {
     int rc = opt_in_smem(reinterpret_cast<const void*>(kern), SMEM);
     if (rc) return rc;
   }
   dim3 grid((p.L + 8 * R - 1) / (8 * R), p.H, p.n_seqs);
-  kern<<<grid, THREADS, SMEM, s>>>(p);
+  kern<<<grid, THREADS * GROUPS, SMEM, s>>>(p);
   return cuda_fail(cudaGetLastError(), "attn_simt launch");
+}
+
+template <typename T, bool TABLES>
+int launch_rows(const AttnParams& p, cudaStream_t s) {
+  // 32 query rows per block re-use each staged row twice as often as 16; 16 rows where 32 would leave SMs without a block.  With at most
+  // two such blocks per SM there is room for a second pair of warps each, which halves the block's chain of key tiles (12 heads, us
+  // per call, one pair and two: 1 x 100 36.2 and 27.4, 2 x 128 38.6 and 33.6, 1 x 200 54.5 and 43.2, 1 x 300 64.9 and 55.1, 2 x 200, which
+  // is 2.1 per SM, 65.6 and 63.0); with more, or one tile, it takes others' place (4 x 128 41.7 and 45.2, 2 x 300 84.8 and 94.3).  Four
+  // pairs gain nothing more below four tiles (1 x 300 64.3, 1 x 512 105.9 against 108.9).
+  int sms = 0, rc;
+  if ((rc = device_sms(&sms))) return rc;
+  const int64_t rows = (int64_t)p.H * p.n_seqs;
+  if ((p.L + 31) / 32 * rows >= 2 * (int64_t)sms) return launch_variant<T, 4, TABLES>(p, s);
+  if (p.L > KT && (p.L + 15) / 16 * rows <= 2 * (int64_t)sms) return launch_variant<T, 2, TABLES, 2>(p, s);
+  return launch_variant<T, 2, TABLES>(p, s);
 }
 
 template <typename T>
 int launch_dtype(const AttnParams& p, cudaStream_t s) {
-  const bool tables = p.flags && !p.c2p_scores && !p.p2c_scores;
-  // 32 query rows per block re-use each staged row twice as often as 16; 16 rows where 32 would leave SMs without a block.
-  int sms = 0, rc;
-  if ((rc = device_sms(&sms))) return rc;
-  const bool small = (int64_t)((p.L + 31) / 32) * p.H * p.n_seqs < 2 * (int64_t)sms;
-  if (tables) return small ? launch_variant<T, 2, true>(p, s) : launch_variant<T, 4, true>(p, s);
-  return small ? launch_variant<T, 2, false>(p, s) : launch_variant<T, 4, false>(p, s);
+  return p.flags && !p.c2p_scores && !p.p2c_scores ? launch_rows<T, true>(p, s) : launch_rows<T, false>(p, s);
 }
 
 }  // namespace
