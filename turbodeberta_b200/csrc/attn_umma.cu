@@ -909,6 +909,7 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap tm_q, c
         // are redone only for rows whose new maximum is more than 2^8 above (or, on the first tile, 2^64 below) it.
         const float m_prev = (it > 0) ? m_run : 0.f;
         float lsum = 0.f;
+        f32x2 sums = 0ull;                   // of even and odd keys (the products in pairs as well: 2 % slower)
         uint32_t pk[KPT / 2];
         // P of this tile goes to tensor memory while it is being formed, eight keys at a time, so the P.V product of
         // the tile before must have finished with the buffer (it has, long ago: it was issued when that tile ended).
@@ -938,7 +939,7 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap tm_q, c
             }
             s[e] = x0; s[e + 1] = x1;
             const float a = ex2(fmaf(x0, sl2, -m_prev)), b = ex2(fmaf(x1, sl2, -m_prev));
-            lsum += a + b;
+            add2(sums, pair(a, b));
             pk[e / 2] = pack_bf16x2(a, b);
             if ((e / 2) % 4 == 3) tmem_st4(tP + (uint32_t)(e / 2 - 3), pk[e / 2 - 3], pk[e / 2 - 2], pk[e / 2 - 1], pk[e / 2]);
             if (fuse && e / 2 == FCB) drain_begin(dc_src);
@@ -956,12 +957,16 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap tm_q, c
             x1 = (e + 1 < nvalid) ? x1 : -CUDART_INF_F;
             s[e] = x0; s[e + 1] = x1;
             const float a = ex2(fmaf(x0, sl2, -m_prev)), b = ex2(fmaf(x1, sl2, -m_prev));
-            lsum += a + b;
+            add2(sums, pair(a, b));
             pk[e / 2] = pack_bf16x2(a, b);
             if ((e / 2) % 4 == 3) tmem_st4(tP + (uint32_t)(e / 2 - 3), pk[e / 2 - 3], pk[e / 2 - 2], pk[e / 2 - 1], pk[e / 2]);
             if (fuse && e / 2 == FCB) drain_begin(dc_src);
             if (fuse && e / 2 > FCB && e / 2 <= FCB + STG_COLS / GROUPS / 8) drain_step(e / 2 - FCB - 1, dc_src, dc_dst);
           }
+        }
+        if (!sat) {
+          const float2 both = halves(sums);
+          lsum = both.x + both.y;
         }
         // Tiles around a saturated one drain the next c2p band here, in one piece (the band product was issued when
         // this tile's p2c band left the buffer, at the top of the tile, and needs about this long).
