@@ -137,8 +137,6 @@ attn_far_kernel(const AttnParams p, int32_t* counter, const __grid_constant__ CU
                 const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_qr) {
   extern __shared__ uint8_t smem_raw[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  wait_for_stream();                                 // behind the near kernel, which lets nothing start early
-  const int total = far_rows(p);
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gbase = smem_raw + (sbase - smem_u32(smem_raw));
   const uint32_t bars = sbase + F_OFF_BAR;
@@ -147,9 +145,6 @@ attn_far_kernel(const AttnParams p, int32_t* counter, const __grid_constant__ CU
   FarWork* ring = reinterpret_cast<FarWork*>(gbase + F_OFF_WORK);
   auto bar = [&](int i) { return bars + 8u * (uint32_t)i; };
   auto wait = [&](int i, uint32_t parity) { return mbar_wait(bar(i), parity, abort_flag, p.status, 201 + i, F_WAIT_NS); };
-  int32_t gave_up_before = 0;
-  if (warp == 2 * GW && lane == 2) gave_up_before = *reinterpret_cast<volatile int32_t*>(p.gave_up);
-
   if (tid == 0) {
     *abort_flag = 0;
     for (int i = 0; i < F_NBARS; ++i) {
@@ -171,6 +166,10 @@ attn_far_kernel(const AttnParams p, int32_t* counter, const __grid_constant__ CU
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  wait_for_stream();                                 // for the near kernel; all of the above ran beside its end
+  const int total = far_rows(p);
+  int32_t gave_up_before = 0;
+  if (warp == 2 * GW && lane == 2) gave_up_before = *reinterpret_cast<volatile int32_t*>(p.gave_up);
 
   auto fetch = [&](int n, FarWork& k) {
     wait(FWORK_FULL + (n % F_RING), (uint32_t)((n / F_RING) & 1));
@@ -554,8 +553,7 @@ int launch_far_variant(const AttnParams& p, dim3 grid, const CUtensorMap* maps, 
   auto kern = attn_far_kernel<C2P, P2C>;
   const int rc = opt_in_smem(reinterpret_cast<const void*>(kern), (int)F_SMEM);
   if (rc) return rc;
-  kern<<<grid, F_THREADS, F_SMEM, s>>>(p, p.counter + 2, maps[0], maps[1], maps[2], maps[3]);
-  return cuda_fail(cudaGetLastError(), "attn_far launch");
+  return cuda_fail(launch_early(kern, grid, F_THREADS, F_SMEM, s, p, p.counter + 2, maps[0], maps[1], maps[2], maps[3]), "attn_far launch");
 }
 
 }  // namespace

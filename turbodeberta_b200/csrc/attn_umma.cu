@@ -115,6 +115,7 @@ __global__ void __launch_bounds__(1024) build_tile_list_kernel(const int32_t* __
   static_assert(LIST_BUCKETS == 1024, "one bucket per thread");
   __shared__ int warp_total[32];
   __shared__ int hist[LIST_BUCKETS];       // tiles per bucket, then the write cursor of the bucket
+  let_next_start();                        // the attention kernel sets itself up meanwhile, and waits for the list
   int2* entries = reinterpret_cast<int2*>(ws + 4);
   for (int i = threadIdx.x; i < LIST_BUCKETS; i += blockDim.x) hist[i] = 0;
   __syncthreads();
@@ -365,6 +366,7 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap tm_q, c
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   wait_for_stream();                       // all of the above ran beside the end of the kernel in front
+  if (SPLIT) let_next_start();             // the far kernel's CTAs, as SMs become free; they wait for the state that all of this leaves
 
   // Item n of this CTA's stream; n_kv < 0 marks the end of the stream.  (Tiles that consist of padded query rows
   // only never enter the ring: the scheduler warp zeroes them itself.)
