@@ -9,13 +9,13 @@
 // gathered (attn_scores.cu does so in bf16); with TDB_FLAG_P2C_MIRRORED the p2c term is read at idx[clamp(k-q)], the reference kernel's convention.
 //
 // Bound by the FMA pipes and, close behind, by shared-memory reads (256 fp32 multiply-adds per score with both terms).
-// A block of two warps owns 8R query rows and walks the keys in tiles of 64.  A thread owns R x 8 scores at rows ti + 8r and
+// A block owns 8R query rows and walks the keys in tiles of 64.  A thread owns R x 8 scores at rows ti + 8r and
 // keys tj + 8s, so that the distance of each of them is (ti - tj) + 8 (r - s): R + 7 table rows per term serve all 8R
 // scores, every product that is formed is a score's own (a band of q.Kr products over all distances of a tile would be
 // twice as many), and nothing has to be skewed or gathered afterwards.  Operand rows are staged fp32, 36-word pitch, half a
-// head (32 columns) at a time: eight consecutive rows fall on different banks, and four blocks fit on an SM, which cover
+// head (32 columns) at a time: eight consecutive rows fall on different banks, and four pairs of warps fit on an SM, which cover
 // each other's loads.  The rows of one query tile stay inside one warp, so the softmax needs shuffles only.
-// One call of 8 x (48..387) fp32 tokens with 12 heads and both terms: 207 us, 26 TFLOP/s (one warp per query row, keys spread
+// One call of 8 x (48..387) fp32 tokens with 12 heads and both terms: 195 us, 28 TFLOP/s (one warp per query row, keys spread
 // over its lanes, every operand read row by row through L1: 1902 us; with one multiply-add per instruction: 234 us).
 //
 // Sums are kept short, because the rounding error of a chain grows with the square root of its length: half a head's terms
@@ -23,6 +23,10 @@
 // 2-norm of the error against float64: 1.7e-7 at 8 x 48..387, 1.8e-7 at 8 x 512, 2.0e-7 at 2 x 2048 (one chain over all terms of a
 // score and over all keys: 3.6e-7, 4.5e-7, 8.3e-7, at the same speed; one warp per query row: 1.9e-7, 2.0e-7, 2.3e-7; without
 // the sum per tile: 1.8e-7, 1.9e-7, 2.6e-7).
+//
+// A block is bound by its own chain of key tiles, some 6 to 9 us each, so two or four pairs of warps (GROUPS) take every second or fourth
+// tile of the same query rows, and their states are added at the end (the rule of the launch has the times).  2 x 128: 35.0 us per
+// call with one pair, 29.4; 8 x (48..387) 208 and 195.
 #include "attn_blocks.cuh"
 #include "ptx_sm100.cuh"
 #include <math_constants.h>
@@ -345,7 +349,7 @@ __global__ void __launch_bounds__(THREADS * GROUPS, 4 / GROUPS) attn_simt_kernel
   }
 }
 
-template <typename T, int R, bool TABLES, int GROUPS = 1>
+template <typename T, int R, bool TABLES, int GROUPS>
 int launch_variant(const AttnParams& p, cudaStream_t s) {
   constexpr int SMEM = smem_floats<R, TABLES, GROUPS> * 4;
   auto kern = attn_simt_kernel<T, R, TABLES, GROUPS>;
@@ -360,17 +364,27 @@ int launch_variant(const AttnParams& p, cudaStream_t s) {
 
 template <typename T, bool TABLES>
 int launch_rows(const AttnParams& p, cudaStream_t s) {
-  // 32 query rows per block re-use each staged row twice as often as 16; 16 rows where 32 would leave SMs without a block.  With at most
-  // two such blocks per SM there is room for a second pair of warps each, which halves the block's chain of key tiles (12 heads, us
-  // per call, one pair and two: 1 x 100 36.2 and 27.4, 2 x 128 38.6 and 33.6, 1 x 200 54.5 and 43.2, 1 x 300 64.9 and 55.1, 2 x 200, which
-  // is 2.1 per SM, 65.6 and 63.0); with more, or one tile, it takes others' place (4 x 128 41.7 and 45.2, 2 x 300 84.8 and 94.3).  Four
-  // pairs gain nothing more below four tiles (1 x 300 64.3, 1 x 512 105.9 against 108.9).
+  // 32 query rows per block re-use each staged row twice as often as 16.  A block is bound by its own chain of key tiles, so two pairs of
+  // warps share them (two blocks of 32 rows per SM instead of four: as many warps, and half the time to wait for the last block); four
+  // pairs while blocks have SMs to themselves, of 16 rows where even those do; one pair for many blocks of two tiles, whose second pair
+  // would be half of the work and all of the staging.  us per call, 12 heads, rows x pairs:
+  //   batch x length    blocks of 32 per SM    16 x 4    32 x 4    32 x 2    32 x 1    16 x 1
+  //   1 x 128           0.3                      28.2      31.9      32.0      44.0      36.6
+  //   1 x 256           0.6                      47.1      37.0      42.3      65.6      54.3
+  //   2 x 200           1.1                      63.0      58.2      55.7      66.4      64.5
+  //   4 x 512 ragged    5.2                     122.6      99.2      96.7     121.4     115.5
+  //   16 x 128          5.2                     131.2     102.1      77.9      79.4      98.7
+  //   32 x 128 ragged   10.4                    168.3     131.8     100.2      88.6     105.0
+  //   8 x 512           10.4                    649.2     468.7     440.9     470.6     615.0
+  // One tile leaves nothing to share: 16 rows where 32 would leave SMs without a block.
   int sms = 0, rc;
   if ((rc = device_sms(&sms))) return rc;
-  const int64_t rows = (int64_t)p.H * p.n_seqs;
-  if ((p.L + 31) / 32 * rows >= 2 * (int64_t)sms) return launch_variant<T, 4, TABLES>(p, s);
-  if (p.L > KT && (p.L + 15) / 16 * rows <= 2 * (int64_t)sms) return launch_variant<T, 2, TABLES, 2>(p, s);
-  return launch_variant<T, 2, TABLES>(p, s);
+  const int64_t rows = (int64_t)p.H * p.n_seqs, blocks16 = (p.L + 15) / 16 * rows, blocks32 = (p.L + 31) / 32 * rows;
+  if (p.L <= KT) return blocks32 < 2 * (int64_t)sms ? launch_variant<T, 2, TABLES, 1>(p, s) : launch_variant<T, 4, TABLES, 1>(p, s);
+  if (blocks16 <= sms) return launch_variant<T, 2, TABLES, 4>(p, s);
+  if (blocks32 <= sms) return launch_variant<T, 4, TABLES, 4>(p, s);
+  if (p.L <= 2 * KT && blocks32 > 6 * (int64_t)sms) return launch_variant<T, 4, TABLES, 1>(p, s);
+  return launch_variant<T, 4, TABLES, 2>(p, s);
 }
 
 template <typename T>
