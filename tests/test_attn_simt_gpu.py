@@ -158,7 +158,8 @@ def test_fp32_error_does_not_grow_with_the_sequence(lengths, c2p, p2c):
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("lengths,padded,heads", [([65], 65, 2), ([128, 64, 1], 128, 2), ([129, 0, 63], 129, 2), ([300, 192, 193], 300, 2),
-                                                  ([257, 320, 64, 0], 320, 3), ([200, 65, 128, 1], 200, 12), ([128, 64, 1, 0] * 20, 128, 3)])
+                                                  ([257, 320, 64, 0], 320, 3), ([200, 65, 128, 1], 200, 12), ([128, 64, 1, 0] * 20, 128, 3),
+                                                  ([128, 64, 1, 0] * 20, 128, 4)])
 @pytest.mark.parametrize("c2p,p2c", [(True, True), (True, False), (False, True), (False, False)])
 def test_pairs_of_warps_share_the_key_tiles(lengths, padded, heads, c2p, p2c, dtype):
     """One, two and four pairs, 16 and 32 rows, at the tiles' edges; sequences with no tile for some of the pairs, and none at all."""

@@ -366,16 +366,18 @@ template <typename T, bool TABLES>
 int launch_rows(const AttnParams& p, cudaStream_t s) {
   // 32 query rows per block re-use each staged row twice as often as 16.  A block is bound by its own chain of key tiles, so two pairs of
   // warps share them (two blocks of 32 rows per SM instead of four: as many warps, and half the time to wait for the last block); four
-  // pairs while blocks have SMs to themselves, of 16 rows where even those do; one pair for many blocks of two tiles, whose second pair
-  // would be half of the work and all of the staging.  us per call, 12 heads, rows x pairs:
+  // pairs while blocks have SMs to themselves, of 16 rows where even those do.  us per call, 12 heads, rows x pairs:
   //   batch x length    blocks of 32 per SM    16 x 4    32 x 4    32 x 2    32 x 1    16 x 1
   //   1 x 128           0.3                      28.2      31.9      32.0      44.0      36.6
   //   1 x 256           0.6                      47.1      37.0      42.3      65.6      54.3
   //   2 x 200           1.1                      63.0      58.2      55.7      66.4      64.5
   //   4 x 512 ragged    5.2                     122.6      99.2      96.7     121.4     115.5
   //   16 x 128          5.2                     131.2     102.1      77.9      79.4      98.7
-  //   32 x 128 ragged   10.4                    168.3     131.8     100.2      88.6     105.0
   //   8 x 512           10.4                    649.2     468.7     440.9     470.6     615.0
+  // With every SM full, an odd tile leaves the second pair waiting, which is one pair's time lost where rows are all as long (two pairs
+  // and one: 5 x 179, 2.4 blocks per SM, 78.2 and 72.5, 8 x 179 92.9 and 74.8; 5 x 300, 4.1 per SM, 161.5 and 167.8, 7 x 300, 5.7, 187.3 and
+  // 169.6; 4 x 448 210.7 and 229.1, 5 x 448 244.0 and 229.8), and so do rows of one tile among ragged ones of up to three (11 x 126
+  // with 16 heads, 4.8 per SM, 51.8 and 49.5, 31 x 128 94.6 and 84.8, 21 x 179 99.4 and 95.9; of four, 15 x 256, 116.9 and 128.3).
   // One tile leaves nothing to share: 16 rows where 32 would leave SMs without a block.
   int sms = 0, rc;
   if ((rc = device_sms(&sms))) return rc;
@@ -383,8 +385,10 @@ int launch_rows(const AttnParams& p, cudaStream_t s) {
   if (p.L <= KT) return blocks32 < 2 * (int64_t)sms ? launch_variant<T, 2, TABLES, 1>(p, s) : launch_variant<T, 4, TABLES, 1>(p, s);
   if (blocks16 <= sms) return launch_variant<T, 2, TABLES, 4>(p, s);
   if (blocks32 <= sms) return launch_variant<T, 4, TABLES, 4>(p, s);
-  if (p.L <= 2 * KT && blocks32 > 6 * (int64_t)sms) return launch_variant<T, 4, TABLES, 1>(p, s);
-  return launch_variant<T, 4, TABLES, 2>(p, s);
+  const int tiles = (p.L + KT - 1) / KT;
+  const bool full = !p.varlen && !p.seqlens;
+  const bool waits = full ? tiles % 2 && blocks32 > (tiles == 3 ? 2 : 5) * (int64_t)sms : tiles <= 3 && blocks32 > (tiles == 2 ? 4 : 5) * (int64_t)sms;
+  return waits ? launch_variant<T, 4, TABLES, 1>(p, s) : launch_variant<T, 4, TABLES, 2>(p, s);
 }
 
 template <typename T>
