@@ -124,7 +124,8 @@ extern "C" {
 // tiles the narrow projections would still gain and the wide ones lose, 48 tokens: 3.2 and 3.3, 4.0 and 4.1, 4.8 and 4.4, 6.5 and
 // 6.7; K 1024 5.6 and 4.8, 5.9 and 5.1; with four all lose (64 tokens: 3.5 and 3.3, 4.2 and 4.0, 5.6 and 4.4, 7.0 and 6.8).  A pass of the
 // base model with and without: 8 tokens 445 and 531 us, 16 tokens 449 and 512, 32 tokens 495 and 507; of the large one: 16 tokens 884
-// and 1057, 32 tokens 999 and 1000.  K up to what a warp's registers hold.
+// and 1057, 32 tokens 999 and 1000 (since encoder_short.cu takes passes of these two sizes as a whole, this is for other sizes and for
+// passes that return every layer).  K up to what a warp's registers hold.
 int tdb_skinny_applies(int64_t T, int64_t K, int64_t N) { return T <= SKINNY_TOKENS && K % KB == 0 && K <= KB * WARPS * 16 && N % 8 == 0; }
 
 int tdb_skinny(const void* x, const void* w, const void* b, int T, int K, int N, int gelu, int early, void* y, void* stream) {
