@@ -347,6 +347,26 @@ def test_far_items_in_a_row(c2p, p2c):
         assert torch.equal(flash_attention_with_disentangled(*args, seqlens=lens, tables=tables, kernel=UMMA), o)
 
 
+@pytest.mark.parametrize("lengths", [[1], [128] * 32, [129, 0, 1] * 11, [5] * 128, [5] * 129, [1100, 3, 640, 0, 256], [640, 127, 128, 129] * 8], ids=lambda x: f"{len(x)}x{max(x)}")
+@pytest.mark.parametrize("told", ["longest", "too short"])
+def test_packed_batches_around_the_rule_of_their_tile_list(lengths, told):
+    """Listed by every CTA for itself or by a kernel in front, with max_seqlen as it is and as a caller may have got it wrong."""
+    from turbodeberta_b200.ops.flash_attention import flash_attention_with_disentangled
+    from turbodeberta_b200.ops.flash_attention_varlen import flash_attention_with_disentangled_varlen
+    L = max(lengths)
+    w = _wl(lengths, L, hidden=128, heads=2, seed=91)
+    q, k, v, rel, P = util.device_inputs(w, DT)
+    tables = util.make_tables(w, rel, P)
+    lens = torch.tensor(lengths, dtype=torch.int32, device="cuda")
+    keep = torch.arange(L, device="cuda")[None] < lens[:, None]
+    cu = torch.tensor(np.concatenate([[0], np.cumsum(lengths)]), dtype=torch.int32, device="cuda")
+    n = L if told == "longest" else max(1, L // 3)
+    got = flash_attention_with_disentangled_varlen(q[keep], k[keep], v[keep], None, None, cu, cu, n, n, False, 0.0722, 256, 512, tables=tables, kernel=UMMA)
+    args = [t.permute(0, 2, 1, 3) for t in (q, k, v)] + [None, None, False, 0.0722, 256, 512]
+    want = flash_attention_with_disentangled(*args, seqlens=lens, tables=tables, kernel=SIMT).permute(0, 2, 1, 3)[keep]
+    assert ((got.float() - want.float()).abs() <= 2.0 ** -7 * want.float().abs() + 8e-3).all()
+
+
 @pytest.mark.parametrize("level", [4.0, 16.0, 60.0])
 def test_far_scores_far_above_the_near_ones(level):
     """Far keys whose scores lie up to hundreds of powers of two above the near tiles': within what the near tiles'

@@ -84,7 +84,8 @@ constexpr int FCB = 9;                          // step of the exponential loop 
 constexpr int FPB = 4;                          // step of the c2p loop at which the fused p2c drain starts
 static_assert(FPB >= 0 && FPB + STG_COLS / GROUPS / 8 <= KPT / 2 - 1, "the fused drain's last step must lie inside the loop");
 static_assert(FCB >= 0 && FCB + STG_COLS / GROUPS / 8 <= KPT / 2 - 1, "the fused drain's last step must lie inside the loop");
-constexpr uint32_t SMEM_BYTES = OFF_PERM + PERM_MAX * 2 + 1024;   // + slack for the 1024-byte alignment of the base
+constexpr int LIST_MAX = 1024;                  // tiles of a packed batch that a CTA lists for itself, in the same place
+constexpr uint32_t SMEM_BYTES = OFF_PERM + (PERM_MAX * 2 > LIST_MAX * 4 ? PERM_MAX * 2 : LIST_MAX * 4) + 1024;   // + slack for the 1024-byte alignment of the base
 static_assert(OFF_STP % 16 == 0 && OFF_XCH % 16 == 0 && OFF_BAR % 16 == 0 && OFF_LX % 16 == 0, "offsets must stay 16-byte aligned");
 static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
 
@@ -248,15 +249,16 @@ struct Work {
   int64_t tok0;
 };
 
-// perm: padded form only, sequences by decreasing length (null: natural order).
-template <bool SPLIT>
-__device__ __forceinline__ bool get_work(const AttnParams& p, int total_tiles, int w, const uint16_t* perm, Work& k) {
+// perm: padded form only, sequences by decreasing length (null: natural order).  list: packed form with OWN, the CTA's own list of tiles
+// (otherwise the one in the workspace).
+template <bool SPLIT, bool OWN>
+__device__ __forceinline__ bool get_work(const AttnParams& p, int total_tiles, int w, const uint16_t* perm, const uint32_t* list, Work& k) {
   const int tile = w / p.H;
   if (tile >= total_tiles) return false;
   k.h = w - tile * p.H;
   if (p.varlen) {
-    const int32_t* ws = reinterpret_cast<const int32_t*>(p.workspace);
-    const int2 e = reinterpret_cast<const int2*>(ws + 4)[tile];
+    const int2 e = OWN ? make_int2((int)(list[tile] >> 16), (int)(list[tile] & 0xffffu) * BQ)
+                       : reinterpret_cast<const int2*>(reinterpret_cast<const int32_t*>(p.workspace) + 4)[tile];
     const int c0 = p.cu_seqlens[e.x];
     k.len = p.cu_seqlens[e.x + 1] - c0; k.rows = e.x; k.tok0 = c0; k.bcoord = 0; k.q0 = e.y;
   } else {
@@ -281,8 +283,9 @@ template <bool SPLIT>
 __device__ __forceinline__ int first_key(const AttnParams& p, int q0) { return SPLIT ? near_first(q0, p.split_sat) * BK : 0; }
 
 // LONG: sequences can be long enough for saturated tiles (compiled out otherwise, which keeps the common kernel lean).
-// SPLIT: they are, and the kernel for far tiles takes those.
-template <bool C2P, bool P2C, bool LONG, bool SPLIT>
+// SPLIT: they are, and the kernel for far tiles takes those.  OWN: a few packed sequences, whose tiles each CTA lists for itself (in the
+// common instantiation the code for it cost 1 to 2 % although it did not run).
+template <bool C2P, bool P2C, bool LONG, bool SPLIT, bool OWN>
 __global__ void __launch_bounds__(threads_of<SPLIT>, 1)
 attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                  const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_kr,
@@ -332,11 +335,41 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap tm_q, c
   // while the other warps set the CTA up: it needs nothing but the lengths in global memory and its own corner of
   // shared memory.
   const uint16_t* perm = nullptr;
+  const uint32_t* list = nullptr;
   int total_tiles = 0;
   int32_t status_at_start = 0;
   if (warp == NCW + 2) {
     wait_for_stream();
-    total_tiles = p.varlen ? reinterpret_cast<const int32_t*>(p.workspace)[0] : p.n_seqs * ((p.L + BQ - 1) / BQ);
+    if constexpr (OWN) {                   // what build_tile_list_kernel does, for a few sequences
+      uint32_t* const lw = reinterpret_cast<uint32_t*>(gbase + OFF_PERM);
+      const int top = p.L > BQ ? (p.L + BQ - 1) / BQ : 1;          // longer ones than the caller has said go with the longest
+      for (int b = top; b >= 1; --b)
+        for (int s0 = 0; s0 < p.n_seqs; s0 += 32) {
+          const int sq = s0 + lane;
+          int nt = 0;
+          if (sq < p.n_seqs) {
+            const int c0 = p.cu_seqlens[sq], c1 = p.cu_seqlens[sq + 1];
+            if (c0 < 0 || c1 < c0 || (int64_t)c1 > p.total_tokens) *reinterpret_cast<volatile int32_t*>(p.status + 1) = 1;
+            else nt = (c1 - c0 + BQ - 1) / BQ;
+          }
+          if ((nt < top ? nt : top) != b) nt = 0;
+          int inc = nt;
+#pragma unroll
+          for (int off = 1; off < 32; off *= 2) {
+            const int o = __shfl_up_sync(0xffffffffu, inc, off);
+            if (lane >= off) inc += o;
+          }
+          const int start = total_tiles + inc - nt;
+          for (int t = 0; t < nt && start + t < LIST_MAX; ++t) lw[start + t] = ((uint32_t)sq << 16) | (uint32_t)t;
+          total_tiles += __shfl_sync(0xffffffffu, inc, 31);
+        }
+      total_tiles = total_tiles < LIST_MAX ? total_tiles : LIST_MAX;
+      if (lane == 0 && p.cu_seqlens[p.n_seqs] != (int32_t)p.total_tokens) *reinterpret_cast<volatile int32_t*>(p.status + 1) = 1;
+      __syncwarp();
+      list = lw;
+    } else {
+      total_tiles = p.varlen ? reinterpret_cast<const int32_t*>(p.workspace)[0] : p.n_seqs * ((p.L + BQ - 1) / BQ);
+    }
     // An earlier CTA gave up: no work is handed out.
     if (lane == 0) status_at_start = *reinterpret_cast<volatile int32_t*>(p.gave_up);
     const int qtiles = (p.L + BQ - 1) / BQ;
@@ -468,7 +501,7 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap tm_q, c
       first = false;
       w = __shfl_sync(0xffffffffu, w, 0);
       Work k;
-      if (!get_work<SPLIT>(p, total_tiles, w, perm, k)) k.n_kv = -1;
+      if (!get_work<SPLIT, OWN>(p, total_tiles, w, perm, list, k)) k.n_kv = -1;
       if (k.n_kv == 0) {
         for (int r = lane; r < BQ; r += 32) {
           if (k.q0 + r >= k.rows) break;
@@ -1114,9 +1147,9 @@ int table_map(CUtensorMap* m, const void* ptr, int rows, int H, int box_rows, co
 
 namespace {
 
-template <bool C2P, bool P2C, bool LONG, bool SPLIT = false>
+template <bool C2P, bool P2C, bool LONG, bool SPLIT = false, bool OWN = false>
 int launch_variant(const AttnParams& p, dim3 grid, const CUtensorMap* maps, cudaStream_t s) {
-  auto kern = attn_umma_kernel<C2P, P2C, LONG, SPLIT>;
+  auto kern = attn_umma_kernel<C2P, P2C, LONG, SPLIT, OWN>;
   const int rc = opt_in_smem(reinterpret_cast<const void*>(kern), (int)SMEM_BYTES);
   if (rc) return rc;
   return cuda_fail(launch_early(kern, grid, threads_of<SPLIT>, SMEM_BYTES, s, p, maps[0], maps[1], maps[2], maps[3], maps[4], maps[5],
@@ -1196,10 +1229,18 @@ int launch_attn_umma(const AttnParams& given, cudaStream_t s) {
   int sms = 0;
   if ((rc = device_sms(&sms))) return rc;
   int64_t tiles;
+  bool own_list = false;
   if (p.varlen) {
     tiles = (p.total_tokens + BQ - 1) / BQ + p.n_seqs + 1;           // upper bound; the device list has the real count
     if (tiles * p.H > 0x7fffffff) { set_error("too many tiles"); return TDB_ERR_SHAPE; }
-    if (!p.tiles_listed) {
+    // A few sequences: listed by each CTA's scheduler warp beside the rest of its set-up, some 300 clocks per step of 32 sequences and one
+    // tile count; the list kernel in front takes 3 us of the GPU and its launch two of the host.  us per call, own list and kernel: 2 x
+    // 50..100 tokens (1 step) 22.2 and 24.7, 20 x 10..64 28.2 and 30.9, 4 x 20..200 24.7 and 26.8, 30 x 60..500 (4) 54.2 and 55.4, 8 x
+    // 60..1000 (8) 37.7 and 38.6; with more than a few items per SM the host's part does not show: 30 x 60..1000 (8) 91.0 and 90.3, 256 x
+    // 8..128 (8) 94.7 and 92.8.
+    const int64_t steps = (int64_t)((p.n_seqs + 31) / 32) * ((p.L + BQ - 1) / BQ);
+    own_list = !split && !lng && !p.lengths_known && tiles <= LIST_MAX && (steps <= 4 || (steps <= 9 && tiles * p.H <= 4 * (int64_t)sms));
+    if (!p.tiles_listed && !own_list) {
       build_tile_list_kernel<<<1, 1024, 0, s>>>(p.cu_seqlens, p.n_seqs, p.total_tokens,
                                                 reinterpret_cast<int32_t*>(p.workspace), (int)tiles, p.status);
       if ((rc = cuda_fail(cudaGetLastError(), "build_tile_list launch"))) return rc;
@@ -1213,7 +1254,12 @@ int launch_attn_umma(const AttnParams& given, cudaStream_t s) {
   // status word 2 as the work counter: start it at zero even if the caller reuses the words
   if (p.counter == p.status + 2 &&
       (rc = cuda_fail(cudaMemsetAsync(p.counter, 0, sizeof(int32_t), s), "cudaMemsetAsync(work counter)"))) return rc;
-  if (c2p && p2c) rc = split ? launch_variant<true, true, false, true>(p, grid, maps, s) : lng ? launch_variant<true, true, true>(p, grid, maps, s) : launch_variant<true, true, false>(p, grid, maps, s);
+  if (own_list)
+    rc = c2p && p2c ? launch_variant<true, true, false, false, true>(p, grid, maps, s)
+         : c2p      ? launch_variant<true, false, false, false, true>(p, grid, maps, s)
+         : p2c      ? launch_variant<false, true, false, false, true>(p, grid, maps, s)
+                    : launch_variant<false, false, false, false, true>(p, grid, maps, s);
+  else if (c2p && p2c) rc = split ? launch_variant<true, true, false, true>(p, grid, maps, s) : lng ? launch_variant<true, true, true>(p, grid, maps, s) : launch_variant<true, true, false>(p, grid, maps, s);
   else if (c2p) rc = split ? launch_variant<true, false, false, true>(p, grid, maps, s) : lng ? launch_variant<true, false, true>(p, grid, maps, s) : launch_variant<true, false, false>(p, grid, maps, s);
   else if (p2c) rc = split ? launch_variant<false, true, false, true>(p, grid, maps, s) : lng ? launch_variant<false, true, true>(p, grid, maps, s) : launch_variant<false, true, false>(p, grid, maps, s);
   else rc = launch_variant<false, false, false>(p, grid, maps, s);
