@@ -109,3 +109,42 @@ def test_bf16_scores_kernel_at_tile_edges(lengths, L, terms, mirrored, width):
     for b, n in enumerate(lengths):
         assert torch.count_nonzero(o[b, :, n:]).item() == 0
         assert n == 0 or (lse[b, :, :n] - lse2[b, :, :n]).abs().max().item() < 1e-3
+
+
+@pytest.mark.parametrize("dtype", [torch.float32])
+@pytest.mark.parametrize("batch,length", [(1, 128), (12, 128), (30, 128), (30, 150), (1, 40)])      # four pairs of 16 and of 32 rows, two, one
+@pytest.mark.parametrize("hidden", ["64:", ":64", "all but 7", "all but 100", "lowest 64:", "lowest :64"])
+@pytest.mark.parametrize("packed", [False, True])
+def test_keys_hidden_by_the_scores(batch, length, hidden, packed, dtype):
+    """Scores of -inf, and two at the lowest finite value whose sum leaves fp32's range, give weight 0: also where they fill a key tile, or all
+    that one pair of warps has of a row."""
+    from turbodeberta_b200.ops.flash_attention import flash_attention_with_disentangled
+    from turbodeberta_b200.ops.flash_attention_varlen import flash_attention_with_disentangled_varlen
+    gen = torch.Generator(device="cuda").manual_seed(9)
+    q, k, v = (torch.randn(batch, length, 2, 64, generator=gen, device="cuda").to(dtype) for _ in range(3))
+    q_pos, k_pos = (torch.randn(batch, length, 2, 128, generator=gen, device="cuda").to(dtype) for _ in range(2))
+    hide = torch.zeros(length, dtype=torch.bool, device="cuda")
+    if hidden.startswith("all"):
+        hide[:] = True
+        hide[int(hidden[8:]) % length] = False
+    else:
+        start, stop = hidden.split()[-1].split(":")
+        hide[int(start or 0):int(stop or length)] = True
+        hide[17 if start else -17] = False           # a sequence within one tile keeps a key
+    lowest = hidden.startswith("lowest")
+    k_pos[:, hide] = torch.finfo(dtype).min if lowest else float("-inf")
+    if lowest:
+        q_pos[:, 5::3] = torch.finfo(dtype).min      # rows of which every score is beyond the others' range
+    if packed:
+        cu = torch.arange(batch + 1, device="cuda", dtype=torch.int32) * length
+        o, lse = flash_attention_with_disentangled_varlen(*(t.flatten(0, 1) for t in (q, k, v, q_pos, k_pos)), cu, cu, length, length, False,
+                                                          0.0722, 64, 128, return_lse=True)
+        o = o.view(batch, length, 2, 64)
+    else:
+        o, lse = flash_attention_with_disentangled(*(t.transpose(1, 2) for t in (q, k, v, q_pos, k_pos)), False, 0.0722, 64, 128, return_lse=True)
+        o = o.transpose(1, 2)
+    assert torch.isfinite(o).all() and torch.isfinite(lse).all()
+    for b in {0, batch - 1}:
+        ref = orc.attention_single_scores(*(util.f64(t[b]) for t in (q, k, v, q_pos, k_pos)), position_buckets=64, max_relative_positions=128,
+                                          sm_scale=0.0722)
+        util.assert_close(o[b], ref, dtype, f"{hidden}, sequence {b}")

@@ -29,6 +29,7 @@
 // call with one pair, 29.4; 8 x (48..387) 208 and 195.
 #include "attn_blocks.cuh"
 #include "ptx_sm100.cuh"
+#include <float.h>
 #include <math_constants.h>
 
 namespace tdb {
@@ -137,10 +138,12 @@ __global__ void __launch_bounds__(THREADS * GROUPS, 4 / GROUPS) attn_simt_kernel
   auto clamped = [&](int delta) { return delta < -dm ? 0 : (delta > dm ? 2 * dm : delta + dm); };
 
   f32x2 o[R][4];                                     // eight output columns
+  // The maximum starts at the lowest finite value: a row whose scores so far are all -inf (score tensors that hide keys, or whose sum leaves
+  // fp32's range) has a reference to take them against, and they get weight 0 instead of exp(-inf + inf).  A row with no other score ends as 0 / 0.
   float m[R], l[R];
 #pragma unroll
   for (int r = 0; r < R; ++r) {
-    m[r] = -CUDART_INF_F; l[r] = 0.f;
+    m[r] = -FLT_MAX; l[r] = 0.f;
 #pragma unroll
     for (int c = 0; c < 4; ++c) o[r][c] = 0ull;
   }
@@ -239,8 +242,8 @@ __global__ void __launch_bounds__(THREADS * GROUPS, 4 / GROUPS) attn_simt_kernel
         }
 #pragma unroll
         for (int off = 1; off < 8; off *= 2) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-        const float mn = fmaxf(m[r], mx);            // finite: every key tile has a valid key
-        corr[r] = expf(m[r] - mn);                   // first tile: m = -inf -> 0
+        const float mn = fmaxf(m[r], mx);
+        corr[r] = expf(m[r] - mn);
         m[r] = mn;
         float sum = 0.f;
 #pragma unroll
