@@ -111,8 +111,8 @@ def test_bf16_scores_kernel_at_tile_edges(lengths, L, terms, mirrored, width):
         assert n == 0 or (lse[b, :, :n] - lse2[b, :, :n]).abs().max().item() < 1e-3
 
 
-@pytest.mark.parametrize("dtype", [torch.float32])
-@pytest.mark.parametrize("batch,length", [(1, 128), (12, 128), (30, 128), (30, 150), (1, 40)])      # four pairs of 16 and of 32 rows, two, one
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("batch,length", [(1, 128), (12, 128), (30, 128), (30, 150), (1, 40)])      # fp32: four pairs of 16 and of 32 rows, two, one
 @pytest.mark.parametrize("hidden", ["64:", ":64", "all but 7", "all but 100", "lowest 64:", "lowest :64"])
 @pytest.mark.parametrize("packed", [False, True])
 def test_keys_hidden_by_the_scores(batch, length, hidden, packed, dtype):

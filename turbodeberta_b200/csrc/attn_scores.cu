@@ -19,6 +19,7 @@
 #include "attn_blocks.cuh"
 #include "attn_warp_mma.cuh"
 #include "ptx_sm100.cuh"
+#include <float.h>
 #include <math_constants.h>
 
 namespace tdb {
@@ -90,7 +91,7 @@ __global__ void __launch_bounds__(S_THREADS, 3) attn_scores_kernel(const AttnPar
 
   // this thread's rows r0 and r0 + 8 of the block, its keys 2 (lane % 4) + {0, 1} of every group of eight
   const int r0 = warp * 16 + lane / 4, kc = 2 * (lane % 4);
-  float o[8][4], m[2] = {-CUDART_INF_F, -CUDART_INF_F}, l[2] = {0.f, 0.f};
+  float o[8][4], m[2] = {-FLT_MAX, -FLT_MAX}, l[2] = {0.f, 0.f};         // not -inf: see attn_simt.cu
 #pragma unroll
   for (int i = 0; i < 8; ++i)
 #pragma unroll
@@ -186,7 +187,7 @@ __global__ void __launch_bounds__(S_THREADS, 3) attn_scores_kernel(const AttnPar
 #pragma unroll
         for (int i = 0; i < 8; ++i) mx = fmaxf(mx, fmaxf(sc[i][2 * r], sc[i][2 * r + 1]));
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));     // finite: every key tile has a valid key
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
         const float corr = ptx::ex2(m[r] - mx);
         m[r] = mx;
         float sum = 0.f;
