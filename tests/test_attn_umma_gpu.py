@@ -347,6 +347,21 @@ def test_far_items_in_a_row(c2p, p2c):
         assert torch.equal(flash_attention_with_disentangled(*args, seqlens=lens, tables=tables, kernel=UMMA), o)
 
 
+@pytest.mark.parametrize("lengths", [[2100, 0, 1300, 2049, 700], [2100] * 4], ids=lambda x: f"{len(x)}x{max(x)}")
+def test_far_items_of_several_groups_of_sequences(lengths):
+    """K and V of a sequence are 13 MB here, so the far kernel takes two sequences at a time, with and without one left over.  Against the
+    exact kernel, tolerance as above."""
+    from turbodeberta_b200.ops.flash_attention import flash_attention_with_disentangled
+    w = _wl(lengths, 2100, hidden=64 * 24, heads=24, buckets=64, maxpos=128)
+    q, k, v, rel, P = util.device_inputs(w, DT)
+    tables = util.make_tables(w, rel, P)
+    lens = torch.tensor(lengths, dtype=torch.int32, device="cuda")
+    args = [t.permute(0, 2, 1, 3) for t in (q, k, v)] + [None, None, False, 0.0722, 64, 128]
+    o = flash_attention_with_disentangled(*args, seqlens=lens, tables=tables, kernel=UMMA)
+    o2 = flash_attention_with_disentangled(*args, seqlens=lens, tables=tables, kernel=SIMT)
+    assert ((o.float() - o2.float()).abs() <= 2.0 ** -7 * o2.float().abs() + 4e-3).all()
+
+
 @pytest.mark.parametrize("lengths", [[1], [128] * 32, [129, 0, 1] * 11, [5] * 128, [5] * 129, [1100, 3, 640, 0, 256], [640, 127, 128, 129] * 8], ids=lambda x: f"{len(x)}x{max(x)}")
 @pytest.mark.parametrize("told", ["longest", "too short"])
 def test_packed_batches_around_the_rule_of_their_tile_list(lengths, told):

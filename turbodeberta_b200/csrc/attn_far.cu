@@ -15,7 +15,7 @@
 // copies while the item is at work (64 KB of outputs per pair of tiles, for which Q has one buffer and not two: the products run
 // ahead of the exponentials by more than Q's way from memory), and the constants are formed one side per thread: read and formed by
 // the groups at the item's ends, they took 6 of the 9.5 thousand clocks between two items.  Padded batches take the outer pairs
-// first, which have most far tiles.  us per call before and after: 4 x 4096 tokens 512 and 502 (this kernel 252 and 237), 1 x 4096
+// first, which have most far tiles (far_work).  us per call before and after: 4 x 4096 tokens 512 and 502 (this kernel 252 and 237), 1 x 4096
 // 212 and 170 (the order), 8 x 2048 350 and 337, 13 x 1200 286 and 270; 64 packed sequences of 2048 to 8192 the same, under the power cap.
 //
 // Bound: the special-function unit, 16384 exponentials per tile = 1024 clocks, beside 768 clocks of tensor work.  What matters
@@ -38,6 +38,7 @@
 // memory is freed and the host reports it.
 #include "attn_common.cuh"
 #include <math_constants.h>
+#include <algorithm>
 
 namespace tdb {
 using namespace ptx;
@@ -72,7 +73,14 @@ struct FarWork {
 static_assert(sizeof(FarWork) == 64, "a ring slot");
 
 // Index space: packed form, the listed tiles (of which every second one of a sequence has nothing to do); padded form, pairs of
-// tiles, from the ends of the sequences inwards: the outer pairs have most far tiles, and the cheapest come last.
+// tiles, from the ends of the sequences inwards: the outer pairs have most far tiles, and the cheapest come last.  That order goes through
+// one group of neighbouring sequences after another (p.far_group of them), because K and V of a whole group are in use at once.  32 MB of
+// them is where more sequences stop helping the tail and begin to cost memory traffic.  us per call, 12 heads, groups of 1, 2, 4, 8 and all
+// sequences (and pairs in their natural order): 16 x 4096 tokens (12.6 MB each) 1870, 1861, 1891, 1945, 1977 (1892); 8 x 8192 (25 MB) 3025,
+// 3046, 3174, 3286 (3025); 64 x 2048 (6.3 MB) 2490, 2494, 2492, 2490, 2533 (2541); 48 x 1000..3000 (9.2 MB) 2292, 2301, 2309, 2321, 2376 (2331);
+// 2 x 4096 265, 261 (312); 3 x 3000 249, 244, of three 240 (277).  Over 36 batches of at most 16384 tokens, 1152 and more each: 0.4 % faster than
+// all sequences at once, from 6 % faster to 1.5 % slower (16 MB 0.3 %, 9 % to 3.3 %; 48 and 64 MB 0.1 %).
+constexpr int64_t GROUP_BYTES = 32 << 20;
 __device__ __forceinline__ int far_rows(const AttnParams& p) {
   return p.varlen ? reinterpret_cast<const int32_t*>(p.workspace)[0] : p.n_seqs * ((p.L + 2 * BQ - 1) / (2 * BQ));
 }
@@ -86,7 +94,8 @@ __device__ __forceinline__ bool far_work(const AttnParams& p, int total, int w, 
     const int c0 = p.cu_seqlens[e.x];
     k.len = p.cu_seqlens[e.x + 1] - c0; k.rows = k.len; k.tok0 = c0; k.bcoord = 0; k.q0 = e.y; k.seq = e.x;
   } else {
-    const int pairs = (p.L + 2 * BQ - 1) / (2 * BQ), rank = tile / p.n_seqs, seq = tile - rank * p.n_seqs;
+    const int pairs = (p.L + 2 * BQ - 1) / (2 * BQ), group = tile / (p.far_group * pairs), first = group * p.far_group;
+    const int seqs = min(p.far_group, p.n_seqs - first), at = tile - first * pairs, rank = at / seqs, seq = first + at - rank * seqs;
     k.q0 = ((rank & 1) ? pairs - 1 - rank / 2 : rank / 2) * (2 * BQ);
     const int len = p.seqlens ? p.seqlens[seq] : p.L;
     k.len = len < 0 ? 0 : (len > p.L ? p.L : len);
@@ -560,7 +569,12 @@ int launch_far_variant(const AttnParams& p, dim3 grid, const CUtensorMap* maps, 
 
 // `tiles`: query tiles of the whole problem (an upper bound in the packed form, whose list says how many there are); at least as many as
 // the kernel's indices.
-int launch_attn_far(const AttnParams& p, int64_t tiles, int sms, cudaStream_t s) {
+int launch_attn_far(const AttnParams& given, int64_t tiles, int sms, cudaStream_t s) {
+  AttnParams p = given;
+  const int64_t kv_bytes = (int64_t)p.L * p.H * 2 * HD * 2;             // of a padded sequence
+  const int most = (int)std::max<int64_t>(1, std::min<int64_t>(p.n_seqs, GROUP_BYTES / std::max<int64_t>(1, kv_bytes)));
+  const int groups = (p.n_seqs + most - 1) / most;
+  p.far_group = (p.n_seqs + groups - 1) / groups;                       // of about the same size
   CUtensorMap maps[4];
   const int64_t tokens = p.varlen ? p.total_tokens : p.L;
   const int B = p.varlen ? 1 : p.n_seqs;

@@ -42,8 +42,8 @@ struct AttnParams {
   int32_t* counter; int32_t* gave_up;
   void* workspace; size_t workspace_bytes;
   // Long sequences on the tensor cores: scratch for the softmax state that the kernel for near key tiles hands to the one for
-  // far tiles, tdb_partial_floats() of fp32, part_ml behind part_o's tiles (null: one kernel does both).  split_sat is the launcher's own.
-  float* part_o; float* part_ml; int split_sat;
+  // far tiles, tdb_partial_floats() of fp32, part_ml behind part_o's tiles (null: one kernel does both).  split_sat and far_group are the launchers' own.
+  float* part_o; float* part_ml; int split_sat; int far_group;
   int lengths_known;                                      // packed form: L is known to be the longest sequence's length
   int direct_tables;                                      // kr and qr are read by index; kr_exp and qr_exp do not exist (kernel for short sequences only)
   int tiles_listed;                                       // packed form: the workspace already holds this batch's tile list
