@@ -175,7 +175,9 @@ attn_far_kernel(const AttnParams p, int32_t* counter, const __grid_constant__ CU
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  wait_for_stream();                                 // for the near kernel; all of the above ran beside its end
+  // For the near kernel, which lets this one start with the end of its last CTA.  Let in earlier, as SMs fall idle, the CTAs of this kernel
+  // made 36 padded batches of 1152 tokens and more 1.0 % slower in the geometric mean (2.8 % slower to 0.3 % faster), packed ones 0 to 0.4 %.
+  wait_for_stream();
   const int total = far_rows(p);
   int32_t gave_up_before = 0;
   if (warp == 2 * GW && lane == 2) gave_up_before = *reinterpret_cast<volatile int32_t*>(p.gave_up);

@@ -399,7 +399,6 @@ attn_umma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap tm_q, c
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   wait_for_stream();                       // all of the above ran beside the end of the kernel in front
-  if (SPLIT) let_next_start();             // the far kernel's CTAs, as SMs become free; they wait for the state that all of this leaves
 
   // Item n of this CTA's stream; n_kv < 0 marks the end of the stream.  (Tiles that consist of padded query rows
   // only never enter the ring: the scheduler warp zeroes them itself.)
