@@ -51,3 +51,19 @@ def test_ids_outside_the_vocabulary_are_reported():
             with pytest.raises(IndexError):
                 model(input_ids=wrong)
         assert torch.equal(model(input_ids=ids).last_hidden_state, want)
+
+
+def test_the_report_of_a_bad_id_leaves_the_others_words_alone():
+    from turbodeberta_b200 import _cabi as cabi
+    from turbodeberta_b200.ops import flash_attention as fa
+    table, v = torch.randn(9, 16, device="cuda"), torch.ones(16, device="cuda")
+    ids, mask = torch.full((2, 4), 9, dtype=torch.long, device="cuda"), torch.ones(2, 4, dtype=torch.long, device="cuda")
+    cabi.host.embed(ids, table, v, v, 1e-7, mask)
+    assert cabi.host.drain_pending() == (0, 0, 0, 1)
+    cabi.host.embed(ids, table, v, v, 1e-7, mask)
+    timed_out = torch.zeros(4, dtype=torch.int32, device="cuda")
+    cabi.check(cabi.lib.tdb_selftest_bounded_wait(cabi.ptr(timed_out), 77, 2000, cabi.stream_ptr(ids.device)))
+    fa._PENDING_STATUS.append(timed_out)
+    with pytest.raises(cabi.TdbError, match="77.*vocabulary"):
+        fa.check_pending_status()
+    fa.check_pending_status()

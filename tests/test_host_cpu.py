@@ -152,6 +152,26 @@ def test_pending_status_blocks_are_folded_never_dropped():
     assert int(torch.stack(blocks).amax(dim=0)[0]) == 7
 
 
+def test_reports_of_several_kinds_are_all_named(monkeypatch):
+    """Words of several calls come together in one check: none of them hides another, from the pool or from a block of a call's own."""
+    from turbodeberta_b200 import _cabi as cabi
+    from turbodeberta_b200.ops import flash_attention as fa
+    pool = []
+    monkeypatch.setattr(cabi.host, "drain_pending", lambda: pool.pop() if pool else None)
+    wait, offsets, token = (302, 0, 0, 0), (0, 1, 0, 0), (0, 0, 0, 1)
+    for pooled, own, error, texts in ((token, None, IndexError, ["vocabulary"]), (offsets, None, ValueError, ["cu_seqlens"]),
+                                      (token, wait, cabi.TdbError, ["302", "vocabulary"]), (wait, token, cabi.TdbError, ["302", "vocabulary"]),
+                                      ((401, 1, 0, 1), offsets, cabi.TdbError, ["401", "cu_seqlens", "vocabulary"]),
+                                      (token, offsets, ValueError, ["cu_seqlens", "vocabulary"])):
+        pool.append(pooled)
+        if own:
+            fa._PENDING_STATUS.append(torch.tensor(own, dtype=torch.int32))
+        with pytest.raises(error) as e:
+            fa.check_pending_status()
+        assert all(t in str(e.value) for t in texts)
+        fa.check_pending_status()                    # nothing is reported twice
+
+
 def test_mask_analysis_refresh_recomputes_lengths_without_changing_the_route():
     from turbodeberta_b200.model import analyse_mask
     m = torch.zeros(2, 6, dtype=torch.long)

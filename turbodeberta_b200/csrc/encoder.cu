@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(128) embed_kernel(const I* __restrict__ ids, c
   if (row >= rows) return;
   int64_t id = ids[row];
   if (id < 0 || id >= vocabulary) {
-    if (lane == 0 && *reinterpret_cast<volatile int32_t*>(status) == 0) *reinterpret_cast<volatile int32_t*>(status) = TDB_BAD_TOKEN;
+    if (lane == 0) *reinterpret_cast<volatile int32_t*>(status + 3) = 1;
     id = 0;
   }
   const float keep = mask_bytes == 8 ? (float)static_cast<const int64_t*>(mask)[row] : (float)static_cast<const uint8_t*>(mask)[row];

@@ -114,12 +114,23 @@ int acquire(int dev) {
   return s;
 }
 
+// What a launch has reported: 0 = code of a wait that gave up, 1 = malformed offsets, 3 = a token id outside the vocabulary.
+struct Words {
+  int w[SLOT_WORDS] = {};
+  bool any() const { return w[0] || w[1] || w[2] || w[3]; }
+  void merge(const Words& o) {
+    for (int i = 0; i < SLOT_WORDS; ++i) w[i] = std::max(w[i], o.w[i]);
+  }
+  py::object to_python() const { return any() ? py::object(py::make_tuple(w[0], w[1], w[2], w[3])) : py::none(); }
+};
+
 // Read the words of a slot whose launch has finished, and hand the slot back clean.
-std::pair<int, int> collect(int dev, int slot, bool keep = false) {
+Words collect(int dev, int slot, bool keep = false) {
   StatusPool& p = g_pools[dev];
   volatile int32_t* w = p.host + slot * SLOT_WORDS;
-  const std::pair<int, int> r(w[0], w[1]);
-  if (r.first || r.second) {
+  Words r;
+  for (int i = 0; i < SLOT_WORDS; ++i) r.w[i] = w[i];
+  if (r.any()) {
     for (int i = 0; i < SLOT_WORDS; ++i) w[i] = 0;
     // a launch that gave up may have left its work counter and flag set
     cudaMemset(p.ctl + slot * SLOT_WORDS, 0, SLOT_WORDS * 4);
@@ -196,7 +207,7 @@ struct Status {
     std::lock_guard<std::mutex> lock(g_pools[dev].mu);
     g_pools[dev].pending.push_back({std::exchange(slot, -1), std::move(mark), false});
   }
-  // What the caller in Python gets to see: None (fine, or deferred into the pool), (word 0, word 1), or the tensor of words.
+  // What the caller in Python gets to see: None (fine, or deferred into the pool), the words, or the tensor of words.
   py::object finish(bool check, c10::cuda::CUDAStream stream) {
     if (slot < 0) return py::cast(own.narrow(0, 0, SLOT_WORDS));
     if (!check) {
@@ -210,16 +221,15 @@ struct Status {
       py::gil_scoped_release nogil;
       e = cudaStreamSynchronize(stream.stream());
     }
-    const auto r = collect(dev, std::exchange(slot, -1));
+    const Words r = collect(dev, std::exchange(slot, -1));
     cuda_ok(e, "cudaStreamSynchronize");
-    if (r.first || r.second) return py::make_tuple(r.first, r.second);
-    return py::none();
+    return r.to_python();
   }
 };
 
 // Words of every launch with a deferred check, all devices: None, or the largest of each word.
 py::object drain_pending() {
-  int w0 = 0, w1 = 0;
+  Words all;
   for (int dev = 0; dev < MAX_DEV; ++dev) {
     StatusPool& p = g_pools[dev];
     std::vector<StatusPool::Pending> take;
@@ -239,14 +249,10 @@ py::object drain_pending() {
         if ((e = t.mark.wait()) != cudaSuccess) break;
       }
     }
-    for (const auto& t : take) {
-      const auto r = collect(dev, t.slot, t.keep);
-      w0 = std::max(w0, r.first); w1 = std::max(w1, r.second);
-    }
+    for (const auto& t : take) all.merge(collect(dev, t.slot, t.keep));
     cuda_ok(e, "synchronisation");
   }
-  if (w0 || w1) return py::make_tuple(w0, w1);
-  return py::none();
+  return all.to_python();
 }
 
 // ------------------------------------------------------------------------------------------------- argument checks
@@ -1330,7 +1336,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     return tdb_gelu(x.data_ptr(), x.numel(), dtype_code(x), c10::cuda::getCurrentCUDAStream().stream());
   });
   m.def("embed", &embed);
-  m.attr("BAD_TOKEN") = TDB_BAD_TOKEN;
   m.def("mask_rows", &mask_rows);
   m.def("pack_rows", &pack_rows);
   m.def("unpack_rows", &unpack_rows);

@@ -35,7 +35,7 @@ struct AttnParams {
   float sm_scale;
   int flags;
   float* lse; int64_t lse_sb, lse_sh;                     // lse[b*lse_sb + h*lse_sh + t] or null
-  int32_t* status;                                        // device-visible words: 0 = gave-up code, 1 = malformed offsets
+  int32_t* status;                                        // device-visible words: 0 = gave-up code, 1 = malformed offsets (3: see tdb_embed)
   // Tensor-core kernel: the device-wide work counter (zero on entry, and zero again once the launch has finished) and the
   // flag that makes CTAs starting after a wait gave up hand out no work.  Null: status words 2 (reset by the launch) and 0.
   // counter[2] is a second counter, of the kernel for far tiles.
@@ -136,9 +136,8 @@ TDB_HOST_API int tdb_expand_pair(const void* kr, const void* qr, const int16_t* 
 // early: as for tdb_skinny, of w and b.
 TDB_HOST_API int tdb_add_layernorm(const void* x, const void* res, const void* w, const void* b, float eps, int64_t rows, int hidden,
                                    int dtype, void* out, int early, void* stream);
-// Embeddings of `rows` tokens (ids of 4 or 8 bytes, a mask of 1 or 8): see embed_kernel.  An id outside the vocabulary is reported
-// in status word 0 as TDB_BAD_TOKEN.
-constexpr int TDB_BAD_TOKEN = 401;
+// Embeddings of `rows` tokens (ids of 4 or 8 bytes, a mask of 1 or 8): see embed_kernel.  An id outside the vocabulary, which is the
+// caller's mistake and not a failure of the device, has a status word of its own: 3.
 TDB_HOST_API int tdb_embed(const void* ids, int id_bytes, const void* table, int64_t vocabulary, const void* w, const void* b, float eps, const void* mask,
                            int mask_bytes, int64_t rows, int hidden, int dtype, void* out, int32_t* status, void* stream);
 TDB_HOST_API int tdb_gelu(void* x, int64_t elements, int dtype, void* stream);

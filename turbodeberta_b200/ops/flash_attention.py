@@ -20,6 +20,7 @@ reproduces the reference kernel's mirrored position->content index (``ops/flash_
 """
 from __future__ import annotations
 
+import itertools
 import math
 
 import torch
@@ -153,14 +154,13 @@ _PENDING_STATUS = _status.PENDING
 def check_pending_status() -> None:
     """Read (one synchronisation) the device status words of every call since the last check that was made
     with ``check_status=False`` and raise if any bounded device wait gave up or any ``cu_seqlens`` was malformed."""
-    pooled = cabi.host.drain_pending()
-    by_dev = {}
+    pooled, blocks = cabi.host.drain_pending(), {}
     for st in _PENDING_STATUS.drain():
-        by_dev.setdefault(st.device, []).append(st)
-    for dev, sts in by_dev.items():
-        _check_status(torch.stack(sts).amax(dim=0))
-    if pooled is not None:
-        _raise_for(pooled)
+        blocks.setdefault(st.device, []).append(st)
+    if pooled is None and not blocks:
+        return
+    words = [torch.stack(sts).amax(dim=0).tolist() for sts in blocks.values()]
+    _raise_for([max(w) for w in itertools.zip_longest(pooled or (0,), *words, fillvalue=0)])
 
 
 def _check_status(status: torch.Tensor):
@@ -169,13 +169,18 @@ def _check_status(status: torch.Tensor):
 
 
 def _raise_for(st):
-    if st[0] == cabi.host.BAD_TOKEN:
-        raise IndexError("a token id lies outside the vocabulary")
+    """The error that status words stand for, if any.  Words of several calls may have come together: the message names
+    every kind, and a wait that gave up, after which no output can be relied on, decides the type before a mistake of a caller's."""
+    found = []
     if st[0]:
-        raise cabi.TdbError(cabi.ERR_TIMEOUT, f"a device-side wait gave up (barrier code {st[0]})")
-    if st[1]:
-        raise ValueError("cu_seqlens is not a non-decreasing sequence ending at the token count (or the key offsets "
-                         "differ from the query offsets, or max_seqlen is smaller than the longest sequence)")
+        found.append((f"a device-side wait gave up (barrier code {st[0]})", lambda text: cabi.TdbError(cabi.ERR_TIMEOUT, text)))
+    if len(st) > 1 and st[1]:
+        found.append(("cu_seqlens is not a non-decreasing sequence ending at the token count (or the key offsets "
+                      "differ from the query offsets, or max_seqlen is smaller than the longest sequence)", ValueError))
+    if len(st) > 3 and st[3]:
+        found.append(("a token id lies outside the vocabulary", IndexError))
+    if found:
+        raise found[0][1]("; and ".join(text for text, _ in found))
 
 
 def finish_status(st, check: bool) -> None:
