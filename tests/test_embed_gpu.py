@@ -67,3 +67,76 @@ def test_the_report_of_a_bad_id_leaves_the_others_words_alone():
     with pytest.raises(cabi.TdbError, match="77.*vocabulary"):
         fa.check_pending_status()
     fa.check_pending_status()
+
+
+def _model():
+    from tests.test_model_gpu import _cfg
+    from turbodeberta_b200.model import FlashDebertaV2Model
+    return FlashDebertaV2Model(_cfg()).eval().to("cuda", torch.bfloat16)
+
+
+def test_a_bad_id_is_reported_to_its_own_caller():
+    """Another thread's pass checks between this pass's embeddings and its own check: it gets its result, and this one the error."""
+    import threading
+    mine, others = _model(), _model()
+    good = torch.randint(0, 500, (2, 20), device="cuda")
+    bad = good.clone()
+    bad[1, 3] = 500
+    run = mine.encoder.forward
+    seen = []
+
+    def other_pass():
+        try:
+            with torch.no_grad():
+                seen.append(others(input_ids=good).last_hidden_state)
+        except Exception as e:                                   # noqa: BLE001
+            seen.append(e)
+
+    def forward(*a, **kw):
+        t = threading.Thread(target=other_pass)
+        t.start()
+        t.join()
+        return run(*a, **kw)
+
+    with torch.no_grad():
+        want = others(input_ids=good).last_hidden_state
+        mine(input_ids=good)
+        mine.encoder.forward = forward
+        with pytest.raises(IndexError):
+            mine(input_ids=bad)
+        assert torch.equal(seen.pop(), want)
+        mine(input_ids=good)
+        assert torch.equal(seen.pop(), want)
+
+
+def test_a_pass_that_ends_early_gives_its_report_back():
+    """More passes than there are pooled words, each with a bad id and an encoder that fails: the words come back clean."""
+    from turbodeberta_b200._cabi import host
+    model = _model()
+    bad = torch.full((2, 20), 1000, device="cuda")
+
+    def fail(*a, **kw):
+        raise RuntimeError("not today")
+
+    run = model.encoder.forward
+    model.encoder.forward = fail
+    with torch.no_grad():
+        for _ in range(300):
+            with pytest.raises(RuntimeError, match="not today"):
+                model(input_ids=bad)
+        model.encoder.forward = run
+        model(input_ids=bad.clamp(max=499))
+        table, v = torch.randn(9, 16, device="cuda"), torch.ones(16, device="cuda")
+        ids = torch.zeros(2, 4, dtype=torch.long, device="cuda")
+        report = host.embed(ids, table, v, v, 1e-7, ids, True)[1]
+        assert isinstance(report, host.Report) and host.drain_pending(report) is None and host.drain_pending(report) is None
+
+
+def test_an_encoder_that_does_not_check_leaves_the_report_to_the_model():
+    model = _model()
+    bad = torch.full((2, 20), 1000, device="cuda")
+    with torch.no_grad():
+        model.encoder.forward = lambda x, *a, **kw: x
+        with pytest.raises(IndexError):
+            model(input_ids=bad)
+        assert model(input_ids=bad.clamp(max=499)).shape[:2] == (2, 20)

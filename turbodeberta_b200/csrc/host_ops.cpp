@@ -207,6 +207,8 @@ struct Status {
     std::lock_guard<std::mutex> lock(g_pools[dev].mu);
     g_pools[dev].pending.push_back({std::exchange(slot, -1), std::move(mark), false});
   }
+  // Leave the check to the holder of the report, or of the tensor of words.
+  py::object report(c10::cuda::CUDAStream stream);
   // What the caller in Python gets to see: None (fine, or deferred into the pool), the words, or the tensor of words.
   py::object finish(bool check, c10::cuda::CUDAStream stream) {
     if (slot < 0) return py::cast(own.narrow(0, 0, SLOT_WORDS));
@@ -227,8 +229,41 @@ struct Status {
   }
 };
 
-// Words of every launch with a deferred check, all devices: None, or the largest of each word.
-py::object drain_pending() {
+// The words of one launch that its caller reads, and nobody else: what a check finds in the pool's list may belong to another thread.
+class Report {
+ public:
+  Report(int dev, int slot, c10::cuda::CUDAStream stream) : dev_(dev), slot_(slot), mark_(stream) {}
+  Report(const Report&) = delete;
+  Report& operator=(const Report&) = delete;
+  ~Report() {                                        // its caller has met an error before the check
+    if (slot_ < 0) return;
+    py::gil_scoped_release nogil;
+    mark_.wait();
+    (void)cudaGetLastError();
+    int before = 0;
+    cudaGetDevice(&before);
+    cudaSetDevice(dev_);
+    collect(dev_, slot_);
+    cudaSetDevice(before);
+  }
+  int device() const { return slot_ < 0 ? -1 : dev_; }
+  const Mark& mark() const { return mark_; }
+  Words take() { return slot_ < 0 ? Words() : collect(dev_, std::exchange(slot_, -1)); }       // the mark has been waited for
+
+ private:
+  int dev_, slot_;
+  Mark mark_;
+};
+
+py::object Status::report(c10::cuda::CUDAStream stream) {
+  if (slot < 0) return py::cast(own.narrow(0, 0, SLOT_WORDS));
+  auto r = std::make_unique<Report>(dev, slot, stream);
+  slot = -1;
+  return py::cast(std::move(r));
+}
+
+// Words of every launch with a deferred check, all devices, and of the caller's own report: None, or the largest of each word.
+py::object drain_pending(Report* own) {
   Words all;
   for (int dev = 0; dev < MAX_DEV; ++dev) {
     StatusPool& p = g_pools[dev];
@@ -237,7 +272,8 @@ py::object drain_pending() {
       std::lock_guard<std::mutex> lock(p.mu);
       take.swap(p.pending);
     }
-    if (take.empty()) continue;
+    const bool with_own = own && own->device() == dev;
+    if (take.empty() && !with_own) continue;
     c10::cuda::CUDAGuard guard((c10::DeviceIndex)dev);
     cudaError_t e = cudaSuccess;
     {
@@ -248,8 +284,10 @@ py::object drain_pending() {
         last = &t.mark;
         if ((e = t.mark.wait()) != cudaSuccess) break;
       }
+      if (with_own && e == cudaSuccess && !(last && own->mark().on(last->stream()) && last->on(own->mark().stream()))) e = own->mark().wait();
     }
     for (const auto& t : take) all.merge(collect(dev, t.slot, t.keep));
+    if (with_own) all.merge(own->take());
     cuda_ok(e, "synchronisation");
   }
   return all.to_python();
@@ -1234,8 +1272,8 @@ py::object mask_rows(const Tensor& mask) {
 }
 
 // A model's input from ids [B, L]: LayerNorm of their embeddings, times the padding mask.  (output, words that somebody has to look at
-// or None), or None where the kernel does not take the tensors as they are.
-py::object embed(const Tensor& ids, const Tensor& table, const Tensor& w, const Tensor& b, double eps, const Tensor& mask) {
+// or None), or None where the kernel does not take the tensors as they are.  own: the words come as a Report, or a tensor, for the caller's own check.
+py::object embed(const Tensor& ids, const Tensor& table, const Tensor& w, const Tensor& b, double eps, const Tensor& mask, bool own) {
   const at::ScalarType t = table.scalar_type();
   const int64_t hidden = table.size(1);
   const bool types = (t == at::kFloat || t == at::kBFloat16) && w.scalar_type() == t && b.scalar_type() == t &&
@@ -1256,7 +1294,7 @@ py::object embed(const Tensor& ids, const Tensor& table, const Tensor& w, const 
                            mask.data_ptr(), (int)mask.element_size(), ids.numel(), (int)hidden, dtype_code(table), out.data_ptr(), reports.status, stream);
   if (rc) st.failed(stream);
   TORCH_CHECK(rc == 0, "libtdb_b200: ", tdb_last_error());
-  return py::make_tuple(out, st.finish(false, stream));
+  return py::make_tuple(out, own ? st.report(stream) : st.finish(false, stream));
 }
 
 // The valid rows of x [B, L, hidden] back to back, and each token's place in that stream (-1: padding).
@@ -1309,7 +1347,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("attn_packed_scores", &attn_packed_scores);
   m.def("expand_pair", &expand_pair);
   m.def("call_tables", &call_tables);
-  m.def("drain_pending", &drain_pending);
+  py::class_<Report>(m, "Report");
+  m.def("drain_pending", &drain_pending, py::arg("own") = py::none());
   py::class_<Watch>(m, "Watch").def(py::init<const py::list&, const py::list&>(), py::arg("modules"), py::arg("settings") = py::list()).def("holds", &Watch::holds);
   py::class_<Encoder>(m, "Encoder")
       .def(py::init<int>())
@@ -1335,7 +1374,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     c10::cuda::CUDAGuard guard(x.device());
     return tdb_gelu(x.data_ptr(), x.numel(), dtype_code(x), c10::cuda::getCurrentCUDAStream().stream());
   });
-  m.def("embed", &embed);
+  m.def("embed", &embed, py::arg("ids"), py::arg("table"), py::arg("w"), py::arg("b"), py::arg("eps"), py::arg("mask"), py::arg("own") = false);
   m.def("mask_rows", &mask_rows);
   m.def("pack_rows", &pack_rows);
   m.def("unpack_rows", &unpack_rows);

@@ -31,7 +31,7 @@ from transformers.models.deberta_v2.modeling_deberta_v2 import (
 
 from . import relpos as _relpos
 from ._cabi import host
-from .ops.flash_attention import _PENDING_STATUS, check_pending_status, flash_attention_with_disentangled
+from .ops.flash_attention import _PENDING_STATUS, _check_pending, flash_attention_with_disentangled
 from .ops.flash_attention_varlen import flash_attention_with_disentangled_varlen
 from .padding import _get_unpad_data, _upad_input, index_first_axis, pad_input
 
@@ -358,7 +358,8 @@ class FlashDebertaV2Encoder(DebertaV2Encoder):
         being captured into a CUDA graph the words stay pending (the graph's replays rewrite them) and the next
         ``check_pending_status()`` outside a capture reads them."""
         if not torch.cuda.is_current_stream_capturing():
-            check_pending_status()
+            report, _PASS.report = _PASS.report, None
+            _check_pending(report)
 
     # -- the whole layer loop in one native call -------------------------------------------------------
     def _native_layers(self):
@@ -532,6 +533,14 @@ class _Wanted(threading.local):
 
 
 _WANTED = _Wanted()
+
+
+class _Pass(threading.local):
+    """The report of the embeddings of this thread's pass, until its check: a bad id is an error of this caller's, whoever else checks."""
+    report = None
+
+
+_PASS = _Pass()
 _PLAIN_ARGUMENTS = frozenset(("input_ids", "attention_mask", "output_hidden_states", "output_attentions", "return_dict"))
 
 
@@ -586,16 +595,25 @@ class FlashDebertaV2Model(DebertaV2Model):
         table, norm = emb.word_embeddings.weight, emb.LayerNorm
         embedded = None
         if norm.weight is not None and norm.bias is not None and tuple(norm.normalized_shape) == table.shape[1:]:
-            embedded = host.embed(input_ids, table, norm.weight, norm.bias, norm.eps, attention_mask)
+            embedded = host.embed(input_ids, table, norm.weight, norm.bias, norm.eps, attention_mask, True)
+        report = None
         if embedded is not None:
-            x, words = embedded
-            if words is not None:
-                _PENDING_STATUS.append(words)
+            x, report = embedded
+            if isinstance(report, torch.Tensor) and torch.cuda.is_current_stream_capturing():       # each replay writes it: left to the next check
+                _PENDING_STATUS.append(report)
+                report = None
         else:
             x = nn.functional.embedding(input_ids, table)
             x = nn.functional.layer_norm(x, norm.normalized_shape, norm.weight, norm.bias, norm.eps)
             x.mul_(attention_mask.to(x.dtype)[..., None])
-        return self.encoder(x, attention_mask, output_hidden_states=False, output_attentions=False, return_dict=True)
+        before, _PASS.report = _PASS.report, report
+        try:
+            out = self.encoder(x, attention_mask, output_hidden_states=False, output_attentions=False, return_dict=True)
+            if _PASS.report is not None:             # an encoder that does not check
+                FlashDebertaV2Encoder._check_status_unless_capturing()
+            return out
+        finally:
+            _PASS.report = before
 
 
 def patch_model(model: nn.Module) -> nn.Module:

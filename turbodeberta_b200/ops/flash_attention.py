@@ -154,13 +154,19 @@ _PENDING_STATUS = _status.PENDING
 def check_pending_status() -> None:
     """Read (one synchronisation) the device status words of every call since the last check that was made
     with ``check_status=False`` and raise if any bounded device wait gave up or any ``cu_seqlens`` was malformed."""
-    pooled, blocks = cabi.host.drain_pending(), {}
+    _check_pending(None)
+
+
+def _check_pending(report) -> None:
+    """``check_pending_status()`` that also reads a report of the caller's own (a native ``Report``, or a tensor of words)."""
+    own = report.tolist() if isinstance(report, torch.Tensor) else ()
+    pooled, blocks = cabi.host.drain_pending() if report is None or own else cabi.host.drain_pending(report), {}
     for st in _PENDING_STATUS.drain():
         blocks.setdefault(st.device, []).append(st)
-    if pooled is None and not blocks:
+    if pooled is None and not blocks and not own:
         return
     words = [torch.stack(sts).amax(dim=0).tolist() for sts in blocks.values()]
-    _raise_for([max(w) for w in itertools.zip_longest(pooled or (0,), *words, fillvalue=0)])
+    _raise_for([max(w) for w in itertools.zip_longest(pooled or (0,), own, *words, fillvalue=0)])
 
 
 def _check_status(status: torch.Tensor):
