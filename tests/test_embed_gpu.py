@@ -140,3 +140,31 @@ def test_an_encoder_that_does_not_check_leaves_the_report_to_the_model():
         with pytest.raises(IndexError):
             model(input_ids=bad)
         assert model(input_ids=bad.clamp(max=499)).shape[:2] == (2, 20)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("ids_of", [lambda x: x, lambda x: x.t().contiguous().t(), lambda x: torch.cat([x, x], 1)[:, :20], lambda x: x.repeat_interleave(2, 1)[:, ::2],
+                                    lambda x: x.int().t().contiguous().t()], ids=["rows", "columns", "wider", "strided", "int32"])
+@pytest.mark.parametrize("mask_of", [lambda m: m, lambda m: m.t().contiguous().t(), lambda m: m.int(), lambda m: m.float(), lambda m: m.bfloat16() * 0.5, lambda m: m.bool().t().contiguous().t()],
+                         ids=["int64", "columns", "int32", "float", "halves", "bool columns"])
+def test_ids_and_masks_of_any_layout_and_type(ids_of, mask_of, dtype, monkeypatch):
+    """The same input as torch's operations form, and the same error for an id outside the vocabulary."""
+    model = _model().to(dtype)
+    ids = torch.randint(0, 500, (3, 20), device="cuda")
+    mask = (torch.arange(20, device="cuda")[None] < torch.tensor([[20], [7], [1]], device="cuda")).long()
+    seen = []
+    model.encoder.forward = lambda x, *a, **kw: seen.append(x) or x
+    with torch.no_grad():
+        emb = model.embeddings
+        want = emb.LayerNorm(emb.word_embeddings(ids)) * mask_of(mask).to(dtype)[..., None]
+
+        def refuse(*a, **kw):                        # a bad id must not get there: its assertion would end the context
+            raise AssertionError("torch's embedding")
+
+        monkeypatch.setattr(torch.nn.functional, "embedding", refuse)
+        model(input_ids=ids_of(ids), attention_mask=mask_of(mask))
+        # bf16: both round the LayerNorm's result and the product once (half a unit each way: 2^-7); fp32: ten roundings of sums
+        assert ((seen[0] - want).abs() <= (2.0 ** -7 if dtype == torch.bfloat16 else 1e-5) * want.abs() + 1e-6).all()
+        ids[2, 0] = 500
+        with pytest.raises(IndexError):
+            model(input_ids=ids_of(ids), attention_mask=mask_of(mask))

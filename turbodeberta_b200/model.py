@@ -595,7 +595,13 @@ class FlashDebertaV2Model(DebertaV2Model):
         table, norm = emb.word_embeddings.weight, emb.LayerNorm
         embedded = None
         if norm.weight is not None and norm.bias is not None and tuple(norm.normalized_shape) == table.shape[1:]:
-            embedded = host.embed(input_ids, table, norm.weight, norm.bias, norm.eps, attention_mask, True)
+            # Rows of a wider tensor, or a mask of another type, must not change what an id outside the vocabulary does: torch's own
+            # embedding ends in an assertion on the device.
+            known = attention_mask.dtype in (torch.int64, torch.bool, torch.uint8)
+            embedded = host.embed(input_ids.contiguous(), table, norm.weight, norm.bias, norm.eps,
+                                  attention_mask.contiguous() if known else torch.ones(input_ids.shape, dtype=torch.bool, device=input_ids.device), True)
+            if embedded is not None and not known:
+                embedded[0].mul_(attention_mask.to(table.dtype)[..., None])
         report = None
         if embedded is not None:
             x, report = embedded
