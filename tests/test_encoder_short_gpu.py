@@ -94,3 +94,63 @@ def test_the_one_kernel_on_several_streams_and_in_a_graph():
         check_pending_status()
         model.encoder.layer[1].output.dense.weight.mul_(1.5)
         assert not torch.equal(model(**kw).last_hidden_state, want)
+
+
+def _stack_of(tokens, hidden, layers, words, limit_ns):
+    """The arguments of tdb_short_stack for one sequence without position terms, as the library lays them out, with random weights."""
+    import ctypes as C
+
+    class Layer(C.Structure):
+        _fields_ = [("tensors", C.c_void_p * 14), ("eps1", C.c_float), ("eps2", C.c_float), ("sm_scale", C.c_float),
+                    ("exp_delta_max", C.c_int), ("exp_rows", C.c_int)]
+
+    class Stack(C.Structure):
+        _fields_ = [("layer", Layer * 48), ("n_layers", C.c_int), ("tokens", C.c_int), ("n_seqs", C.c_int), ("length", C.c_int),
+                    ("x", C.c_void_p), ("out", C.c_void_p), ("scratch", C.c_void_p * 5), ("cu_seqlens", C.c_void_p),
+                    ("status", C.c_void_p), ("counter", C.c_void_p), ("gave_up", C.c_void_p), ("limit_ns", C.c_uint64)]
+
+    def random(*shape):
+        return torch.randn(shape, device="cuda", dtype=torch.bfloat16) * 0.05
+    shapes = [(3 * hidden, hidden), (3 * hidden,), (hidden, hidden), (hidden,), (hidden,), (hidden,), (4 * hidden, hidden), (4 * hidden,),
+              (hidden, 4 * hidden), (hidden,), (hidden,), (hidden,)]                  # q/k/v, output, norm, up, down, norm
+    p, keep = Stack(), []
+    torch.manual_seed(5)
+    for i in range(layers):
+        w = [random(*s) for s in shapes]
+        keep += w
+        p.layer[i] = Layer((C.c_void_p * 14)(*[t.data_ptr() for t in w]), 1e-7, 1e-7, 0.07, 0, 0)
+    x, out = random(tokens, hidden), torch.zeros(tokens, hidden, device="cuda", dtype=torch.bfloat16)
+    scratch = [torch.zeros(tokens, n * hidden, device="cuda", dtype=torch.bfloat16) for n in (3, 1, 1, 4, 1)]
+    p.n_layers, p.tokens, p.n_seqs, p.length, p.limit_ns = layers, tokens, 1, tokens, limit_ns
+    p.x, p.out, p.scratch = x.data_ptr(), out.data_ptr(), (C.c_void_p * 5)(*[t.data_ptr() for t in scratch])
+    p.status, p.counter, p.gave_up = words.data_ptr(), words.data_ptr() + 16, words.data_ptr() + 20       # as a call's own words lie
+    return p, out, keep + [x] + scratch
+
+
+@pytest.mark.parametrize("tokens", [16, 32])
+@pytest.mark.parametrize("hidden", [512, 768, 1024])
+def test_a_meeting_that_nobody_completes_is_given_up(hidden, tokens):
+    """The counter begins one short, so the first meeting's limit of 5 ms runs out: every block leaves, the code is reported, and with the
+    words cleared the next pass on them is right."""
+    import ctypes as C
+    import time
+    from turbodeberta_b200 import _cabi as cabi
+    words = torch.zeros(8, dtype=torch.int32, device="cuda")
+    p, out, keep = _stack_of(tokens, hidden, 2, words, 5_000_000)
+
+    def run():
+        cabi.check(cabi.lib.tdb_short_stack(C.byref(p), hidden, C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+        torch.cuda.synchronize()
+    run()
+    want = out.clone()
+    assert words.tolist() == [0] * 8 and torch.isfinite(want.float()).all() and torch.count_nonzero(want).item() > 0
+    out.zero_()
+    words[4] = -1
+    torch.cuda.synchronize()
+    t0 = time.time()
+    run()
+    assert time.time() - t0 < 0.5
+    assert words[0].item() == 302 and words[5].item() == 1 and torch.count_nonzero(out).item() == 0
+    words.zero_()
+    run()
+    assert words.tolist() == [0] * 8 and torch.equal(out, want)

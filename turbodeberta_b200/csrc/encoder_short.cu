@@ -44,7 +44,6 @@ constexpr int KS = 8;                                // warps that share a produ
 constexpr int TT = SKINNY_TOKENS;                    // tokens at most, and rows of an attention tile
 constexpr int TB = 52;                               // pitch of a band row in floats (48 distances)
 constexpr uint32_t ATT_BYTES = 3 * TT * SP * 2 + 2 * TT * TB * 4, TAB_BYTES = 2 * 2 * TT * SP * 2;
-constexpr uint64_t MEET_NS = 1000ull * 1000ull * 1000ull;
 
 // Rows in shared memory are 64 bytes longer than a multiple of 128, so that the 16-byte loads of two rows by four lanes each
 // fall on different banks.
@@ -82,11 +81,11 @@ __device__ __forceinline__ void warp_sums(float* x) {          // of two values
   }
 }
 // Out of line, like the LayerNorm: the kernel's code runs once per layer, so what is not in it need not be fetched again.
-__device__ __noinline__ void wait_longer(uint32_t bar, uint32_t phase, volatile int* abort_flag, int32_t* status) {
-  mbar_wait(bar, phase, abort_flag, status, 301, MEET_NS);
+__device__ __noinline__ bool wait_longer(uint32_t bar, uint32_t phase, volatile int* abort_flag, int32_t* status, uint64_t limit_ns) {
+  return mbar_wait(bar, phase, abort_flag, status, 301, limit_ns);
 }
-// Until the counter has come to `expected`; gives up with the others, or after a second.
-__device__ __noinline__ void meet_others(int32_t* counter, int expected, int32_t* gave_up, int32_t* status, volatile int* abort_flag) {
+// Until the counter has come to `expected`; gives up with the others, or after the limit.
+__device__ __noinline__ void meet_others(int32_t* counter, int expected, int32_t* gave_up, int32_t* status, volatile int* abort_flag, uint64_t limit_ns) {
   const uint64_t t0 = globaltimer_ns();
 #pragma unroll 1
   for (int i = 1;; ++i) {
@@ -94,7 +93,7 @@ __device__ __noinline__ void meet_others(int32_t* counter, int expected, int32_t
     asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(now) : "l"(counter) : "memory");
     if (now >= expected) return;
     if (i % 64) continue;
-    const bool late = globaltimer_ns() - t0 > MEET_NS;
+    const bool late = globaltimer_ns() - t0 > limit_ns;
     if (!late && *reinterpret_cast<volatile int32_t*>(gave_up) == 0) continue;
     *abort_flag = 1;
     if (late) {
@@ -303,35 +302,42 @@ __global__ void __launch_bounds__(MT * KS * 32, 1) short_stack_kernel(const __gr
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid / 32, 0), lane = tid % 32, g = lane / 4, t = lane % 4;
   const int ks = warp % KS, mt = warp / KS, block = blockIdx.x, blocks = gridDim.x;
   const uint32_t base = smem_u32(smem), sX = base + P::OFF_X, sA = base + P::OFF_A, sB = base + P::OFF_B, sN = base + P::OFF_N;
-  const uint32_t barA = base + P::OFF_BAR, barB = barA + 8, barN = barA + 16;
+  enum { A, B, N, BARS };                            // the barrier of each buffer that bulk copies go to
+  const uint32_t bars = base + P::OFF_BAR;
 
   if (tid == 0) {
     s_abort = 0;
-    mbar_init(barA, 1); mbar_init(barB, 1); mbar_init(barN, 1);
+    for (int i = 0; i < BARS; ++i) mbar_init(bars + 8u * i, 1);
     fence_mbar_init();
   }
   __syncthreads();
   // This block's rows of a weight matrix to shared memory (by the first warp, a row per lane; whoever read or wrote the buffer is
   // behind a barrier).
-  auto bring = [&](uint32_t dst, uint32_t pitch, uint32_t bar, int rows, uint32_t bytes, const bf16* mine) {
-    if (warp != 0) return;
+  uint32_t phase[BARS] = {}, late = 0;               // late: a bit for each barrier whose wait was given up
+  auto bring = [&](uint32_t dst, uint32_t pitch, int i, int rows, uint32_t bytes, const bf16* mine) {
+    const uint32_t bar = bars + 8u * i;
+    if (warp != 0 || (late >> i & 1u)) return;
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     if (lane == 0) mbar_expect_tx(bar, (uint32_t)rows * bytes);
     __syncwarp();
     if (lane < rows) bulk_load(dst + (uint32_t)lane * pitch, mine, bytes, bar);
   };
   auto bring_qkv = [&](const ShortLayer& l) {
-    bring(sA, P::PITCH, barA, 24, 2 * H, l.qkv_w + ((int64_t)(lane >> 3) * H + 8 * block + (lane & 7)) * H);
+    bring(sA, P::PITCH, A, 24, 2 * H, l.qkv_w + ((int64_t)(lane >> 3) * H + 8 * block + (lane & 7)) * H);
   };
-  auto bring_up = [&](const ShortLayer& l) { bring(sA, P::PITCH, barA, 32, 2 * H, l.up_w + (int64_t)(32 * block + lane) * H); };
-  auto bring_out = [&](const ShortLayer& l) { bring(sB, P::PITCH, barB, 8, 2 * H, l.out_w + (int64_t)(8 * block + (lane & 7)) * H); };
-  auto bring_down = [&](const ShortLayer& l) { bring(sB, P::PITCH4, barB, 8, 8 * H, l.down_w + (int64_t)(8 * block + (lane & 7)) * 4 * H); };
-  auto bring_norm = [&](const bf16* w, const bf16* b) { bring(sN, 2 * H, barN, 2, 2 * H, lane ? b : w); };
-  uint32_t phase_a = 0, phase_b = 0, phase_n = 0;
-  auto landed = [&](uint32_t bar, uint32_t& phase) {
-    if (__any_sync(0xffffffffu, !mbar_try_wait(bar, phase))) wait_longer(bar, phase, &s_abort, p.status);
+  auto bring_up = [&](const ShortLayer& l) { bring(sA, P::PITCH, A, 32, 2 * H, l.up_w + (int64_t)(32 * block + lane) * H); };
+  auto bring_out = [&](const ShortLayer& l) { bring(sB, P::PITCH, B, 8, 2 * H, l.out_w + (int64_t)(8 * block + (lane & 7)) * H); };
+  auto bring_down = [&](const ShortLayer& l) { bring(sB, P::PITCH4, B, 8, 8 * H, l.down_w + (int64_t)(8 * block + (lane & 7)) * 4 * H); };
+  auto bring_norm = [&](const bf16* w, const bf16* b) { bring(sN, 2 * H, N, 2, 2 * H, lane ? b : w); };
+  auto landed = [&](int i) {
+    const uint32_t bar = bars + 8u * i;
+    if (__any_sync(0xffffffffu, !mbar_try_wait(bar, phase[i])) &&
+        __any_sync(0xffffffffu, !wait_longer(bar, phase[i], &s_abort, p.status, p.limit_ns))) {
+      late |= 1u << i;
+      phase[i] ^= 1;                                 // the copy's phase is still the one to wait for
+    }
     __syncwarp();
-    phase ^= 1;
+    phase[i] ^= 1;
   };
 
   // The blocks' meeting: everything written before an arrival is there after a wait for it.
@@ -344,7 +350,7 @@ __global__ void __launch_bounds__(MT * KS * 32, 1) short_stack_kernel(const __gr
     }
   };
   auto meet = [&]() {                                // false: somebody gave up
-    if (warp == 0) meet_others(p.counter, expected, p.gave_up, p.status, &s_abort);       // all its lanes, so that it stays in step
+    if (warp == 0) meet_others(p.counter, expected, p.gave_up, p.status, &s_abort, p.limit_ns);       // all its lanes, so that it stays in step
     __syncwarp();
     __syncthreads();
     return !__any_sync(0xffffffffu, *reinterpret_cast<volatile int*>(&s_abort));
@@ -436,7 +442,7 @@ __global__ void __launch_bounds__(MT * KS * 32, 1) short_stack_kernel(const __gr
   }
   auto from_x = [&](int r, int b) { return ld16s(sX + (uint32_t)(16 * mt + g + 8 * r) * P::PITCH + 64u * (uint32_t)b + 16u * (uint32_t)t); };
   auto normalise = [&](const bf16* s, float eps) {
-    landed(barN, phase_n);
+    landed(N);
     const int row = (warp + block) % (MT * KS);
     if (row < p.tokens) norm_rows<NB>(s, row, MT * KS, p.tokens, sX, P::PITCH, sN, sN + 2 * H, eps);
     __syncthreads();
@@ -450,6 +456,7 @@ __global__ void __launch_bounds__(MT * KS * 32, 1) short_stack_kernel(const __gr
   auto from_l2 = [&](int r, int b) { return ld16g(rows_of[r] + 32 * b); };
 
   bool good = true;
+  uint32_t due = 0;                                  // the barriers whose copies are on their way when the block gives up
   float acc[4][4];
   uint32_t bias = bias_of(p.layer[0].qkv_b + 8 * block, 12, H);
   __syncthreads();
@@ -458,7 +465,7 @@ __global__ void __launch_bounds__(MT * KS * 32, 1) short_stack_kernel(const __gr
     const bool last = i + 1 == p.n_layers;
     // 1: q, k, v
     if (i > 0) normalise(p.z, p.layer[i - 1].eps2);
-    landed(barA, phase_a);
+    landed(A);
     product(three, narrow, sA, P::PITCH, from_x, acc);
     finish(three, sA, acc, bias,
            [&](int row, int c, float a, float b) { put(p.qkv + (int64_t)row * 3 * H + (c >> 3) * H + 8 * block + (c & 7), a, b); });
@@ -467,7 +474,7 @@ __global__ void __launch_bounds__(MT * KS * 32, 1) short_stack_kernel(const __gr
     bias = bias_of(l.out_b + 8 * block, 4, 0);
     // 2: attention
     if (block < takers) {
-      if (!(good = meet())) break;
+      if (!(good = meet())) { due = 1 << B; break; }
       for (int pair = block; pair < pairs; pair += blocks) {
         const int seq = pair / (H / 64), h = pair - seq * (H / 64);
         int tok0 = seq * p.length, len = p.length;
@@ -485,10 +492,10 @@ __global__ void __launch_bounds__(MT * KS * 32, 1) short_stack_kernel(const __gr
     }
     expected += takers;
     bring_up(l);
-    if (!(good = meet())) break;
+    if (!(good = meet())) { due = 1 << A | 1 << B; break; }
     // 3: output projection
     activations(p.ctx, H);
-    landed(barB, phase_b);
+    landed(B);
     product(one, narrow, sB, P::PITCH, from_l2, acc);
     finish(one, sB, acc, bias,
            [&](int row, int c, float a, float b) { put(p.y + (int64_t)row * H + 8 * block + c, a, b); });
@@ -497,10 +504,10 @@ __global__ void __launch_bounds__(MT * KS * 32, 1) short_stack_kernel(const __gr
     bring_down(l);
     bring_norm(l.ln1_w, l.ln1_b);
     bias = bias_of(l.up_b + 32 * block, 16, 8);
-    if (!(good = meet())) break;
+    if (!(good = meet())) { due = 1 << A | 1 << B | 1 << N; break; }
     // 4: intermediate projection
     normalise(p.y, l.eps1);
-    landed(barA, phase_a);
+    landed(A);
     product(four, narrow, sA, P::PITCH, from_x, acc);
     finish(four, sA, acc, bias,
            [&](int row, int c, float a, float b) { put(p.u + (int64_t)row * 4 * H + 32 * block + c, gelu(a, bf16()), gelu(b, bf16())); });
@@ -508,10 +515,10 @@ __global__ void __launch_bounds__(MT * KS * 32, 1) short_stack_kernel(const __gr
     expected += blocks;
     if (!last) bring_qkv(p.layer[i + 1]);
     bias = bias_of(l.down_b + 8 * block, 4, 0);
-    if (!(good = meet())) break;
+    if (!(good = meet())) { due = (last ? 0 : 1 << A) | 1 << B; break; }
     // 5: second projection
     activations(p.u, 4 * H);
-    landed(barB, phase_b);
+    landed(B);
     product(one, wide, sB, P::PITCH4, from_l2, acc);
     finish(one, sB, acc, bias, [&](int row, int c, float a, float b) { put(p.z + (int64_t)row * H + 8 * block + c, a, b); });
     arrive();
@@ -520,10 +527,10 @@ __global__ void __launch_bounds__(MT * KS * 32, 1) short_stack_kernel(const __gr
     bring_norm(l.ln2_w, l.ln2_b);
     if (!last) bias = bias_of(p.layer[i + 1].qkv_b + 8 * block, 12, H);
     if (!last && block < takers) copy_tables(tables, p.layer[i + 1], block % (H / 64));
-    if (!(good = meet())) break;
+    if (!(good = meet())) { due = (last ? 0 : 1 << A | 1 << B) | 1 << N; break; }
   }
   if (good) {                                        // the last layer's LayerNorm: a row per block
-    landed(barN, phase_n);
+    landed(N);
     if (warp == 0 && block < p.tokens) {
       norm_rows<NB>(p.z, block, p.tokens, p.tokens, sX, P::PITCH, sN, sN + 2 * H, p.layer[p.n_layers - 1].eps2);
       __syncwarp();
@@ -533,9 +540,15 @@ __global__ void __launch_bounds__(MT * KS * 32, 1) short_stack_kernel(const __gr
     // the last block to leave puts the counters back to zero: all have left their last meeting
     if (tid == 0 && atomicInc(reinterpret_cast<unsigned int*>(p.counter + 3), (unsigned int)(blocks - 1)) == (unsigned int)(blocks - 1))
       *reinterpret_cast<volatile int32_t*>(p.counter) = 0;
-  } else {                                           // copies that may still be in flight: time to land
-    const uint64_t t0 = globaltimer_ns();
-    while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
+  }
+  if (!good || late) {                               // copies that are still on their way come in before the block's memory is another's
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    if (tid == 0)
+#pragma unroll
+      for (int i = 0; i < BARS; ++i) {
+        const uint64_t t0 = globaltimer_ns();
+        while (((due | late) >> i & 1u) && !mbar_try_wait_parked(bars + 8u * i, phase[i], 20000u) && globaltimer_ns() - t0 < p.limit_ns) {}
+      }
   }
 }
 

@@ -1000,6 +1000,7 @@ class Encoder {
     tdb::AttnParams reports{};
     Status st(x.get_device(), reports);
     p.status = reports.status; p.counter = reports.counter; p.gave_up = reports.gave_up;
+    p.limit_ns = 1000ull * 1000ull * 1000ull;
     if (tdb_short_stack(&p, (int)hidden, stream.stream())) {      // not all of its blocks can be resident here
       st.failed(stream.stream());
       return {};

@@ -118,6 +118,7 @@ struct ShortStack {
   __nv_bfloat16 *out, *qkv, *ctx, *y, *u, *z;
   const int32_t* cu_seqlens;
   int32_t *status, *counter, *gave_up;                // as in AttnParams; counter[0] and counter[3] are zero on entry and again at the end
+  uint64_t limit_ns;                                  // of a wait, after which the kernel gives up
 };
 }  // namespace tdb
 
