@@ -154,3 +154,29 @@ def test_a_meeting_that_nobody_completes_is_given_up(hidden, tokens):
     words.zero_()
     run()
     assert words.tolist() == [0] * 8 and torch.equal(out, want)
+
+
+def test_a_launch_that_fails_is_reported_once():
+    """What a refused launch leaves behind is not the next kernel's error.  (The launch takes its grid from the feature count: 0 is refused on
+    the host.)  A capture that has become invalid refuses the whole-stack kernel, which is not the answer of a device that is too small."""
+    import ctypes as C
+    from turbodeberta_b200 import _cabi as cabi
+    rt = C.CDLL("libcudart.so.12")                    # the one that torch has loaded
+    words = torch.zeros(8, dtype=torch.int32, device="cuda")
+    p, out, keep = _stack_of(16, 512, 1, words, 5_000_000)
+    idx = torch.full((513,), -1, device="cuda", dtype=torch.int16)
+    torch.cuda.synchronize()
+    current = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    where = C.c_void_p(out.data_ptr())
+    assert cabi.lib.tdb_skinny(where, where, where, 16, 512, 0, 0, 0, where, current) == cabi.ERR_CUDA
+    assert cabi.lib.tdb_bucket_table(0, 256, 256, cabi.ptr(idx), current) == 0
+    stream, graph = C.c_void_p(), C.c_void_p()
+    assert rt.cudaStreamCreateWithFlags(C.byref(stream), 1) == 0
+    assert rt.cudaStreamBeginCapture(stream, 2) == 0              # relaxed
+    assert rt.cudaStreamSynchronize(stream) != 0                  # not allowed in a capture, which ends it
+    assert cabi.lib.tdb_short_stack(C.byref(p), 512, stream) == cabi.ERR_CUDA
+    assert rt.cudaStreamEndCapture(stream, C.byref(graph)) != 0 and not graph.value
+    rt.cudaGetLastError()
+    assert rt.cudaStreamDestroy(stream) == 0
+    torch.cuda.synchronize()
+    assert (idx >= 0).all() and torch.count_nonzero(out).item() == 0

@@ -563,7 +563,27 @@ int launch_short(const ShortStack& p, cudaStream_t s) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(32 * NB); cfg.blockDim = dim3(Plan<MT, NB>::THREADS); cfg.dynamicSmemBytes = Plan<MT, NB>::SMEM; cfg.stream = s;
   cfg.attrs = &attr; cfg.numAttrs = 1;
-  return cuda_fail(cudaLaunchKernelEx(&cfg, kern, p), "short stack launch");
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, p);
+  const int failed = cuda_fail(e, "short stack launch");
+  return e == cudaErrorCooperativeLaunchTooLarge ? TDB_ERR_UNSUPPORTED : failed;
+}
+
+// Whether all blocks can be resident at once on the current device; asked once per device.
+template <int MT, int NB>
+bool resident() {
+  constexpr int MAX_DEV = 64;
+  static int known[MAX_DEV] = {};                    // 1: they can, 2: they cannot; same value from every thread
+  int dev = 0, sms = 0, cooperative = 0, per_sm = 0;
+  if (cuda_fail(cudaGetDevice(&dev), "cudaGetDevice")) return false;
+  if (dev < MAX_DEV && known[dev]) return known[dev] == 1;
+  auto kern = short_stack_kernel<MT, NB>;
+  if (device_sms(&sms) || opt_in_smem(reinterpret_cast<const void*>(kern), (int)Plan<MT, NB>::SMEM) ||
+      cuda_fail(cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, dev), "cudaDeviceGetAttribute") ||
+      cuda_fail(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, Plan<MT, NB>::THREADS, Plan<MT, NB>::SMEM), "occupancy of the short stack"))
+    return false;
+  const bool fits = cooperative && per_sm * sms >= 32 * NB;
+  if (dev < MAX_DEV) known[dev] = fits ? 1 : 2;
+  return fits;
 }
 
 }  // namespace
@@ -576,10 +596,12 @@ extern "C" {
 
 // Hidden sizes whose columns the eight warps can share in whole blocks of 32, with a block per eight columns resident at once.
 int tdb_short_stack_applies(int64_t tokens, int64_t hidden, int64_t inner, int64_t layers) {
-  int sms = 0;
   if (tokens < 1 || tokens > SKINNY_TOKENS || layers < 1 || layers > SHORT_LAYERS || inner != 4 * hidden) return 0;
-  if (hidden != 512 && hidden != 768 && hidden != 1024) return 0;
-  return device_sms(&sms) == 0 && hidden / 8 <= sms;
+  const bool one = tokens <= 16;
+  if (hidden == 512) return one ? resident<1, 2>() : resident<2, 2>();
+  if (hidden == 768) return one ? resident<1, 3>() : resident<2, 3>();
+  if (hidden == 1024) return one ? resident<1, 4>() : resident<2, 4>();
+  return 0;
 }
 
 int tdb_short_stack(const ShortStack* p, int hidden, void* stream) {

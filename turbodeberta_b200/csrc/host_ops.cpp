@@ -1001,9 +1001,10 @@ class Encoder {
     Status st(x.get_device(), reports);
     p.status = reports.status; p.counter = reports.counter; p.gave_up = reports.gave_up;
     p.limit_ns = 1000ull * 1000ull * 1000ull;
-    if (tdb_short_stack(&p, (int)hidden, stream.stream())) {      // not all of its blocks can be resident here
+    if (const int rc = tdb_short_stack(&p, (int)hidden, stream.stream())) {
       st.failed(stream.stream());
-      return {};
+      if (rc == TDB_ERR_UNSUPPORTED) return {};      // a part of the device that is too small for all of its blocks
+      ok(rc);
     }
     st.defer(stream, words);
     return y;

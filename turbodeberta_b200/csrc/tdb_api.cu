@@ -19,6 +19,7 @@ void set_error(const char* fmt, ...) {
 int cuda_fail(cudaError_t e, const char* what) {
   if (e == cudaSuccess) return TDB_OK;
   set_error("%s: %s", what, cudaGetErrorString(e));
+  (void)cudaGetLastError();                        // this library's runtime would report it again, to the next launch
   return TDB_ERR_CUDA;
 }
 

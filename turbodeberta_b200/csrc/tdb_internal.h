@@ -146,7 +146,8 @@ TDB_HOST_API int tdb_gelu(void* x, int64_t elements, int dtype, void* stream);
 // then must not be what wrote W (W is read before the wait for it).
 TDB_HOST_API int tdb_skinny_applies(int64_t T, int64_t K, int64_t N);
 TDB_HOST_API int tdb_skinny(const void* x, const void* w, const void* b, int T, int K, int N, int gelu, int early, void* y, void* stream);
-// All layers for at most SKINNY_TOKENS tokens in one kernel whose blocks wait for one another.
+// All layers for at most SKINNY_TOKENS tokens in one kernel whose blocks wait for one another.  TDB_ERR_UNSUPPORTED: not all of them can be
+// resident where the stream may run.
 TDB_HOST_API int tdb_short_stack_applies(int64_t tokens, int64_t hidden, int64_t inner, int64_t layers);
 TDB_HOST_API int tdb_short_stack(const tdb::ShortStack* p, int hidden, void* stream);
 TDB_HOST_API int tdb_mask_rows(const void* mask, int elem_bytes, int B, int L, int32_t* seqlens, int32_t* cu, int32_t* ticket,
