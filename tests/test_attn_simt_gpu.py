@@ -169,3 +169,21 @@ def test_pairs_of_warps_share_the_key_tiles(lengths, padded, heads, c2p, p2c, dt
     util.assert_close(o, ref, dtype, f"{lengths} c2p={c2p} p2c={p2c}")
     for b, n in enumerate(lengths):
         assert torch.count_nonzero(o[b, n:]).item() == 0
+
+
+def test_a_calls_own_tables_are_not_expanded_for_the_exact_kernel():
+    """It reads them by index in either type: the call allocates its output, not the tensor-core kernels' copies of the tables (0.8 MB here)."""
+    from turbodeberta_b200.ops.flash_attention import flash_attention_with_disentangled
+    w = workloads.make_attention_workload("own", seed=23, hidden_size=128, num_heads=2, lengths=[40], padded_len=40, dtype=torch.bfloat16)
+    q, k, v, rel, P = util.device_inputs(w, torch.bfloat16)
+    t = util.make_tables(w, rel, P)
+    q, k, v = (x.permute(0, 2, 1, 3) for x in (q, k, v))
+    run = lambda **kw: flash_attention_with_disentangled(q, k, v, kw.pop("q_pos", None), kw.pop("k_pos", None), False, 0.07, w.position_buckets,
+                                                         w.max_relative_positions, kernel=SIMT, **kw)
+    run(q_pos=t.kr, k_pos=t.qr)
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    got = run(q_pos=t.kr, k_pos=t.qr)
+    assert torch.cuda.max_memory_allocated() - before < 100_000
+    assert torch.equal(got, run(tables=t))

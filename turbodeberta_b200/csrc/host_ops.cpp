@@ -403,9 +403,10 @@ Tensor expand_both(const OptTensor& kr, const OptTensor& qr, const Tensor& idx, 
   if (rc) throw std::runtime_error(std::string("libtdb_b200: ") + tdb_last_error());
   return both;
 }
-// Tables of one call are expanded only for a kernel that reads them so.  Returns the expanded ones, for p to point into.
+// Tables of one call are expanded only for a kernel that reads them so (the CUDA-core kernel does not, in either type).  Returns the
+// expanded ones, for p to point into.
 Tensor expand_for(tdb::AttnParams& p, const Tables* tables, int dtype, int kernel) {
-  if (!tables || !tables->one_call || dtype != TDB_DTYPE_BF16) return {};
+  if (!tables || !tables->one_call || dtype != TDB_DTYPE_BF16 || kernel == TDB_KERNEL_SIMT) return {};
   p.direct_tables = tdb_takes_direct_tables(&p, dtype, kernel);
   if (p.direct_tables) return {};
   const Tensor both = expand_both(tables->kr, tables->qr, *tables->idx, tables->exp_delta_max);
