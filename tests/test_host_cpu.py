@@ -184,6 +184,16 @@ def test_mask_analysis_refresh_recomputes_lengths_without_changing_the_route():
     assert analyse_mask(m, 2, 6) is b                      # the refreshed analysis is what later calls see
 
 
+def test_mask_analysis_after_the_native_one_has_the_validity_too():
+    """The native analysis of a mask of ones keeps what the encoder needs of it; whoever asks for the rest afterwards gets it."""
+    from turbodeberta_b200 import model as M
+    m = torch.ones(2, 6, dtype=torch.long)
+    M._mask_cache_put(m, M.MaskInfo(True, True, torch.tensor([6, 6], dtype=torch.int32), None, (12, 6, None)))
+    info = M.analyse_mask(m, 2, 6)
+    assert info.all_ones and info.right_padded and info.seqlens.tolist() == [6, 6] and torch.equal(info.key_mask, m != 0)
+    assert M.analyse_mask(m, 2, 6) is info
+
+
 def _small_config(**kw):
     from transformers import DebertaV2Config
     return DebertaV2Config(**{**dict(vocab_size=50, hidden_size=128, num_hidden_layers=4, num_attention_heads=2,

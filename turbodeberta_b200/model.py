@@ -92,7 +92,7 @@ def analyse_mask(attention_mask: torch.Tensor | None, batch: int, length: int, r
     if hit is not None:
         ref, version, cached = hit
         if ref() is attention_mask and version == attention_mask._version:     # same live tensor object, unmodified
-            if not refresh:
+            if not refresh and cached.key_mask is not None:            # the native analysis leaves it out
                 return cached
             flags = (cached.all_ones, cached.right_padded)
     m = attention_mask
