@@ -168,3 +168,32 @@ def test_ids_and_masks_of_any_layout_and_type(ids_of, mask_of, dtype, monkeypatc
         ids[2, 0] = 500
         with pytest.raises(IndexError):
             model(input_ids=ids_of(ids), attention_mask=mask_of(mask))
+
+
+class _Halves(torch.Tensor):
+    """A tensor that holds half of its values: it has no memory of its own for a kernel to read."""
+    @staticmethod
+    def __new__(cls, inner):
+        return torch.Tensor._make_wrapper_subclass(cls, inner.shape, dtype=inner.dtype, device=inner.device)
+
+    def __init__(self, inner):
+        self.inner = inner
+
+    @classmethod
+    def __torch_dispatch__(cls, func, types, args=(), kwargs=None):
+        if func is torch.ops.aten.detach.default:
+            return cls(args[0].inner)
+        return func(*[a.inner * 2 if isinstance(a, cls) else a for a in args], **(kwargs or {}))
+
+
+def test_a_table_of_another_tensor_class_is_left_to_torch(monkeypatch):
+    from turbodeberta_b200 import model as M
+    model = _model()
+    ids = torch.randint(0, 500, (2, 20), device="cuda")
+    with torch.no_grad():
+        want = model(input_ids=ids).last_hidden_state.float()
+        words = model.embeddings.word_embeddings
+        words.weight = torch.nn.Parameter(_Halves(words.weight.detach() / 2), requires_grad=False)
+        monkeypatch.setattr(M.host, "embed", lambda *a: pytest.fail("not a tensor that the kernel can read"))
+        got = model(input_ids=ids).last_hidden_state.float()
+    assert ((got - want).norm() / want.norm()).item() < 1e-2         # the two routes round the same tensors to bf16

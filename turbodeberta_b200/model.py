@@ -541,6 +541,7 @@ class _Pass(threading.local):
 
 
 _PASS = _Pass()
+_PLAIN_TENSORS = frozenset((torch.Tensor, nn.Parameter))      # other classes may keep their values elsewhere (quantised, sharded)
 _PLAIN_ARGUMENTS = frozenset(("input_ids", "attention_mask", "output_hidden_states", "output_attentions", "return_dict"))
 
 
@@ -594,7 +595,8 @@ class FlashDebertaV2Model(DebertaV2Model):
             attention_mask = torch.ones(input_ids.shape, dtype=torch.long, device=input_ids.device)
         table, norm = emb.word_embeddings.weight, emb.LayerNorm
         embedded = None
-        if norm.weight is not None and norm.bias is not None and tuple(norm.normalized_shape) == table.shape[1:]:
+        if (norm.weight is not None and norm.bias is not None and tuple(norm.normalized_shape) == table.shape[1:]
+                and all(type(t) in _PLAIN_TENSORS for t in (input_ids, attention_mask, table, norm.weight, norm.bias))):
             # Rows of a wider tensor, or a mask of another type, must not change what an id outside the vocabulary does: torch's own
             # embedding ends in an assertion on the device.
             known = attention_mask.dtype in (torch.int64, torch.bool, torch.uint8)
