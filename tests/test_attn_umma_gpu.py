@@ -96,15 +96,23 @@ def test_umma_varlen():
     assert torch.equal(o, o3)
 
 
-def test_umma_bad_cu_seqlens_reported():
+@pytest.mark.parametrize("n_seqs,max_seqlen", [(2, 64), (300, 64), (2, 1280)])      # listed by each CTA; by a kernel, for their number and for their length
+@pytest.mark.parametrize("change", ["a negative length", "past the end", "a negative offset", "too few"])
+def test_umma_bad_cu_seqlens_reported(n_seqs, max_seqlen, change):
+    """Whichever side lists the tiles: a sequence that does not lie in the stream is dropped and reported."""
     from turbodeberta_b200.ops.flash_attention_varlen import flash_attention_with_disentangled_varlen
-    w = _wl([64, 64], None)
+    lengths = [max_seqlen] + [2] * (n_seqs - 1)
+    w = _wl([sum(lengths)], None)
     q, k, v, rel, P = util.device_inputs(w, DT)
     tables = util.make_tables(w, rel, P)
-    cu = torch.tensor([0, 80, 64], dtype=torch.int32, device="cuda")
+    cu = torch.tensor([0] + lengths, dtype=torch.int32).cumsum(0, dtype=torch.int32)
+    run = lambda: flash_attention_with_disentangled_varlen(q, k, v, None, None, cu.cuda(), cu.cuda(), max_seqlen, max_seqlen, False, 0.07, 256, 512,
+                                                           tables=tables, kernel=UMMA)
+    assert torch.isfinite(run()).all()
+    at, value = {"a negative length": (1, cu[2] + 1), "past the end": (1, cu[-1] + 5), "a negative offset": (0, -3), "too few": (-1, cu[-1] - 1)}[change]
+    cu[at] = value
     with pytest.raises(ValueError):
-        flash_attention_with_disentangled_varlen(q, k, v, None, None, cu, cu, 64, 64, False, 0.07, 256, 512,
-                                                 tables=tables, kernel=UMMA)
+        run()
 
 
 def test_empty_and_degenerate_inputs():
