@@ -187,3 +187,32 @@ def test_a_calls_own_tables_are_not_expanded_for_the_exact_kernel():
     got = run(q_pos=t.kr, k_pos=t.qr)
     assert torch.cuda.max_memory_allocated() - before < 100_000
     assert torch.equal(got, run(tables=t))
+
+
+@pytest.mark.parametrize("form", ["tables", "content", "scores"])
+@pytest.mark.parametrize("ragged", [False, True])
+@pytest.mark.parametrize("batch,length", [(3, 192), (4, 192), (4, 129), (9, 65), (12, 128), (4, 300), (3, 449), (14, 128), (27, 128), (14, 256), (40, 65)])
+def test_both_sides_of_the_rule_for_rows_and_pairs(batch, length, ragged, form):
+    """Around the lines between 16 and 32 rows and between one and two pairs of warps (148 SMs, 12 heads): every block's rows, against torch in float64."""
+    from turbodeberta_b200.ops.flash_attention import flash_attention_with_disentangled
+    g = torch.Generator(device="cuda").manual_seed(37)
+    q, k, v = (torch.randn(batch, 12, length, 64, generator=g, device="cuda") for _ in range(3))
+    lens = torch.randint(1, length + 1, (batch,), generator=g, device="cuda", dtype=torch.int32) if ragged else None
+    kr, qr = (torch.randn(12, 64, 64, generator=g, device="cuda") for _ in range(2))
+    at = torch.arange(length, device="cuda")
+    row = (at[:, None] - at[None, :] + 32).clamp(0, 63)                      # of query i and key j, without buckets
+    pos, both = None, None
+    if form != "content":
+        c = torch.einsum("bhid,hrd->bhir", q.double(), kr.double()).float()
+        p = torch.einsum("bhjd,hrd->bhjr", k.double(), qr.double()).float()
+        pos = c.double().gather(-1, row.expand(batch, 12, -1, -1)) + p.double().gather(-1, row.t().expand(batch, 12, -1, -1)).transpose(-1, -2)
+        both = (kr, qr) if form == "tables" else (c, p)
+    got = flash_attention_with_disentangled(q, k, v, *(both or (None, None)), False, 0.07, 0, 32, seqlens=lens)
+    s = torch.einsum("bhid,bhjd->bhij", q.double(), k.double())
+    s = (s if pos is None else s + pos) * 0.07
+    if ragged:
+        s.masked_fill_(at >= lens[:, None, None, None], float("-inf"))
+    want = torch.einsum("bhij,bhjd->bhid", s.softmax(-1), v.double())
+    if ragged:
+        want.masked_fill_((at >= lens[:, None])[:, None, :, None], 0.0)
+    assert ((got.double() - want).norm() / want.norm()).item() < 1e-6            # fp32 sums: some 2e-7

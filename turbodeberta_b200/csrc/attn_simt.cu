@@ -373,25 +373,43 @@ int launch_rows(const AttnParams& p, cudaStream_t s) {
   //   batch x length    blocks of 32 per SM    16 x 4    32 x 4    32 x 2    32 x 1    16 x 1
   //   1 x 128           0.3                      28.2      31.9      32.0      44.0      36.6
   //   1 x 256           0.6                      47.1      37.0      42.3      65.6      54.3
-  //   2 x 200           1.1                      63.0      58.2      55.7      66.4      64.5
-  //   4 x 512 ragged    5.2                     122.6      99.2      96.7     121.4     115.5
+  //   2 x 256           1.3                      63.3      59.0      55.5      66.8      65.8
+  //   3 x 192           1.5                      57.7      56.1      55.2      54.4      53.3
+  //   4 x 256           2.6                     110.7      81.8      80.2      92.0     108.1
+  //   4 x 300           3.2                     185.8     151.8     131.1     112.5     149.2
+  //   6 x 256           3.9                     143.9     104.4      96.4      94.2     125.7
   //   16 x 128          5.2                     131.2     102.1      77.9      79.4      98.7
-  //   8 x 512           10.4                    649.2     468.7     440.9     470.6     615.0
-  // With every SM full, an odd tile leaves the second pair waiting, which is one pair's time lost where rows are all as long (two pairs
-  // and one: 5 x 179, 2.4 blocks per SM, 78.2 and 72.5, 8 x 179 92.9 and 74.8; 5 x 300, 4.1 per SM, 161.5 and 167.8, 7 x 300, 5.7, 187.3 and
-  // 169.6; 4 x 448 210.7 and 229.1, 5 x 448 244.0 and 229.8), and so do rows of one tile among ragged ones of up to three (11 x 126
-  // with 16 heads, 4.8 per SM, 51.8 and 49.5, 31 x 128 94.6 and 84.8, 21 x 179 99.4 and 95.9; of four, 15 x 256, 116.9 and 128.3).
+  //   8 x 512           10.4                    647.9     468.6     439.1     469.4     613.3
+  //   14 x 384          13.6                    722.3     498.3     419.7     417.5     579.5
+  // An SM runs four pairs at a time, so a call is rounds of four blocks of one pair, or of two blocks of two.  Where the last round of four is
+  // nearly full, two pairs save nothing: they take twice as many rounds of half the length, adding their states up comes on top, and with an odd
+  // number of tiles the second pair waits for a tile's time in each of them.  So rows that are all as long have one pair per block where more than
+  // three of the last four slots are taken; with an odd number of tiles also beyond two (three tiles) or five blocks per SM; in long calls
+  // also where the last round has more than one block and at most two, which is a whole round of two.  Three tiles and few blocks: 16 rows.
+  // Among ragged rows those of one tile leave the second pair waiting: up to three tiles, and of four in long calls (one pair and two: 11 x 126
+  // with 16 heads 49.5 and 51.8, 31 x 128 84.8 and 94.6, 21 x 179 95.9 and 99.4, 13 x 128..256 157 and 175, 21 x 128..256 220 and 237; 15 x 32..256
+  // 128.3 and 116.9).  185 calls of full rows and 142 of ragged ones take 7 and 9 % less time in the geometric mean than with one pair throughout
+  // (16 rows up to two blocks per SM, then 32), and no full one takes longer; before the last round was looked at 20 of those took 2 to 17 % longer.
+  // Gathered scores: the loads of the score rows are what a block waits for, and of 16 rows (168 registers for 250) six fit on an SM instead of four and
+  // cover each other's; from two blocks of 32 per SM on, but for a single round that four fill.  16 x 1, 32 x 1 and 32 x 2:
+  // 3 x 300 81.7, 109.2, 116.1; 8 x 256 130.5, 159.1, 144.3; 13 x 512 733, 918, 882; 4 x 300 123.7, 109.1, 126.4; 2 x 256 61.0, 82.2, 57.1.  Content
+  // alone stands between the two: 16 rows up to three blocks per SM (9 x 128 38.0, 42.3, 41.0), and then as with tables.
   // One tile leaves nothing to share: 16 rows where 32 would leave SMs without a block.
-  int sms = 0, rc;
-  if ((rc = device_sms(&sms))) return rc;
-  const int64_t rows = (int64_t)p.H * p.n_seqs, blocks16 = (p.L + 15) / 16 * rows, blocks32 = (p.L + 31) / 32 * rows;
-  if (p.L <= KT) return blocks32 < 2 * (int64_t)sms ? launch_variant<T, 2, TABLES, 1>(p, s) : launch_variant<T, 4, TABLES, 1>(p, s);
+  int device = 0, rc;
+  if ((rc = device_sms(&device))) return rc;
+  const int64_t sms = device, rows = (int64_t)p.H * p.n_seqs, blocks16 = (p.L + 15) / 16 * rows, blocks32 = (p.L + 31) / 32 * rows;
+  if (p.L <= KT) return blocks32 < 2 * sms ? launch_variant<T, 2, TABLES, 1>(p, s) : launch_variant<T, 4, TABLES, 1>(p, s);
   if (blocks16 <= sms) return launch_variant<T, 2, TABLES, 4>(p, s);
   if (blocks32 <= sms) return launch_variant<T, 4, TABLES, 4>(p, s);
   const int tiles = (p.L + KT - 1) / KT;
-  const bool full = !p.varlen && !p.seqlens;
-  const bool waits = full ? tiles % 2 && blocks32 > (tiles == 3 ? 2 : 5) * (int64_t)sms : tiles <= 3 && blocks32 > (tiles == 2 ? 4 : 5) * (int64_t)sms;
-  return waits ? launch_variant<T, 4, TABLES, 1>(p, s) : launch_variant<T, 4, TABLES, 2>(p, s);
+  const bool full = !p.varlen && !p.seqlens, gathers = p.c2p_scores || p.p2c_scores;
+  if (tiles == 3 && blocks16 <= (TABLES ? 3 : 4) * sms) return launch_variant<T, 2, TABLES, 1>(p, s);
+  if (!TABLES && ((blocks32 > 2 * sms && blocks32 <= 3 * sms) || (gathers && blocks32 > 4 * sms))) return launch_variant<T, 2, TABLES, 1>(p, s);
+  const int64_t last = (blocks32 - 1) % (4 * sms) + 1;         // blocks of the last round of four per SM
+  bool one;
+  if (full || gathers) one = last > 3 * sms || (tiles % 2 ? blocks32 > (tiles == 3 ? 2 : 5) * sms : blocks32 > 8 * sms && last > sms && last <= 2 * sms);
+  else one = tiles == 4 ? blocks32 > 8 * sms : tiles <= 3 && blocks32 > (tiles == 2 ? 4 : 5) * sms;
+  return one ? launch_variant<T, 4, TABLES, 1>(p, s) : launch_variant<T, 4, TABLES, 2>(p, s);
 }
 
 template <typename T>
