@@ -1223,7 +1223,7 @@ int launch_attn_umma(const AttnParams& given, cudaStream_t s) {
     if (lng && (rc = table_map(&maps[6], p.qr_exp, p.exp_rows, p.H, SATN, "qr_exp (saturated tiles)"))) return rc;
   } else { maps[4] = maps[0]; maps[6] = maps[0]; }
 
-  // Persistent CTAs: one per SM (201 KB of shared memory and all 512 tensor-memory columns each), never more
+  // Persistent CTAs: one per SM (SMEM_BYTES, 225 KB, of shared memory and all 512 tensor-memory columns each), never more
   // than there are work items (query tiles x heads).
   int sms = 0;
   if ((rc = device_sms(&sms))) return rc;
@@ -1233,12 +1233,12 @@ int launch_attn_umma(const AttnParams& given, cudaStream_t s) {
     tiles = (p.total_tokens + BQ - 1) / BQ + p.n_seqs + 1;           // upper bound; the device list has the real count
     if (tiles * p.H > 0x7fffffff) { set_error("too many tiles"); return TDB_ERR_SHAPE; }
     // A few sequences: listed by each CTA's scheduler warp beside the rest of its set-up, some 300 clocks per step of 32 sequences and one
-    // tile count; the list kernel in front takes 3 us of the GPU and its launch two of the host.  us per call, own list and kernel: 2 x
-    // 50..100 tokens (1 step) 22.2 and 24.7, 20 x 10..64 28.2 and 30.9, 4 x 20..200 24.7 and 26.8, 30 x 60..500 (4) 54.2 and 55.4, 8 x
-    // 60..1000 (8) 37.7 and 38.6; with more than a few items per SM the host's part does not show: 30 x 60..1000 (8) 91.0 and 90.3, 256 x
-    // 8..128 (8) 94.7 and 92.8.
+    // tile count; the list kernel in front takes 3 us of the GPU and its launch two of the host, which beyond four steps no longer show.
+    // us per call, own list and kernel: 2 x 50..100 tokens (1 step) 27.9 and 32.3, 20 x 10..64 28.2 and 30.6, 4 x 20..200 (2) 30.4 and 35.0, 8 x 60..500
+    // (4) 42.6 and 43.4, 30 x 60..500 83.3 and 84.2; of 16 heads, 60 x 60..256 93.6 and 93.2, 5 x 500..640 (5) 70.2 and 66.6; 4 x 100..1000 (8) 56.1 and
+    // 55.5, 8 x 60..1000 74.4 and 72.1.
     const int64_t steps = (int64_t)((p.n_seqs + 31) / 32) * ((p.L + BQ - 1) / BQ);
-    own_list = !split && !lng && !p.lengths_known && tiles <= LIST_MAX && (steps <= 4 || (steps <= 9 && tiles * p.H <= 4 * (int64_t)sms));
+    own_list = !split && !lng && !p.lengths_known && tiles <= LIST_MAX && steps <= 4;
     if (!p.tiles_listed && !own_list) {
       build_tile_list_kernel<<<1, 1024, 0, s>>>(p.cu_seqlens, p.n_seqs, p.total_tokens,
                                                 reinterpret_cast<int32_t*>(p.workspace), (int)tiles, p.status);
