@@ -1,8 +1,8 @@
 // Sequences of at most 128 tokens, bf16, projected tables: one block per sequence, head and 64 query rows.
 //
 // Such a call is bound by latency, not by any unit: one or two score tiles per block.  The persistent tensor-memory kernel takes 7.3 us
-// for 64 tokens and 7.8 for 128 (scheduler ring, tensor-memory allocation and a chain of nine hand-offs between its roles); here a tile
-// is four barriers long.  Both bands are formed by the warp-level tensor instruction, q.Kr for the 80 distances of a warp's 16 query
+// for 64 tokens and 7.8 for 128 (scheduler ring, tensor-memory allocation and a chain of nine hand-offs between its roles); here one tile
+// is two barriers long, and two are six.  Both bands are formed by the warp-level tensor instruction, q.Kr for the 80 distances of a warp's 16 query
 // rows and k.Qr for those of 16 key rows, kept in fp32 in shared memory and read back along the diagonal:
 //
 //   s[i][j] = (Q[i].K[j] + C[i][i - j] + P2[j][i - j]) * scale ;  P as bf16 ;  O = P . V

@@ -18,7 +18,7 @@
 // through the weights' buffer.  The order of the columns inside a product is free as long as both operands share it, so a
 // thread's fragments of two k16 steps are one 16-byte load.
 //
-// Base model, one pass of 32 tokens from ids to hidden states: 515 us as a replayed recording of 84 kernels, 406 here (the kernel
+// Base model, one pass of 32 tokens from ids to hidden states: 447 us as a replayed recording of 84 kernels, 306 here, back to back (the kernel
 // itself 240: 20 us per layer, of which the five meetings 5.6, the LayerNorms 3.4, the products 5.0 - the second projection, whose 196 KB of
 // activations come in at 55 bytes per clock, 2.6 - the sums of their parts with the way to memory 3.4, and the attention 2.4); 16 tokens 16 us
 // per layer.  Tried and left out: clusters of four that share the LayerNorms over distributed shared memory (a row's four
@@ -27,7 +27,7 @@
 // took for converged: its ten shuffles cost 5 us.
 //
 // The blocks wait for one another, so the launch is a cooperative one (all of them run at the same time, or the launch
-// fails), and every wait has a limit, after which all blocks leave and the host reports it.
+// fails), and every wait has a limit, after which all blocks leave, behind their own copies, and the host reports it.
 #include "attn_warp_mma.cuh"
 #include "gelu.cuh"
 #include "ptx_sm100.cuh"
@@ -594,7 +594,10 @@ using namespace tdb;
 
 extern "C" {
 
-// Hidden sizes whose columns the eight warps can share in whole blocks of 32, with a block per eight columns resident at once.
+// Hidden sizes whose columns the eight warps can share in whole blocks of 32, with a block per eight columns resident at once.  The tokens end at
+// 32 because the attention has one tile of 32 keys, for which all score and band fragments are a warp's each; the shared memory would hold 48 at a hidden
+// size of 768.  us per pass on both sides of the line, 32 tokens here and 40 by the layer loop's recording: 165 and 200 (512, six layers), 306 and 416 (768,
+// twelve), 639 and 874 (1024, 24).  Many short sequences cost a block several heads in turn: 32 sequences of one token 367 (768), as a recording 494.
 int tdb_short_stack_applies(int64_t tokens, int64_t hidden, int64_t inner, int64_t layers) {
   if (tokens < 1 || tokens > SKINNY_TOKENS || layers < 1 || layers > SHORT_LAYERS || inner != 4 * hidden) return 0;
   const bool one = tokens <= 16;

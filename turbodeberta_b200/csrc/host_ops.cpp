@@ -1012,14 +1012,13 @@ class Encoder {
   }
 
   // Small passes that the one kernel does not take are bound by the host: eight launches per layer of some 4 us each, for kernels of
-  // 2 to 8 us.  A shape that
-  // comes a second time on a stream is recorded into a CUDA graph, which belongs to that stream (its buffers are in use until
+  // 2 to 8 us.  A shape that comes a second time on a stream is recorded into a CUDA graph, which belongs to that stream (its buffers are in use until
   // the replay is over), as long as the weights stay where they are.  At most GRAPHS of them.  A shape then has to come COMEBACKS
   // times while the longest unused recording does not come once: only then does it take that one's place.  With any number of
   // shapes in turn the first GRAPHS stay recorded and the others stay eager.
-  // us per pass, eager and replayed, and what the pass that records costs beyond an eager one: base model, 128 tokens 659, 562, 730; 2048 tokens 1027, 899, 700; large model, 128 tokens 1271, 1086, 1150; 2048 tokens 2337, 2081,
-  // 1040.  So a recording has paid for itself after six to eight replays (COMEBACKS), 25 where the projections are kernels of our
-  // own.  Twelve shapes in turn of some 30 tokens each, before the one kernel took those: 502 us per pass; 40 shapes 574; all new ones
+  // us per pass, eager and replayed, and what the pass that records costs beyond an eager one: base model, 128 tokens 659, 562, 730; 2048
+  // tokens 1027, 899, 700; large model, 128 tokens 1271, 1086, 1150; 2048 tokens 2337, 2081, 1040.  So a recording has paid for itself after
+  // six to eight replays (COMEBACKS).  Twelve shapes in turn of some 30 tokens each, before the one kernel took those: 502 us per pass; 40 shapes 574; all new ones
   // 632 (when every shape that came back pushed the oldest out: 1070 and 1277).  Beyond GRAPH_MAX_ELEMENTS the gain falls (6 M elements 5 %, 9 to 12 M 1 to 2 %) and the
   // buffers grow: a recording at the limit holds 52 MB, and each stream with one 32 MB of workspace.
   static constexpr int GRAPHS = 8, COMEBACKS = 8, SEEN = 64, BLOCK = 128;
