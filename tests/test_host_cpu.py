@@ -194,6 +194,14 @@ def test_mask_analysis_after_the_native_one_has_the_validity_too():
     assert M.analyse_mask(m, 2, 6) is info
 
 
+@pytest.mark.parametrize("tokens,columns,features,own", [(32, 1024, 4096, 1), (33, 1024, 4096, 0), (32, 4096, 1024, 1), (8, 1024, 4104, 1), (1, 1280, 3840, 0), (1, 1280, 1280, 1),
+                                                         (32, 768, 3072, 1), (16, 768, 4, 0), (16, 760, 8, 0)])
+def test_which_projections_are_kernels_of_our_own(tokens, columns, features, own):
+    import ctypes as C
+    from turbodeberta_b200 import _cabi as cabi
+    assert cabi.lib.tdb_skinny_applies(C.c_int64(tokens), C.c_int64(columns), C.c_int64(features)) == own
+
+
 def _small_config(**kw):
     from transformers import DebertaV2Config
     return DebertaV2Config(**{**dict(vocab_size=50, hidden_size=128, num_hidden_layers=4, num_attention_heads=2,

@@ -122,11 +122,15 @@ extern "C" {
 // memory, this kernel against the library's.  32 tokens: K 768 and N 768 2.5 and 3.3, N 2304 3.0 and 3.9, N 3072 4.1 and 4.2, K 3072
 // and N 768 5.8 and 6.6; K 1024 and N 3072 4.7 and 4.7, N 4096 5.5 and 5.0 (where GELU in the epilogue saves a launch).  With three token
 // tiles the narrow projections would still gain and the wide ones lose, 48 tokens: 3.2 and 3.3, 4.0 and 4.1, 4.8 and 4.4, 6.5 and
-// 6.7; K 1024 5.6 and 4.8, 5.9 and 5.1; with four all lose (64 tokens: 3.5 and 3.3, 4.2 and 4.0, 5.6 and 4.4, 7.0 and 6.8).  A pass of the
-// base model with and without: 8 tokens 445 and 531 us, 16 tokens 449 and 512, 32 tokens 495 and 507; of the large one: 16 tokens 884
-// and 1057, 32 tokens 999 and 1000 (since encoder_short.cu takes passes of these two sizes as a whole, this is for other sizes and for
-// passes that return every layer).  K up to what a warp's registers hold.
-int tdb_skinny_applies(int64_t T, int64_t K, int64_t N) { return T <= SKINNY_TOKENS && K % KB == 0 && K <= KB * WARPS * 16 && N % 8 == 0; }
+// 6.7; K 1024 5.6 and 4.8, 5.9 and 5.1; with four all lose (64 tokens: 3.5 and 3.3, 4.2 and 4.0, 5.6 and 4.4, 7.0 and 6.8).  Larger weights
+// than those lose too: a pass of twelve layers of hidden size 1280, 32 tokens, without a limit, with it, and with the library for all 603, 548,
+// 544; of 1536 682, 601, 595; six layers of 2048, 8 tokens 467, 435, 437, 32 tokens 497, 408, 408.  Passes of 8, 16 and 32 tokens with this kernel, and with
+// the library: twelve layers of hidden size 384 324, 314, 322 and 384, 361, 362; of 640 392, 399, 419 and 465, 440, 435; and where
+// encoder_short.cu does not come in because every layer is returned, the base model 635, 644, 668 and 843, 790, 785, the large one 1095, 1119, 1214
+// and 1404, 1415, 1379.  K up to what a warp's registers hold.
+int tdb_skinny_applies(int64_t T, int64_t K, int64_t N) {
+  return T <= SKINNY_TOKENS && K % KB == 0 && K <= KB * WARPS * 16 && N % 8 == 0 && K * N <= 4500000;
+}
 
 int tdb_skinny(const void* x, const void* w, const void* b, int T, int K, int N, int gelu, int early, void* y, void* stream) {
   cudaStream_t s = (cudaStream_t)stream;
