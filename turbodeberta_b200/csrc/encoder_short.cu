@@ -18,8 +18,8 @@
 // through the weights' buffer.  The order of the columns inside a product is free as long as both operands share it, so a
 // thread's fragments of two k16 steps are one 16-byte load.
 //
-// Base model, one pass of 32 tokens from ids to hidden states: 447 us as a replayed recording of 84 kernels, 306 here, back to back (the kernel
-// itself 240: 20 us per layer, of which the five meetings 5.6, the LayerNorms 3.4, the products 5.0 - the second projection, whose 196 KB of
+// Base model, one pass of 32 tokens from ids to hidden states: 447 us as a replayed recording of 84 kernels, 306 here (with a new padding mask for
+// each pass 508 and 354; the kernel itself 240: 20 us per layer, of which the five meetings 5.6, the LayerNorms 3.4, the products 5.0 - the second projection, whose 196 KB of
 // activations come in at 55 bytes per clock, 2.6 - the sums of their parts with the way to memory 3.4, and the attention 2.4); 16 tokens 16 us
 // per layer.  Tried and left out: clusters of four that share the LayerNorms over distributed shared memory (a row's four
 // copies cost what forming it four times does) and split the second projection's columns (1.3 of its 5 thousand clocks).
@@ -596,7 +596,7 @@ extern "C" {
 
 // Hidden sizes whose columns the eight warps can share in whole blocks of 32, with a block per eight columns resident at once.  The tokens end at
 // 32 because the attention has one tile of 32 keys, for which all score and band fragments are a warp's each; the shared memory would hold 48 at a hidden
-// size of 768.  us per pass on both sides of the line, 32 tokens here and 40 by the layer loop's recording: 165 and 200 (512, six layers), 306 and 416 (768,
+// size of 768.  us per pass with a known mask on both sides of the line, 32 tokens here and 40 by the layer loop's recording: 165 and 200 (512, six layers), 306 and 416 (768,
 // twelve), 639 and 874 (1024, 24).  Many short sequences cost a block several heads in turn: 32 sequences of one token 367 (768), as a recording 494.
 int tdb_short_stack_applies(int64_t tokens, int64_t hidden, int64_t inner, int64_t layers) {
   if (tokens < 1 || tokens > SKINNY_TOKENS || layers < 1 || layers > SHORT_LAYERS || inner != 4 * hidden) return 0;
