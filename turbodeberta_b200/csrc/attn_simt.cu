@@ -386,14 +386,15 @@ int launch_rows(const AttnParams& p, cudaStream_t s) {
   // number of tiles the second pair waits for a tile's time in each of them.  So rows that are all as long have one pair per block where more than
   // three of the last four slots are taken; with an odd number of tiles also beyond two (three tiles) or five blocks per SM; in long calls
   // also where the last round has more than one block and at most two, which is a whole round of two.  Three tiles and few blocks: 16 rows.
-  // Among ragged rows those of one tile leave the second pair waiting: up to three tiles, and of four in long calls (one pair and two: 11 x 126
-  // with 16 heads 49.5 and 51.8, 31 x 128 84.8 and 94.6, 21 x 179 95.9 and 99.4, 13 x 128..256 157 and 175, 21 x 128..256 220 and 237; 15 x 32..256
-  // 128.3 and 116.9).  185 calls of full rows and 142 of ragged ones take 7 and 9 % less time in the geometric mean than with one pair throughout
-  // (16 rows up to two blocks per SM, then 32), and no full one takes longer; before the last round was looked at 20 of those took 2 to 17 % longer.
+  // Among ragged rows those of one tile leave the second pair waiting, up to three tiles in all (one pair and two: 11 x 126 with 16 heads 49.5 and
+  // 51.8, 31 x 128 84.8 and 94.6, 21 x 179 95.9 and 99.4; of four tiles, 15 x 32..256, 128.3 and 116.9, four draws of 14 x 256 0.97 to 1.14 times two pairs').  185 calls of
+  // full rows and 178 of ragged ones take 7 and 8 % less time in the geometric mean than with one pair throughout (16 rows up to two
+  // blocks per SM, then 32), and no full one takes longer; before the last round was looked at 20 of those took 2 to 17 % longer.
   // Gathered scores: the loads of the score rows are what a block waits for, and of 16 rows (168 registers for 250) six fit on an SM instead of four and
   // cover each other's; from two blocks of 32 per SM on, but for a single round that four fill.  16 x 1, 32 x 1 and 32 x 2:
-  // 3 x 300 81.7, 109.2, 116.1; 8 x 256 130.5, 159.1, 144.3; 13 x 512 733, 918, 882; 4 x 300 123.7, 109.1, 126.4; 2 x 256 61.0, 82.2, 57.1.  Content
-  // alone stands between the two: 16 rows up to three blocks per SM (9 x 128 38.0, 42.3, 41.0), and then as with tables.
+  // 3 x 300 81.7, 109.2, 116.1; 8 x 256 130.5, 159.1, 144.3; 13 x 512 733, 918, 882; 4 x 300 123.7, 109.1, 126.4; 2 x 256 61.0, 82.2, 57.1.  Ragged
+  // rows of more than three tiles gain from six blocks per SM on (four draws of 8 x 32..256 and up take 0.92 to 1.12 of the time of two pairs,
+  // of 11 x 256 0.82 to 0.96, of 18 x 256 0.80 to 0.86).  Content alone stands between the two: 16 rows up to three blocks per SM (9 x 128 38.0, 42.3, 41.0), and then as with tables.
   // One tile leaves nothing to share: 16 rows where 32 would leave SMs without a block.
   int device = 0, rc;
   if ((rc = device_sms(&device))) return rc;
@@ -404,11 +405,14 @@ int launch_rows(const AttnParams& p, cudaStream_t s) {
   const int tiles = (p.L + KT - 1) / KT;
   const bool full = !p.varlen && !p.seqlens, gathers = p.c2p_scores || p.p2c_scores;
   if (tiles == 3 && blocks16 <= (TABLES ? 3 : 4) * sms) return launch_variant<T, 2, TABLES, 1>(p, s);
-  if (!TABLES && ((blocks32 > 2 * sms && blocks32 <= 3 * sms) || (gathers && blocks32 > 4 * sms))) return launch_variant<T, 2, TABLES, 1>(p, s);
+  if (!TABLES) {
+    const bool by16 = full ? (blocks32 > 2 * sms && blocks32 <= 3 * sms) || (gathers && blocks32 > 4 * sms) : gathers && blocks32 > (tiles <= 3 ? 2 : 6) * sms;
+    if (by16) return launch_variant<T, 2, TABLES, 1>(p, s);
+  }
   const int64_t last = (blocks32 - 1) % (4 * sms) + 1;         // blocks of the last round of four per SM
   bool one;
-  if (full || gathers) one = last > 3 * sms || (tiles % 2 ? blocks32 > (tiles == 3 ? 2 : 5) * sms : blocks32 > 8 * sms && last > sms && last <= 2 * sms);
-  else one = tiles == 4 ? blocks32 > 8 * sms : tiles <= 3 && blocks32 > (tiles == 2 ? 4 : 5) * sms;
+  if (full) one = last > 3 * sms || (tiles % 2 ? blocks32 > (tiles == 3 ? 2 : 5) * sms : blocks32 > 8 * sms && last > sms && last <= 2 * sms);
+  else one = tiles <= 3 && blocks32 > (tiles == 2 ? 4 : 5) * sms;
   return one ? launch_variant<T, 4, TABLES, 1>(p, s) : launch_variant<T, 4, TABLES, 2>(p, s);
 }
 
