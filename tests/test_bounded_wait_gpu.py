@@ -34,3 +34,21 @@ def test_selftest_argument_errors():
     assert cabi.lib.tdb_selftest_bounded_wait(None, 1, 10, None) == cabi.ERR_ARG
     assert cabi.lib.tdb_selftest_bounded_wait(cabi.ptr(status), 0, 10, None) == cabi.ERR_ARG
     assert cabi.lib.tdb_selftest_bounded_wait(cabi.ptr(status), 1, 10 ** 7, None) == cabi.ERR_ARG
+
+
+def test_words_of_another_stream_are_waited_for():
+    """A check in one thread reads what calls of others have left: on streams that may not have come to them yet."""
+    from turbodeberta_b200 import status as st
+    stream = torch.cuda.Stream()
+    for pending in (1, st.PendingStatus.FOLD_AT + 3):                # read one by one, and folded on the way
+        words = torch.zeros(4, dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        with torch.cuda.stream(stream):
+            torch.cuda._sleep(100_000_000)                           # some 50 ms
+            words[0].fill_(77)
+            fa._PENDING_STATUS.append(words)
+        for _ in range(pending - 1):
+            fa._PENDING_STATUS.append(torch.zeros(4, dtype=torch.int32, device="cuda"))
+        with pytest.raises(cabi.TdbError, match="77"):
+            fa.check_pending_status()
+    fa.check_pending_status()
