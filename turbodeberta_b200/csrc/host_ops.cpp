@@ -1274,8 +1274,10 @@ py::object mask_rows(const Tensor& mask) {
 }
 
 // A model's input from ids [B, L]: LayerNorm of their embeddings, times the padding mask.  (output, words that somebody has to look at
-// or None), or None where the kernel does not take the tensors as they are.  own: the words come as a Report, or a tensor, for the caller's own check.
-py::object embed(const Tensor& ids, const Tensor& table, const Tensor& w, const Tensor& b, double eps, const Tensor& mask, bool own) {
+// or None), or None where the kernel does not take the tensors.  own: ids and mask of any layout, and the words come as a Report, or a tensor, for the
+// caller's own check.
+py::object embed(const Tensor& given_ids, const Tensor& table, const Tensor& w, const Tensor& b, double eps, const Tensor& given_mask, bool own) {
+  const Tensor ids = own ? given_ids.contiguous() : given_ids, mask = own ? given_mask.contiguous() : given_mask;
   const at::ScalarType t = table.scalar_type();
   const int64_t hidden = table.size(1);
   const bool types = (t == at::kFloat || t == at::kBFloat16) && w.scalar_type() == t && b.scalar_type() == t &&

@@ -542,6 +542,7 @@ class _Pass(threading.local):
 
 _PASS = _Pass()
 _PLAIN_TENSORS = frozenset((torch.Tensor, nn.Parameter))      # other classes may keep their values elsewhere (quantised, sharded)
+_MASK_TYPES = (torch.int64, torch.bool, torch.uint8)
 _PLAIN_ARGUMENTS = frozenset(("input_ids", "attention_mask", "output_hidden_states", "output_attentions", "return_dict"))
 
 
@@ -580,14 +581,15 @@ class FlashDebertaV2Model(DebertaV2Model):
                                            or attention_mask.device != input_ids.device):
             return None
         emb = self.embeddings
-        watch, of = _PLANS.get(self, (None, None))
+        watch, of, plain = _PLANS.get(self, (None, None, None))
         if watch is None or of is not emb:
             if (type(emb) is not DebertaV2Embeddings or type(emb.word_embeddings) is not nn.Embedding
                     or type(emb.LayerNorm) is not nn.LayerNorm or emb.word_embeddings.max_norm is not None
                     or any(getattr(emb, n, None) is not None for n in ("position_embeddings", "token_type_embeddings", "embed_proj"))):
                 return None
             watch = host.Watch(list(emb.modules()), [(emb.word_embeddings, ("max_norm",))])
-            _PLANS[self] = (watch, emb)
+            plain = all(type(p) is nn.Parameter for p in emb.parameters())      # the watch knows them by identity
+            _PLANS[self] = (watch, emb, plain)
         if not watch.holds():
             _PLANS.pop(self, None)
             return None
@@ -595,13 +597,13 @@ class FlashDebertaV2Model(DebertaV2Model):
             attention_mask = torch.ones(input_ids.shape, dtype=torch.long, device=input_ids.device)
         table, norm = emb.word_embeddings.weight, emb.LayerNorm
         embedded = None
-        if (norm.weight is not None and norm.bias is not None and tuple(norm.normalized_shape) == table.shape[1:]
-                and all(type(t) in _PLAIN_TENSORS for t in (input_ids, attention_mask, table, norm.weight, norm.bias))):
+        if (plain and type(input_ids) in _PLAIN_TENSORS and type(attention_mask) in _PLAIN_TENSORS and norm.weight is not None
+                and norm.bias is not None and tuple(norm.normalized_shape) == table.shape[1:]):
             # Rows of a wider tensor, or a mask of another type, must not change what an id outside the vocabulary does: torch's own
             # embedding ends in an assertion on the device.
-            known = attention_mask.dtype in (torch.int64, torch.bool, torch.uint8)
-            embedded = host.embed(input_ids.contiguous(), table, norm.weight, norm.bias, norm.eps,
-                                  attention_mask.contiguous() if known else torch.ones(input_ids.shape, dtype=torch.bool, device=input_ids.device), True)
+            known = attention_mask.dtype in _MASK_TYPES
+            embedded = host.embed(input_ids, table, norm.weight, norm.bias, norm.eps,
+                                  attention_mask if known else torch.ones(input_ids.shape, dtype=torch.bool, device=input_ids.device), True)
             if embedded is not None and not known:
                 embedded[0].mul_(attention_mask.to(table.dtype)[..., None])
         report = None

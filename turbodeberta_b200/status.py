@@ -28,6 +28,8 @@ class PendingStatus:
 
     def drain(self) -> list:
         """All blocks, for the current stream of each device to read."""
+        if not self._by_dev:                         # as after nearly every pass
+            return []
         with self._lock:
             taken, self._by_dev = self._by_dev, {}
         return [st for blocks in taken.values() for st in self._ready(blocks)]
